@@ -78,6 +78,7 @@ def _declare(lib):
         "gefen_b200_muon_apply": (i32, [vp, vp, i32, i64, dbl, dbl, vp, i32, vp]),
         "gefen_b200_step_tensor_size": (i32, []),
         "gefen_b200_step_tensor_class": (i32, [vp, i32]),
+        "gefen_b200_step_launch_class": (i32, [vp, i32]),
         "gefen_b200_step_status": (i32, [vp, i32]),
         "gefen_b200_debug_set_stage_spin_limit": (i32, [i64]),
         "gefen_b200_exact_histogram": (i32, [vp, i32, i64, i64, vp, i32, vp]),

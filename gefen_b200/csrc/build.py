@@ -35,6 +35,7 @@ NVCC_FLAGS = [
     "-gencode",
     "arch=compute_100a,code=sm_100a",
     "-lineinfo",
+    "-split-compile=0",
     "-Xcompiler",
     "-fPIC",
 ]

@@ -11,16 +11,21 @@
 //   p_i  -= cb[code'_i] * mag' * step * lr,   step = (1/bc1) / (sqrt(v/bc2) + eps)
 //
 // Two kernels:
-//  * step_vec_kernel  - the fast path, in two kinds that are compiled and launched separately: one warp
-//    owns one block, or several blocks when they are not longer than 1024 elements (see
-//    lanes_per_block). Codes and gradients are read once
-//    (128-bit loads), the updated momenta wait in the warp's slice of shared memory while the
-//    block's absmax is reduced with shuffles, then they are re-encoded and the parameters updated:
-//    codes, gradients and params cross HBM exactly once (8 B/element in bf16, 14 B/element in
-//    fp32). Codebook, thresholds and the quantisation table arrive in shared memory by one bulk
-//    (TMA) copy per CTA. No __syncthreads after set-up; the loops are short so the code stays in
+//  * step_vec_kernel  - the fast path: one warp owns one block, or several blocks when they are not longer than 1024
+//    elements (see lanes_shift). Codes and gradients are read once in chunks of eight elements (four, two or one
+//    where the block length or a pointer is a multiple of no more), the updated momenta wait in the warp's slice of
+//    shared memory while the block's absmax is reduced with shuffles, then they are re-encoded and the parameters
+//    updated: codes, gradients and params cross HBM exactly once (8 B/element in bf16, 14 B/element in fp32).
+//    Codebook and thresholds arrive by one bulk (TMA) copy per CTA, which turns them into tables with a copy per
+//    lane (see LaneTables). No __syncthreads after set-up; the loops are short so the code stays in
 //    the instruction cache.
-//  * step_generic_kernel - any period, alignment and dtype (fp64 included), period-1 tensors and
+//    What bounds it: for two-byte types the issue of instructions (31 per element) together with the latency that
+//    sixteen warps per SM can cover, for fp32 HBM. 134 M elements in blocks of 2048 bf16: 0.259 -> 0.221 ms = 0.75 of
+//    the measured copy bandwidth (the tables without bank conflicts, arithmetic on pairs, loops without per-lane
+//    bounds tests); blocks of 512 0.275 -> 0.230 ms, of 128 0.455 -> 0.315 ms; fp32 of 768 / 2048 0.193 -> 0.192 /
+//    0.182 -> 0.183 ms (67 M elements). Rows that are no multiples of eight, which the generic kernel used to take:
+//    120 M bf16 elements in blocks of 300 1.87 -> 0.37 ms, 135 M of 1500 2.26 -> 0.32 ms, 59 M of 147 0.98 -> 0.46 ms.
+//  * step_generic_kernel - blocks of more than 8192 elements, fp64, period-1 tensors and
 //    4-bit packed codes: two passes with scalar accesses, the second pass re-reading from L1/L2.
 // Both take their tensors from a descriptor table (one launch for many tensors); a single-tensor
 // call passes a one-row table inside the kernel parameters. For data-parallel ranks whose buffers
@@ -78,31 +83,46 @@ struct StepLaunch {
 };
 
 // Set (never cleared by a kernel) when a bounded wait ran out and the CTA left without doing its
-// share of the step: bit 0 = the table staging of a step kernel. Read and cleared by
+// share of the step: bit 0 = the table staging of a step kernel, bit 1 = its shared-memory layout does not fit. Read and cleared by
 // gefen_b200_step_status on the host.
 __device__ int g_step_status;
+
+// Two fp32 operations in one instruction (sm_100: each half is the IEEE operation of its own, so the results
+// are those of the scalar forms). The step kernels are bound by instruction issue; their arithmetic runs on pairs.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpair(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
 
 template <typename T> __device__ __forceinline__ T* peer_ptr(T* p, long long delta) {
     return reinterpret_cast<T*>(reinterpret_cast<uintptr_t>(p) + delta);
 }
 
-constexpr int kSmemWs = GEFEN_B200_CODEBOOK_WS_BYTES;
+// Every step kernel stages the head of the codebook workspace: codebook, thresholds, size.
+constexpr int kSmemWs = kWsLutOff;
+static_assert(kSmemWs % 16 == 0, "bulk copies move multiples of 16 bytes");
 constexpr int kMaxSmem = 227 * 1024;
-// The fast path reads the codebook twice per element with data-dependent indices. One copy per
-// lane (entry e of lane c at word 32*e + c, a 128-byte row per entry) makes every such read
-// conflict-free, against the ~3.5-way conflict of a single 1 KB table.
-constexpr int kRepCopies = 32;
-constexpr int kSmemRep = kMaxCodebook * kRepCopies * 4;
 
 struct SmemView {
     const float* cb;             // 256, padded with the last entry
     const float* thr;            // 256, padded with +inf
-    const unsigned char* lut;    // kLutBytes
-    const float* rep;            // fast path only: kRepCopies interleaved copies of cb, offset by the lane's copy
     int k;                       // true codebook size
 };
 
-// Stages the workspace with one bulk copy. Returns false (uniformly for the CTA) if the copy did
+// Stages the tables with one bulk copy. Returns false (uniformly for the CTA) if the copy did
 // not land within `spin_limit` polls of its barrier; the status word is raised then, and the CTA
 // still gives the copy a second, long bounded wait before it returns, so that it does not leave
 // while a copy into its shared memory is in flight.
@@ -128,8 +148,6 @@ __device__ __forceinline__ bool stage_tables(const unsigned char* ws, unsigned c
     __syncthreads();
     view.cb = reinterpret_cast<const float*>(smem + kWsCodebookOff);
     view.thr = reinterpret_cast<const float*>(smem + kWsThresholdOff);
-    view.lut = smem + kWsLutOff;
-    view.rep = nullptr;
     view.k = 1;
     if (!ok) return false;
     view.k = reinterpret_cast<const int*>(smem + kWsMetaOff)[0];
@@ -187,158 +205,362 @@ template <> __device__ __forceinline__ uint4 multimem_load_sum16<float>(const vo
     return v;
 }
 
-template <typename S> struct Chunk;
-template <> struct Chunk<__nv_bfloat16> {
-    uint4 raw;
-    __device__ __forceinline__ void load_sum(const void* mc_base, long long chunk) {
-        raw = multimem_load_sum16<__nv_bfloat16>(reinterpret_cast<const uint4*>(mc_base) + chunk);
+// Storage form of one element: widening to fp32 and rounding back, two at a time.
+template <typename S> struct Packed;
+template <> struct Packed<__nv_bfloat16> {
+    static __device__ __forceinline__ void unpack(uint32_t w, float& lo, float& hi) {
+        lo = __uint_as_float(w << 16);
+        hi = __uint_as_float(w & 0xFFFF0000u);
     }
-    __device__ __forceinline__ void store_all(void* mc_base, long long chunk) const {
-        multimem_store16(reinterpret_cast<uint4*>(mc_base) + chunk, raw);
-    }
-    __device__ __forceinline__ void load(const void* base, long long chunk) {
-        raw = __ldcs(reinterpret_cast<const uint4*>(base) + chunk);
-    }
-    __device__ __forceinline__ void store(void* base, long long chunk) const {
-        reinterpret_cast<uint4*>(base)[chunk] = raw;
-    }
-    __device__ __forceinline__ void unpack(float (&f)[8]) const {
-        const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            f[2 * i] = __uint_as_float(w[i] << 16);
-            f[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
-        }
-    }
-    __device__ __forceinline__ void pack(const float (&f)[8]) {
-        uint32_t w[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const __nv_bfloat162 h = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
-            w[i] = *reinterpret_cast<const uint32_t*>(&h);
-        }
-        raw = make_uint4(w[0], w[1], w[2], w[3]);
+    static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+        return *reinterpret_cast<const uint32_t*>(&h);
     }
 };
-template <> struct Chunk<__half> {
-    uint4 raw;
-    __device__ __forceinline__ void load_sum(const void* mc_base, long long chunk) {
-        raw = multimem_load_sum16<__half>(reinterpret_cast<const uint4*>(mc_base) + chunk);
+template <> struct Packed<__half> {
+    static __device__ __forceinline__ void unpack(uint32_t w, float& lo, float& hi) {
+        const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&w));
+        lo = v.x;
+        hi = v.y;
     }
-    __device__ __forceinline__ void store_all(void* mc_base, long long chunk) const {
-        multimem_store16(reinterpret_cast<uint4*>(mc_base) + chunk, raw);
-    }
-    __device__ __forceinline__ void load(const void* base, long long chunk) {
-        raw = __ldcs(reinterpret_cast<const uint4*>(base) + chunk);
-    }
-    __device__ __forceinline__ void store(void* base, long long chunk) const {
-        reinterpret_cast<uint4*>(base)[chunk] = raw;
-    }
-    __device__ __forceinline__ void unpack(float (&f)[8]) const {
-        const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
-            f[2 * i] = v.x;
-            f[2 * i + 1] = v.y;
-        }
-    }
-    __device__ __forceinline__ void pack(const float (&f)[8]) {
-        uint32_t w[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const __half2 h = __floats2half2_rn(f[2 * i], f[2 * i + 1]);
-            w[i] = *reinterpret_cast<const uint32_t*>(&h);
-        }
-        raw = make_uint4(w[0], w[1], w[2], w[3]);
-    }
-};
-template <> struct Chunk<float> {
-    float4 lo, hi;
-    __device__ __forceinline__ void load_sum(const void* mc_base, long long chunk) {
-        const uint4 a = multimem_load_sum16<float>(reinterpret_cast<const uint4*>(mc_base) + 2 * chunk);
-        const uint4 b = multimem_load_sum16<float>(reinterpret_cast<const uint4*>(mc_base) + 2 * chunk + 1);
-        lo = make_float4(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z), __uint_as_float(a.w));
-        hi = make_float4(__uint_as_float(b.x), __uint_as_float(b.y), __uint_as_float(b.z), __uint_as_float(b.w));
-    }
-    __device__ __forceinline__ void store_all(void* mc_base, long long chunk) const {
-        multimem_store16(reinterpret_cast<uint4*>(mc_base) + 2 * chunk,
-                         make_uint4(__float_as_uint(lo.x), __float_as_uint(lo.y), __float_as_uint(lo.z), __float_as_uint(lo.w)));
-        multimem_store16(reinterpret_cast<uint4*>(mc_base) + 2 * chunk + 1,
-                         make_uint4(__float_as_uint(hi.x), __float_as_uint(hi.y), __float_as_uint(hi.z), __float_as_uint(hi.w)));
-    }
-    __device__ __forceinline__ void load(const void* base, long long chunk) {
-        lo = __ldcs(reinterpret_cast<const float4*>(base) + 2 * chunk);
-        hi = __ldcs(reinterpret_cast<const float4*>(base) + 2 * chunk + 1);
-    }
-    __device__ __forceinline__ void store(void* base, long long chunk) const {
-        __stcs(reinterpret_cast<float4*>(base) + 2 * chunk, lo);   // measured: streaming stores pay for fp32 only
-        __stcs(reinterpret_cast<float4*>(base) + 2 * chunk + 1, hi);
-    }
-    __device__ __forceinline__ void unpack(float (&f)[8]) const {
-        f[0] = lo.x; f[1] = lo.y; f[2] = lo.z; f[3] = lo.w;
-        f[4] = hi.x; f[5] = hi.y; f[6] = hi.z; f[7] = hi.w;
-    }
-    __device__ __forceinline__ void pack(const float (&f)[8]) {
-        lo = make_float4(f[0], f[1], f[2], f[3]);
-        hi = make_float4(f[4], f[5], f[6], f[7]);
+    static __device__ __forceinline__ uint32_t pack(float lo, float hi) {
+        const __half2 h = __floats2half2_rn(lo, hi);
+        return *reinterpret_cast<const uint32_t*>(&h);
     }
 };
 
-// Pulls the lines of this warp's NEXT block towards L2 while the current block is being worked on,
-// so that its loads later pay an L2 hit instead of a DRAM round trip (shared memory takes almost
-// all of L1, and the registers are busy: a hint costs neither).
-__device__ __forceinline__ void prefetch_l2_range(const void* base, long long bytes, int lane) {
-    const char* p = static_cast<const char*>(base);
-    for (long long off = static_cast<long long>(lane) * 128; off < bytes; off += 32 * 128) {
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(p + off));
+// V consecutive elements of a tensor: V code bytes and V * sizeof(S) bytes of gradients or parameters, aligned to
+// the smaller of that and 16. V = 8 is the usual chunk; 4, 2 and 1 serve blocks and pointers that are multiples of
+// no more than that.
+template <typename S, int V> struct Chunk {
+    static constexpr int kBytes = V * static_cast<int>(sizeof(S));
+    static constexpr int kWords = kBytes < 4 ? 1 : kBytes / 4;
+    uint32_t w[kWords];
+    __device__ __forceinline__ void load(const void* base, long long chunk) {
+        const char* p = static_cast<const char*>(base) + chunk * kBytes;
+        if constexpr (kBytes >= 16) {
+#pragma unroll
+            for (int q = 0; q < kBytes / 16; ++q) {
+                const uint4 v = __ldcs(reinterpret_cast<const uint4*>(p) + q);
+                w[4 * q] = v.x; w[4 * q + 1] = v.y; w[4 * q + 2] = v.z; w[4 * q + 3] = v.w;
+            }
+        } else if constexpr (kBytes == 8) {
+            const uint2 v = __ldcs(reinterpret_cast<const uint2*>(p));
+            w[0] = v.x; w[1] = v.y;
+        } else if constexpr (kBytes == 4) {
+            w[0] = __ldcs(reinterpret_cast<const unsigned int*>(p));
+        } else {
+            w[0] = __ldcs(reinterpret_cast<const unsigned short*>(p));
+        }
     }
+    __device__ __forceinline__ void store(void* base, long long chunk) const {
+        char* p = static_cast<char*>(base) + chunk * kBytes;
+        if constexpr (kBytes >= 16) {
+#pragma unroll
+            for (int q = 0; q < kBytes / 16; ++q) {
+                const uint4 v = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+                if constexpr (sizeof(S) == 4) __stcs(reinterpret_cast<uint4*>(p) + q, v);   // measured: streaming stores pay for fp32 only
+                else reinterpret_cast<uint4*>(p)[q] = v;
+            }
+        } else if constexpr (kBytes == 8) {
+            *reinterpret_cast<uint2*>(p) = make_uint2(w[0], w[1]);
+        } else if constexpr (kBytes == 4) {
+            *reinterpret_cast<unsigned int*>(p) = w[0];
+        } else {
+            *reinterpret_cast<unsigned short*>(p) = static_cast<unsigned short>(w[0]);
+        }
+    }
+    // the element-wise sum over a multicast address; a store that reaches every GPU's copy (V = 8)
+    __device__ __forceinline__ void load_sum(const void* mc_base, long long chunk) {
+#pragma unroll
+        for (int q = 0; q < kBytes / 16; ++q) {
+            const uint4 v = multimem_load_sum16<S>(reinterpret_cast<const uint4*>(mc_base) + chunk * (kBytes / 16) + q);
+            w[4 * q] = v.x; w[4 * q + 1] = v.y; w[4 * q + 2] = v.z; w[4 * q + 3] = v.w;
+        }
+    }
+    __device__ __forceinline__ void store_all(void* mc_base, long long chunk) const {
+#pragma unroll
+        for (int q = 0; q < kBytes / 16; ++q)
+            multimem_store16(reinterpret_cast<uint4*>(mc_base) + chunk * (kBytes / 16) + q,
+                             make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]));
+    }
+    __device__ __forceinline__ void unpack(float (&f)[V]) const {
+        if constexpr (sizeof(S) == 4) {
+#pragma unroll
+            for (int i = 0; i < V; ++i) f[i] = __uint_as_float(w[i]);
+        } else if constexpr (V == 1) {
+            float unused;
+            Packed<S>::unpack(w[0], f[0], unused);
+        } else {
+#pragma unroll
+            for (int i = 0; i < V; i += 2) Packed<S>::unpack(w[i / 2], f[i], f[i + 1]);
+        }
+    }
+    __device__ __forceinline__ void pack(const float (&f)[V]) {
+        if constexpr (sizeof(S) == 4) {
+#pragma unroll
+            for (int i = 0; i < V; ++i) w[i] = __float_as_uint(f[i]);
+        } else if constexpr (V == 1) {
+            w[0] = Packed<S>::pack(f[0], 0.0f);
+        } else {
+#pragma unroll
+            for (int i = 0; i < V; i += 2) w[i / 2] = Packed<S>::pack(f[i], f[i + 1]);
+        }
+    }
+};
+
+// The V code bytes of a chunk, in one or two words.
+template <int V> struct CodeChunk {
+    uint32_t w[V == 8 ? 2 : 1];
+    __device__ __forceinline__ void load(const uint8_t* base, long long chunk) {
+        if constexpr (V == 8) {
+            const uint2 v = __ldcs(reinterpret_cast<const uint2*>(base) + chunk);
+            w[0] = v.x; w[1] = v.y;
+        } else if constexpr (V == 4) w[0] = __ldcs(reinterpret_cast<const unsigned int*>(base) + chunk);
+        else if constexpr (V == 2) w[0] = __ldcs(reinterpret_cast<const unsigned short*>(base) + chunk);
+        else w[0] = __ldcs(base + chunk);
+    }
+    __device__ __forceinline__ void store(uint8_t* base, long long chunk) const {
+        if constexpr (V == 8) reinterpret_cast<uint2*>(base)[chunk] = make_uint2(w[0], w[1]);
+        else if constexpr (V == 4) reinterpret_cast<uint32_t*>(base)[chunk] = w[0];
+        else if constexpr (V == 2) reinterpret_cast<unsigned short*>(base)[chunk] = static_cast<unsigned short>(w[0]);
+        else base[chunk] = static_cast<uint8_t>(w[0]);
+    }
+};
+
+// Pulls the lines of this warp's NEXT block towards L2 while the current block is being worked on, so that its
+// loads later pay an L2 hit instead of a DRAM round trip: one instruction of one lane for a whole range (widened
+// to 16-byte boundaries).
+__device__ __forceinline__ void prefetch_l2_range(const void* base, long long bytes) {
+    const uintptr_t first = reinterpret_cast<uintptr_t>(base) & ~static_cast<uintptr_t>(15);
+    const uintptr_t last = (reinterpret_cast<uintptr_t>(base) + bytes + 15) & ~static_cast<uintptr_t>(15);
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(first), "r"(static_cast<uint32_t>(last - first)) : "memory");
 }
 
-// The updated momenta of chunk c, from the warp's staging slice.
-__device__ __forceinline__ void staged_momenta(const float4* stage_a, const float4* stage_b, int c, float (&m)[8]) {
-    const float4 ma = stage_a[c], mb = stage_b[c];
-    m[0] = ma.x; m[1] = ma.y; m[2] = ma.z; m[3] = ma.w;
-    m[4] = mb.x; m[5] = mb.y; m[6] = mb.z; m[7] = mb.w;
+// A block's updated momenta in the warp's staging slice: chunks of V floats; for V = 8 the first halves of all
+// chunks, then the second halves (`half` floats further on), so that the 128-bit accesses of a full warp are
+// conflict-free.
+template <int V> __device__ __forceinline__ void stage_store(float* stage, int half, int c, const float (&m)[V]) {
+    if constexpr (V == 8) {
+        *reinterpret_cast<float4*>(stage + 4 * c) = make_float4(m[0], m[1], m[2], m[3]);
+        *reinterpret_cast<float4*>(stage + half + 4 * c) = make_float4(m[4], m[5], m[6], m[7]);
+    } else if constexpr (V == 4) *reinterpret_cast<float4*>(stage + 4 * c) = make_float4(m[0], m[1], m[2], m[3]);
+    else if constexpr (V == 2) *reinterpret_cast<float2*>(stage + 2 * c) = make_float2(m[0], m[1]);
+    else stage[c] = m[0];
+}
+template <int V> __device__ __forceinline__ void stage_load(const float* stage, int half, int c, float (&m)[V]) {
+    if constexpr (V >= 4) {
+        const float4 a = *reinterpret_cast<const float4*>(stage + 4 * c);
+        m[0] = a.x; m[1] = a.y; m[2] = a.z; m[3] = a.w;
+        if constexpr (V == 8) {
+            const float4 b = *reinterpret_cast<const float4*>(stage + half + 4 * c);
+            m[4] = b.x; m[5] = b.y; m[6] = b.z; m[7] = b.w;
+        }
+    } else if constexpr (V == 2) {
+        const float2 a = *reinterpret_cast<const float2*>(stage + 2 * c);
+        m[0] = a.x; m[1] = a.y;
+    } else m[0] = stage[c];
 }
 
 // --------------------------------------------------------------------------- fast path
-// lut_query_fast with the table's shared-memory address folded into the rounding constant: the low mantissa
-// bits of fma(x, 16384, magic) are then the address of x's table entry itself (the address is a multiple of
-// eight, so the cell, the value with its low three bits cleared, is the same one) and the query needs no add.
-__device__ __forceinline__ float lut_magic(const unsigned char* lut) {
-    return 12582912.0f + 16384.0f + static_cast<float>(static_cast<uint32_t>(__cvta_generic_to_shared(lut)));
+// The quantiser of the fast path. Data-dependent shared-memory reads are what it would be bound by (the data pipe
+// serves one 128-byte row per cycle; a single table answers 32 random lanes in 3.5 to 6.6 rows), so every lane has
+// copies of its own, on its own bank, and every read is one row:
+//   rows   256 rows of 256 bytes: thr[e] of all 32 lanes, then cb[e] of all 32 lanes. A lane's address of entry e is
+//          (e << 8) + 4 * lane, one byte permute from a code byte.
+//   cells  256 words per lane; byte j of word r counts the thresholds below cell (j << 8) + r of 1024 uniform
+//          cells over [-1, 1].
+// x lies in cell N >> 7 with N = round(65472 x) + 65536 (the low mantissa bits of one FMA; 64 <= N <= 131008),
+// a map that is monotone in x, so its entry is the count of its cell plus the thresholds of the same cell below
+// x: `rounds` comparisons with the threshold of the entry so far, where rounds is the most thresholds that share a
+// cell (one or two for codebooks of the fit; a comparison too many is always false). Codebooks that put more than
+// kMaxRounds into a cell, or end below 1 (where the rule is not monotone), go through the binary search of exact_row.
+constexpr int kRowBytes = 256;
+constexpr int kSmemRows = kMaxCodebook * kRowBytes;
+constexpr int kCells = 1024;
+constexpr int kSmemCells = kCells * 32;
+constexpr int kMaxRounds = 6;
+// The tables lie at fixed shared-memory addresses, so that a read needs no address arithmetic beyond the row itself:
+// the offsets are immediates of the loads. Dynamic shared memory starts behind the 1024 bytes that the system keeps
+// and the kernels' static variables (at most 256 bytes; checked at run time, see fast_smem).
+constexpr int kFixed = 1024 + 256;
+constexpr int kRowsAt = kFixed, kCellsAt = kRowsAt + kSmemRows, kWsAt = kCellsAt + kSmemCells;
+constexpr int kStageAt = kWsAt + kSmemWs;       // the warps' staging slices follow
+constexpr int kSmemTables = kStageAt - 1024;    // dynamic shared memory up to the slices
+static_assert(kFixed % 128 == 0 && kStageAt % 16 == 0, "a lane's words lie on its own bank, the staging slices hold float4");
+
+extern __shared__ __align__(128) unsigned char g_smem[];
+// The generic pointer of a fixed shared-memory address.
+__device__ __forceinline__ unsigned char* fast_smem(int address) { return g_smem + (address - static_cast<int>(smem_u32(g_smem))); }
+
+__device__ __forceinline__ float cell_position(float x) { return fmaf(x, 65472.0f, 8388608.0f + 65536.0f); }
+__device__ __forceinline__ int threshold_cell(float t) {   // -1: below every x; kCells: above or equal to every x
+    if (t < -1.0f) return -1;
+    if (!(t < 1.0f)) return kCells;
+    return static_cast<int>((__float_as_uint(cell_position(t)) & 0x1FFFFu) >> 7);
 }
-__device__ __forceinline__ uint32_t lut_query_shared(float x, float magic) {
-    const uint32_t addr = __float_as_uint(fmaf(x, 16384.0f, magic)) & 0x3FFF8u;
-    uint32_t thr_bits, below;
-    asm("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(thr_bits), "=r"(below) : "r"(addr));
-    return below + (x > __uint_as_float(thr_bits) ? 1u : 0u);
+
+// This lane's view of the tables.
+struct LaneTables {
+    uint32_t lane4;       // 4 * lane
+    int rounds;           // 0: no fast answer, exact_row
+    int k;                // true codebook size
+    // row address of the entry in byte `i` of w
+    __device__ __forceinline__ uint32_t row_of_byte(uint32_t w, int i) const { return __byte_perm(w, lane4, 0x6504u | (i << 4)); }
+    __device__ __forceinline__ uint32_t row_of_entry(uint32_t e) const { return row_of_byte(e, 0); }
+    __device__ __forceinline__ float value(uint32_t row) const {
+        float f;
+        asm("ld.shared.f32 %0, [%1 + %2];" : "=f"(f) : "r"(row), "n"(kRowsAt + 128));
+        return f;
+    }
+    __device__ __forceinline__ float threshold(uint32_t row) const {
+        float f;
+        asm("ld.shared.f32 %0, [%1 + %2];" : "=f"(f) : "r"(row), "n"(kRowsAt));
+        return f;
+    }
+    // y = cell_position(x): the row of the count of thresholds in lower cells (the exponent bits of y come off in
+    // the load's offset)
+    __device__ __forceinline__ uint32_t cell_row(float y) const {
+        const uint32_t bits = __float_as_uint(y);
+        const uint32_t at = ((bits & 0x7F80u) | lane4) + (bits >> 15);
+        uint32_t below;
+        asm("ld.shared.u8 %0, [%1 + %2];" : "=r"(below) : "r"(at), "n"(kCellsAt - (0x4B000000 >> 15)));
+        return row_of_byte(below, 0);
+    }
+    __device__ __forceinline__ uint32_t refine(float x, uint32_t row) const { return row + (x > threshold(row) ? kRowBytes : 0u); }
+    // entry_exact (any codebook, NaN and values above the last entry included), reading this lane's copies
+    __device__ __forceinline__ uint32_t exact_row(float x) const {
+        const uint32_t last = row_of_entry(k - 1);
+        if (x > value(last)) {
+            const uint32_t left = k >= 2 ? last - kRowBytes : last;
+            return fabsf(x - value(left)) <= fabsf(x - value(last)) ? left : last;
+        }
+        uint32_t row = lane4;
+#pragma unroll
+        for (uint32_t step = 128; step > 0; step >>= 1) {
+            if (threshold(row + (step - 1) * kRowBytes) < x) row += step * kRowBytes;
+        }
+        return row;
+    }
+};
+
+// Fills rows and cells from the staged codebook and thresholds; every thread of the CTA. `scratch`: 1028 bytes of
+// shared memory that are free until the next __syncthreads after the call.
+__device__ __forceinline__ LaneTables build_lane_tables(const SmemView& s, unsigned char* scratch) {
+    unsigned char* below = scratch;
+    int* most = reinterpret_cast<int*>(scratch + kCells);
+    if (threadIdx.x == 0) *most = 1;
+    __syncthreads();
+    for (int i = threadIdx.x; i < kMaxCodebook; i += blockDim.x) {
+        const int c = threshold_cell(s.thr[i]);
+        const int before = i == 0 ? -1 : threshold_cell(s.thr[i - 1]);
+        for (int cell = before + 1; cell <= c && cell < kCells; ++cell) below[cell] = static_cast<unsigned char>(i);
+        if (c >= 0 && c < kCells) {
+            int run = 1;
+            while (run <= kMaxRounds && i + run < kMaxCodebook && threshold_cell(s.thr[i + run]) == c) ++run;
+            if (run > 1) atomicMax(most, run);
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kSmemRows / 16; i += blockDim.x) {
+        const float v = (i & 8) ? s.cb[i >> 4] : s.thr[i >> 4];
+        reinterpret_cast<float4*>(fast_smem(kRowsAt))[i] = make_float4(v, v, v, v);
+    }
+    for (int i = threadIdx.x; i < kSmemCells / 16; i += blockDim.x) {
+        const int r = i >> 3;
+        const uint32_t w = below[r] | (below[256 + r] << 8) | (below[512 + r] << 16) | (static_cast<uint32_t>(below[768 + r]) << 24);
+        reinterpret_cast<uint4*>(fast_smem(kCellsAt))[i] = make_uint4(w, w, w, w);
+    }
+    LaneTables t;
+    t.lane4 = (threadIdx.x & 31u) * 4u;
+    t.k = s.k;
+    t.rounds = __shfl_sync(0xffffffffu, (*most > kMaxRounds || s.cb[s.k - 1] < 1.0f) ? 0 : *most, 0);
+    __syncthreads();
+    asm volatile("" : "+r"(t.lane4)::"memory");   // every read of the tables depends on lane4: none before this point
+    return t;
+}
+
+// The same two-operation form for the last element of an odd chunk: the second half is not used.
+template <int V> __device__ __forceinline__ f32x2 pair_at(const float (&f)[V], int i) { return pair(f[i], f[i + 1 < V ? i + 1 : i]); }
+template <int V> __device__ __forceinline__ void unpair_at(f32x2 v, float (&f)[V], int i) {
+    float spare;
+    if (i + 1 < V) unpair(v, f[i], f[i + 1]); else unpair(v, f[i], spare);
+}
+
+// Row addresses of the entries of a chunk of momenta (quotients m / absmax through the block's reciprocal, see
+// div_by_block_constant). ONE: t.rounds == 1, the usual codebook.
+template <int V, bool ONE>
+__device__ __forceinline__ void encode(const float (&m)[V], f32x2 neg_absmax2, f32x2 rinv2, const LaneTables& t,
+                                       uint32_t (&row)[V]) {
+    float x[V];
+#pragma unroll
+    for (int i = 0; i < V; i += 2) {
+        const f32x2 m2 = pair_at(m, i);
+        const f32x2 q0 = mul2(m2, rinv2);
+        unpair_at(fma2(fma2(q0, neg_absmax2, m2), rinv2, q0), x, i);
+    }
+#pragma unroll
+    for (int i = 0; i < V; ++i) row[i] = t.cell_row(cell_position(x[i]));
+#pragma unroll
+    for (int i = 0; i < V; ++i) row[i] = t.refine(x[i], row[i]);
+    if constexpr (!ONE) {
+        if (t.rounds == 0) {
+#pragma unroll
+            for (int i = 0; i < V; ++i) row[i] = t.exact_row(x[i]);
+        } else {
+            for (int r = 1; r < t.rounds; ++r) {
+#pragma unroll
+                for (int i = 0; i < V; ++i) row[i] = t.refine(x[i], row[i]);
+            }
+        }
+    }
+}
+// The code bytes of a chunk's row addresses.
+template <int V> __device__ __forceinline__ CodeChunk<V> row_codes(const uint32_t (&row)[V]) {
+    CodeChunk<V> c;
+    if constexpr (V >= 4) {
+#pragma unroll
+        for (int i = 0; i < V; i += 4)
+            c.w[i / 4] = __byte_perm(__byte_perm(row[i], row[i + 1], 0x0051), __byte_perm(row[i + 2], row[i + 3], 0x0051), 0x5410);
+    } else if constexpr (V == 2) c.w[0] = __byte_perm(row[0], row[1], 0x0051);
+    else c.w[0] = row[0] >> 8;
+    return c;
 }
 
 // Lanes that share one block, a power of two, so that a warp works on 32 / lanes blocks at once. A lane takes
 // several chunks of its block, which keeps as many loads in flight and shares the per-block work (reductions,
-// step size, reciprocal, descriptor reads) between more elements: about eight chunks per lane for blocks of
-// more than 256 elements, as in a 2048-element block (8 lanes for 512 elements, 16 for 1024, all 32 from 1032
-// elements on; measured on 512-element blocks: 0.43 ms -> 0.32 ms per 134 M elements), up to four for 136 to
-// 256 elements (8 lanes; 256-element bf16 blocks: 0.25 -> 0.50 of the copy bandwidth against one chunk per
-// lane), two below that (bf16, 128 / 64 / 32 elements: 0.23 -> 0.37 / 0.36 / 0.35; four per lane there puts the
-// staging slices of a warp's blocks on the same shared-memory banks and is slower for 2-byte elements).
-__host__ __device__ __forceinline__ int lanes_per_block(long long period) {
-    const long long nchunks = period >> 3;
-    const long long want = nchunks > 32 ? (nchunks + 7) >> 3 : (nchunks > 16 ? (nchunks + 3) >> 2 : (nchunks + 1) >> 1);
-    int lanes = 1;
-    while (lanes < 32 && lanes < want) lanes <<= 1;
-    return lanes;
+// step size, reciprocal) between more elements: about eight chunks of eight elements per lane for blocks of more
+// than 256 elements, as in a 2048-element block (8 lanes for 512 elements, 16 for 1024, all 32 from 1032 on), up to
+// four below that (134 M bf16 elements in blocks of 128 / 64 / 32: 0.315 / 0.331 / 0.332 ms, with up to two chunks
+// per lane 0.46 / 0.47 / 0.50; fp32 keeps two for blocks of 64 and less, whose lanes would otherwise each read
+// 128 bytes of their own: 67 M elements 0.233 against 0.427 ms).
+__host__ __device__ __forceinline__ int lanes_shift(long long nchunks, int v, int es) {   // log2 of the lanes; chunks of v elements of es bytes
+    if (v < 8) {   // smaller chunks: about sixteen per lane, eight of them in flight
+        int shift = 0;
+        while (shift < 5 && (16 << shift) < nchunks) ++shift;
+        return shift;
+    }
+    const long long want = nchunks > 32 ? (nchunks + 7) >> 3 : ((es == 4 && nchunks <= 8) ? (nchunks + 1) >> 1 : (nchunks + 3) >> 2);
+    int shift = 0;
+    while (shift < 5 && (1 << shift) < want) ++shift;
+    return shift;
 }
-// Elements of one work unit of a tensor (what a warp stages at a time).
-__host__ __device__ __forceinline__ long long unit_elements(long long period) {
-    return period * (32 / lanes_per_block(period));
+// Elements of one work unit of a tensor (what a warp stages at a time), blocks of nchunks chunks of v elements.
+__host__ __device__ __forceinline__ long long unit_elements(long long period, int v, int es) { return period << (5 - lanes_shift(period / v, v, es)); }
+// Floats from one block's staged momenta to the next one's in a warp's slice. Eight lanes make one 128-byte access;
+// where they belong to several blocks (fewer than eight lanes per block), the blocks' slices start on different banks.
+__host__ __device__ __forceinline__ int slice_stride(int period, int shift, int v) {
+    return v < 8 || shift >= 3 ? period : ((period + 31) & ~31) + (4 << shift);
+}
+// Floats that a warp stages for one unit.
+__host__ __device__ __forceinline__ long long unit_floats(long long period, int v, int es) {
+    const int shift = lanes_shift(period / v, v, es);
+    return static_cast<long long>(slice_stride(static_cast<int>(period), shift, v)) << (5 - shift);
 }
 // Work units (one warp pass each) of a tensor on the fast path.
-__host__ __device__ __forceinline__ long long vec_units(long long num_blocks, long long period) {
-    const int group = 32 / lanes_per_block(period);
-    return (num_blocks + group - 1) / group;
+__host__ __device__ __forceinline__ long long vec_units(long long num_blocks, long long period, int v, int es) {
+    const int shift = 5 - lanes_shift(period / v, v, es);
+    return (num_blocks + (1 << shift) - 1) >> shift;
 }
 
 // Reductions over aligned groups of `lanes` lanes (a power of two); every lane of the warp calls them.
@@ -358,21 +580,57 @@ __device__ __forceinline__ float group_sum(float v, int lanes) {
     return v;
 }
 
+// What the passes need of a tensor, in a shared-memory slot of the warp: its descriptor lives in global memory, where
+// the passes' stores might alias it as far as the compiler can tell, and is read again only when the warp comes to
+// another tensor. (In registers it would cost some 25 of them for values that are used once per block.)
+template <typename S> struct alignas(8) TensorSlot {
+    const S* g;
+    S* p;
+    uint8_t* codes;
+    void* mag;
+    void* v;
+    long long first, units, num_blocks;   // in the launch's work units; blocks
+    int period, mag_dtype, v_dtype;
+    uint32_t flags;
+    float beta1, beta2, inv_bc1, bc2, eps, lr, wd_mul;
+    __device__ __forceinline__ void load(const gefen_b200_step_tensor_t* t, int v_elems) {
+        g = static_cast<const S*>(t->g);
+        p = static_cast<S*>(t->p);
+        codes = t->codes;
+        mag = t->mag;
+        v = t->v;
+        first = t->first_block;
+        num_blocks = t->num_blocks;
+        period = static_cast<int>(t->period);   // at most kFastMaxPeriod
+        flags = t->flags;
+        units = vec_units(num_blocks, period, v_elems, sizeof(S));
+        mag_dtype = t->mag_dtype;
+        v_dtype = t->v_dtype;
+        beta1 = t->beta1;
+        beta2 = t->beta2;
+        inv_bc1 = 1.0f / t->bc1;
+        bc2 = t->bc2;
+        eps = t->eps;
+        lr = t->lr;
+        wd_mul = t->wd_mul;
+    }
+};
+
 // First pass over U chunks of one lane (chunks c0, c0 + LANES, ...): all loads first, then the
 // moment update, the running absmax and sum of squares, and the staging of the updated momenta.
 // SUMMED: g_blk is the multicast address of the block's gradients; a load returns the sum over the ranks,
 // which is scaled by `scale` and rounded to the gradient dtype as a reduce-scatter into it would leave it.
-template <typename S, int U, bool GUARD, bool SUMMED>
-__device__ __forceinline__ void first_pass_group(const S* g_blk, const uint2* codes_in, float4* stage_a, float4* stage_b,
-                                                 const float* rep, int c0, int LANES, int nchunks, float old_mag,
-                                                 float beta1, float omb1, float scale, float& absmax, float& sumsq) {
-    uint2 craw[U];
-    Chunk<S> graw[U];
+template <typename S, int V, int U, bool GUARD, bool SUMMED>
+__device__ __forceinline__ void first_pass_group(const S* g_blk, const uint8_t* codes_in, float* stage, int half,
+                                                 const LaneTables& t, int c0, int LANES, int nchunks, f32x2 mag2,
+                                                 f32x2 beta2_, f32x2 omb2_, float scale, float& absmax, f32x2& sumsq2) {
+    CodeChunk<V> craw[U];
+    Chunk<S, V> graw[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
         const int c = c0 + LANES * u;
         if (!GUARD || c < nchunks) {
-            craw[u] = __ldcs(codes_in + c);
+            craw[u].load(codes_in, c);
             if (SUMMED) graw[u].load_sum(g_blk, c);
             else graw[u].load(g_blk, c);
         }
@@ -381,26 +639,34 @@ __device__ __forceinline__ void first_pass_group(const S* g_blk, const uint2* co
     for (int u = 0; u < U; ++u) {
         const int c = c0 + LANES * u;
         if (!GUARD || c < nchunks) {
-            float g[8], m[8];
+            float g[V], m[V];
             graw[u].unpack(g);
             if (SUMMED) {
 #pragma unroll
-                for (int i = 0; i < 8; ++i) g[i] *= scale;
-                Chunk<S> rounded;
+                for (int i = 0; i < V; ++i) g[i] *= scale;
+                Chunk<S, V> rounded;
                 rounded.pack(g);
                 rounded.unpack(g);
             }
-            const uint32_t cw[2] = {craw[u].x, craw[u].y};
+            if constexpr (V == 1) {
+                const float cur = t.value(t.row_of_byte(craw[u].w[0], 0));
+                float lo, spare;
+                unpair(fma2(beta2_, mul2(mag2, pair(cur, cur)), mul2(omb2_, pair(g[0], g[0]))), lo, spare);
+                m[0] = lo;
+                absmax = max_abs_nan(absmax, lo);
+                sumsq2 = fma2(pair(g[0], 0.0f), pair(g[0], 0.0f), sumsq2);
+            } else {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const uint32_t code = __byte_perm(cw[i >> 2], 0u, 0x4440u + (i & 3));   // byte i & 3, zero-extended
-                const float cur = old_mag * rep[code * kRepCopies];
-                m[i] = ema_update(beta1, cur, omb1, g[i]);
-                absmax = max_abs_nan(absmax, m[i]);
-                sumsq = fmaf(g[i], g[i], sumsq);
+                for (int i = 0; i < V; i += 2) {
+                    const f32x2 g2 = pair(g[i], g[i + 1]);
+                    const f32x2 cur = mul2(mag2, pair(t.value(t.row_of_byte(craw[u].w[i >> 2], i & 3)),
+                                                      t.value(t.row_of_byte(craw[u].w[i >> 2], (i & 3) + 1))));
+                    unpair(fma2(beta2_, cur, mul2(omb2_, g2)), m[i], m[i + 1]);   // ema_update
+                    absmax = max_abs_nan(max_abs_nan(absmax, m[i]), m[i + 1]);
+                    sumsq2 = fma2(g2, g2, sumsq2);
+                }
             }
-            stage_a[c] = make_float4(m[0], m[1], m[2], m[3]);
-            stage_b[c] = make_float4(m[4], m[5], m[6], m[7]);
+            stage_store<V>(stage, half, c, m);
         }
     }
 }
@@ -410,8 +676,8 @@ __device__ __forceinline__ void first_pass_group(const S* g_blk, const uint2* co
 // a chunk are added batch after batch, in the order given.
 // EXACT: there are exactly NSRC sources (no test per source).
 template <typename S, int NSRC, bool EXACT = false>
-__device__ __forceinline__ void reduce_pass(const StepLaunch& L, const S* g_blk, const uint2* codes_in, float4* stage_a,
-                                            float4* stage_b, const float* rep, int lane, int LANES, int nchunks,
+__device__ __forceinline__ void reduce_pass(const StepLaunch& L, const S* g_blk, const uint8_t* codes_in, float* stage, int half,
+                                            const LaneTables& t, int lane, int LANES, int nchunks,
                                             float old_mag, float beta1, float omb1, float& absmax, float& sumsq) {
     constexpr int kSlots = sizeof(S) == 2 ? 4 : 2;
     constexpr int BS = NSRC < kSlots ? NSRC : kSlots;
@@ -420,17 +686,17 @@ __device__ __forceinline__ void reduce_pass(const StepLaunch& L, const S* g_blk,
     const float scale = L.grad_scale;
     for (int c0 = lane; c0 < nchunks; c0 += LANES * U) {
         float acc[U][8];
-        uint2 craw[U];   // the codes travel with the first batch of gradient loads
+        CodeChunk<8> craw[U];   // the codes travel with the first batch of gradient loads
 #pragma unroll
         for (int u = 0; u < U; ++u) {
 #pragma unroll
             for (int i = 0; i < 8; ++i) acc[u][i] = 0.0f;
-            if (c0 + LANES * u < nchunks) craw[u] = __ldcs(codes_in + c0 + LANES * u);
+            if (c0 + LANES * u < nchunks) craw[u].load(codes_in, c0 + LANES * u);
         }
 #pragma unroll
         for (int r0 = 0; r0 < NSRC; r0 += BS) {
             if (r0 < n_src) {
-                Chunk<S> src[U * BS];
+                Chunk<S, 8> src[U * BS];
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     const int c = c0 + LANES * u;
@@ -459,86 +725,101 @@ __device__ __forceinline__ void reduce_pass(const StepLaunch& L, const S* g_blk,
             if (c < nchunks) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) acc[u][i] *= scale;
-                Chunk<S> rounded;
+                Chunk<S, 8> rounded;
                 rounded.pack(acc[u]);
                 float g[8], m[8];
                 rounded.unpack(g);
-                const uint32_t cw[2] = {craw[u].x, craw[u].y};
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                    const uint32_t code = __byte_perm(cw[i >> 2], 0u, 0x4440u + (i & 3));   // byte i & 3, zero-extended
-                    const float cur = old_mag * rep[code * kRepCopies];
+                    const float cur = old_mag * t.value(t.row_of_byte(craw[u].w[i >> 2], i & 3));
                     m[i] = ema_update(beta1, cur, omb1, g[i]);
                     absmax = max_abs_nan(absmax, m[i]);
                     sumsq = fmaf(g[i], g[i], sumsq);
                 }
-                stage_a[c] = make_float4(m[0], m[1], m[2], m[3]);
-                stage_b[c] = make_float4(m[4], m[5], m[6], m[7]);
+                stage_store<8>(stage, half, c, m);
             }
         }
     }
 }
 
-// The re-encode and update loop of the common case (finite block, Gefen update of the parameters) with
-// everything that is fixed per launch or per tensor decided at compile time, so that the loop body carries no
-// branch but the rare one into the exact quantiser: WD = the decoupled weight decay of the reference's
-// separate multiply, STORE = 0 this GPU's copy only, 1 peer stores as well, 2 one multicast store.
-// The parameters of the next chunk are fetched while this one is encoded.
-template <typename S, bool WD, int STORE>
-__device__ __forceinline__ void second_pass_common(const StepLaunch& L, const SmemView& s, const float* rep,
-                                                   const float4* stage_a, const float4* stage_b, uint2* codes_out,
-                                                   S* p_blk, Chunk<S> pnext, int lane, int LANES, int nchunks,
-                                                   float absmax, float rinv, float step, float lr, float wd_mul) {
-    const float neg_step = -step;
-    const float magic = lut_magic(s.lut);
-    for (int c = lane; c < nchunks; c += LANES) {
-        Chunk<S> praw = pnext;
-        if (c + LANES < nchunks) pnext.load(p_blk, c + LANES);
-        float m[8];
-        staged_momenta(stage_a, stage_b, c, m);
-        uint32_t code[8];
-        uint32_t any = 0u;
+// One chunk of the re-encode and update of the common case (finite block, Gefen update of the parameters) with
+// everything that is fixed per launch or per tensor decided at compile time: WD = the decoupled weight decay of the
+// reference's separate multiply, STORE = 0 this GPU's copy only, 1 peer stores as well, 2 one multicast store, ONE =
+// see encode.
+struct BlockScalars {
+    f32x2 neg_absmax2, rinv2, step2, lr2, wd2;
+};
+template <typename S, int V, bool WD, int STORE, bool ONE>
+__device__ __forceinline__ void update_chunk(const StepLaunch& L, const LaneTables& t, const float* stage, int half,
+                                             uint8_t* codes, S* p_blk, Chunk<S, V> praw, int c, const BlockScalars& b) {
+    float m[V];
+    stage_load<V>(stage, half, c, m);
+    uint32_t row[V];
+    encode<V, ONE>(m, b.neg_absmax2, b.rinv2, t, row);
+    row_codes<V>(row).store(codes, c);
+    float pv[V];
+    praw.unpack(pv);
+    if (WD) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float x = div_by_block_constant(m[i], absmax, rinv);
-            code[i] = lut_query_shared(x, magic);
-            any |= code[i];
-        }
-        if (any & kLutSlowBit) {   // rare: a cell with two thresholds, or values above the last entry
+        for (int i = 0; i < V; i += 2) unpair_at(mul2(pair_at(pv, i), b.wd2), pv, i);
+        Chunk<S, V> rounded;       // the separate multiply of the reference rounds to the parameter dtype
+        rounded.pack(pv);
+        rounded.unpack(pv);
+    }
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                if (code[i] & kLutSlowBit) {
-                    const float x = div_by_block_constant(m[i], absmax, rinv);
-                    code[i] = static_cast<uint32_t>(entry_exact(x, s.thr, s.cb, s.k));
-                }
-            }
+    for (int i = 0; i < V; i += 2) {
+        const f32x2 neg_q = mul2(pair(t.value(row[i]), t.value(row[i + 1 < V ? i + 1 : i])), b.neg_absmax2);
+        unpair_at(fma2(mul2(neg_q, b.step2), b.lr2, pair_at(pv, i)), pv, i);   // fma(-(q * step), lr, p)
+    }
+    praw.pack(pv);
+    if (STORE == 2) {
+        praw.store_all(peer_ptr(p_blk, L.param_mc_delta), c);   // every rank's copy, this one included
+    } else {
+        praw.store(p_blk, c);
+        if (STORE == 1) {
+            const int n_peers = L.n_peers;
+            for (int r = 0; r < n_peers; ++r) praw.store(peer_ptr(p_blk, L.peer_delta[r]), c);
         }
-        uint2 cw;
-        cw.x = __byte_perm(__byte_perm(code[0], code[1], 0x0040), __byte_perm(code[2], code[3], 0x0040), 0x5410);
-        cw.y = __byte_perm(__byte_perm(code[4], code[5], 0x0040), __byte_perm(code[6], code[7], 0x0040), 0x5410);
-        codes_out[c] = cw;
-        float pv[8];
-        praw.unpack(pv);
-        if (WD) {
+    }
+}
+// Parameters (GefenMuon: gradients) of a lane's chunks that are requested ahead of the re-encoding: the next chunk of
+// eight elements, the next eight of the smaller chunks, whose work is too short to cover the latency of a load.
+template <typename S, int V> struct Ahead {
+    static constexpr int kDepth = V < 8 ? (V * sizeof(S) > 8 ? 4 : 8) : 1;
+    Chunk<S, V> slot[kDepth];
+    __device__ __forceinline__ void start(const S* blk, int lane, int LANES, int nchunks) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) pv[i] *= wd_mul;
-            Chunk<S> rounded;       // the separate multiply of the reference rounds to the parameter dtype
-            rounded.pack(pv);
-            rounded.unpack(pv);
+        for (int u = 0; u < kDepth; ++u)
+            if (lane + u * LANES < nchunks) slot[u].load(blk, lane + u * LANES);
+    }
+    // hands out slot u (chunk c) and requests the chunk that comes to it next
+    __device__ __forceinline__ Chunk<S, V> take(int u, const S* blk, int c, int LANES, int nchunks) {
+        const Chunk<S, V> now = slot[u];
+        if (c + kDepth * LANES < nchunks) slot[u].load(blk, c + kDepth * LANES);
+        return now;
+    }
+};
+// The chunks of one block: `full` rounds in which every lane of the warp has one, then the guarded rest. The
+// parameters of the next chunks are fetched while this one is encoded.
+template <typename S, int V, bool WD, int STORE, bool ONE>
+__device__ __forceinline__ void second_pass_common(const StepLaunch& L, const LaneTables& t, const float* stage,
+                                                   int half, uint8_t* codes, S* p_blk, Ahead<S, V>& ahead, int lane, int LANES,
+                                                   int nchunks, int full, int rounds_all, const BlockScalars& b) {
+    constexpr int D = Ahead<S, V>::kDepth;
+    int c = lane;
+    int it = 0;
+    if constexpr (D == 1) {
+        for (; it < full; ++it, c += LANES) {
+            const Chunk<S, V> praw = ahead.take(0, p_blk, c, LANES, nchunks);
+            update_chunk<S, V, WD, STORE, ONE>(L, t, stage, half, codes, p_blk, praw, c, b);
         }
+    }
+    for (; it < rounds_all; it += D, c += D * LANES) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float q = rep[code[i] * kRepCopies] * absmax;
-            pv[i] = fmaf(q * neg_step, lr, pv[i]);   // = fma(-(q * step), lr, p)
-        }
-        praw.pack(pv);
-        if (STORE == 2) {
-            praw.store_all(peer_ptr(p_blk, L.param_mc_delta), c);   // every rank's copy, this one included
-        } else {
-            praw.store(p_blk, c);
-            if (STORE == 1) {
-                const int n_peers = L.n_peers;
-                for (int r = 0; r < n_peers; ++r) praw.store(peer_ptr(p_blk, L.peer_delta[r]), c);
+        for (int u = 0; u < D; ++u) {
+            if (c + u * LANES < nchunks) {
+                const Chunk<S, V> praw = ahead.take(u, p_blk, c + u * LANES, LANES, nchunks);
+                update_chunk<S, V, WD, STORE, ONE>(L, t, stage, half, codes, p_blk, praw, c + u * LANES, b);
             }
         }
     }
@@ -548,138 +829,129 @@ __device__ __forceinline__ void second_pass_common(const StepLaunch& L, const Sm
 // with the gradient when asked (torch: m.mul_(momentum).add_(g, alpha=1-momentum) on the rounded momentum,
 // reference gefen_muon.py:312-314; alpha travels in the descriptor's beta2), goes where the Gefen step keeps
 // the parameters. The gradient chunk of the next iteration is requested while this one is encoded.
-template <typename S, bool NESTEROV>
-__device__ __forceinline__ void second_pass_muon(const SmemView& s, const float* rep, const float4* stage_a,
-                                                 const float4* stage_b, uint2* codes_out, const S* g_blk, S* out_blk,
-                                                 int lane, int LANES, int nchunks, float absmax, float rinv,
-                                                 float beta1, float alpha) {
-    const float magic = lut_magic(s.lut);
-    Chunk<S> gnext;
-    if (NESTEROV && lane < nchunks) gnext.load(g_blk, lane);
-    for (int c = lane; c < nchunks; c += LANES) {
-        Chunk<S> graw = gnext;
-        if (NESTEROV && c + LANES < nchunks) gnext.load(g_blk, c + LANES);
-        float m[8];
-        staged_momenta(stage_a, stage_b, c, m);
-        uint32_t code[8];
-        uint32_t any = 0u;
+template <typename S, int V, bool NESTEROV>
+__device__ __forceinline__ void second_pass_muon(const LaneTables& t, const float* stage, int half, uint8_t* codes,
+                                                 const S* g_blk, S* out_blk, int lane, int LANES, int nchunks, float absmax,
+                                                 f32x2 neg_absmax2, f32x2 rinv2, float beta1, float alpha) {
+    constexpr int D = Ahead<S, V>::kDepth;
+    Ahead<S, V> ahead;
+    if (NESTEROV) ahead.start(g_blk, lane, LANES, nchunks);
+    for (int c0 = lane; c0 < nchunks; c0 += D * LANES) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float x = div_by_block_constant(m[i], absmax, rinv);
-            code[i] = lut_query_shared(x, magic);
-            any |= code[i];
-        }
-        if (any & kLutSlowBit) {   // rare: a cell with two thresholds, or values above the last entry
+        for (int u = 0; u < D; ++u) {
+        const int c = c0 + u * LANES;
+        if (c >= nchunks) break;
+        Chunk<S, V> graw;
+        if (NESTEROV) graw = ahead.take(u, g_blk, c, LANES, nchunks);
+        float m[V];
+        stage_load<V>(stage, half, c, m);
+        uint32_t row[V];
+        encode<V, false>(m, neg_absmax2, rinv2, t, row);
+        row_codes<V>(row).store(codes, c);
+        float q[V];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                if (code[i] & kLutSlowBit) {
-                    const float x = div_by_block_constant(m[i], absmax, rinv);
-                    code[i] = static_cast<uint32_t>(entry_exact(x, s.thr, s.cb, s.k));
-                }
-            }
-        }
-        uint2 cw;
-        cw.x = __byte_perm(__byte_perm(code[0], code[1], 0x0040), __byte_perm(code[2], code[3], 0x0040), 0x5410);
-        cw.y = __byte_perm(__byte_perm(code[4], code[5], 0x0040), __byte_perm(code[6], code[7], 0x0040), 0x5410);
-        codes_out[c] = cw;
-        float q[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) q[i] = rep[code[i] * kRepCopies] * absmax;
+        for (int i = 0; i < V; ++i) q[i] = t.value(row[i]) * absmax;
         if (NESTEROV) {
-            float g[8];
+            float g[V];
             graw.unpack(g);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
+            for (int i = 0; i < V; ++i) {
                 const float m1 = ScalarIO<S>::round(ScalarIO<S>::round(q[i]) * beta1);
                 q[i] = fmaf(alpha, g[i], m1);
             }
         }
-        Chunk<S> out;
+        Chunk<S, V> out;
         out.pack(q);
         out.store(out_blk, c);
+        }
     }
 }
 
-// One warp, one unit: 32 / LANES consecutive blocks of t.period = 8 * nchunks elements, LANES lanes
-// each (LANES = lanes_per_block(t.period), uniform over the warp; FULL fixes it to 32 at compile
-// time, for blocks of more than 1024 elements). A block's slice of `stage` holds period floats: the first halves of all chunks, then the
-// second halves, so that the 128-bit shared accesses of a full warp are conflict-free.
-// The descriptor lives in global or parameter memory, which the stores below might alias as far as
-// the compiler can tell: everything the loops need from it is copied into locals first.
+// One warp, one unit: 32 / LANES consecutive blocks of t.period = V * chunks elements, LANES lanes
+// each (a power of two, uniform over the warp; FULL fixes it to 32 at compile
+// time, for blocks of more than 1024 elements). A block's slice of `stage` holds period floats (see stage_store).
 // GSRC: where the gradients come from: 0 = this GPU's buffer, 1 = averaged over the ranks' buffers with peer
 // loads, 2 = summed by the switch through the multicast mapping (StepLaunch::grad_mc_delta).
-template <typename S, int GSRC, bool FULL>
-__device__ __forceinline__ void warp_block_step(const gefen_b200_step_tensor_t& t, long long unit, const StepLaunch& L,
-                                                const SmemView& s, float* stage, int warp_lane) {
+template <typename S, int V, int GSRC, bool FULL>
+__device__ __forceinline__ void warp_block_step(const TensorSlot<S>& t, long long unit, const StepLaunch& L, const LaneTables& tables,
+                                                float* stage, int warp_lane) {
     const float* const stepsize = L.stepsize;
-    const int n_peers = L.n_peers;
-    const long long param_mc = L.param_mc_delta;
-    const int period = static_cast<int>(t.period);     // at most kFastMaxPeriod
-    const int LANES = FULL ? 32 : lanes_per_block(period);
+    const int n_peers = GSRC == 0 && V < 8 ? 0 : L.n_peers;            // (chunks below 8 serve this GPU's buffers only)
+    const long long param_mc = GSRC == 0 && V < 8 ? 0 : L.param_mc_delta;
+    // (the shuffle tells the compiler that the period is the same in all lanes, which the loops' bounds profit from)
+    const int period = __shfl_sync(0xffffffffu, t.period, 0);
+    const int chunks = period / V;                     // of a block
+    const int shift = FULL ? 5 : lanes_shift(chunks, V, sizeof(S));
+    const int LANES = 1 << shift;
     const int lane = warp_lane & (LANES - 1);          // lane within the block's group
-    const int member = warp_lane >> (31 - __clz(LANES));   // which block of the unit
-    const long long b = unit * (32 / LANES) + member;
-    const bool valid = b < t.num_blocks;               // the last unit of a tensor may be short
-    const int nchunks = valid ? (period >> 3) : 0;
-    stage += member * period;
+    const int member = warp_lane >> shift;             // which block of the unit
+    const long long b = (unit << (5 - shift)) + member;
+    const bool all_valid = FULL || ((unit + 1) << (5 - shift)) <= t.num_blocks;   // the last unit of a tensor may be short
+    const bool valid = FULL || b < t.num_blocks;
+    const int nchunks = valid ? chunks : 0;
+    stage += member * slice_stride(period, shift, V);
+    const int half = period >> 1;
     const long long elem0 = b * static_cast<long long>(period);
-    const uint2* const codes_in = reinterpret_cast<const uint2*>(t.codes + elem0);
-    uint2* const codes_out = reinterpret_cast<uint2*>(t.codes + elem0);
-    const S* const g_blk = static_cast<const S*>(t.g) + elem0;   // chunk c of the block = 8 elements at g_blk + 8 c
-    S* const p_blk = static_cast<S*>(t.p) + elem0;
+    uint8_t* const codes = t.codes + elem0;
+    const S* const g_blk = t.g + elem0;   // chunk c of the block = V elements at g_blk + V c
+    S* const p_blk = t.p + elem0;
     const uint32_t flags = t.flags;
     const bool muon = (flags & GEFEN_B200_STEP_MUON) != 0;
 
     const float beta1 = t.beta1;
     const float omb1 = 1.0f - beta1;
     const float old_mag = valid ? load_state(t.mag, b, t.mag_dtype) : 0.0f;
-    float4* const stage_a = reinterpret_cast<float4*>(stage);
-    float4* const stage_b = stage_a + (period >> 3);
-    const float* rep = s.rep;  // this lane's copy of the codebook: entry e at rep[e * kRepCopies]
 
     // Everything the block needs from HBM besides codes and gradients is requested now, so that its
     // latency overlaps the first pass: the second moment and, where the registers allow it (2-byte
     // types), the first chunk of parameters.
     constexpr bool kEarlyParams = sizeof(S) == 2;
     const float lr = t.lr;
-    const float wd_mul = t.wd_mul;
-    const float nesterov_alpha = t.beta2;
     const bool do_update = muon || lr != 0.0f;
     const bool load_p = !muon && do_update;
     float v_in = 1.0f;
     if (!muon && valid) v_in = stepsize != nullptr ? stepsize[b] : load_state(t.v, b, t.v_dtype);
-    Chunk<S> pnext;
-    if (kEarlyParams && load_p && lane < nchunks) pnext.load(p_blk, lane);
+    Ahead<S, V> ahead;
+    if (kEarlyParams && load_p) ahead.start(p_blk, lane, LANES, nchunks);
 
     // ---- pass over codes and gradients (the only read of both)
     float absmax = 0.0f;
     float sumsq = 0.0f;
-    if (GSRC == 2) {
-        constexpr int U = 4;
-        const S* const g_sum = peer_ptr(g_blk, L.grad_mc_delta);
-        for (int c0 = lane; c0 < nchunks; c0 += LANES * U)
-            first_pass_group<S, U, true, true>(g_sum, codes_in, stage_a, stage_b, rep, c0, LANES, nchunks, old_mag, beta1, omb1,
-                                               L.grad_scale, absmax, sumsq);
-    } else if (GSRC == 1) {
+    f32x2 sumsq2 = pair(0.0f, 0.0f);
+    if (GSRC == 1) {
         // The gradient of this block is the average over the ranks' buffers (this GPU's and the
         // peers', read over NVLink), summed in fp32 in rank order and rounded to the gradient dtype,
         // as a reduce-scatter into that dtype would leave it.
-        const int n_src = L.n_grad_srcs;
-        if (n_src == 2) reduce_pass<S, 2, true>(L, g_blk, codes_in, stage_a, stage_b, rep, lane, LANES, nchunks, old_mag, beta1, omb1, absmax, sumsq);
-        else if (n_src < 2) reduce_pass<S, 2>(L, g_blk, codes_in, stage_a, stage_b, rep, lane, LANES, nchunks, old_mag, beta1, omb1, absmax, sumsq);
-        else if (n_src == 4) reduce_pass<S, 4, true>(L, g_blk, codes_in, stage_a, stage_b, rep, lane, LANES, nchunks, old_mag, beta1, omb1, absmax, sumsq);
-        else if (n_src < 4) reduce_pass<S, 4>(L, g_blk, codes_in, stage_a, stage_b, rep, lane, LANES, nchunks, old_mag, beta1, omb1, absmax, sumsq);
-        else reduce_pass<S, 8>(L, g_blk, codes_in, stage_a, stage_b, rep, lane, LANES, nchunks, old_mag, beta1, omb1, absmax, sumsq);
+        if constexpr (GSRC == 1) {
+            const int n_src = L.n_grad_srcs;
+#define GEFEN_REDUCE_PASS(...) reduce_pass<S, __VA_ARGS__>(L, g_blk, codes, stage, half, tables, lane, LANES, nchunks, old_mag, beta1, omb1, absmax, sumsq)
+            if (n_src == 2) GEFEN_REDUCE_PASS(2, true);
+            else if (n_src < 2) GEFEN_REDUCE_PASS(2);
+            else if (n_src == 4) GEFEN_REDUCE_PASS(4, true);
+            else if (n_src < 4) GEFEN_REDUCE_PASS(4);
+            else GEFEN_REDUCE_PASS(8);
+#undef GEFEN_REDUCE_PASS
+        }
     } else {
-        // up to four chunks in flight per lane (blocks of up to 256 elements have one chunk per lane). With the
-        // kernels of the two block kinds compiled apart, four fit the registers of both (measured on blocks of
-        // 512 / 1024 bf16 elements: 0.549 -> 0.599 / 0.566 -> 0.620 of the copy bandwidth against one in flight)
-        constexpr int U = (sizeof(S) == 4 && !FULL) ? 2 : 4;   // (fp32 blocks that share a warp: see vec_max_threads)
-        // (a separate loop without bounds tests for the complete groups was measured: slower, it
-        // costs registers)
-        for (int c0 = lane; c0 < nchunks; c0 += LANES * U)
-            first_pass_group<S, U, true, false>(g_blk, codes_in, stage_a, stage_b, rep, c0, LANES, nchunks, old_mag, beta1, omb1,
-                                                1.0f, absmax, sumsq);
+        // Up to four chunks in flight per lane; complete groups of four in every lane without bounds tests, which
+        // cost four instructions each and sit on the one path that every element takes.
+        constexpr int U = V < 8 ? 8 : 4;
+        constexpr bool SUMMED = GSRC == 2;
+        const S* const g_src = SUMMED ? peer_ptr(g_blk, L.grad_mc_delta) : g_blk;
+        const float scale = SUMMED ? L.grad_scale : 1.0f;
+        const f32x2 mag2 = pair(old_mag, old_mag), beta2_ = pair(beta1, beta1), omb2_ = pair(omb1, omb1);
+        int c0 = 0;
+        if (all_valid && sizeof(S) == 2) {   // (fp32: the second copy of the loop costs registers; measured slower)
+            for (; c0 + LANES * U <= chunks; c0 += LANES * U)
+                first_pass_group<S, V, U, false, SUMMED>(g_src, codes, stage, half, tables, c0 + lane, LANES, nchunks, mag2, beta2_, omb2_,
+                                                         scale, absmax, sumsq2);
+        }
+        for (; c0 < chunks; c0 += LANES * U)
+            first_pass_group<S, V, U, true, SUMMED>(g_src, codes, stage, half, tables, c0 + lane, LANES, nchunks, mag2, beta2_, omb2_,
+                                                    scale, absmax, sumsq2);
+        float even, odd;
+        unpair(sumsq2, even, odd);
+        sumsq = even + odd;
     }
     absmax = group_max_nan(absmax, LANES);
 
@@ -697,7 +969,7 @@ __device__ __forceinline__ void warp_block_step(const gefen_b200_step_tensor_t& 
                 if (lane == 0 && valid) v = store_state(t.v, b, t.v_dtype, nv);
                 v = __shfl_sync(0xffffffffu, v, warp_lane & ~(LANES - 1));
             }
-            step = adam_step_size(v, t.bc1, t.bc2, t.eps);
+            step = t.inv_bc1 / (sqrtf(v / t.bc2) + t.eps);   // adam_step_size
         }
     }
     __syncwarp();  // staged momenta are visible to the whole warp; every lane has read the old magnitude
@@ -708,10 +980,10 @@ __device__ __forceinline__ void warp_block_step(const gefen_b200_step_tensor_t& 
     if (__any_sync(0xffffffffu, !(absmax <= 3.0e38f))) {   // warp-uniform: the reduction below shuffles
         float mx = 0.0f;
         for (int c = lane; c < nchunks; c += LANES) {
-            float m[8];
-            staged_momenta(stage_a, stage_b, c, m);
+            float m[V];
+            stage_load<V>(stage, half, c, m);
 #pragma unroll
-            for (int i = 0; i < 8; ++i) mx = fmaxf(mx, fabsf(m[i]));
+            for (int i = 0; i < V; ++i) mx = fmaxf(mx, fabsf(m[i]));
         }
         absmax = group_max(mx, LANES);
         exact_path = true;
@@ -723,104 +995,94 @@ __device__ __forceinline__ void warp_block_step(const gefen_b200_step_tensor_t& 
     const float rinv = fastdiv ? 1.0f / absmax : 0.0f;
     const bool wd = (flags & GEFEN_B200_STEP_WEIGHT_DECAY) != 0;
     const bool nesterov = (flags & GEFEN_B200_STEP_NESTEROV) != 0;
+    const float wd_mul = t.wd_mul;
+    const BlockScalars bs = {pair(-absmax, -absmax), pair(rinv, rinv), pair(step, step), pair(lr, lr), pair(wd_mul, wd_mul)};
 
     // ---- re-encode and update; the parameters of the next chunk are fetched while this one is encoded
-    if (!kEarlyParams && load_p && lane < nchunks) pnext.load(p_blk, lane);
+    if (!kEarlyParams && load_p) ahead.start(p_blk, lane, LANES, nchunks);
     // The common case takes the loop that was compiled for it (the conditions are uniform over the warp: they
     // come from the launch and the tensor's descriptor, and a warp's blocks go one way together).
     if (__all_sync(0xffffffffu, fastdiv || !valid) && !muon && do_update) {
-        const int store = param_mc != 0 ? 2 : (n_peers > 0 ? 1 : 0);
-#define GEFEN_SECOND_PASS(WD_, STORE_)                                                                                      \
-    second_pass_common<S, WD_, STORE_>(L, s, rep, stage_a, stage_b, codes_out, p_blk, pnext, lane, LANES, nchunks, absmax, \
-                                       rinv, step, lr, wd_mul)
-        if (store == 0) { if (wd) GEFEN_SECOND_PASS(true, 0); else GEFEN_SECOND_PASS(false, 0); }
-        else if (store == 1) { if (wd) GEFEN_SECOND_PASS(true, 1); else GEFEN_SECOND_PASS(false, 1); }
-        else { if (wd) GEFEN_SECOND_PASS(true, 2); else GEFEN_SECOND_PASS(false, 2); }
+        const int rounds_all = (chunks + LANES - 1) >> shift, full = all_valid ? chunks >> shift : 0;
+#define GEFEN_SECOND_PASS(WD_, STORE_, ONE_)                                                                                       \
+    second_pass_common<S, V, WD_, STORE_, ONE_>(L, tables, stage, half, codes, p_blk, ahead, lane, LANES, nchunks, full,        \
+                                                rounds_all, bs)
+        if constexpr (V == 8) {
+            const int store = param_mc != 0 ? 2 : (n_peers > 0 ? 1 : 0);
+            if (store == 0) {
+                if (tables.rounds == 1) { if (wd) GEFEN_SECOND_PASS(true, 0, true); else GEFEN_SECOND_PASS(false, 0, true); }
+                else { if (wd) GEFEN_SECOND_PASS(true, 0, false); else GEFEN_SECOND_PASS(false, 0, false); }
+            } else if (store == 1) { if (wd) GEFEN_SECOND_PASS(true, 1, false); else GEFEN_SECOND_PASS(false, 1, false); }
+            else { if (wd) GEFEN_SECOND_PASS(true, 2, false); else GEFEN_SECOND_PASS(false, 2, false); }
+        } else {
+            if (wd) GEFEN_SECOND_PASS(true, 0, false); else GEFEN_SECOND_PASS(false, 0, false);
+        }
 #undef GEFEN_SECOND_PASS
         __syncwarp();  // the staging slice is free for this warp's next block
         return;
     }
     if (GSRC == 0 && muon && __all_sync(0xffffffffu, fastdiv || !valid)) {
-        if (nesterov) second_pass_muon<S, true>(s, rep, stage_a, stage_b, codes_out, g_blk, p_blk, lane, LANES, nchunks, absmax,
-                                                rinv, beta1, nesterov_alpha);
-        else second_pass_muon<S, false>(s, rep, stage_a, stage_b, codes_out, g_blk, p_blk, lane, LANES, nchunks, absmax, rinv,
-                                        beta1, nesterov_alpha);
+        if (nesterov) second_pass_muon<S, V, true>(tables, stage, half, codes, g_blk, p_blk, lane, LANES, nchunks, absmax,
+                                                   bs.neg_absmax2, bs.rinv2, beta1, t.beta2);
+        else second_pass_muon<S, V, false>(tables, stage, half, codes, g_blk, p_blk, lane, LANES, nchunks, absmax, bs.neg_absmax2,
+                                           bs.rinv2, beta1, t.beta2);
         __syncwarp();  // the staging slice is free for this warp's next block
         return;
     }
     // Everything else (lr == 0, blocks that are all zero or hold NaN or Inf, magnitudes outside the range of the
     // reciprocal, GefenMuon's momentum over averaged gradients): the general loop.
     for (int c = lane; c < nchunks; c += LANES) {
-        Chunk<S> praw = pnext;
-        if (load_p && c + LANES < nchunks) pnext.load(p_blk, c + LANES);
-        float m[8];
-        staged_momenta(stage_a, stage_b, c, m);
-        uint32_t code[8];
-        float q[8];
+        Chunk<S, V> praw;
+        if (load_p) praw.load(p_blk, c);
+        float m[V];
+        stage_load<V>(stage, half, c, m);
+        uint32_t row[V];
+        float q[V];
         if (fastdiv) {
-            uint32_t any = 0u;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float x = div_by_block_constant(m[i], absmax, rinv);
-                code[i] = lut_query_fast(x, s.lut);
-                any |= code[i];
-            }
-            if (any & kLutSlowBit) {   // rare: a cell with two thresholds, or values above the last entry
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    if (code[i] & kLutSlowBit) {
-                        const float x = div_by_block_constant(m[i], absmax, rinv);
-                        code[i] = static_cast<uint32_t>(entry_exact(x, s.thr, s.cb, s.k));
-                    }
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < 8; ++i) q[i] = rep[code[i] * kRepCopies] * absmax;
+            encode<V, false>(m, bs.neg_absmax2, bs.rinv2, tables, row);
         } else {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
+            for (int i = 0; i < V; ++i) {
                 float x = 0.0f;
                 if (nonzero) x = m[i] / absmax;
-                code[i] = static_cast<uint32_t>(entry_exact(x, s.thr, s.cb, s.k));
-                q[i] = s.cb[code[i]] * absmax;
+                row[i] = tables.exact_row(x);
             }
         }
-        uint2 cw;
-        cw.x = __byte_perm(__byte_perm(code[0], code[1], 0x0040), __byte_perm(code[2], code[3], 0x0040), 0x5410);
-        cw.y = __byte_perm(__byte_perm(code[4], code[5], 0x0040), __byte_perm(code[6], code[7], 0x0040), 0x5410);
-        codes_out[c] = cw;
+#pragma unroll
+        for (int i = 0; i < V; ++i) q[i] = tables.value(row[i]) * absmax;
+        row_codes<V>(row).store(codes, c);
         if (muon) {
             if (nesterov) {
                 // torch: m.mul_(momentum).add_(g, alpha=1-momentum) on the rounded momentum
                 // (reference: gefen_muon.py:312-314); alpha travels in t.beta2.
-                Chunk<S> g2;
+                Chunk<S, V> g2;
                 g2.load(g_blk, c);
-                float g[8];
+                float g[V];
                 g2.unpack(g);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
+                for (int i = 0; i < V; ++i) {
                     const float m1 = ScalarIO<S>::round(ScalarIO<S>::round(q[i]) * beta1);
-                    q[i] = fmaf(nesterov_alpha, g[i], m1);
+                    q[i] = fmaf(t.beta2, g[i], m1);
                 }
             }
-            Chunk<S> out;
+            Chunk<S, V> out;
             out.pack(q);
             out.store(p_blk, c);
         } else if (do_update) {
-            float pv[8];
+            float pv[V];
             praw.unpack(pv);
             if (wd) {
 #pragma unroll
-                for (int i = 0; i < 8; ++i) pv[i] *= wd_mul;
-                Chunk<S> rounded;       // the separate multiply of the reference rounds to the parameter dtype
+                for (int i = 0; i < V; ++i) pv[i] *= wd_mul;
+                Chunk<S, V> rounded;       // the separate multiply of the reference rounds to the parameter dtype
                 rounded.pack(pv);
                 rounded.unpack(pv);
             }
 #pragma unroll
-            for (int i = 0; i < 8; ++i) pv[i] = fmaf(-(q[i] * step), lr, pv[i]);
+            for (int i = 0; i < V; ++i) pv[i] = fmaf(-(q[i] * step), lr, pv[i]);
             praw.pack(pv);
-            if (param_mc != 0) {
-                praw.store_all(peer_ptr(p_blk, param_mc), c);   // every rank's copy, this one included
+            if (V == 8 && param_mc != 0) {
+                if constexpr (V == 8) praw.store_all(peer_ptr(p_blk, param_mc), c);   // every rank's copy, this one included
             } else {
                 praw.store(p_blk, c);
                 for (int r = 0; r < n_peers; ++r) praw.store(peer_ptr(p_blk, L.peer_delta[r]), c);
@@ -830,63 +1092,56 @@ __device__ __forceinline__ void warp_block_step(const gefen_b200_step_tensor_t& 
     __syncwarp();  // the staging slice is free for this warp's next block
 }
 
-// Warps per CTA of the staged kernel: twenty for 2-byte types (96 registers per thread), sixteen for
-// fp32, whose wider chunks need the full 128.
-// The variant that averages gradients over NVLink holds more loads in flight per thread and is not
-// bound by occupancy: sixteen warps of 128 registers for every type.
-// fp32 tensors whose blocks share a warp are bound by the latency of their loads: there twenty warps of 96
-// registers with two chunks in flight beat sixteen of 128 with four (measured on 768-element blocks: 0.725
-// against 0.703 of the copy bandwidth).
-template <typename S, int GSRC, bool FULL> __host__ __device__ constexpr int vec_max_threads() {
-    if (sizeof(S) == 4 && GSRC == 0 && !FULL) return 640;
-    return (sizeof(S) == 2 && GSRC != 1) ? 640 : 512;
-}
+// Threads per CTA: sixteen warps of 128 registers; the tables leave room for sixteen staging slices of 2048 elements.
+constexpr int kVecThreads = 512;
 
-// GSRC: see warp_block_step. FULL: every tensor of the launch has whole-warp blocks (lanes_per_block == 32);
-// otherwise none has. The two kinds are separate kernels so that each is compiled (registers, code size) for
+// GSRC: see warp_block_step. FULL: every tensor of the launch has whole-warp blocks (32 lanes per block);
+// otherwise none has. The kinds are separate kernels so that each is compiled (registers, code size) for
 // its own loop structure.
-template <typename S, int GSRC, bool FULL>
-__global__ void __launch_bounds__(vec_max_threads<S, GSRC, FULL>(), 1) step_vec_kernel(const __grid_constant__ StepLaunch L,
-                                                           const __grid_constant__ gefen_b200_step_tensor_t single) {
-    extern __shared__ __align__(128) unsigned char smem[];
+template <typename S, int V, int GSRC, bool FULL>
+__global__ void __launch_bounds__(kVecThreads, 1) step_vec_kernel(const __grid_constant__ StepLaunch L,
+                                                                  const __grid_constant__ gefen_b200_step_tensor_t single) {
     SmemView s;
-    if (!stage_tables(L.ws, smem, s, L.spin_limit)) return;
+    if (smem_u32(g_smem) > kFixed) {   // (static variables have outgrown their share: nothing is done, the status says so)
+        if (threadIdx.x == 0) atomicOr(&g_step_status, 2);
+        return;
+    }
+    if (!stage_tables(L.ws, fast_smem(kWsAt), s, L.spin_limit)) return;
     const gefen_b200_step_tensor_t* table = L.table != nullptr ? L.table : &single;
 
     const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
     const int warps = blockDim.x >> 5;
-    {
-        float* rep = reinterpret_cast<float*>(smem + kSmemWs);
-        for (int i = threadIdx.x; i < kMaxCodebook * kRepCopies; i += blockDim.x) rep[i] = s.cb[i / kRepCopies];
-        s.rep = rep + (lane & (kRepCopies - 1));
-        __syncthreads();
-    }
-    float* stage = reinterpret_cast<float*>(smem + kSmemWs + kSmemRep) + static_cast<size_t>(warp) * L.stage_floats;
+    const LaneTables tables = build_lane_tables(s, fast_smem(kStageAt));
+    float* stage = reinterpret_cast<float*>(fast_smem(kStageAt)) + static_cast<size_t>(warp) * L.stage_floats;
     const long long warp_global = static_cast<long long>(blockIdx.x) * warps + warp;
     const long long warp_stride = static_cast<long long>(gridDim.x) * warps;
-    const gefen_b200_step_tensor_t* __restrict__ tp = table;
     // On this path first_block and total_blocks count work units (see vec_units), not blocks.
-    long long t_first = tp->first_block, t_count = vec_units(tp->num_blocks, tp->period);
+    // the warp's slot lies where the codebook was staged (build_lane_tables has consumed it)
+    TensorSlot<S>& t = reinterpret_cast<TensorSlot<S>*>(fast_smem(kWsAt))[warp];
+    static_assert(sizeof(TensorSlot<S>) * (kVecThreads / 32) <= kSmemWs, "a slot per warp");
+    long long t_first = 0, t_units = 0;
     for (long long gb = warp_global; gb < L.total_blocks; gb += warp_stride) {
-        if (gb < t_first || gb >= t_first + t_count) {
-            tp = table + find_tensor(table, L.n_tensors, gb);
-            t_first = tp->first_block;
-            t_count = vec_units(tp->num_blocks, tp->period);
+        if (gb < t_first || gb >= t_first + t_units) {
+            const gefen_b200_step_tensor_t* found = table + find_tensor(table, L.n_tensors, gb);
+            if (lane == 0) t.load(found, V);
+            __syncwarp();
+            t_first = t.first;
+            t_units = t.units;
         }
-        const gefen_b200_step_tensor_t& t = *tp;
-        const long long nb_local = gb - t_first;
-        const long long next = nb_local + warp_stride;
+        const long long unit = gb - t_first;
+        const long long next = unit + warp_stride;
         // same tensor: hint the next block of this warp (measured: pays for 2-byte dtypes with long blocks only)
-        const long long unit_elems = unit_elements(t.period);
-        if (GSRC == 0 && sizeof(S) == 2 && unit_elems >= 1024 && next + 1 < t_count) {   // (not a ragged last unit)
-            const long long elem0 = next * unit_elems;
-            prefetch_l2_range(t.codes + elem0, unit_elems, lane);
-            prefetch_l2_range(static_cast<const char*>(t.g) + elem0 * sizeof(S), unit_elems * sizeof(S), lane);
-            if (!(t.flags & GEFEN_B200_STEP_MUON))
-                prefetch_l2_range(static_cast<const char*>(t.p) + elem0 * sizeof(S), unit_elems * sizeof(S), lane);
+        if (GSRC == 0 && lane == 0 && next + 1 < t_units) {   // (not a ragged last unit)
+            const long long unit_elems = unit_elements(t.period, V, sizeof(S));
+            if (unit_elems >= 1024 || V < 8) {
+                const long long elem0 = next * unit_elems;
+                prefetch_l2_range(t.codes + elem0, unit_elems);
+                prefetch_l2_range(t.g + elem0, unit_elems * sizeof(S));
+                if (!(t.flags & GEFEN_B200_STEP_MUON) && unit_elems * static_cast<int>(sizeof(S)) < 8192) prefetch_l2_range(t.p + elem0, unit_elems * sizeof(S));
+            }
         }
-        warp_block_step<S, GSRC, FULL>(t, nb_local, L, s, stage, lane);
+        warp_block_step<S, V, GSRC, FULL>(t, unit, L, tables, stage, lane);
     }
 }
 
@@ -908,11 +1163,10 @@ constexpr int kWarps = kThreads / 32;
 template <typename S, int GROUP>
 __global__ void __launch_bounds__(kThreads) step_generic_kernel(const __grid_constant__ StepLaunch L,
                                                                 const __grid_constant__ gefen_b200_step_tensor_t single) {
-    extern __shared__ __align__(128) unsigned char smem[];
     __shared__ float red_max[kWarps];
     __shared__ float red_sum[kWarps];
     SmemView s;
-    if (!stage_tables(L.ws, smem, s, L.spin_limit)) return;
+    if (!stage_tables(L.ws, g_smem, s, L.spin_limit)) return;
     const gefen_b200_step_tensor_t* table = L.table != nullptr ? L.table : &single;
 
     const int lane = threadIdx.x & 31;
@@ -1111,7 +1365,7 @@ __global__ void __launch_bounds__(kThreads) multicast_sum_kernel(void* __restric
                                                                  long long chunks, float scale) {
     const long long stride = static_cast<long long>(gridDim.x) * kThreads;
     for (long long c = static_cast<long long>(blockIdx.x) * kThreads + threadIdx.x; c < chunks; c += stride) {
-        Chunk<S> v;
+        Chunk<S, 8> v;
         v.load_sum(src_mc, c);
         float f[8];
         v.unpack(f);
@@ -1135,7 +1389,7 @@ __global__ void __launch_bounds__(kThreads) muon_apply_kernel(S* __restrict__ p,
     const long long tid = static_cast<long long>(blockIdx.x) * kThreads + threadIdx.x;
     const long long chunks = vec ? numel >> 3 : 0;
     for (long long c = tid; c < chunks; c += stride) {
-        Chunk<S> pr, ur;
+        Chunk<S, 8> pr, ur;
         pr.load(p, c);
         ur.load(u, c);
         float pv[8], uv[8];
@@ -1201,11 +1455,10 @@ static int warps_override() {
 constexpr unsigned int kDefaultStageSpinLimit = 4000000u;
 static unsigned int g_stage_spin_limit = kDefaultStageSpinLimit;
 
-template <typename S, int GSRC, bool FULL>
-static int launch_vec_variant(StepLaunch L, const gefen_b200_step_tensor_t& single, long long max_period,
-                              cudaStream_t stream) {
+template <typename S, int V, int GSRC, bool FULL>
+static int launch_vec_variant(StepLaunch L, const gefen_b200_step_tensor_t& single, long long max_unit, cudaStream_t stream) {
     static bool configured[kMaxDevices];
-    auto kernel = step_vec_kernel<S, GSRC, FULL>;
+    auto kernel = step_vec_kernel<S, V, GSRC, FULL>;
     {
         int dev = 0;
         const int rc = current_device(&dev);
@@ -1217,15 +1470,15 @@ static int launch_vec_variant(StepLaunch L, const gefen_b200_step_tensor_t& sing
         }
     }
     // a warp stages one unit: one long block, or the 32 / lanes shorter blocks that share the warp
-    // (max_period: the largest unit of the launch, see unit_elements)
-    const long long stage_bytes = (max_period > 256 ? max_period : 256) * 4;
-    int max_warps = vec_max_threads<S, GSRC, FULL>() / 32;
+    // (max_unit: the largest need of the launch, see unit_floats; a slice starts on 16 bytes)
+    const long long stage_bytes = ((max_unit > 256 ? max_unit : 256) * 4 + 15) / 16 * 16;
+    int max_warps = kVecThreads / 32;
     if (warps_override() > 0 && warps_override() < max_warps) max_warps = warps_override();
-    int warps = static_cast<int>((kMaxSmem - kStaticSmemSlack - kSmemWs - kSmemRep) / stage_bytes);
+    int warps = static_cast<int>((kMaxSmem - kStaticSmemSlack - kSmemTables) / stage_bytes);
     if (warps > max_warps) warps = max_warps;
-    if (warps < 1) return fail(GEFEN_B200_EINVAL, "internal: period %lld too large for the staged path", max_period);
+    if (warps < 1) return fail(GEFEN_B200_EINVAL, "internal: unit of %lld elements too large for the staged path", max_unit);
     if (L.total_blocks < warps) warps = static_cast<int>(L.total_blocks);
-    const int smem = kSmemWs + kSmemRep + static_cast<int>(stage_bytes) * warps;
+    const int smem = kSmemTables + static_cast<int>(stage_bytes) * warps;
     int ctas_per_sm = (kMaxSmem + kCtaReservedSmem) / (smem + kStaticSmemSlack + kCtaReservedSmem);
     if (ctas_per_sm > 2) ctas_per_sm = 2;
     if (ctas_per_sm < 1) ctas_per_sm = 1;
@@ -1236,11 +1489,19 @@ static int launch_vec_variant(StepLaunch L, const gefen_b200_step_tensor_t& sing
     return GEFEN_B200_OK;
 }
 
-template <typename S, bool FULL>
-static int launch_vec(StepLaunch L, const gefen_b200_step_tensor_t& single, long long max_period, cudaStream_t stream) {
-    if (L.grad_mc_delta != 0) return launch_vec_variant<S, 2, FULL>(L, single, max_period, stream);
-    if (L.n_grad_srcs > 0) return launch_vec_variant<S, 1, FULL>(L, single, max_period, stream);
-    return launch_vec_variant<S, 0, FULL>(L, single, max_period, stream);
+template <typename S>
+static int launch_vec(int cls, StepLaunch L, const gefen_b200_step_tensor_t& single, long long max_unit, cudaStream_t stream) {
+    if (cls == 3) return launch_vec_variant<S, 4, 0, false>(L, single, max_unit, stream);
+    if (cls == 4) return launch_vec_variant<S, 2, 0, false>(L, single, max_unit, stream);
+    if (cls == 5) return launch_vec_variant<S, 1, 0, false>(L, single, max_unit, stream);
+    if (cls == 1) {
+        if (L.grad_mc_delta != 0) return launch_vec_variant<S, 8, 2, true>(L, single, max_unit, stream);
+        if (L.n_grad_srcs > 0) return launch_vec_variant<S, 8, 1, true>(L, single, max_unit, stream);
+        return launch_vec_variant<S, 8, 0, true>(L, single, max_unit, stream);
+    }
+    if (L.grad_mc_delta != 0) return launch_vec_variant<S, 8, 2, false>(L, single, max_unit, stream);
+    if (L.n_grad_srcs > 0) return launch_vec_variant<S, 8, 1, false>(L, single, max_unit, stream);
+    return launch_vec_variant<S, 8, 0, false>(L, single, max_unit, stream);
 }
 
 template <typename S>
@@ -1270,37 +1531,37 @@ static int launch_generic(bool cta_per_block, const StepLaunch& L, const gefen_b
     return GEFEN_B200_OK;
 }
 
-// Class of a tensor: 1 = vectorised staged path with whole-warp blocks, 2 = the same path with several blocks
-// per warp pass (blocks of up to 1024 elements), 0 = generic warp per block, -1 = generic CTA per block.
+// Class of a tensor: 1 = staged path in chunks of eight with whole-warp blocks, 2 = the same with several blocks
+// per warp pass (blocks of up to 1024 elements), 3 / 4 / 5 = staged path in chunks of four, two, one (the most that
+// divides the block length and the alignment of all pointers), 0 = generic warp per block, -1 = generic CTA per block.
+static int generic_class(const gefen_b200_step_tensor_t& t) { return t.period > 2048 ? -1 : 0; }
+static int class_chunk(int cls) { return cls <= 2 ? 8 : (cls == 3 ? 4 : (cls == 4 ? 2 : 1)); }
 static int tensor_class(const gefen_b200_step_tensor_t& t, int dtype) {
     const bool vec_dtype = dtype == GEFEN_B200_F32 || dtype == GEFEN_B200_BF16 || dtype == GEFEN_B200_F16;
-    const bool period1 = (t.flags & GEFEN_B200_STEP_PERIOD1) != 0;
-    const bool packed = (t.flags & GEFEN_B200_STEP_PACKED) != 0;
-    if (vec_dtype && !period1 && !packed && t.period % 8 == 0 && t.period <= kFastMaxPeriod && aligned16(t.g) && aligned16(t.p) &&
-        (reinterpret_cast<uintptr_t>(t.codes) & 7u) == 0) {
-        return lanes_per_block(t.period) == 32 ? 1 : 2;
+    if (!vec_dtype || (t.flags & (GEFEN_B200_STEP_PERIOD1 | GEFEN_B200_STEP_PACKED)) != 0 || t.period > kFastMaxPeriod) return generic_class(t);
+    const uintptr_t ptrs = reinterpret_cast<uintptr_t>(t.g) | reinterpret_cast<uintptr_t>(t.p);
+    for (int cls = 2; cls <= 5; ++cls) {
+        const int v = class_chunk(cls);
+        const uintptr_t bytes = static_cast<uintptr_t>(v * dtype_size(dtype) < 16 ? v * dtype_size(dtype) : 16);
+        if (t.period % v != 0 || ptrs % bytes != 0 || reinterpret_cast<uintptr_t>(t.codes) % v != 0) continue;
+        return cls == 2 && lanes_shift(t.period / 8, 8, dtype_size(dtype)) == 5 ? 1 : cls;
     }
-    return t.period > 2048 ? -1 : 0;
+    return generic_class(t);   // (a pointer that is not aligned to its own type)
 }
 // Units of a tensor in its launch's index space: passes of a warp on the staged path, blocks elsewhere.
 // (4-bit codes with an odd period: a pair of blocks is one unit, see step_generic_kernel)
-static long long class_units(const gefen_b200_step_tensor_t& t, int cls) {
-    if (cls >= 1) return vec_units(t.num_blocks, t.period);
+static long long class_units(const gefen_b200_step_tensor_t& t, int cls, int dtype) {
+    if (cls >= 1) return vec_units(t.num_blocks, t.period, class_chunk(cls), dtype_size(dtype));
     const bool paired = (t.flags & GEFEN_B200_STEP_PACKED) != 0 && (t.period & 1) != 0;
     return paired ? (t.num_blocks + 1) / 2 : t.num_blocks;
 }
 
 static int launch_class(int cls, int dtype, const StepLaunch& L, const gefen_b200_step_tensor_t& single,
-                        long long max_period, cudaStream_t stream) {
-    if (cls == 1) {
-        if (dtype == GEFEN_B200_BF16) return launch_vec<__nv_bfloat16, true>(L, single, max_period, stream);
-        if (dtype == GEFEN_B200_F16) return launch_vec<__half, true>(L, single, max_period, stream);
-        return launch_vec<float, true>(L, single, max_period, stream);
-    }
-    if (cls == 2) {
-        if (dtype == GEFEN_B200_BF16) return launch_vec<__nv_bfloat16, false>(L, single, max_period, stream);
-        if (dtype == GEFEN_B200_F16) return launch_vec<__half, false>(L, single, max_period, stream);
-        return launch_vec<float, false>(L, single, max_period, stream);
+                        long long max_unit, cudaStream_t stream) {
+    if (cls >= 1) {
+        if (dtype == GEFEN_B200_BF16) return launch_vec<__nv_bfloat16>(cls, L, single, max_unit, stream);
+        if (dtype == GEFEN_B200_F16) return launch_vec<__half>(cls, L, single, max_unit, stream);
+        return launch_vec<float>(cls, L, single, max_unit, stream);
     }
     const bool cta = cls < 0;
     switch (dtype) {
@@ -1336,7 +1597,7 @@ static int run_single(gefen_b200_step_tensor_t& t, int param_dtype, const float*
     L.n_tensors = 1;
     L.stage_floats = 0;
     const int cls = tensor_class(t, param_dtype);
-    L.total_blocks = class_units(t, cls);
+    L.total_blocks = class_units(t, cls, param_dtype);
     L.ws = static_cast<const unsigned char*>(ws);
     L.stepsize = stepsize;
     L.n_peers = 0;
@@ -1345,7 +1606,7 @@ static int run_single(gefen_b200_step_tensor_t& t, int param_dtype, const float*
     L.grad_mc_delta = 0;
     L.param_mc_delta = 0;
     L.spin_limit = g_stage_spin_limit;
-    return launch_class(cls, param_dtype, L, t, cls >= 1 ? unit_elements(t.period) : t.period, stream);
+    return launch_class(cls, param_dtype, L, t, cls >= 1 ? unit_floats(t.period, class_chunk(cls), dtype_size(param_dtype)) : t.period, stream);
 }
 
 }  // namespace gefen
@@ -1531,6 +1792,12 @@ int gefen_b200_step_tensor_size(void) { return static_cast<int>(sizeof(gefen_b20
 
 int gefen_b200_step_tensor_class(const gefen_b200_step_tensor_t* host_entry, int param_dtype) {
     if (host_entry == nullptr) return -2;
+    const int cls = tensor_class(*host_entry, param_dtype);
+    return cls >= 3 ? generic_class(*host_entry) : cls;
+}
+
+int gefen_b200_step_launch_class(const gefen_b200_step_tensor_t* host_entry, int param_dtype) {
+    if (host_entry == nullptr) return -2;
     return tensor_class(*host_entry, param_dtype);
 }
 
@@ -1660,14 +1927,17 @@ int gefen_b200_multi_tensor_step_multicast(gefen_b200_step_tensor_t* host_table,
                         "Tensor %d: 4-bit codes are not defined for period-1 tensors.", i);
         GEFEN_CHECK_ARG(n_grad_srcs == 0 || !(t.flags & GEFEN_B200_STEP_MUON),
                         "Tensor %d: the momentum-only step does not average gradients over ranks.", i);
-        t.reserved_[0] = tensor_class(t, param_dtype);
+        int cls = tensor_class(t, param_dtype);
+        // chunks below eight serve this GPU's buffers only; with peers the generic kernels do (same order of rows)
+        if (cls >= 3 && (n_peers > 0 || n_grad_srcs > 0)) cls = generic_class(t);
+        t.reserved_[0] = cls;
     }
     for (int begin = 0; begin < n_tensors;) {
         int end = begin;
         long long first = 0;
         while (end < n_tensors && host_table[end].reserved_[0] == host_table[begin].reserved_[0]) {
             host_table[end].first_block = first;   // in work units on the staged path, in blocks elsewhere
-            first += class_units(host_table[end], host_table[end].reserved_[0]);
+            first += class_units(host_table[end], host_table[end].reserved_[0], param_dtype);
             ++end;
         }
         host_table[begin].reserved_[1] = end - begin;  // run length, read back below
@@ -1678,10 +1948,11 @@ int gefen_b200_multi_tensor_step_multicast(gefen_b200_step_tensor_t* host_table,
     for (int begin = 0; begin < n_tensors;) {
         const int run = host_table[begin].reserved_[1];
         const gefen_b200_step_tensor_t& last = host_table[begin + run - 1];
-        const long long total = last.first_block + class_units(last, last.reserved_[0]);
+        const long long total = last.first_block + class_units(last, last.reserved_[0], param_dtype);
         long long max_period = 0;   // largest staging need of a warp: the elements of one unit on the staged path
         for (int i = begin; i < begin + run; ++i) {
-            const long long need = host_table[begin].reserved_[0] >= 1 ? unit_elements(host_table[i].period) : host_table[i].period;
+            const int cls = host_table[begin].reserved_[0];
+            const long long need = cls >= 1 ? unit_floats(host_table[i].period, class_chunk(cls), dtype_size(param_dtype)) : host_table[i].period;
             max_period = need > max_period ? need : max_period;
         }
         if (total > 0) {

@@ -482,7 +482,8 @@ class Gefen(torch.optim.Optimizer):
                 rows[r]["p"] = local_p.data_ptr() + b0 * block * local_p.element_size()
                 rows[r]["g"] = grad.data_ptr() + b0 * block * grad.element_size()
             classes = [lib.gefen_b200_step_tensor_class(rows[r:r + 1].ctypes.data, tag) for r in range(len(idxs))]
-            order = sorted(range(len(idxs)), key=lambda r: classes[r])
+            launch = [lib.gefen_b200_step_launch_class(rows[r:r + 1].ctypes.data, tag) for r in range(len(idxs))]
+            order = sorted(range(len(idxs)), key=lambda r: launch[r])
             rows = np.ascontiguousarray(rows[order])
             tables.append({
                 "tag": tag,

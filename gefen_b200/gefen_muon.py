@@ -130,7 +130,7 @@ class GefenMuon(Gefen):
             rows[r]["flags"] = flags
             state["step"] += 1
         tag = _lib.dtype_tag(chunk[0][4].dtype)
-        classes = [lib.gefen_b200_step_tensor_class(rows[r:r + 1].ctypes.data, tag) for r in range(len(chunk))]
+        classes = [lib.gefen_b200_step_launch_class(rows[r:r + 1].ctypes.data, tag) for r in range(len(chunk))]
         order = sorted(range(len(chunk)), key=lambda r: classes[r])
         rows = np.ascontiguousarray(rows[order])
         device = chunk[0][4].device

@@ -191,11 +191,14 @@ int gefen_b200_multicast_sum(void* dst, const void* src_multicast, int dtype, in
                              void* stream);
 /* sizeof(gefen_b200_step_tensor_t) as compiled, for binding-side layout checks. */
 int gefen_b200_step_tensor_size(void);
-/* Kernel class the library would use for one table entry: 1 = vectorised staged path with one block per
+/* Kind of block of one table entry: 1 = staged path in chunks of eight elements with one block per
  * warp pass, 2 = the same path with several blocks (of up to 1024 elements) per warp pass,
- * 0 = generic warp-per-block, -1 = generic CTA-per-block. Rows of equal
- * class that are adjacent in the table share one launch. */
+ * 0 = any other block of up to 2048 elements, -1 = any other longer block. */
 int gefen_b200_step_tensor_class(const gefen_b200_step_tensor_t* host_entry, int param_dtype);
+/* The launch a table entry goes to: 1 and 2 as above, 3 / 4 / 5 = staged path in chunks of four, two, one
+ * element (blocks and pointers that are multiples of no more than that), 0 / -1 = generic kernels. Rows
+ * of equal launch class that are adjacent in the table share one launch. */
+int gefen_b200_step_launch_class(const gefen_b200_step_tensor_t* host_entry, int param_dtype);
 
 /* Error status of the step kernels on the CURRENT device. Every wait inside them is bounded; a CTA
  * whose wait for its staged tables runs out leaves without doing its share of the step and raises
