@@ -39,6 +39,14 @@ STEP_TENSOR_DTYPE = np.dtype(
     ]
 )
 
+# numpy mirror of gefen_b200_ns_matrix_t
+NS_MATRIX_DTYPE = np.dtype(
+    [
+        ("src", "<u8"), ("p", "<u8"), ("x0", "<u8"), ("x1", "<u8"), ("gram", "<u8"), ("poly", "<u8"),
+        ("rows", "<i8"), ("cols", "<i8"), ("wd_mul", "<f4"), ("alpha", "<f4"), ("decay", "<i4"), ("reserved", "<i4"),
+    ]
+)
+
 _lib = None
 
 
@@ -94,6 +102,11 @@ def _declare(lib):
         "gefen_b200_exact_dp": (i32, [vp, vp, vp, i32, i32, i32, vp, vp, vp]),
         "gefen_b200_ns_gemm_tn": (i32, [vp, vp, vp, vp, vp, i32, i32, i32, i64, i64, i64, i64, i64, dbl, dbl, i32, vp, vp]),
         "gefen_b200_newton_schulz": (i32, [vp, vp, vp, vp, i32, i32, i32, dbl, dbl, dbl, vp, vp]),
+        "gefen_b200_ns_matrix_size": (i32, []),
+        "gefen_b200_ns_group_plan_bytes": (i64, [vp, i32]),
+        "gefen_b200_ns_group_plan": (i32, [vp, i32, vp]),
+        "gefen_b200_ns_group": (i32, [vp, i32, vp, vp, vp, i32, i32, dbl, dbl, dbl, dbl, vp, vp]),
+        "gefen_b200_ns_group_apply": (i32, [vp, i32, vp, i32, i32, vp, i32, vp]),
         "gefen_b200_ns_gemm_nn": (i32, [vp, vp, vp, vp, i32, i32, i32, i64, i64, i64, i64, dbl, dbl, vp, vp]),
         "gefen_b200_ns_gemm_tt": (i32, [vp, vp, vp, vp, i32, i32, i32, i64, i64, i64, i64, dbl, dbl, i32, vp, vp]),
     }
@@ -119,6 +132,8 @@ def load():
         EXPORTED_SYMBOLS = sorted(_declare(lib).keys())
         if lib.gefen_b200_step_tensor_size() != STEP_TENSOR_DTYPE.itemsize:
             raise GefenB200Error("step-tensor layout mismatch between the library and its Python mirror")
+        if lib.gefen_b200_ns_matrix_size() != NS_MATRIX_DTYPE.itemsize:
+            raise GefenB200Error("matrix-table layout mismatch between the library and its Python mirror")
         _lib = lib
     return _lib
 

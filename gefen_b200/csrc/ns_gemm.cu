@@ -24,11 +24,15 @@
 
 #include <stdio.h>
 #include <stdlib.h>
+#include <string.h>
 
 #include <cuda.h>
+#include <algorithm>
 #include <map>
 #include <mutex>
+#include <new>
 #include <tuple>
+#include <vector>
 
 namespace gefen {
 
@@ -37,7 +41,23 @@ constexpr int kBK = 64;                 // 64 bf16 = one 128-byte swizzle row
 constexpr int kGemmThreads = 192;
 constexpr uint32_t kSpinLimit = 20000000u;
 
+// One product of a group (see ns_group below): its operands' tensor maps and its matrices.
+struct alignas(64) GroupEntry {
+    CUtensorMap a, b;
+    const __nv_bfloat16* c;
+    __nv_bfloat16* d;
+    int M, N, K;
+    int ldc, ldd;
+    int reserved_[7];
+};
+static_assert(sizeof(GroupEntry) == 320, "tensor maps start on 64 bytes");
+struct GroupTile {
+    int entry, m0, n0, reserved_;
+};
+
 struct GemmArgs {
+    const GroupEntry* entries;   // GROUP only: the products of the launch, and their tiles in the order they are taken
+    const GroupTile* tiles;
     const __nv_bfloat16* c;
     __nv_bfloat16* d;
     __nv_bfloat16* dt;
@@ -149,7 +169,17 @@ __host__ __device__ inline bool tile_coords(int M, int N, int bn, int symmetric,
 // tall matrix, Y^T Y, without transposing Y.
 // Variants whose ring is at most 96 KB run two CTAs per SM: the epilogue of one overlaps the main
 // loop of the other (each holds BN <= 256 of the 512 TMEM columns).
-template <int BN, int STAGES, bool A_MN, bool B_MN, bool PERSIST>
+// GROUP (a persistent variant): the launch computes the products of many matrices; a tile names its product, whose
+// tensor maps and sizes come from global memory (the host has copied them there before the launch).
+struct TileView {
+    const CUtensorMap* map_a;
+    const CUtensorMap* map_b;
+    const __nv_bfloat16* c;
+    __nv_bfloat16* d;
+    int M, N, K, m0, n0;
+    long long ldc, ldd;
+};
+template <int BN, int STAGES, bool A_MN, bool B_MN, bool PERSIST, bool GROUP = false>
 __global__ void __launch_bounds__(kGemmThreads, (STAGES * (kBM + BN) * kBK * 2 <= 96 * 1024) ? 2 : 1) ns_gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a,
                                                                      const __grid_constant__ CUtensorMap map_b,
                                                                      const __grid_constant__ GemmArgs args) {
@@ -168,18 +198,36 @@ __global__ void __launch_bounds__(kGemmThreads, (STAGES * (kBM + BN) * kBK * 2 <
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     constexpr int kTmemCols = PERSIST ? 2 * BN : BN;
-    const int k_blocks = (args.K + kBK - 1) / kBK;
     if (!PERSIST && args.symmetric && static_cast<int>(blockIdx.x) * BN + BN <= static_cast<int>(blockIdx.y) * kBM)
         return;   // tile entirely below the diagonal: its mirror image computes it
     // li-th tile of this CTA
-    auto my_tile = [&](int li, int* m0, int* n0) -> bool {
+    auto my_tile = [&](int li, TileView& t) -> bool {
+        const long long index = static_cast<long long>(blockIdx.x) + static_cast<long long>(li) * gridDim.x;
+        if constexpr (GROUP) {
+            if (index >= args.n_tiles) return false;
+            const GroupTile g = args.tiles[index];
+            const GroupEntry* e = args.entries + g.entry;
+            t.map_a = &e->a;
+            t.map_b = &e->b;
+            t.c = e->c;
+            t.d = e->d;
+            t.M = e->M; t.N = e->N; t.K = e->K;
+            t.ldc = e->ldc; t.ldd = e->ldd;
+            t.m0 = g.m0; t.n0 = g.n0;
+            return true;
+        }
+        t.map_a = &map_a;
+        t.map_b = &map_b;
+        t.c = args.c;
+        t.d = args.d;
+        t.M = args.M; t.N = args.N; t.K = args.K;
+        t.ldc = args.ldc; t.ldd = args.ldd;
         if (!PERSIST) {
-            *m0 = blockIdx.y * kBM;
-            *n0 = blockIdx.x * BN;
+            t.m0 = blockIdx.y * kBM;
+            t.n0 = blockIdx.x * BN;
             return li == 0;
         }
-        const long long t = static_cast<long long>(blockIdx.x) + static_cast<long long>(li) * gridDim.x;
-        return t < args.n_tiles && tile_coords(args.M, args.N, BN, args.symmetric, t, m0, n0);
+        return index < args.n_tiles && tile_coords(args.M, args.N, BN, args.symmetric, index, &t.m0, &t.n0);
     };
 
     if (threadIdx.x == 0) {
@@ -200,12 +248,19 @@ __global__ void __launch_bounds__(kGemmThreads, (STAGES * (kBM + BN) * kBK * 2 <
     if (warp == 4) {
         // ---------------- producer
         if (lane == 0) {
-            asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
-            asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
+            if constexpr (!GROUP) {
+                asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
+                asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
+            }
             uint32_t it = 0;   // k-blocks issued so far, over all tiles: ring slot and phase
             bool ok = true;
-            int m0, n0;
-            for (int li = 0; ok && my_tile(li, &m0, &n0); ++li)
+            TileView t;
+            for (int li = 0; ok && my_tile(li, t); ++li) {
+            const int m0 = t.m0, n0 = t.n0, k_blocks = (t.K + kBK - 1) / kBK;
+            if constexpr (GROUP) {   // maps in global memory: make the host's copy visible to the tensor-map proxy
+                asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(t.map_a) : "memory");
+                asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(t.map_b) : "memory");
+            }
             for (int kb = 0; kb < k_blocks; ++kb, ++it) {
                 const int s = it % STAGES;
                 const uint32_t parity = ((it / STAGES) & 1) ^ 1;
@@ -213,19 +268,24 @@ __global__ void __launch_bounds__(kGemmThreads, (STAGES * (kBM + BN) * kBK * 2 <
                 mbar_expect_tx(&full_bar[s], kStageBytes);
                 unsigned char* a_dst = smem + s * kStageBytes;
                 if (!A_MN) {
-                    tma_load_2d(a_dst, &map_a, kb * kBK, m0, &full_bar[s]);
+                    tma_load_2d(a_dst, t.map_a, kb * kBK, m0, &full_bar[s]);
                 } else {
 #pragma unroll
                     for (int j = 0; j < kBM / 64; ++j)
-                        tma_load_2d(a_dst + j * (kBK * 128), &map_a, m0 + 64 * j, kb * kBK, &full_bar[s]);
+                        tma_load_2d(a_dst + j * (kBK * 128), t.map_a, m0 + 64 * j, kb * kBK, &full_bar[s]);
                 }
-                if (!B_MN) {
-                    tma_load_2d(a_dst + kABytes, &map_b, kb * kBK, n0, &full_bar[s]);
+                if (!B_MN && GROUP) {   // (one map serves both operands: boxes of 128 rows)
+#pragma unroll
+                    for (int j = 0; j < BN / kBM; ++j)
+                        tma_load_2d(a_dst + kABytes + j * kABytes, t.map_b, kb * kBK, n0 + kBM * j, &full_bar[s]);
+                } else if (!B_MN) {
+                    tma_load_2d(a_dst + kABytes, t.map_b, kb * kBK, n0, &full_bar[s]);
                 } else {
 #pragma unroll
                     for (int j = 0; j < BN / 64; ++j)   // 64 K-rows x 64 N-columns per box
-                        tma_load_2d(a_dst + kABytes + j * (kBK * 128), &map_b, n0 + 64 * j, kb * kBK, &full_bar[s]);
+                        tma_load_2d(a_dst + kABytes + j * (kBK * 128), t.map_b, n0 + 64 * j, kb * kBK, &full_bar[s]);
                 }
+            }
             }
         }
         __syncwarp();
@@ -237,8 +297,9 @@ __global__ void __launch_bounds__(kGemmThreads, (STAGES * (kBM + BN) * kBK * 2 <
                                        (static_cast<uint32_t>(BN >> 3) << 17) | (static_cast<uint32_t>(kBM >> 4) << 24);
             bool ok = true;
             uint32_t it = 0;
-            int m0, n0;
-            for (int li = 0; ok && my_tile(li, &m0, &n0); ++li) {
+            TileView t;
+            for (int li = 0; ok && my_tile(li, t); ++li) {
+            const int k_blocks = (t.K + kBK - 1) / kBK;
             const int buf = PERSIST ? (li & 1) : 0;
             const uint32_t tmem_acc = tmem_base + static_cast<uint32_t>(buf * BN);
             if (PERSIST) {   // the epilogue has drained this buffer (passes at once for the first two tiles)
@@ -270,20 +331,21 @@ __global__ void __launch_bounds__(kGemmThreads, (STAGES * (kBM + BN) * kBK * 2 <
         __syncwarp();
     } else {
         // ---------------- epilogue: warp w owns TMEM lanes (rows) 32w .. 32w+31
-        int m0, n0;
-        for (int li = 0; my_tile(li, &m0, &n0); ++li) {
+        TileView t;
+        for (int li = 0; my_tile(li, t); ++li) {
+        const int m0 = t.m0, n0 = t.n0;
         const int buf = PERSIST ? (li & 1) : 0;
         const int row = m0 + warp * 32 + lane;
-        const bool row_ok = row < args.M;
+        const bool row_ok = row < t.M;
         // C does not depend on the accumulators: the first chunk's row segment is fetched while the main
         // loop runs, and chunk j+1's while chunk j is converted and stored.
         const bool use_c = row_ok && args.beta != 0.0f;
-        const __nv_bfloat16* crow_base = use_c ? args.c + static_cast<long long>(row) * args.ldc : nullptr;
-        const bool c_vec = use_c && ((reinterpret_cast<uintptr_t>(crow_base) & 15u) == 0) && (args.ldc % 8 == 0) && (n0 % 8 == 0);
+        const __nv_bfloat16* crow_base = use_c ? t.c + static_cast<long long>(row) * t.ldc : nullptr;
+        const bool c_vec = use_c && ((reinterpret_cast<uintptr_t>(crow_base) & 15u) == 0) && (t.ldc % 8 == 0) && (n0 % 8 == 0);
         uint4 cnext[4];
         auto fetch_c = [&](int j) {
             const int col0 = n0 + j * 32;
-            if (c_vec && col0 + 32 <= args.N) {
+            if (c_vec && col0 + 32 <= t.N) {
 #pragma unroll
                 for (int q = 0; q < 4; ++q) cnext[q] = reinterpret_cast<const uint4*>(crow_base + col0)[q];
             }
@@ -313,8 +375,8 @@ __global__ void __launch_bounds__(kGemmThreads, (STAGES * (kBM + BN) * kBK * 2 <
                 if (j + 1 < BN / 32) fetch_c(j + 1);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 const int col0 = n0 + j * 32;
-                if (col0 >= args.N) continue;
-                const bool full_cols = col0 + 32 <= args.N;
+                if (col0 >= t.N) continue;
+                const bool full_cols = col0 + 32 <= t.N;
                 float v[32];
 #pragma unroll
                 for (int i = 0; i < 32; ++i) v[i] = args.alpha * __uint_as_float(r[i]);
@@ -334,16 +396,16 @@ __global__ void __launch_bounds__(kGemmThreads, (STAGES * (kBM + BN) * kBK * 2 <
                     } else {
 #pragma unroll
                         for (int i = 0; i < 32; ++i)
-                            if (col0 + i < args.N) v[i] = fmaf(args.beta, __bfloat162float(crow[i]), v[i]);
+                            if (col0 + i < t.N) v[i] = fmaf(args.beta, __bfloat162float(crow[i]), v[i]);
                     }
                 }
                 if (row_ok) {
-                    __nv_bfloat16* drow = args.d + static_cast<long long>(row) * args.ldd + col0;
+                    __nv_bfloat16* drow = t.d + static_cast<long long>(row) * t.ldd + col0;
                     if (args.symmetric && col0 < row) {
                         // chunk crosses or lies left of the diagonal: only the elements with column >= row
 #pragma unroll
                         for (int i = 0; i < 32; ++i)
-                            if (col0 + i < args.N && col0 + i >= row) drow[i] = __float2bfloat16_rn(v[i]);
+                            if (col0 + i < t.N && col0 + i >= row) drow[i] = __float2bfloat16_rn(v[i]);
                     } else if (full_cols && ((reinterpret_cast<uintptr_t>(drow) & 15u) == 0)) {
 #pragma unroll
                         for (int q = 0; q < 4; ++q) {
@@ -358,20 +420,20 @@ __global__ void __launch_bounds__(kGemmThreads, (STAGES * (kBM + BN) * kBK * 2 <
                     } else {
 #pragma unroll
                         for (int i = 0; i < 32; ++i)
-                            if (col0 + i < args.N) drow[i] = __float2bfloat16_rn(v[i]);
+                            if (col0 + i < t.N) drow[i] = __float2bfloat16_rn(v[i]);
                     }
                     if (args.dt != nullptr) {
                         // transposed copy: for a fixed column the lanes of a warp write consecutive addresses
 #pragma unroll
                         for (int i = 0; i < 32; ++i)
-                            if (col0 + i < args.N)
+                            if (col0 + i < t.N)
                                 args.dt[static_cast<long long>(col0 + i) * args.lddt + row] = __float2bfloat16_rn(v[i]);
                     }
                 }
                 if (args.symmetric) {
                     // mirror: element (row, c) with c > row also goes to (c, row)
                     const int warp_row0 = m0 + warp * 32;
-                    if (col0 > warp_row0 + 31 && warp_row0 + 31 < args.M && full_cols) {
+                    if (col0 > warp_row0 + 31 && warp_row0 + 31 < t.M && full_cols) {
                         // the whole chunk is right of every row of this warp (warp-uniform): lanes pair up so
                         // that each store carries two consecutive rows of one column (4 bytes)
                         const bool odd = (lane & 1) != 0;
@@ -383,13 +445,13 @@ __global__ void __launch_bounds__(kGemmThreads, (STAGES * (kBM + BN) * kBK * 2 <
                             const float hi = odd ? v[i + 1] : recv;      // value of the odd row
                             const int c = col0 + i + (odd ? 1 : 0);
                             const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
-                            *reinterpret_cast<__nv_bfloat162*>(args.d + static_cast<long long>(c) * args.ldd + (row & ~1)) = h;
+                            *reinterpret_cast<__nv_bfloat162*>(t.d + static_cast<long long>(c) * t.ldd + (row & ~1)) = h;
                         }
                     } else if (row_ok && col0 + 31 > row) {
 #pragma unroll
                         for (int i = 0; i < 32; ++i)
-                            if (col0 + i < args.N && col0 + i > row)
-                                args.d[static_cast<long long>(col0 + i) * args.ldd + row] = __float2bfloat16_rn(v[i]);
+                            if (col0 + i < t.N && col0 + i > row)
+                                t.d[static_cast<long long>(col0 + i) * t.ldd + row] = __float2bfloat16_rn(v[i]);
                     }
                 }
             }
@@ -456,19 +518,19 @@ static int count_tiles(int M, int N, int bn, int symmetric) {
     return total;
 }
 
-template <int BN, int STAGES, bool A_MN, bool B_MN, bool PERSIST>
+template <int BN, int STAGES, bool A_MN, bool B_MN, bool PERSIST, bool GROUP = false>
 static int launch_gemm_variant(const CUtensorMap& ma, const CUtensorMap& mb, GemmArgs args, cudaStream_t stream) {
     constexpr int smem = STAGES * (kBM * kBK * 2 + BN * kBK * 2) + 1024;
     static bool configured[64];
     int dev = 0;
     GEFEN_CHECK_CUDA(cudaGetDevice(&dev));
-    auto kernel = ns_gemm_tn_kernel<BN, STAGES, A_MN, B_MN, PERSIST>;
+    auto kernel = ns_gemm_tn_kernel<BN, STAGES, A_MN, B_MN, PERSIST, GROUP>;
     if (dev < 64 && !configured[dev]) {
         GEFEN_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         configured[dev] = true;
     }
-    args.n_tiles = count_tiles(args.M, args.N, BN, args.symmetric);
-    dim3 grid((args.N + BN - 1) / BN, (args.M + kBM - 1) / kBM);
+    if (!GROUP) args.n_tiles = count_tiles(args.M, args.N, BN, args.symmetric);
+    dim3 grid(GROUP ? 1 : (args.N + BN - 1) / BN, GROUP ? 1 : (args.M + kBM - 1) / kBM);
     if (PERSIST) grid = dim3(args.n_tiles < sm_count() ? args.n_tiles : sm_count(), 1);
     kernel<<<grid, kGemmThreads, smem, stream>>>(ma, mb, args);
     GEFEN_CHECK_CUDA(cudaGetLastError());
@@ -528,7 +590,7 @@ static int ns_gemm(const void* a, bool a_is_km, const void* b, bool b_is_kn, con
     if (rc != GEFEN_B200_OK) return rc;
     rc = b_is_kn ? make_map(&mb, b, K, N, ldb, kBK) : make_map(&mb, b, N, K, ldb, bn);
     if (rc != GEFEN_B200_OK) return rc;
-    GemmArgs args;
+    GemmArgs args = {};
     args.c = static_cast<const __nv_bfloat16*>(c);
     args.d = static_cast<__nv_bfloat16*>(d);
     args.dt = static_cast<__nv_bfloat16*>(dt);
@@ -679,4 +741,395 @@ extern "C" int gefen_b200_ns_gemm_tt(const void* a, const void* b, const void* c
                                      int64_t lda, int64_t ldb, int64_t ldc, int64_t ldd, double alpha, double beta,
                                      int symmetric, int* status, void* stream) {
     return ns_gemm(a, true, b, true, c, d, nullptr, M, N, K, lda, ldb, ldc, ldd, 0, alpha, beta, symmetric, status, stream);
+}
+
+// --------------------------------------------------------------------------- many matrices at once
+// The matrices of an optimizer step go through the iteration together: one launch per product for all of them, so
+// that the tiles of small matrices fill the GPU (one 768 x 768 Gram matrix has 12 tiles of 128 x 256 for 148 SMs) and
+// the last wave is paid once per product instead of once per matrix and product, and so that the host enqueues
+// 3 * steps + 3 launches instead of that many per matrix. Measured, whole GefenMuon steps: 24 matrices of a 768-wide
+// transformer 3.86 -> 1.25 ms, four matrices of 64 to 1026 rows 0.61 -> 0.27 ms, 28 Qwen3-1.7B-shaped matrices
+// 9.5 -> 8.3 ms (there the products themselves, 1060 TFLOP/s, are what is left). Tall matrices enter transposed (Y^T Y = X X^T for X = Y^T), so
+// every product has one of two forms: A * B^T with both operands K-major, or A * B with B MN-major.
+namespace gefen {
+
+// What the element-wise kernels read of a matrix; uploaded with every call (the step's scalars are in it).
+typedef gefen_b200_ns_matrix_t NsMatrix;
+
+constexpr int kNormParts = 64;      // CTAs per matrix of the norm
+constexpr int kElemThreads = 256;
+constexpr int kTile = 64;           // transposing tile
+
+__device__ __forceinline__ bool ns_tall(const NsMatrix& m) { return m.rows > m.cols; }
+__device__ __forceinline__ int ns_wide_rows(const NsMatrix& m) { return (static_cast<int>(m.rows < m.cols ? m.rows : m.cols) + 7) / 8 * 8; }
+__device__ __forceinline__ int ns_wide_cols(const NsMatrix& m) { return (static_cast<int>(m.rows < m.cols ? m.cols : m.rows) + 7) / 8 * 8; }
+
+template <typename S> __device__ __forceinline__ float as_bf16(const S* p) { return __bfloat162float(__float2bfloat16_rn(ScalarIO<S>::load(p))); }
+
+// Partial sums of squares of the matrix rounded to bf16, in a fixed order.
+template <typename S>
+__global__ void __launch_bounds__(kElemThreads) ns_norm_kernel(const NsMatrix* __restrict__ table, float* __restrict__ parts) {
+    __shared__ float red[kElemThreads / 32];
+    const NsMatrix& m = table[blockIdx.y];
+    const long long n = m.rows * m.cols;
+    const S* src = static_cast<const S*>(m.src);
+    constexpr int kVec = 16 / static_cast<int>(sizeof(S));
+    const long long per = ((n + kNormParts - 1) / kNormParts + kVec - 1) / kVec * kVec;   // (src starts on 16 bytes)
+    const long long begin = per * blockIdx.x;
+    const long long end = begin + per < n ? begin + per : n;
+    float acc = 0.0f;
+    long long i = begin + static_cast<long long>(threadIdx.x) * kVec;
+    for (; i + kVec <= end; i += kElemThreads * kVec) {
+        const uint4 raw = *reinterpret_cast<const uint4*>(src + i);
+        const S* v = reinterpret_cast<const S*>(&raw);
+#pragma unroll
+        for (int e = 0; e < kVec; ++e) { const float f = as_bf16(v + e); acc = fmaf(f, f, acc); }
+    }
+    for (; i < end; ++i) { const float f = as_bf16(src + i); acc = fmaf(f, f, acc); }   // (at most one thread)
+    acc = warp_sum(acc);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float t = 0.0f;
+        for (int w = 0; w < kElemThreads / 32; ++w) t += red[w];
+        parts[blockIdx.y * kNormParts + blockIdx.x] = t;
+    }
+}
+
+// x0 <- bf16(src) / max(norm, eps), wide and padded with zeros; norm and quotient rounded to bf16 as torch's
+// x.div_(x.norm().clamp(min=eps)) on a bf16 tensor rounds them (reference: gefen_muon.py:38).
+template <typename S>
+__global__ void __launch_bounds__(kElemThreads) ns_normalise_kernel(const NsMatrix* __restrict__ table, const float* __restrict__ parts, float eps) {
+    __shared__ __nv_bfloat16 tile[kTile][kTile + 2];
+    __shared__ float norm_shared;
+    const NsMatrix& m = table[blockIdx.y];
+    if (threadIdx.x < 32) {
+        float t = parts[blockIdx.y * kNormParts + threadIdx.x] + parts[blockIdx.y * kNormParts + 32 + threadIdx.x];
+        t = warp_sum(t);
+        if (threadIdx.x == 0)
+            norm_shared = fmaxf(__bfloat162float(__float2bfloat16_rn(sqrtf(t))), __bfloat162float(__float2bfloat16_rn(eps)));
+    }
+    __syncthreads();
+    const float norm = norm_shared;
+    const S* src = static_cast<const S*>(m.src);
+    __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(m.x0);
+    const int rows = static_cast<int>(m.rows), cols = static_cast<int>(m.cols);
+    const int wr = ns_wide_rows(m), wc = ns_wide_cols(m);
+    if (!ns_tall(m) && wr == rows && wc == cols) {
+        const long long chunks = m.rows * m.cols / 8;
+        for (long long c = static_cast<long long>(blockIdx.x) * kElemThreads + threadIdx.x; c < chunks; c += static_cast<long long>(gridDim.x) * kElemThreads) {
+            uint32_t w[4];
+            alignas(16) S v[8];
+            if constexpr (sizeof(S) == 2) *reinterpret_cast<uint4*>(v) = reinterpret_cast<const uint4*>(src)[c];
+            else {
+                reinterpret_cast<uint4*>(v)[0] = reinterpret_cast<const uint4*>(src)[2 * c];
+                reinterpret_cast<uint4*>(v)[1] = reinterpret_cast<const uint4*>(src)[2 * c + 1];
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const __nv_bfloat162 h = __floats2bfloat162_rn(as_bf16(v + 2 * e) / norm, as_bf16(v + 2 * e + 1) / norm);
+                w[e] = *reinterpret_cast<const uint32_t*>(&h);
+            }
+            reinterpret_cast<uint4*>(dst)[c] = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+        return;
+    }
+    // any other matrix tile by tile of the wide result, through shared memory where it is transposed
+    const int tiles_c = (wc + kTile - 1) / kTile, tiles = tiles_c * ((wr + kTile - 1) / kTile);
+    const int x = threadIdx.x % kTile, y0 = threadIdx.x / kTile;
+    for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const int r0 = t / tiles_c * kTile, c0 = t % tiles_c * kTile;
+        if (ns_tall(m)) {
+            __syncthreads();
+            for (int y = y0; y < kTile; y += kElemThreads / kTile) {   // source row c0 + y, column r0 + x
+                float f = 0.0f;
+                if (c0 + y < rows && r0 + x < cols) f = as_bf16(src + static_cast<long long>(c0 + y) * cols + r0 + x) / norm;
+                tile[y][x] = __float2bfloat16_rn(f);
+            }
+            __syncthreads();
+            for (int y = y0; y < kTile; y += kElemThreads / kTile)
+                if (r0 + y < wr && c0 + x < wc) dst[static_cast<long long>(r0 + y) * wc + c0 + x] = tile[x][y];
+        } else {
+            for (int y = y0; y < kTile; y += kElemThreads / kTile) {
+                if (r0 + y >= wr || c0 + x >= wc) continue;
+                float f = 0.0f;
+                if (r0 + y < rows && c0 + x < cols) f = as_bf16(src + static_cast<long long>(r0 + y) * cols + c0 + x) / norm;
+                dst[static_cast<long long>(r0 + y) * wc + c0 + x] = __float2bfloat16_rn(f);
+            }
+        }
+    }
+}
+
+struct ApplyPeers {
+    int n;
+    long long delta[GEFEN_B200_MAX_PEERS];
+};
+
+// p <- round(p * wd_mul); p <- round(p + alpha * u), u the (bf16) result of the iteration, which lies wide: what
+// muon_apply_kernel does for one matrix (reference: gefen_muon.py:326-329), peer stores included.
+template <typename S>
+__global__ void __launch_bounds__(kElemThreads) ns_apply_kernel(const NsMatrix* __restrict__ table, int in_x1, const __grid_constant__ ApplyPeers peers) {
+    __shared__ __nv_bfloat16 tile[kTile][kTile + 2];
+    const NsMatrix& m = table[blockIdx.y];
+    const __nv_bfloat16* u = static_cast<const __nv_bfloat16*>(in_x1 ? m.x1 : m.x0);
+    S* p = static_cast<S*>(m.p);
+    const float wd_mul = m.wd_mul, alpha = m.alpha;
+    const bool decay = m.decay != 0;
+    const int rows = static_cast<int>(m.rows), cols = static_cast<int>(m.cols);
+    const int wr = ns_wide_rows(m), wc = ns_wide_cols(m);
+    auto update = [&](float pv, float uv) {
+        if (decay) pv = ScalarIO<S>::round(pv * wd_mul);
+        return fmaf(alpha, uv, pv);
+    };
+    auto put = [&](long long at, float v) {
+        ScalarIO<S>::store(p + at, v);
+        for (int r = 0; r < peers.n; ++r) ScalarIO<S>::store(reinterpret_cast<S*>(reinterpret_cast<uintptr_t>(p + at) + peers.delta[r]), v);
+    };
+    if (!ns_tall(m) && wc == cols && wr == rows && (reinterpret_cast<uintptr_t>(p) & 15u) == 0) {
+        const long long chunks = m.rows * m.cols / 8;
+        for (long long c = static_cast<long long>(blockIdx.x) * kElemThreads + threadIdx.x; c < chunks; c += static_cast<long long>(gridDim.x) * kElemThreads) {
+            const uint4 raw = reinterpret_cast<const uint4*>(u)[c];
+            const __nv_bfloat16* uv = reinterpret_cast<const __nv_bfloat16*>(&raw);
+            constexpr int kWide = static_cast<int>(sizeof(S)) / 2;   // 16-byte pieces of eight parameters
+            alignas(16) S v[8];
+#pragma unroll
+            for (int q = 0; q < kWide; ++q) reinterpret_cast<uint4*>(v)[q] = reinterpret_cast<const uint4*>(p)[kWide * c + q];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) ScalarIO<S>::store(v + e, update(ScalarIO<S>::load(v + e), __bfloat162float(uv[e])));
+#pragma unroll
+            for (int q = 0; q < kWide; ++q) {
+                reinterpret_cast<uint4*>(p)[kWide * c + q] = reinterpret_cast<uint4*>(v)[q];
+                for (int r = 0; r < peers.n; ++r)
+                    reinterpret_cast<uint4*>(reinterpret_cast<uintptr_t>(p) + peers.delta[r])[kWide * c + q] = reinterpret_cast<uint4*>(v)[q];
+            }
+        }
+        return;
+    }
+    const int tiles_c = (cols + kTile - 1) / kTile, tiles = tiles_c * ((rows + kTile - 1) / kTile);   // of the parameter
+    const int x = threadIdx.x % kTile, y0 = threadIdx.x / kTile;
+    for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const int r0 = t / tiles_c * kTile, c0 = t % tiles_c * kTile;
+        if (ns_tall(m)) {
+            __syncthreads();
+            for (int y = y0; y < kTile; y += kElemThreads / kTile)   // u row c0 + y, column r0 + x
+                if (c0 + y < wr && r0 + x < wc) tile[y][x] = u[static_cast<long long>(c0 + y) * wc + r0 + x];
+            __syncthreads();
+            for (int y = y0; y < kTile; y += kElemThreads / kTile) {
+                if (r0 + y >= rows || c0 + x >= cols) continue;
+                const long long at = static_cast<long long>(r0 + y) * cols + c0 + x;
+                put(at, update(ScalarIO<S>::load(p + at), __bfloat162float(tile[x][y])));
+            }
+        } else {
+            for (int y = y0; y < kTile; y += kElemThreads / kTile) {
+                if (r0 + y >= rows || c0 + x >= cols) continue;
+                const long long at = static_cast<long long>(r0 + y) * cols + c0 + x;
+                put(at, update(ScalarIO<S>::load(p + at), __bfloat162float(u[static_cast<long long>(r0 + y) * wc + c0 + x])));
+            }
+        }
+    }
+}
+
+// The plan of a group: five lists of products (Gram matrix of x0 / of x1, polynomial, update x0 -> x1 / x1 -> x0) and
+// two lists of tiles (of the symmetric m x m results, of the m x k results).
+struct GroupShape {
+    int bn;
+    int64_t gram_tiles, update_tiles, entries_bytes, bytes;
+};
+static void wide_dims(const NsMatrix& m, int* wr, int* wc) {
+    const int64_t a = (m.rows + 7) / 8 * 8, b = (m.cols + 7) / 8 * 8;
+    *wr = static_cast<int>(std::min(a, b));
+    *wc = static_cast<int>(std::max(a, b));
+}
+static GroupShape group_shape(const NsMatrix* mats, int n) {
+    GroupShape g;
+    for (g.bn = 256;; g.bn = 128) {
+        g.gram_tiles = g.update_tiles = 0;
+        for (int i = 0; i < n; ++i) {
+            int m, k;
+            wide_dims(mats[i], &m, &k);
+            g.gram_tiles += count_tiles(m, m, g.bn, 1);
+            g.update_tiles += count_tiles(m, k, g.bn, 0);
+        }
+        // tiles of 128 x 256 have the better ratio of operand bytes to work; where they do not fill the SMs, 128 x 128
+        if (g.bn == 128 || g.gram_tiles >= sm_count()) break;
+    }
+    g.entries_bytes = static_cast<int64_t>(5) * n * static_cast<int64_t>(sizeof(GroupEntry));
+    g.bytes = g.entries_bytes + (g.gram_tiles + g.update_tiles) * static_cast<int64_t>(sizeof(GroupTile));
+    return g;
+}
+static int check_group(const NsMatrix* mats, int n) {
+    GEFEN_CHECK_ARG(n >= 1 && n <= 4096 && mats != nullptr, "Expected between 1 and 4096 matrices, got %d.", n);
+    for (int i = 0; i < n; ++i) {
+        GEFEN_CHECK_ARG(mats[i].rows > 0 && mats[i].cols > 0 && mats[i].rows <= (1 << 24) && mats[i].cols <= (1 << 24),
+                        "Matrix %d has bad dimensions.", i);
+        GEFEN_CHECK_ARG(mats[i].x0 && mats[i].x1 && mats[i].gram && mats[i].poly, "Matrix %d has a null buffer.", i);
+        GEFEN_CHECK_ARG(aligned16(mats[i].x0) && aligned16(mats[i].x1) && aligned16(mats[i].gram) && aligned16(mats[i].poly),
+                        "Matrix %d has a buffer that is not 16-byte aligned.", i);
+    }
+    return GEFEN_B200_OK;
+}
+
+static int build_group_plan(const NsMatrix* mats, int n, const GroupShape& g, std::vector<unsigned char>& image) {
+    image.assign(static_cast<size_t>(g.bytes), 0);
+    GroupEntry* entries = reinterpret_cast<GroupEntry*>(image.data());
+    GroupTile* gram_tiles = reinterpret_cast<GroupTile*>(image.data() + g.entries_bytes);
+    GroupTile* update_tiles = gram_tiles + g.gram_tiles;
+    std::vector<int> order(n);   // longest products first: the last wave is made of the short ones
+    for (int i = 0; i < n; ++i) order[i] = i;
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
+        return std::max(mats[x].rows, mats[x].cols) > std::max(mats[y].rows, mats[y].cols);
+    });
+    int64_t gt = 0, ut = 0;
+    for (int i = 0; i < n; ++i) {
+        const NsMatrix& mat = mats[order[i]];
+        int m, k;
+        wide_dims(mat, &m, &k);
+        CUtensorMap x[2], x_mn[2], gram, poly;
+        void* xs[2] = {mat.x0, mat.x1};
+        int rc;
+        for (int q = 0; q < 2; ++q) {
+            if ((rc = make_map(&x[q], xs[q], m, k, k, kBM)) != GEFEN_B200_OK) return rc;
+            if ((rc = make_map(&x_mn[q], xs[q], m, k, k, kBK)) != GEFEN_B200_OK) return rc;
+        }
+        if ((rc = make_map(&gram, mat.gram, m, m, m, kBM)) != GEFEN_B200_OK) return rc;
+        if ((rc = make_map(&poly, mat.poly, m, m, m, kBM)) != GEFEN_B200_OK) return rc;
+        auto fill = [&](int list, const CUtensorMap& a, const CUtensorMap& b, const void* c, void* d, int N, int K) {
+            GroupEntry& e = entries[list * n + i];
+            e.a = a;
+            e.b = b;
+            e.c = static_cast<const __nv_bfloat16*>(c);
+            e.d = static_cast<__nv_bfloat16*>(d);
+            e.M = m; e.N = N; e.K = K;
+            e.ldc = N; e.ldd = N;
+        };
+        fill(0, x[0], x[0], nullptr, mat.gram, m, k);
+        fill(1, x[1], x[1], nullptr, mat.gram, m, k);
+        fill(2, gram, gram, mat.gram, mat.poly, m, m);
+        fill(3, poly, x_mn[0], mat.x0, mat.x1, k, m);
+        fill(4, poly, x_mn[1], mat.x1, mat.x0, k, m);
+        int m0, n0;
+        for (int64_t t = 0; tile_coords(m, m, g.bn, 1, t, &m0, &n0); ++t) gram_tiles[gt++] = {i, m0, n0, 0};
+        for (int64_t t = 0; tile_coords(m, k, g.bn, 0, t, &m0, &n0); ++t) update_tiles[ut++] = {i, m0, n0, 0};
+    }
+    return GEFEN_B200_OK;
+}
+
+template <bool B_MN>
+static int launch_group(const GroupShape& g, GemmArgs args, cudaStream_t stream) {
+    const CUtensorMap none = {};
+    if (g.bn == 256) return launch_gemm_variant<256, 4, false, B_MN, true, true>(none, none, args, stream);
+    return launch_gemm_variant<128, 6, false, B_MN, true, true>(none, none, args, stream);
+}
+
+}  // namespace gefen
+
+extern "C" int gefen_b200_ns_matrix_size(void) { return static_cast<int>(sizeof(gefen_b200_ns_matrix_t)); }
+
+extern "C" int64_t gefen_b200_ns_group_plan_bytes(const gefen_b200_ns_matrix_t* mats, int n) {
+    if (check_group(mats, n) != GEFEN_B200_OK) return 0;
+    return group_shape(mats, n).bytes;
+}
+
+extern "C" int gefen_b200_ns_group_plan(const gefen_b200_ns_matrix_t* mats, int n, void* host_plan) {
+    int rc = check_group(mats, n);
+    if (rc != GEFEN_B200_OK) return rc;
+    GEFEN_CHECK_ARG(host_plan != nullptr, "Expected a non-null plan buffer.");
+    try {
+        std::vector<unsigned char> image;
+        const GroupShape g = group_shape(mats, n);
+        rc = build_group_plan(mats, n, g, image);
+        if (rc == GEFEN_B200_OK) memcpy(host_plan, image.data(), image.size());
+        return rc;
+    } catch (const std::bad_alloc&) {
+        return fail(GEFEN_B200_ERUNTIME, "Out of host memory for the plan of %d matrices.", n);
+    }
+}
+
+extern "C" int gefen_b200_ns_group(const gefen_b200_ns_matrix_t* mats, int n, const void* device_mats, const void* device_plan,
+                                   float* partials, int src_dtype, int steps, double a, double b, double c, double eps, int* status,
+                                   void* stream_) {
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+    int rc = check_group(mats, n);
+    if (rc != GEFEN_B200_OK) return rc;
+    GEFEN_CHECK_ARG(device_mats && device_plan && partials && aligned16(device_mats) && (reinterpret_cast<uintptr_t>(device_plan) & 63u) == 0,
+                    "Expected non-null tables, the plan on a 64-byte boundary.");
+    GEFEN_CHECK_ARG(steps >= 0 && steps < 100, "Number of steps must be less than 100.");
+    for (int i = 0; i < n; ++i) GEFEN_CHECK_ARG(mats[i].src != nullptr && aligned16(mats[i].src), "Matrix %d needs a 16-byte aligned source.", i);
+    const GroupShape g = group_shape(mats, n);
+    const NsMatrix* table = static_cast<const NsMatrix*>(device_mats);
+    int64_t most = 1;
+    for (int i = 0; i < n; ++i) most = std::max(most, (mats[i].rows + 7) * (mats[i].cols + 7));
+    const dim3 elem(static_cast<unsigned>(std::min<int64_t>((most + 4095) / 4096, 4 * sm_count())), static_cast<unsigned>(n));
+    switch (src_dtype) {
+#define GEFEN_NS_SRC(tag, S)                                                                         \
+    case tag:                                                                                        \
+        ns_norm_kernel<S><<<dim3(kNormParts, n), kElemThreads, 0, stream>>>(table, partials);        \
+        ns_normalise_kernel<S><<<elem, kElemThreads, 0, stream>>>(table, partials, static_cast<float>(eps)); \
+        break;
+        GEFEN_NS_SRC(GEFEN_B200_F32, float)
+        GEFEN_NS_SRC(GEFEN_B200_F16, __half)
+        GEFEN_NS_SRC(GEFEN_B200_BF16, __nv_bfloat16)
+        GEFEN_NS_SRC(GEFEN_B200_F64, double)
+#undef GEFEN_NS_SRC
+        default: return fail(GEFEN_B200_EINVAL, "Unsupported source dtype tag %d.", src_dtype);
+    }
+    GEFEN_CHECK_CUDA(cudaGetLastError());
+    const GroupEntry* entries = static_cast<const GroupEntry*>(device_plan);
+    const GroupTile* tiles = reinterpret_cast<const GroupTile*>(static_cast<const unsigned char*>(device_plan) + g.entries_bytes);
+    for (int it = 0; it < steps; ++it) {
+        GemmArgs args = {};
+        args.status = status;
+        // G = X X^T ; B = b G + c G G ; X' = a X + B X
+        args.tiles = tiles;
+        args.n_tiles = static_cast<int>(g.gram_tiles);
+        args.symmetric = 1;
+        args.entries = entries + (it & 1) * n;
+        args.alpha = 1.0f;
+        args.beta = 0.0f;
+        if ((rc = launch_group<false>(g, args, stream)) != GEFEN_B200_OK) return rc;
+        args.entries = entries + 2 * n;
+        args.alpha = static_cast<float>(c);
+        args.beta = static_cast<float>(b);
+        if ((rc = launch_group<false>(g, args, stream)) != GEFEN_B200_OK) return rc;
+        args.tiles = tiles + g.gram_tiles;
+        args.n_tiles = static_cast<int>(g.update_tiles);
+        args.symmetric = 0;
+        args.entries = entries + (3 + (it & 1)) * n;
+        args.alpha = 1.0f;
+        args.beta = static_cast<float>(a);
+        if ((rc = launch_group<true>(g, args, stream)) != GEFEN_B200_OK) return rc;
+    }
+    return GEFEN_B200_OK;
+}
+
+extern "C" int gefen_b200_ns_group_apply(const gefen_b200_ns_matrix_t* mats, int n, const void* device_mats, int dtype, int steps,
+                                         const int64_t* peer_deltas, int n_peers, void* stream_) {
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+    int rc = check_group(mats, n);
+    if (rc != GEFEN_B200_OK) return rc;
+    GEFEN_CHECK_ARG(device_mats != nullptr, "Expected a non-null table.");
+    GEFEN_CHECK_ARG(n_peers >= 0 && n_peers <= GEFEN_B200_MAX_PEERS, "Expected between 0 and %d peers, got %d.", GEFEN_B200_MAX_PEERS, n_peers);
+    GEFEN_CHECK_ARG(n_peers == 0 || peer_deltas != nullptr, "Expected peer offsets for %d peers.", n_peers);
+    ApplyPeers peers = {};
+    peers.n = n_peers;
+    for (int r = 0; r < n_peers; ++r) {
+        GEFEN_CHECK_ARG(peer_deltas[r] % 16 == 0, "Peer offset %d is not a multiple of 16 bytes.", r);
+        peers.delta[r] = peer_deltas[r];
+    }
+    int64_t most = 1;
+    for (int i = 0; i < n; ++i) {
+        GEFEN_CHECK_ARG(mats[i].p != nullptr, "Matrix %d has no parameter.", i);
+        most = std::max(most, mats[i].rows * mats[i].cols);
+    }
+    const dim3 elem(static_cast<unsigned>(std::min<int64_t>((most + 4095) / 4096, 4 * sm_count())), static_cast<unsigned>(n));
+    const NsMatrix* table = static_cast<const NsMatrix*>(device_mats);
+    const int in_x1 = steps & 1;
+    switch (dtype) {
+        case GEFEN_B200_F32: ns_apply_kernel<float><<<elem, kElemThreads, 0, stream>>>(table, in_x1, peers); break;
+        case GEFEN_B200_F16: ns_apply_kernel<__half><<<elem, kElemThreads, 0, stream>>>(table, in_x1, peers); break;
+        case GEFEN_B200_BF16: ns_apply_kernel<__nv_bfloat16><<<elem, kElemThreads, 0, stream>>>(table, in_x1, peers); break;
+        default: return fail(GEFEN_B200_EINVAL, "The GefenMuon apply supports fp32, fp16 and bf16 parameters.");
+    }
+    GEFEN_CHECK_CUDA(cudaGetLastError());
+    return GEFEN_B200_OK;
 }

@@ -4,7 +4,7 @@ Per 2-D parameter and step: dequantise the momentum, m <- beta*m + (1-beta)*g, r
 same block kernel as Gefen, writing the dequantised new momentum), Nesterov blend, Newton-Schulz
 orthogonalisation in bf16, decoupled weight decay and the update with the shape-adjusted learning
 rate. The momentum kernel runs once for all matrices of a chunk (one multi-tensor launch, Nesterov
-fused); Newton-Schulz and the apply run per matrix.
+fused); Newton-Schulz and the apply run for groups of matrices.
 """
 from __future__ import annotations
 
@@ -17,7 +17,7 @@ import torch.nn as nn
 
 from . import _lib
 from .gefen import Gefen
-from .newton_schulz import orthogonalize_all
+from . import newton_schulz
 
 EPS = 1e-7
 DEFAULT_A = 3.4445
@@ -80,6 +80,8 @@ class GefenMuon(Gefen):
                     raise ValueError("GefenMuon only supports 2D parameters whereas we found a parameter with size: {}"
                                      .format(p.size()))
         self._scratch = None
+        self._ns_scratch = None     # buffers of the Newton-Schulz groups, and the launch tables over them by shapes
+        self._ns_groups = {}
 
     # ------------------------------------------------------------------ momentum
     def _momentum_scratch(self, numel: int, dtype, device) -> torch.Tensor:
@@ -98,8 +100,6 @@ class GefenMuon(Gefen):
     def check(self) -> None:
         """As `Gefen.check`, and also raises if a Newton-Schulz GEMM gave up one of its bounded waits."""
         super().check()
-        from . import newton_schulz
-
         for device in {p.device for g in self.param_groups for p in g["params"] if p.device.type == "cuda"}:
             newton_schulz.check_status(device)
 
@@ -170,36 +170,57 @@ class GefenMuon(Gefen):
             cur_elems += n
         if cur:
             chunks.append(cur)
-        lib = _lib.load()
         for chunk in chunks:
             total = sum((it[4].numel() + 7) // 8 * 8 for it in chunk)
             scratch = self._momentum_scratch(total, chunk[0][4].dtype, chunk[0][4].device)
             outs = self._quantized_momentum(chunk, scratch)
 
-            peers = getattr(self, "_peer_param_deltas", None)
-            n_peers = 0 if peers is None else len(peers)
+            # all matrices of a run share the launches; the iteration's arguments must be the same for them
+            keys = [(tuple(group["ns_coefficients"]), group["ns_steps"], group["eps"]) for group, name, p, local_p, grad in chunk]
+            for begin, end in newton_schulz.group_runs(keys, [out.numel() for out in outs]):
+                self._orthogonalize_and_apply(chunk[begin:end], outs[begin:end])
 
-            def apply(i, ortho):
-                # decoupled weight decay and the update (reference: gefen_muon.py:325-329), one kernel; for a
-                # ZeRO-1 rank it also stores the updated matrix into the other ranks' parameter buffers
-                group, name, p, local_p, grad = chunk[i]
-                lr = group["lr"]
-                adjusted_lr = _adjust_lr(lr, group["adjust_lr_fn"], p.shape)
-                wd_mul = 1 - float(lr) * group["weight_decay"] if group["weight_decay"] > 0.0 else 1.0
-                if ortho.dtype != local_p.dtype or not local_p.is_contiguous():
-                    if wd_mul != 1.0:
-                        local_p.mul_(wd_mul)
-                    local_p.add_(ortho, alpha=-adjusted_lr)
-                    return
-                if not ortho.is_contiguous():
-                    ortho = ortho.contiguous()
-                with _lib.device_guard(local_p.device):
-                    _lib.check(lib.gefen_b200_muon_apply(
-                        _lib.ptr(local_p), _lib.ptr(ortho), _lib.dtype_tag(local_p.dtype), local_p.numel(), wd_mul,
-                        -adjusted_lr, peers.ctypes.data if n_peers else None, n_peers, _lib.current_stream(local_p.device)))
+    def _matrix_group(self, shapes, device) -> "newton_schulz.MatrixGroup":
+        """Launch tables for matrices of these shapes, kept between steps over one scratch buffer that grows on demand
+        (work on one stream is ordered, so the groups of a step share it)."""
+        need = newton_schulz.group_scratch_elements(shapes)
+        if self._ns_scratch is None or self._ns_scratch.numel() < need or self._ns_scratch.device != device:
+            self._ns_scratch = torch.empty(need, dtype=torch.bfloat16, device=device)
+            self._ns_groups.clear()
+        found = self._ns_groups.get(shapes)
+        if found is None:
+            if len(self._ns_groups) >= 256:   # callers whose set of matrices keeps changing
+                self._ns_groups.clear()
+            found = self._ns_groups[shapes] = newton_schulz.MatrixGroup(shapes, self._ns_scratch)
+        return found
 
-            orthogonalize_all([(update, group["ns_coefficients"], group["ns_steps"], group["eps"])
-                               for (group, name, p, local_p, grad), update in zip(chunk, outs)], apply)
+    def _orthogonalize_and_apply(self, run, updates) -> None:
+        """Newton-Schulz, decoupled weight decay and the update (reference: gefen_muon.py:325-329) of one group; for a
+        ZeRO-1 rank the apply also stores the updated matrices into the other ranks' parameter buffers."""
+        first = run[0][0]
+        newton_schulz.check_arguments(first["ns_coefficients"], first["ns_steps"])
+        wd_muls, alphas = [], []
+        for group, name, p, local_p, grad in run:
+            lr = group["lr"]
+            alphas.append(-_adjust_lr(lr, group["adjust_lr_fn"], p.shape))
+            wd_muls.append(1 - float(lr) * group["weight_decay"] if group["weight_decay"] > 0.0 else 1.0)
+        peers = getattr(self, "_peer_param_deltas", None)
+        device = updates[0].device
+        shapes = tuple(tuple(update.shape) for update in updates)
+        if any(min(shape) == 0 for shape in shapes):
+            return
+        matrices = self._matrix_group(shapes, device)
+        together = all(local_p.is_contiguous() for group, name, p, local_p, grad in run)
+        if together:
+            matrices.update_of([local_p for group, name, p, local_p, grad in run], wd_muls, alphas)
+        matrices.run(updates, first["ns_coefficients"], first["ns_steps"], first["eps"])
+        if together:
+            matrices.apply(updates[0].dtype, peers)
+            return
+        for i, (group, name, p, local_p, grad) in enumerate(run):
+            if wd_muls[i] != 1.0:
+                local_p.mul_(wd_muls[i])
+            local_p.add_(matrices.result(i), alpha=alphas[i])
 
     @torch.no_grad()
     def step(self, closure=None):

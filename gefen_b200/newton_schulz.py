@@ -4,16 +4,17 @@ X <- X / max(||X||_F, eps); then `steps` times: A = X X^T, B = b*A + c*A*A, X <-
 bf16 with fp32 accumulation, on the wide orientation (rows <= cols; taller inputs are transposed).
 Each product rounds its result to bf16 once, as the reference's torch.addmm / `@` calls do.
 
-The products run on the library's tcgen05 GEMMs (`gefen_b200_newton_schulz`: K-major and MN-major
-operands, so no transposed copy is ever made). The kernels take dimensions that are multiples of 8
-(16-byte rows); any other matrix is padded with zero rows and columns, which the iteration maps to
-zero rows and columns (they add nothing to X X^T), and the result is cut back. There is no library
-GEMM behind this module.
+The products run on the library's tcgen05 GEMMs, all matrices of a group in one launch per product
+(`gefen_b200_ns_group`: K-major and MN-major operands, so no transposed copy is made between
+products). The kernels take dimensions that are multiples of 8 (16-byte rows); any other matrix is
+padded with zero rows and columns, which the iteration maps to zero rows and columns (they add
+nothing to X X^T), and the result is cut back. There is no library GEMM behind this module.
 """
 from __future__ import annotations
 
-from typing import Optional, Tuple
+from typing import List, Optional, Sequence, Tuple
 
+import numpy as np
 import torch
 
 from . import _lib
@@ -21,19 +22,9 @@ from . import _lib
 _STATUS = {}
 
 
-_SCRATCH = {}
-LANES = 2   # matrices orthogonalised side by side (see `orthogonalize_all`)
-
-
-def _scratch(device, numel: int, lane: int = 0) -> torch.Tensor:
-    """Per-device, per-lane bf16 scratch for the iteration (Gram matrix, polynomial, both iterates), grown on
-    demand. Work on one stream is ordered, so successive matrices of a lane can share it."""
-    key = (device.index, lane)
-    t = _SCRATCH.get(key)
-    if t is None or t.numel() < numel:
-        t = torch.empty(numel, dtype=torch.bfloat16, device=device)
-        _SCRATCH[key] = t
-    return t[:numel]
+# Elements of all matrices that go through the iteration together: enough tiles for several waves of the GPU's SMs
+# (two layers of a 1.7 B model), and a bound on the iterates' memory (4 bytes per element, the Gram matrices on top).
+GROUP_ELEMENTS = 1 << 27
 
 
 def _status(device) -> torch.Tensor:
@@ -102,84 +93,139 @@ def gemm_tt(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None
     return out
 
 
-def _newton_schulz_into_scratch(grad: torch.Tensor, ns_coefficients, ns_steps: int, eps: float, lane: int) -> torch.Tensor:
-    """The iteration on the current stream; returns a VIEW of the lane's scratch that holds the result (valid
-    until the lane's next matrix is enqueued)."""
+def _wide(shape) -> Tuple[int, int]:
+    """Rows and columns of a matrix as the iteration holds it: wide, each a multiple of 8."""
+    a, b = (shape[0] + 7) // 8 * 8, (shape[1] + 7) // 8 * 8
+    return min(a, b), max(a, b)
+
+
+def group_scratch_elements(shapes: Sequence[Tuple[int, int]]) -> int:
+    """bf16 elements of the buffers of a group: both iterates, Gram matrix and polynomial of every matrix."""
+    return sum(2 * m * k + 2 * m * m for m, k in map(_wide, shapes))
+
+
+class MatrixGroup:
+    """The launch tables of a group of matrices of given shapes over one scratch buffer (at least
+    `group_scratch_elements` bf16 elements). It can be kept and run again as long as the shapes repeat; its work is
+    ordered by the stream it runs on."""
+
+    def __init__(self, shapes: Sequence[Tuple[int, int]], scratch: torch.Tensor):
+        lib = _lib.load()
+        self.scratch = scratch
+        self.device = scratch.device
+        self.mats = np.zeros(len(shapes), dtype=_lib.NS_MATRIX_DTYPE)
+        self._places = []
+        base, offset = scratch.data_ptr(), 0
+        for row, (rows, cols) in zip(self.mats, shapes):
+            m, k = _wide((rows, cols))
+            self._places.append(offset)
+            row["rows"], row["cols"] = rows, cols
+            for field, n in (("x0", m * k), ("x1", m * k), ("gram", m * m), ("poly", m * m)):
+                row[field] = base + 2 * offset
+                offset += n
+        if offset > scratch.numel():
+            raise ValueError("Expected {} elements of scratch for the group, got {}".format(offset, scratch.numel()))
+        nbytes = lib.gefen_b200_ns_group_plan_bytes(self.mats.ctypes.data, len(shapes))
+        host = torch.empty(max(nbytes, 1), dtype=torch.uint8)
+        _lib.check(lib.gefen_b200_ns_group_plan(self.mats.ctypes.data, len(shapes), _lib.ptr(host)))
+        self.plan = host.to(self.device)
+        self.table = torch.empty(self.mats.nbytes, dtype=torch.uint8, device=self.device)
+        self.partials = torch.empty(64 * len(shapes), dtype=torch.float32, device=self.device)
+        self.steps = 0
+
+    def run(self, sources: Sequence[torch.Tensor], ns_coefficients, ns_steps: int, eps: float) -> None:
+        """Normalises the (contiguous, 16-byte aligned, equally typed) sources and iterates. `update_of` set the
+        scalars of `apply` beforehand, if that follows."""
+        a, b, c = ns_coefficients
+        self.mats["src"] = [t.data_ptr() for t in sources]
+        self.table.copy_(torch.from_numpy(self.mats.view(np.uint8)), non_blocking=True)
+        self.steps = int(ns_steps)
+        with _lib.device_guard(self.device):
+            _lib.check(_lib.load().gefen_b200_ns_group(
+                self.mats.ctypes.data, len(self.mats), _lib.ptr(self.table), _lib.ptr(self.plan), _lib.ptr(self.partials),
+                _lib.dtype_tag(sources[0].dtype), self.steps, float(a), float(b), float(c), float(eps),
+                _lib.ptr(_status(self.device)), _lib.current_stream(self.device)))
+
+    def update_of(self, params: Sequence[torch.Tensor], wd_muls, alphas) -> None:
+        self.mats["p"] = [p.data_ptr() for p in params]
+        self.mats["wd_mul"], self.mats["alpha"] = wd_muls, alphas
+        self.mats["decay"] = [int(w != 1.0) for w in wd_muls]
+
+    def apply(self, dtype: torch.dtype, peers=None) -> None:
+        """Weight decay and update of the parameters given to `update_of` (before `run`)."""
+        n_peers = 0 if peers is None else len(peers)
+        with _lib.device_guard(self.device):
+            _lib.check(_lib.load().gefen_b200_ns_group_apply(
+                self.mats.ctypes.data, len(self.mats), _lib.ptr(self.table), _lib.dtype_tag(dtype), self.steps,
+                peers.ctypes.data if n_peers else None, n_peers, _lib.current_stream(self.device)))
+
+    def result(self, i: int) -> torch.Tensor:
+        """The orthogonalised matrix i: a view of the scratch."""
+        rows, cols = int(self.mats[i]["rows"]), int(self.mats[i]["cols"])
+        m, k = _wide((rows, cols))
+        start = self._places[i] + (m * k if self.steps % 2 else 0)
+        x = self.scratch[start:start + m * k].view(m, k)
+        return x[:rows, :cols] if rows <= cols else x[:cols, :rows].t()
+
+
+def check_arguments(ns_coefficients, ns_steps: int) -> None:
     if ns_steps >= 100:
         raise ValueError("Number of steps must be less than 100 for computational efficiency")
-    if len(grad.shape) != 2:
-        raise ValueError("Input tensor gradient must be a 2D matrix")
     if len(ns_coefficients) != 3:
         raise ValueError("Coefficients must be a tuple of exactly 3 values")
+
+
+def _checked_source(grad: torch.Tensor, ns_coefficients, ns_steps: int) -> torch.Tensor:
+    check_arguments(ns_coefficients, ns_steps)
+    if len(grad.shape) != 2:
+        raise ValueError("Input tensor gradient must be a 2D matrix")
     if grad.device.type != "cuda":
         raise ValueError("gefen_b200 runs Newton-Schulz on the GPU only, got device {}".format(grad.device))
-    a, b, c = ns_coefficients
-    x = grad.bfloat16()
-    rows, cols = x.shape
-    if rows == 0 or cols == 0:
-        return x
-    # bf16 norm and quotient, as the reference's div_ (the Frobenius norm does not care about orientation).
-    # Both iterates live in the lane's scratch: the same addresses for every matrix of a shape, which lets
-    # the native driver replay the chain of products as one graph.
-    prow, pcol = (rows + 7) // 8 * 8, (cols + 7) // 8 * 8
-    m = min(prow, pcol)
-    scratch = _scratch(x.device, 2 * m * m + 2 * prow * pcol, lane)
-    gram = scratch[: m * m]
-    poly = scratch[m * m: 2 * m * m]
-    nxt = scratch[2 * m * m: 2 * m * m + prow * pcol].view(prow, pcol)
-    first = scratch[2 * m * m + prow * pcol: 2 * m * m + 2 * prow * pcol].view(prow, pcol)
-    if (prow, pcol) != (rows, cols):
-        first.zero_()
-        nxt.zero_()
-    torch.div(x, x.norm().clamp(min=eps), out=first[:rows, :cols])
-    if ns_steps > 0:
-        with _lib.device_guard(x.device):
-            _lib.check(_lib.load().gefen_b200_newton_schulz(
-                _lib.ptr(first), _lib.ptr(nxt), _lib.ptr(gram), _lib.ptr(poly), prow, pcol, int(ns_steps), float(a), float(b),
-                float(c), _lib.ptr(_status(x.device)), _lib.current_stream(x.device)))
-    result = first if ns_steps % 2 == 0 else nxt
-    return result[:rows, :cols]
+    if grad.dtype not in (torch.float32, torch.float16, torch.bfloat16):
+        grad = grad.bfloat16()
+    grad = grad.contiguous()
+    return grad if grad.data_ptr() % 16 == 0 else grad.clone()
 
 
 def zeropower_via_newtonschulz(grad: torch.Tensor, ns_coefficients: Tuple[float, float, float], ns_steps: int,
                                eps: float) -> torch.Tensor:
     """reference: gefen_muon.py:16-51. Returns a new tensor."""
-    return _newton_schulz_into_scratch(grad, ns_coefficients, ns_steps, eps, 0).clone()
+    out = []
+    orthogonalize_all([(grad, ns_coefficients, ns_steps, eps)],
+                      lambda i, ortho: out.append(ortho.clone(memory_format=torch.contiguous_format)))
+    return out[0]
 
 
-_LANE_STREAMS = {}
-
-
-def _lane_streams(device):
-    streams = _LANE_STREAMS.get(device.index)
-    if streams is None:
-        streams = _LANE_STREAMS[device.index] = [torch.cuda.Stream(device) for _ in range(LANES)]
-    return streams
+def group_runs(keys: Sequence, numels: Sequence[int]) -> List[Tuple[int, int]]:
+    """Cuts a sequence of matrices into runs of equal keys and at most GROUP_ELEMENTS elements (one at least)."""
+    runs, begin, total = [], 0, 0
+    for i, (key, n) in enumerate(zip(keys, numels)):
+        if i > begin and (key != keys[begin] or total + n > GROUP_ELEMENTS):
+            runs.append((begin, i))
+            begin, total = i, 0
+        total += n
+    if len(numels) > begin:
+        runs.append((begin, len(numels)))
+    return runs
 
 
 def orthogonalize_all(items, consume) -> None:
-    """Newton-Schulz for many matrices, LANES of them side by side.
+    """Newton-Schulz for many matrices, grouped (see MatrixGroup).
 
-    items: list of (matrix, ns_coefficients, ns_steps, eps); consume(i, ortho) is called with the
-    orthogonalised matrix i (a view of scratch memory: use it at once, on the current stream). The two
-    symmetric products of an iteration have fewer output tiles than the GPU has SMs (72 tiles of 128 x 256
-    for a 2048-row Gram matrix); running the chains of two matrices on two streams lets those launches
-    share the SMs. Every lane stream starts after the work already on the caller's stream and the caller's
-    stream waits for all lanes at the end, so to the caller this is one ordered piece of work."""
-    if not items:
-        return
-    device = items[0][0].device
-    cur = torch.cuda.current_stream(device)
-    streams = _lane_streams(device)
-    start = torch.cuda.Event()
-    start.record(cur)
-    for lane, stream in enumerate(streams):
-        stream.wait_event(start)
-    for i, (matrix, coefficients, steps, eps) in enumerate(items):
-        lane = i % LANES
-        with torch.cuda.stream(streams[lane]):
-            consume(i, _newton_schulz_into_scratch(matrix, coefficients, steps, eps, lane))
-    for stream in streams:
-        done = torch.cuda.Event()
-        done.record(stream)
-        cur.wait_event(done)
+    items: list of (matrix, ns_coefficients, ns_steps, eps); consume(i, ortho) is called in order with the
+    orthogonalised matrix i (a view of scratch memory: use it at once, on the current stream)."""
+    sources = [_checked_source(matrix, coefficients, steps) for matrix, coefficients, steps, _ in items]
+    keys = [(s.dtype, s.device, tuple(item[1]), int(item[2]), float(item[3]), s.numel() == 0) for s, item in zip(sources, items)]
+    for begin, end in group_runs(keys, [s.numel() for s in sources]):
+        run = sources[begin:end]
+        if run[0].numel() == 0:
+            for i in range(begin, end):
+                consume(i, sources[i].bfloat16())
+            continue
+        shapes = [tuple(s.shape) for s in run]
+        scratch = torch.empty(group_scratch_elements(shapes), dtype=torch.bfloat16, device=run[0].device)
+        group = MatrixGroup(shapes, scratch)
+        _, coefficients, steps, eps = items[begin]
+        group.run(run, coefficients, steps, eps)
+        for i in range(begin, end):
+            consume(i, group.result(i - begin))

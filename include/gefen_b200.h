@@ -310,6 +310,35 @@ int gefen_b200_ns_gemm_tt(const void* a, const void* b, const void* c, void* d, 
                           int K, int64_t lda, int64_t ldb, int64_t ldc, int64_t ldd, double alpha,
                           double beta, int symmetric, int* status, void* stream);
 
+/* Newton-Schulz for many matrices at once (reference: gefen_muon.py:16-51, 325-329 for each of them). One entry per
+ * matrix; the buffers are the caller's: x0 and x1 hold the iterates, gram and poly m x m, all bf16 and 16-byte
+ * aligned, m and k the smaller and the larger of rows and cols, each rounded up to a multiple of 8 (a tall matrix is
+ * held transposed). src: the matrix, contiguous, 16-byte aligned. p (apply only): the contiguous parameter. */
+typedef struct gefen_b200_ns_matrix {
+    const void* src;
+    void* p;
+    void* x0;
+    void* x1;
+    void* gram;
+    void* poly;
+    int64_t rows, cols;
+    float wd_mul, alpha;   /* p <- round(p * wd_mul) if decay; p <- round(p + alpha * result) */
+    int32_t decay, reserved_;
+} gefen_b200_ns_matrix_t;
+int gefen_b200_ns_matrix_size(void);
+/* The plan depends on the shapes and buffers only: plan_bytes bytes, filled on the host by ns_group_plan, copied by the
+ * caller to a 64-byte aligned device buffer before ns_group runs. 0 bytes: bad arguments. */
+int64_t gefen_b200_ns_group_plan_bytes(const gefen_b200_ns_matrix_t* mats, int n);
+int gefen_b200_ns_group_plan(const gefen_b200_ns_matrix_t* mats, int n, void* host_plan);
+/* Normalises every matrix and runs `steps` iterations; the results lie in x0 (even number of steps) or x1. device_mats:
+ * a copy of mats in device memory; partials: 64 floats per matrix of device scratch; status: see ns_gemm_tn. */
+int gefen_b200_ns_group(const gefen_b200_ns_matrix_t* mats, int n, const void* device_mats, const void* device_plan,
+                        float* partials, int src_dtype, int steps, double a, double b, double c, double eps,
+                        int* status, void* stream);
+/* Weight decay and update of every p from the results (see gefen_b200_muon_apply); dtype: of the parameters. */
+int gefen_b200_ns_group_apply(const gefen_b200_ns_matrix_t* mats, int n, const void* device_mats, int dtype, int steps,
+                              const int64_t* peer_deltas, int n_peers, void* stream);
+
 /* `steps` Newton-Schulz iterations (reference: gefen_muon.py:38-47) of one already normalised bf16
  * matrix [rows, cols] (row-major, contiguous, dimensions multiples of 8), enqueued as 3 * steps
  * GEMMs: G = X X^T, B = b G + c G G, X <- a X + B X on the wide orientation, or the mirrored form

@@ -1,0 +1,54 @@
+"""Newton-Schulz for groups of matrices: every matrix comes out as it does alone, whatever else is in its group, and
+the fused update equals torch's two operations on that result."""
+import pytest
+import torch
+
+SHAPES = [(300, 500), (1000, 300), (127, 64), (64, 127), (513, 1026), (8, 8), (1, 40), (40, 1), (256, 256), (2048, 192), (129, 2056)]
+NS = (3.4445, -4.7750, 2.0315)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("steps", [0, 1, 4, 5])
+def test_group_equals_single_runs_and_the_torch_update(cuda_device, dtype, steps):
+    from gefen_b200 import newton_schulz as ns
+
+    gen = torch.Generator(device=cuda_device).manual_seed(steps)
+    grads = [(torch.randn(s, generator=gen, device=cuda_device) * 0.1).to(dtype) for s in SHAPES]
+    params = [(torch.randn(s, generator=gen, device=cuda_device) * 0.02).to(dtype) for s in SHAPES]
+    scratch = torch.full((ns.group_scratch_elements(SHAPES),), float("nan"), dtype=torch.bfloat16, device=cuda_device)
+    group = ns.MatrixGroup(SHAPES, scratch)
+    wd = [1.0 if i % 3 == 0 else 0.998 for i in range(len(SHAPES))]
+    alpha = [-0.02 * (1 + i) for i in range(len(SHAPES))]
+    mine = [p.clone() for p in params]
+    for _ in range(2):   # the second run over the same buffers starts again from the sources
+        group.update_of(mine, wd, alpha)
+        group.run(grads, NS, steps, 1e-7)
+    group.apply(dtype)
+    ns.check_status(cuda_device)
+    for i, (g, p, got) in enumerate(zip(grads, params, mine)):
+        ortho = group.result(i).clone()
+        assert ortho.shape == g.shape
+        assert torch.equal(ortho, ns.zeropower_via_newtonschulz(g, NS, steps, 1e-7)), SHAPES[i]
+        x = g.bfloat16()
+        x = x / x.norm().clamp(min=1e-7)
+        x = x.T if g.shape[0] > g.shape[1] else x
+        for _ in range(steps):
+            gram = x @ x.T
+            x = torch.addmm(x, torch.addmm(gram, gram, gram, beta=NS[1], alpha=NS[2]), x, beta=NS[0])
+        want = (x.T if g.shape[0] > g.shape[1] else x).float()
+        assert float((ortho.float() - want).norm() / want.norm()) <= 2e-2, SHAPES[i]
+        if wd[i] != 1.0:
+            p.mul_(wd[i])
+        p.add_(ortho, alpha=alpha[i])
+        assert torch.equal(got, p), SHAPES[i]
+
+
+def test_runs_of_a_group():
+    from gefen_b200 import newton_schulz as ns
+
+    cap = ns.GROUP_ELEMENTS
+    assert ns.group_runs([], []) == []
+    assert ns.group_runs("aab", [1, 2, 3]) == [(0, 2), (2, 3)]
+    assert ns.group_runs("aaaa", [cap, 1, cap - 1, 1]) == [(0, 1), (1, 3), (3, 4)]
+    assert ns.group_runs("aa", [2 * cap, 2 * cap]) == [(0, 1), (1, 2)]
