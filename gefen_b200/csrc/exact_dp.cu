@@ -27,23 +27,74 @@ __device__ __forceinline__ double segment_cost(const double* pw, const double* p
     return __dsub_rn(swx2, __ddiv_rn(__dmul_rn(swx, swx), sw));
 }
 
-// One CTA per end index e. dp_prev = dp[.][c-1], dp_cur = dp[.][c].
+// One warp per end index e. dp_prev = dp[.][c-1], dp_cur = dp[.][c], starts_prev = the best starts of stage c - 1.
+//
+// Only the starts that can be the minimum are evaluated (a stage of 4096 points has 8.4 M candidates otherwise, each
+// with a double-precision division; the 256 stages took 5.6 ms). With U the candidate at the previous stage's best
+// start, a start s is out if dp_prev[s-1] > U + margin (the segment's cost is not negative) and all larger starts with
+// it (dp_prev grows with s), or if cost(s, e) > U + margin (dp_prev is not negative) and all smaller starts with it
+// (a segment's cost grows as it is extended). These hold exactly for exact costs; computed ones differ by rounding:
+// a prefix sum carries at most n 2^-53 of the total T = sum w + sum w x^2 (by Cauchy-Schwarz no other
+// sum is larger) where errors do not cancel, typically sqrt(n) 2^-53 T, a cost a few of those, and dp_prev a
+// cost's error per stage. The differences that matter are those between prefixes that all candidates read from the same
+// arrays; the functions above are evaluated on these arrays as they are, so what is left is the rounding of the
+// differences, product, quotient and sums: at most 8 * 2^-53 T per cost and K times that in dp_prev, 2.3e-13 T for 256
+// stages. margin = 1e-10 T (clusters are 1e-8 T and more) covers it, and the accumulated error of the prefixes
+// (4096 * 2^-53 T = 4.5e-13 T per element at the very worst), several hundred times over. Every start whose value is U
+// or less is therefore evaluated, with the expressions and the tie rule as before: the tables are the same bits.
+constexpr double kMargin = 1e-10;
+
 __global__ void __launch_bounds__(kDpThreads) dp_stage_kernel(const double* __restrict__ pw, const double* __restrict__ pwx,
                                                               const double* __restrict__ pwx2, int num_points, int c,
                                                               int mode, const double* __restrict__ dp_prev,
+                                                              const int* __restrict__ starts_prev,
                                                               double* __restrict__ dp_cur, int* __restrict__ backtrack,
                                                               int first_end) {
-    __shared__ double red_v[kDpThreads / 32];
-    __shared__ int red_i[kDpThreads / 32];
-    const int e = first_end + static_cast<int>(blockIdx.x);
+    const int lane = threadIdx.x & 31;
+    const int e = first_end + static_cast<int>(blockIdx.x) * (kDpThreads / 32) + (threadIdx.x >> 5);
     if (e > num_points) return;
     if (e < c) {
-        if (threadIdx.x == 0) { dp_cur[e] = INFINITY; backtrack[e] = -1; }
+        if (lane == 0) { dp_cur[e] = INFINITY; backtrack[e] = -1; }
         return;
+    }
+    int lo = c, hi = e;      // candidates [lo, hi]
+    if (c == 1) {
+        hi = 1;              // dp[s - 1][0] is infinite for every other start
+    } else {
+        const int guess = starts_prev[e] > c ? starts_prev[e] : c;
+        const double bound = dp_prev[guess - 1] + segment_cost(pw, pwx, pwx2, guess, e, mode) +
+                             kMargin * (pw[num_points] + pwx2[num_points]);
+        if (isfinite(bound)) {
+            // starts below `lo` cost too much: 32 probes over [lo, guess], twice
+            for (int round = 0; round < 2; ++round) {
+                const int step = (guess - lo) / 32 + 1;
+                const int probe = lo + lane * step;
+                const bool out = probe < guess && segment_cost(pw, pwx, pwx2, probe, e, mode) > bound;
+                const unsigned votes = __ballot_sync(0xffffffffu, out);
+                if (votes != 0u) lo = lo + (31 - __clz(votes)) * step + 1;
+                if (step == 1) break;
+            }
+            // starts above `hi` have too much before them
+            int low = guess;
+            for (int round = 0; round < 2; ++round) {
+                const int step = (hi - low) / 32 + 1;
+                const int probe = low + (lane + 1) * step;
+                const bool out = probe <= hi && dp_prev[probe - 1] > bound;
+                const unsigned votes = __ballot_sync(0xffffffffu, out);
+                if (votes != 0u) {
+                    const int first = __ffs(votes) - 1;
+                    hi = low + (first + 1) * step - 1;
+                    low = low + first * step;
+                } else {
+                    low = low + 31 * step < hi ? low + 31 * step : hi;
+                }
+                if (step == 1) break;
+            }
+        }
     }
     double best = INFINITY;
     int best_s = -1;
-    for (int s = c + static_cast<int>(threadIdx.x); s <= e; s += kDpThreads) {
+    for (int s = lo + lane; s <= hi; s += 32) {
         const double cand = __dadd_rn(dp_prev[s - 1], segment_cost(pw, pwx, pwx2, s, e, mode));
         if (cand < best) { best = cand; best_s = s; }
     }
@@ -54,14 +105,7 @@ __global__ void __launch_bounds__(kDpThreads) dp_stage_kernel(const double* __re
         const int os = __shfl_xor_sync(0xffffffffu, best_s, o);
         if (os >= 0 && (best_s < 0 || ov < best || (ov == best && os < best_s))) { best = ov; best_s = os; }
     }
-    if ((threadIdx.x & 31) == 0) { red_v[threadIdx.x >> 5] = best; red_i[threadIdx.x >> 5] = best_s; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < kDpThreads / 32; ++w) {
-            const double ov = red_v[w];
-            const int os = red_i[w];
-            if (os >= 0 && (best_s < 0 || ov < best || (ov == best && os < best_s))) { best = ov; best_s = os; }
-        }
+    if (lane == 0) {
         dp_cur[e] = best;
         backtrack[e] = best_s;
     }
@@ -130,8 +174,9 @@ int gefen_b200_exact_dp(const double* prefix_w, const double* prefix_wx, const d
         // only dp[num_points][K] is read from the last stage
         const int first_end = (c == num_codebooks) ? num_points : 0;
         const int n_ends = num_points - first_end + 1;
-        dp_stage_kernel<<<n_ends, kDpThreads, 0, stream>>>(prefix_w, prefix_wx, prefix_wx2, num_points, c, mode, prev, cur,
-                                                          backtrack + static_cast<int64_t>(c) * n1, first_end);
+        dp_stage_kernel<<<(n_ends + kDpThreads / 32 - 1) / (kDpThreads / 32), kDpThreads, 0, stream>>>(
+            prefix_w, prefix_wx, prefix_wx2, num_points, c, mode, prev, backtrack + static_cast<int64_t>(c - 1) * n1, cur,
+            backtrack + static_cast<int64_t>(c) * n1, first_end);
         GEFEN_CHECK_CUDA(cudaGetLastError());
         double* t = prev; prev = cur; cur = t;
     }
