@@ -11,7 +11,10 @@
 // a block's elements, where one is needed, comes from L1.
 #include "common.cuh"
 
+#include <string.h>
+
 #include <algorithm>
+#include <new>
 #include <vector>
 
 namespace gefen {
@@ -276,117 +279,258 @@ __global__ void adjacent_diff_final_kernel(const double* __restrict__ partial, i
     }
 }
 
-// out[j] = sum of `ratio` consecutive entries of in[], added left to right: the block sums of period
-// p from those of a divisor q of p (ratio = p / q). Logs are taken once per element, not once per
-// candidate period.
-__global__ void __launch_bounds__(kThreads) regroup_sums_kernel(const double* __restrict__ in, long long ratio,
-                                                                long long num_out, double* __restrict__ out) {
-    const int lane = threadIdx.x & 31;
-    if (ratio >= 64) {
-        const long long w0 = static_cast<long long>(blockIdx.x) * kWarps + (threadIdx.x >> 5);
-        const long long stride = static_cast<long long>(gridDim.x) * kWarps;
-        for (long long j = w0; j < num_out; j += stride) {
-            const double* src = in + j * ratio;
-            double acc = 0.0;
-            for (long long i = lane; i < ratio; i += 32) acc += src[i];
-            acc = warp_sum(acc);
-            if (lane == 0) out[j] = acc;
+// ------------------------------------------------------------------------------- scan of many periods
+// All candidate periods of many tensors in a handful of launches. The block sums of a candidate are formed from those
+// of a smaller candidate that divides it; the candidates that no other one divides ("bases": 8, 9 and 12 for a tensor
+// of 768 x 2304 elements) read the tensor themselves.
+//
+// A base takes one logarithm per block, not per element: the sum of log x_i is the logarithm of the product, which is
+// kept as a mantissa in [1, 2) and an exponent (split off every eight factors; with eps >= 2^-120 and |g| < 2^63 eight
+// factors neither overflow nor underflow, other values take their own logarithm). One rounding of 2^-53 per factor is
+// less than what adding up logarithms of about -25 costs (2^-49 per term). Two double-precision operations per
+// element remain, and the tensor is read once per base instead of a double per element written and read back.
+struct LogProduct {
+    double mantissa, slow;
+    int exponent;
+    __device__ __forceinline__ LogProduct() : mantissa(1.0), slow(0.0), exponent(0) {}
+    __device__ __forceinline__ void split() {
+        const int hi = __double2hiint(mantissa);
+        exponent += (hi >> 20) - 1023;
+        mantissa = __hiloint2double((hi & 0x000FFFFF) | 0x3FF00000, __double2loint(mantissa));
+    }
+    // |f| as a double, built from the bits (the conversion instruction runs at a quarter of the arithmetic's rate).
+    // Subnormal and zero values come out as at most 2^-126, whose square vanishes beside eps >= 2^-120.
+    static __device__ __forceinline__ double magnitude(uint32_t bits) {
+        return __hiloint2double(static_cast<int>(((bits & 0x7FFFFFFFu) >> 3) + 0x38000000u), static_cast<int>(bits << 29));
+    }
+    // up to eight values; the first n count
+    template <bool SQUARED>
+    __device__ __forceinline__ void add(const float (&f)[8], int n, double eps, bool eps_ok, unsigned long long& invalid) {
+        uint32_t most = 0u;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const uint32_t bits = __float_as_uint(f[i]) & (SQUARED ? 0xFFFFFFFFu : 0x7FFFFFFFu);   // (negative: largest)
+            most = i < n && bits > most ? bits : most;
         }
-    } else {
-        const long long t0 = static_cast<long long>(blockIdx.x) * kThreads + threadIdx.x;
-        const long long stride = static_cast<long long>(gridDim.x) * kThreads;
-        for (long long j = t0; j < num_out; j += stride) {
-            const double* src = in + j * ratio;
-            double acc = 0.0;
-            for (long long i = 0; i < ratio; ++i) acc += src[i];
-            out[j] = acc;
+        if (eps_ok && most < (SQUARED ? 0x71800000u : 0x5F000000u)) {   // 2^100 / 2^63; NaN and infinity are above
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const double v = magnitude(__float_as_uint(f[i]));
+                const double x = SQUARED ? v + eps : fma(v, v, eps);
+                mantissa *= i < n ? x : 1.0;
+            }
+            split();
+        } else {
+            for (int i = 0; i < n; ++i) slow += log_term<float, SQUARED>(f + i, eps, invalid);
         }
     }
-}
-
-// ---- the same three kernels for all candidate periods of a scan at once (blockIdx.y = candidate): a scan of 72
-// candidates is then a dozen launches instead of two hundred. The arithmetic per candidate, and therefore every
-// score, is that of the single-candidate kernels above: an output of the regrouping depends on no launch
-// parameter, and the partial sums are cut by the candidate's own number of partials, not by the grid.
-struct ScanCandidate {
-    long long src;        // offset (in doubles from the scratch base) of the sums this candidate is regrouped from
-    long long dst;        // offset of its own sums
-    long long ratio;      // period / parent period; 0: the sums are the base sums themselves, nothing to regroup
-    long long nb;         // blocks of this period
-    long long partial;    // offset of its partial sums (n_partial doubles)
-    double period;
-    int n_partial;
-    int stats;            // index of its pair of outputs
+    __device__ __forceinline__ void combine_warp() {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            mantissa *= __shfl_xor_sync(0xffffffffu, mantissa, o);   // at most 2^32
+            exponent += __shfl_xor_sync(0xffffffffu, exponent, o);
+            slow += __shfl_xor_sync(0xffffffffu, slow, o);
+        }
+    }
+    __device__ __forceinline__ double value() const { return log(mantissa) + (static_cast<double>(exponent) * 0.693147180559945309417 + slow); }
 };
 
-__global__ void __launch_bounds__(kThreads) regroup_sums_batch_kernel(double* __restrict__ scratch,
-                                                                      const ScanCandidate* __restrict__ table, int first) {
-    const ScanCandidate c = table[first + blockIdx.y];
-    if (c.ratio == 0) return;
-    const double* in = scratch + c.src;
-    double* out = scratch + c.dst;
-    const long long ratio = c.ratio, num_out = c.nb;
-    const int lane = threadIdx.x & 31;
-    if (ratio >= 64) {
-        const long long w0 = static_cast<long long>(blockIdx.x) * kWarps + (threadIdx.x >> 5);
-        const long long stride = static_cast<long long>(gridDim.x) * kWarps;
-        for (long long j = w0; j < num_out; j += stride) {
-            const double* src = in + j * ratio;
-            double acc = 0.0;
-            for (long long i = lane; i < ratio; i += 32) acc += src[i];
-            acc = warp_sum(acc);
-            if (lane == 0) out[j] = acc;
-        }
+struct ScanBase {
+    const void* values;
+    long long dst;         // offset of its sums (in doubles from the scratch base)
+    long long period, nb;
+    long long first_unit;  // in the index space of the launch
+    int dtype, tensor;
+    int count_invalid;     // one base per tensor counts the non-positive logarithm inputs
+    int vec;               // eight elements per load
+};
+struct ScanCandidate {
+    long long src;         // offset of the sums that this candidate is regrouped from
+    long long dst;         // offset of its own sums
+    long long ratio;       // period / parent period; 0: a base
+    long long nb;          // blocks of this period
+    long long first_unit;  // of its level's regrouping launch
+    long long first_partial;   // number of its first partial sum
+    double period;
+    int n_partial;
+    int tensor;
+};
+
+constexpr int kThreadPeriod = 64;       // shorter blocks: one thread each; longer ones: one warp,
+constexpr int kCtaPeriod = 16384;       // from here on one CTA
+// Blocks of one unit of work (a CTA's turn).
+__host__ __device__ inline long long base_unit_blocks(long long period) {
+    if (period < kThreadPeriod) return 2 * kThreads;
+    if (period >= kCtaPeriod) return 1;
+    return period >= 1024 ? kWarps : kWarps * 4;
+}
+
+template <typename S> __device__ __forceinline__ float scan_value(const S* p) { return ScalarIO<S>::load(p); }
+
+// The product over elements first, first + stride, ... (stride counted in elements; VEC: runs of eight) of one block.
+template <typename S, bool SQUARED>
+__device__ __forceinline__ void block_product(const S* v, long long period, int index, int count, bool vec, double eps, bool eps_ok,
+                                              LogProduct& p, unsigned long long& invalid) {
+    if constexpr (sizeof(S) == 8) {
+        for (long long i = index; i < period; i += count) p.slow += log_term<S, SQUARED>(v + i, eps, invalid);
     } else {
-        const long long t0 = static_cast<long long>(blockIdx.x) * kThreads + threadIdx.x;
-        const long long stride = static_cast<long long>(gridDim.x) * kThreads;
-        for (long long j = t0; j < num_out; j += stride) {
-            const double* src = in + j * ratio;
-            double acc = 0.0;
-            for (long long i = 0; i < ratio; ++i) acc += src[i];
-            out[j] = acc;
+        float f[8];
+        if (vec) {
+            for (long long c = index; c < period / 8; c += count) {
+                load8<S>(v + 8 * c, f);
+                p.template add<SQUARED>(f, 8, eps, eps_ok, invalid);
+            }
+        } else {
+            for (long long i0 = index; i0 < period; i0 += 8LL * count) {
+                const long long left = (period - i0 + count - 1) / count;
+                const int n = left < 8 ? static_cast<int>(left) : 8;
+#pragma unroll
+                for (int u = 0; u < 8; ++u) f[u] = u < n ? scan_value(v + i0 + static_cast<long long>(u) * count) : 0.0f;
+                p.template add<SQUARED>(f, n, eps, eps_ok, invalid);
+            }
         }
     }
 }
 
-__global__ void __launch_bounds__(kThreads) adjacent_diff_partial_batch_kernel(double* __restrict__ scratch,
-                                                                               const ScanCandidate* __restrict__ table) {
+template <typename S, bool SQUARED>
+__device__ __forceinline__ void scan_base_unit(const ScanBase& b, long long unit, double eps, bool eps_ok, double* sums,
+                                               unsigned long long& invalid) {
+    const S* values = static_cast<const S*>(b.values);
+    const long long period = b.period, first = unit * base_unit_blocks(period);
+    if (period < kThreadPeriod) {
+        for (int r = 0; r < 2; ++r) {
+            const long long j = first + r * kThreads + threadIdx.x;
+            if (j >= b.nb) return;
+            LogProduct p;
+            block_product<S, SQUARED>(values + j * period, period, 0, 1, b.vec != 0, eps, eps_ok, p, invalid);
+            sums[j] = p.value();
+        }
+    } else if (period < kCtaPeriod) {
+        const int lane = threadIdx.x & 31;
+        const long long end = first + base_unit_blocks(period) < b.nb ? first + base_unit_blocks(period) : b.nb;
+        for (long long j = first + (threadIdx.x >> 5); j < end; j += kWarps) {
+            LogProduct p;
+            block_product<S, SQUARED>(values + j * period, period, lane, 32, b.vec != 0, eps, eps_ok, p, invalid);
+            p.combine_warp();
+            if (lane == 0) sums[j] = p.value();
+        }
+    } else {
+        __shared__ double red[kWarps];
+        LogProduct p;
+        block_product<S, SQUARED>(values + first * period, period, threadIdx.x, kThreads, b.vec != 0, eps, eps_ok, p, invalid);
+        p.combine_warp();
+        __syncthreads();   // the previous unit's sum has been read
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = p.value();
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double t = 0.0;
+            for (int w = 0; w < kWarps; ++w) t += red[w];
+            sums[first] = t;
+        }
+    }
+}
+
+// Entry of a table sorted by `key` (the first unit of each entry) that holds `unit`.
+template <typename T, typename F> __device__ __forceinline__ int find_entry(const T* table, int n, long long unit, F key) {
+    int lo = 0, hi = n - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (key(table[mid]) <= unit) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
+
+template <bool SQUARED>
+__global__ void __launch_bounds__(kThreads) scan_base_kernel(double* __restrict__ scratch, const ScanBase* __restrict__ table, int n,
+                                                             long long units, double eps, unsigned long long* __restrict__ invalid_out) {
+    // 2^-120; squared inputs: 2^-70 (zeros and subnormal values count as up to 2^-126 themselves, not squared)
+    const bool eps_ok = eps >= (SQUARED ? 8.470329472543003e-22 : 7.52316384526264e-37);
+    for (long long u = blockIdx.x; u < units; u += gridDim.x) {
+        const ScanBase& b = table[find_entry(table, n, u, [](const ScanBase& e) { return e.first_unit; })];
+        const long long unit = u - b.first_unit;
+        double* sums = scratch + b.dst;
+        unsigned long long invalid = 0;
+        switch (b.dtype) {
+            case GEFEN_B200_F32: scan_base_unit<float, SQUARED>(b, unit, eps, eps_ok, sums, invalid); break;
+            case GEFEN_B200_F16: scan_base_unit<__half, SQUARED>(b, unit, eps, eps_ok, sums, invalid); break;
+            case GEFEN_B200_BF16: scan_base_unit<__nv_bfloat16, SQUARED>(b, unit, eps, eps_ok, sums, invalid); break;
+            default: scan_base_unit<double, SQUARED>(b, unit, eps, eps_ok, sums, invalid); break;
+        }
+        if (invalid != 0 && b.count_invalid) atomicAdd(&invalid_out[b.tensor], invalid);
+    }
+}
+
+constexpr int kRegroupUnit = 4 * kThreads;   // outputs of a unit whose outputs are formed by one thread each
+__host__ __device__ inline long long regroup_units(long long ratio, long long nb) {
+    return ratio >= 64 ? (nb + kWarps - 1) / kWarps : (nb + kRegroupUnit - 1) / kRegroupUnit;
+}
+// One level: out[j] = sum of `ratio` consecutive sums of the parent, added left to right.
+__global__ void __launch_bounds__(kThreads) scan_regroup_kernel(double* __restrict__ scratch, const ScanCandidate* __restrict__ table,
+                                                                int n, long long units) {
+    for (long long u = blockIdx.x; u < units; u += gridDim.x) {
+        const ScanCandidate& c = table[find_entry(table, n, u, [](const ScanCandidate& e) { return e.first_unit; })];
+        const double* in = scratch + c.src;
+        double* out = scratch + c.dst;
+        const long long ratio = c.ratio, nb = c.nb, unit = u - c.first_unit;
+        if (ratio >= 64) {
+            const int lane = threadIdx.x & 31;
+            const long long j = unit * kWarps + (threadIdx.x >> 5);
+            if (j >= nb) continue;
+            double acc = 0.0;
+            for (long long i = lane; i < ratio; i += 32) acc += in[j * ratio + i];
+            acc = warp_sum(acc);
+            if (lane == 0) out[j] = acc;
+        } else {
+            for (int r = 0; r < kRegroupUnit / kThreads; ++r) {
+                const long long j = unit * kRegroupUnit + r * kThreads + threadIdx.x;
+                if (j >= nb) break;
+                double acc = 0.0;
+                for (long long i = 0; i < ratio; ++i) acc += in[j * ratio + i];
+                out[j] = acc;
+            }
+        }
+    }
+}
+
+// Partial sums of |S[j+1] - S[j]| (the mean difference is that over the period), cut by the candidate's own number of
+// partials: reproducible.
+__global__ void __launch_bounds__(kThreads) scan_partial_kernel(const double* __restrict__ scratch, const ScanCandidate* __restrict__ table,
+                                                                int n, double* __restrict__ partials) {
     __shared__ double red[kWarps];
-    const ScanCandidate c = table[blockIdx.y];
-    if (static_cast<int>(blockIdx.x) >= c.n_partial) return;
+    const long long u = blockIdx.x;
+    const ScanCandidate& c = table[find_entry(table, n, u, [](const ScanCandidate& e) { return e.first_partial; })];
     const double* sums = scratch + c.dst;
     const long long num_pairs = c.nb - 1;
-    const double period = c.period;
-    const long long per_cta = (num_pairs + c.n_partial - 1) / c.n_partial;
-    const long long begin = static_cast<long long>(blockIdx.x) * per_cta;
-    long long end = begin + per_cta;
-    if (end > num_pairs) end = num_pairs;
+    const long long per = (num_pairs + c.n_partial - 1) / c.n_partial;
+    const long long begin = (u - c.first_partial) * per;
+    const long long end = begin + per < num_pairs ? begin + per : num_pairs;
     double acc = 0.0;
-    for (long long j = begin + threadIdx.x; j < end; j += kThreads) {
-        const double cur = sums[j] / period;
-        const double nxt = sums[j + 1] / period;
-        acc += fabs(nxt - cur);
-    }
+    for (long long j = begin + threadIdx.x; j < end; j += kThreads) acc += fabs(sums[j + 1] - sums[j]);
     acc = warp_sum(acc);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
     __syncthreads();
     if (threadIdx.x == 0) {
         double t = 0.0;
         for (int w = 0; w < kWarps; ++w) t += red[w];
-        scratch[c.partial + blockIdx.x] = t;
+        partials[u] = t;
     }
 }
 
-__global__ void adjacent_diff_final_batch_kernel(const double* __restrict__ scratch, const ScanCandidate* __restrict__ table,
-                                                 const unsigned long long* __restrict__ invalid,
-                                                 double* __restrict__ stats) {
-    if (threadIdx.x != 0) return;
-    const ScanCandidate c = table[blockIdx.x];
-    const double* partial = scratch + c.partial;
+// stats[candidate] = (score, invalid inputs of its tensor); one warp per candidate. `place`: where in stats.
+__global__ void __launch_bounds__(kThreads) scan_final_kernel(const double* __restrict__ partials, const ScanCandidate* __restrict__ table,
+                                                              const int* __restrict__ place, int n,
+                                                              const unsigned long long* __restrict__ invalid, double* __restrict__ stats) {
+    const int i = blockIdx.x * kWarps + (threadIdx.x >> 5);
+    if (i >= n) return;
+    const ScanCandidate& c = table[i];
+    const int lane = threadIdx.x & 31;
     double t = 0.0;
-    for (int i = 0; i < c.n_partial; ++i) t += partial[i];
-    stats[2 * c.stats] = t / static_cast<double>(c.nb - 1);
-    stats[2 * c.stats + 1] = static_cast<double>(*invalid);
+    for (int k = lane; k < c.n_partial; k += 32) t += partials[c.first_partial + k];
+    t = warp_sum(t);
+    if (lane == 0) {
+        stats[2 * place[i]] = t / c.period / static_cast<double>(c.nb - 1);
+        stats[2 * place[i] + 1] = static_cast<double>(invalid[c.tensor]);
+    }
 }
 
 // Mean within-block variance / coefficient of variation of x (= v or v*v), fp32 sums
@@ -693,58 +837,96 @@ static int adjacent_score(const void* values, int dtype, int64_t numel, int64_t 
     return launch_adjacent_score(block_sums, nb, period, invalid, partial, stats, stream);
 }
 
-static int64_t gcd64(int64_t a, int64_t b) { while (b) { const int64_t t = a % b; a = b; b = t; } return a; }
-
-// Plan of the hierarchical scan: the base period (gcd of all candidates), and for every candidate
-// the largest smaller candidate (or the base) that divides it. Offsets index one scratch array:
-// [invalid | partials | base sums | sums of candidate 0 | sums of candidate 1 | ...].
+// Plan of a scan: for every tensor the bases, and for every other candidate its parent. Offsets index one scratch
+// array: [invalid counts | sums | partial sums | tables].
 struct ScanPlan {
-    int64_t base;
-    std::vector<int> order;        // candidate indices by ascending period
-    std::vector<int> parent;       // per candidate: index of the parent candidate, -1 = base
-    std::vector<int64_t> offset;   // per candidate: offset of its sums (== base offset if period == base)
-    std::vector<int> level;        // per candidate: regrouping steps between the base sums and its own
-    std::vector<int> n_partial;    // per candidate: partial sums of its score
-    std::vector<int64_t> partial;  // per candidate: offset of those
-    int64_t table_offset;          // the device copy of the candidates' descriptors
-    int64_t base_offset;
-    int64_t total;
+    std::vector<ScanBase> bases;
+    std::vector<ScanCandidate> candidates;   // by level, bases first
+    std::vector<int> place;                  // index of each in the caller's order
+    std::vector<int> level_begin;            // first candidate of each level, and the end
+    std::vector<int64_t> level_units;
+    int64_t base_units = 0, partials = 0;
+    int64_t partial_offset = 0, bases_offset = 0, candidates_offset = 0, place_offset = 0, total = 0;   // doubles
 };
 
+static int64_t doubles_for(size_t bytes) { return static_cast<int64_t>((bytes + 7) / 8); }
 
-static ScanPlan make_scan_plan(int64_t numel, const int64_t* periods, int n) {
+static ScanPlan make_scan_plan(int n_tensors, const uint64_t* values, const int32_t* dtypes, const int64_t* numels,
+                               const int32_t* offsets, const int64_t* periods) {
+    struct Item { int tensor, index, parent, level; int64_t period; };
     ScanPlan plan;
-    plan.base = 0;
-    for (int i = 0; i < n; ++i) plan.base = gcd64(plan.base, periods[i]);
-    plan.order.resize(n);
-    for (int i = 0; i < n; ++i) plan.order[i] = i;
-    std::sort(plan.order.begin(), plan.order.end(), [&](int x, int y) { return periods[x] < periods[y]; });
-    plan.parent.assign(n, -1);
-    plan.offset.assign(n, 0);
-    plan.base_offset = 1 + kMaxPartials;
-    int64_t cursor = plan.base_offset + numel / plan.base;
-    for (int oi = 0; oi < n; ++oi) {
-        const int i = plan.order[oi];
-        if (periods[i] == plan.base) { plan.offset[i] = plan.base_offset; continue; }
-        for (int oj = oi - 1; oj >= 0; --oj) {
-            const int j = plan.order[oj];
-            if (periods[j] < periods[i] && periods[i] % periods[j] == 0) { plan.parent[i] = j; break; }
+    std::vector<Item> items;
+    int levels = 1;
+    for (int t = 0; t < n_tensors; ++t) {
+        const int first = static_cast<int>(items.size());
+        for (int i = offsets[t]; i < offsets[t + 1]; ++i) items.push_back({t, i, -1, 0, periods[i]});
+        std::stable_sort(items.begin() + first, items.end(), [](const Item& x, const Item& y) { return x.period < y.period; });
+        for (int i = first; i < static_cast<int>(items.size()); ++i) {
+            // the parent: a divisor of at least a sixteenth with the shortest way to the tensor, else the largest divisor
+            int best = -1, largest = -1;
+            for (int j = i - 1; j >= first; --j) {
+                if (items[j].period == items[i].period || items[i].period % items[j].period != 0) continue;
+                if (largest < 0) largest = j;
+                if (items[i].period / items[j].period <= 16 && (best < 0 || items[j].level < items[best].level)) best = j;
+            }
+            items[i].parent = best >= 0 ? best : largest;
+            items[i].level = items[i].parent < 0 ? 0 : items[items[i].parent].level + 1;
+            levels = std::max(levels, items[i].level + 1);
         }
-        plan.offset[i] = cursor;
-        cursor += numel / periods[i];
     }
-    plan.level.assign(n, 0);
-    plan.n_partial.assign(n, 1);
-    plan.partial.assign(n, 0);
-    for (int oi = 0; oi < n; ++oi) {   // ascending periods: a parent comes before its children
-        const int i = plan.order[oi];
-        plan.level[i] = periods[i] == plan.base ? 0 : (plan.parent[i] < 0 ? 1 : plan.level[plan.parent[i]] + 1);
-        plan.n_partial[i] = partials_for(numel / periods[i] - 1);
-        plan.partial[i] = cursor;
-        cursor += plan.n_partial[i];
+    const int n = static_cast<int>(items.size());
+    int64_t cursor = n_tensors;
+    std::vector<int64_t> dst(n);
+    for (int i = 0; i < n; ++i) { dst[i] = cursor; cursor += numels[items[i].tensor] / items[i].period; }
+    std::vector<bool> counted(n_tensors, false);
+    for (int level = 0; level < levels; ++level) {
+        plan.level_begin.push_back(static_cast<int>(plan.candidates.size()));
+        int64_t units = 0;
+        for (int i = 0; i < n; ++i) {
+            const Item& it = items[i];
+            if (it.level != level) continue;
+            ScanCandidate c = {};
+            c.nb = numels[it.tensor] / it.period;
+            c.dst = dst[i];
+            c.period = static_cast<double>(it.period);
+            c.tensor = it.tensor;
+            c.n_partial = partials_for(c.nb - 1);
+            c.first_partial = plan.partials;
+            plan.partials += c.n_partial;
+            if (level == 0) {
+                ScanBase b = {};
+                b.values = reinterpret_cast<const void*>(static_cast<uintptr_t>(values[it.tensor]));
+                b.dst = c.dst;
+                b.period = it.period;
+                b.nb = c.nb;
+                b.first_unit = plan.base_units;
+                b.dtype = dtypes[it.tensor];
+                b.tensor = it.tensor;
+                b.count_invalid = counted[it.tensor] ? 0 : 1;
+                counted[it.tensor] = true;
+                b.vec = it.period % 8 == 0 && aligned16(b.values) && b.dtype != GEFEN_B200_F64;
+                plan.base_units += (b.nb + base_unit_blocks(b.period) - 1) / base_unit_blocks(b.period);
+                plan.bases.push_back(b);
+            } else {
+                c.src = dst[it.parent];
+                c.ratio = it.period / items[it.parent].period;
+                c.first_unit = units;
+                units += regroup_units(c.ratio, c.nb);
+            }
+            plan.candidates.push_back(c);
+            plan.place.push_back(it.index);
+        }
+        plan.level_units.push_back(units);
     }
-    plan.table_offset = cursor;
-    cursor += (static_cast<int64_t>(n) * static_cast<int64_t>(sizeof(ScanCandidate)) + 7) / 8;
+    plan.level_begin.push_back(n);
+    plan.partial_offset = cursor;
+    cursor += plan.partials;
+    plan.bases_offset = cursor;
+    cursor += doubles_for(plan.bases.size() * sizeof(ScanBase));
+    plan.candidates_offset = cursor;
+    cursor += doubles_for(plan.candidates.size() * sizeof(ScanCandidate));
+    plan.place_offset = cursor;
+    cursor += doubles_for(plan.place.size() * sizeof(int));
     plan.total = cursor;
     return plan;
 }
@@ -842,81 +1024,113 @@ int gefen_b200_average_adjacent_log_block_mean_difference(const void* values, in
     return adjacent_score(values, dtype, numel, period, input_is_squared != 0, epsilon, stats, block_sums, stream);
 }
 
+int64_t gefen_b200_period_scan_many_scratch_doubles(int n_tensors, const int64_t* numels, const int32_t* offsets,
+                                                    const int64_t* periods) {
+    if (n_tensors <= 0 || numels == nullptr || offsets == nullptr || periods == nullptr) return 0;
+    for (int t = 0; t < n_tensors; ++t) {
+        if (numels[t] <= 0 || offsets[t + 1] < offsets[t]) return 0;
+        for (int i = offsets[t]; i < offsets[t + 1]; ++i)
+            if (periods[i] <= 0 || numels[t] % periods[i] != 0) return 0;
+    }
+    try {
+        const std::vector<uint64_t> values(n_tensors, 0);
+        const std::vector<int32_t> dtypes(n_tensors, GEFEN_B200_F32);
+        return make_scan_plan(n_tensors, values.data(), dtypes.data(), numels, offsets, periods).total;
+    } catch (const std::bad_alloc&) {
+        return 0;
+    }
+}
+
 int64_t gefen_b200_period_scan_scratch_doubles(int64_t numel, const int64_t* host_periods, int n_periods) {
-    if (numel <= 0 || n_periods <= 0 || host_periods == nullptr) return 0;
-    for (int i = 0; i < n_periods; ++i)
-        if (host_periods[i] <= 0 || numel % host_periods[i] != 0) return 0;
-    return make_scan_plan(numel, host_periods, n_periods).total;
+    if (n_periods <= 0) return 0;
+    const int32_t offsets[2] = {0, n_periods};
+    return gefen_b200_period_scan_many_scratch_doubles(1, &numel, offsets, host_periods);
+}
+
+int gefen_b200_period_scan_many(int n_tensors, const uint64_t* values, const int32_t* dtypes, const int64_t* numels,
+                                const int32_t* offsets, const int64_t* periods, int input_is_squared, double epsilon,
+                                double* stats, double* scratch, void* stream_) {
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+    GEFEN_CHECK_ARG(n_tensors >= 0, "Expected a non-negative number of tensors.");
+    if (n_tensors == 0) return GEFEN_B200_OK;
+    GEFEN_CHECK_ARG(values && dtypes && numels && offsets && periods && stats && scratch, "Expected non-null arguments.");
+    GEFEN_CHECK_ARG(epsilon > 0.0, "Expected a positive epsilon.");
+    for (int t = 0; t < n_tensors; ++t) {
+        GEFEN_CHECK_ARG(offsets[t + 1] >= offsets[t], "Expected ascending offsets.");
+        for (int i = offsets[t]; i < offsets[t + 1]; ++i) {
+            const int rc = check_flat(reinterpret_cast<const void*>(static_cast<uintptr_t>(values[t])), dtypes[t], numels[t], periods[i]);
+            if (rc != GEFEN_B200_OK) return rc;
+            GEFEN_CHECK_ARG(numels[t] / periods[i] >= 2, "Expected at least two blocks for period %lld.", static_cast<long long>(periods[i]));
+        }
+    }
+    try {
+        const ScanPlan plan = make_scan_plan(n_tensors, values, dtypes, numels, offsets, periods);
+        const int n = static_cast<int>(plan.candidates.size());
+        if (n == 0) return GEFEN_B200_OK;
+        unsigned long long* invalid = reinterpret_cast<unsigned long long*>(scratch);
+        ScanBase* bases = reinterpret_cast<ScanBase*>(scratch + plan.bases_offset);
+        ScanCandidate* table = reinterpret_cast<ScanCandidate*>(scratch + plan.candidates_offset);
+        int* place = reinterpret_cast<int*>(scratch + plan.place_offset);
+        // one copy for the three tables, which lie one after the other
+        std::vector<double> image(static_cast<size_t>(plan.total - plan.bases_offset), 0.0);
+        memcpy(image.data(), plan.bases.data(), plan.bases.size() * sizeof(ScanBase));
+        memcpy(image.data() + (plan.candidates_offset - plan.bases_offset), plan.candidates.data(), plan.candidates.size() * sizeof(ScanCandidate));
+        memcpy(image.data() + (plan.place_offset - plan.bases_offset), plan.place.data(), plan.place.size() * sizeof(int));
+        GEFEN_CHECK_CUDA(cudaMemsetAsync(invalid, 0, sizeof(unsigned long long) * n_tensors, stream));
+        GEFEN_CHECK_CUDA(cudaMemcpyAsync(bases, image.data(), image.size() * 8, cudaMemcpyHostToDevice, stream));
+        const int64_t cap = static_cast<int64_t>(sm_count()) * 8;
+        const int n_bases = static_cast<int>(plan.bases.size());
+        const int grid = static_cast<int>(std::min(plan.base_units, 4 * cap));
+        if (input_is_squared) scan_base_kernel<true><<<grid, kThreads, 0, stream>>>(scratch, bases, n_bases, plan.base_units, epsilon, invalid);
+        else scan_base_kernel<false><<<grid, kThreads, 0, stream>>>(scratch, bases, n_bases, plan.base_units, epsilon, invalid);
+        GEFEN_CHECK_CUDA(cudaGetLastError());
+        for (size_t level = 1; level + 1 < plan.level_begin.size(); ++level) {
+            const int64_t units = plan.level_units[level];
+            scan_regroup_kernel<<<static_cast<int>(std::min(units, 4 * cap)), kThreads, 0, stream>>>(
+                scratch, table + plan.level_begin[level], plan.level_begin[level + 1] - plan.level_begin[level], units);
+            GEFEN_CHECK_CUDA(cudaGetLastError());
+        }
+        double* partials = scratch + plan.partial_offset;
+        scan_partial_kernel<<<static_cast<unsigned>(plan.partials), kThreads, 0, stream>>>(scratch, table, n, partials);
+        GEFEN_CHECK_CUDA(cudaGetLastError());
+        scan_final_kernel<<<(n + kWarps - 1) / kWarps, kThreads, 0, stream>>>(partials, table, place, n, invalid, stats);
+        GEFEN_CHECK_CUDA(cudaGetLastError());
+        return GEFEN_B200_OK;
+    } catch (const std::bad_alloc&) {
+        return fail(GEFEN_B200_ERUNTIME, "Out of host memory for the plan of the period scan.");
+    }
 }
 
 int gefen_b200_period_scan(const void* values, int dtype, int64_t numel, int input_is_squared, double epsilon,
                            const int64_t* host_periods, int n_periods, double* stats, double* scratch,
-                           void* stream_) {
-    cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+                           void* stream) {
     GEFEN_CHECK_ARG(n_periods >= 0, "Expected a non-negative number of periods.");
     if (n_periods == 0) return GEFEN_B200_OK;
     GEFEN_CHECK_ARG(host_periods != nullptr && stats != nullptr && scratch != nullptr,
                     "Expected non-null periods, stats and scratch.");
-    GEFEN_CHECK_ARG(epsilon > 0.0, "Expected a positive epsilon.");
-    for (int i = 0; i < n_periods; ++i) {
-        int rc = check_flat(values, dtype, numel, host_periods[i]);
-        if (rc != GEFEN_B200_OK) return rc;
-        GEFEN_CHECK_ARG(numel / host_periods[i] >= 2, "Expected at least two blocks for period %lld.",
-                        static_cast<long long>(host_periods[i]));
+    const uint64_t pointer = static_cast<uint64_t>(reinterpret_cast<uintptr_t>(values));
+    const int32_t offsets[2] = {0, n_periods}, tag = dtype;
+    return gefen_b200_period_scan_many(1, &pointer, &tag, &numel, offsets, host_periods, input_is_squared, epsilon, stats, scratch, stream);
+}
+
+int gefen_b200_divisors(int64_t n, int64_t* out, int capacity) {
+    if (n <= 0 || (out == nullptr && capacity > 0)) return 0;
+    int count = 0;   // ascending: the small divisors, then their cofactors backwards
+    int64_t root = 0;
+    for (int64_t i = 1; i * i <= n; ++i) {
+        if (n % i != 0) continue;
+        if (count < capacity) out[count] = i;
+        ++count;
+        root = i;
     }
-    const ScanPlan plan = make_scan_plan(numel, host_periods, n_periods);
-    unsigned long long* invalid = reinterpret_cast<unsigned long long*>(scratch);
-    GEFEN_CHECK_CUDA(cudaMemsetAsync(invalid, 0, sizeof(unsigned long long), stream));
-    // the only pass over the tensor: log sums at the base granularity
-    int rc = launch_block_logsums(values, dtype, numel, plan.base, input_is_squared != 0, epsilon,
-                                  scratch + plan.base_offset, invalid, stream);
-    if (rc != GEFEN_B200_OK) return rc;
-    // the candidates in the order of their launches: by regrouping level (a parent is one level above its
-    // children), so that each level is one launch over a run of the table
-    std::vector<int> exec(plan.order);
-    std::stable_sort(exec.begin(), exec.end(), [&](int x, int y) { return plan.level[x] < plan.level[y]; });
-    std::vector<ScanCandidate> table(n_periods);
-    int max_level = 0, max_partial = 1;
-    for (int e = 0; e < n_periods; ++e) {
-        const int i = exec[e];
-        const int64_t p = host_periods[i];
-        ScanCandidate& c = table[e];
-        const int64_t q = plan.parent[i] < 0 ? plan.base : host_periods[plan.parent[i]];
-        c.src = plan.parent[i] < 0 ? plan.base_offset : plan.offset[plan.parent[i]];
-        c.dst = plan.offset[i];
-        c.ratio = p == plan.base ? 0 : p / q;
-        c.nb = numel / p;
-        c.partial = plan.partial[i];
-        c.period = static_cast<double>(p);
-        c.n_partial = plan.n_partial[i];
-        c.stats = i;
-        max_level = std::max(max_level, plan.level[i]);
-        max_partial = std::max(max_partial, c.n_partial);
+    const int small = count;
+    for (int s = small - 1; s >= 0; --s) {
+        if (s >= capacity) return -1;
+        if (s == small - 1 && root * root == n) continue;
+        if (count < capacity) out[count] = n / out[s];
+        ++count;
     }
-    ScanCandidate* dev_table = reinterpret_cast<ScanCandidate*>(scratch + plan.table_offset);
-    GEFEN_CHECK_CUDA(cudaMemcpyAsync(dev_table, table.data(), sizeof(ScanCandidate) * n_periods, cudaMemcpyHostToDevice, stream));
-    for (int level = 1; level <= max_level; ++level) {
-        int first = -1, count = 0;
-        int64_t most = 1;
-        for (int e = 0; e < n_periods; ++e) {
-            if (plan.level[exec[e]] != level) continue;
-            if (first < 0) first = e;
-            ++count;
-            const int64_t groups = table[e].ratio >= 64 ? (table[e].nb + kWarps - 1) / kWarps : (table[e].nb + kThreads - 1) / kThreads;
-            most = std::max(most, groups);
-        }
-        if (count == 0) continue;
-        const int64_t cap = static_cast<int64_t>(sm_count()) * 8;
-        const dim3 grid(static_cast<unsigned>(std::min(most, cap)), static_cast<unsigned>(count));
-        regroup_sums_batch_kernel<<<grid, kThreads, 0, stream>>>(scratch, dev_table, first);
-        GEFEN_CHECK_CUDA(cudaGetLastError());
-    }
-    adjacent_diff_partial_batch_kernel<<<dim3(static_cast<unsigned>(max_partial), static_cast<unsigned>(n_periods)), kThreads, 0,
-                                         stream>>>(scratch, dev_table);
-    GEFEN_CHECK_CUDA(cudaGetLastError());
-    adjacent_diff_final_batch_kernel<<<n_periods, 32, 0, stream>>>(scratch, dev_table, invalid, stats);
-    GEFEN_CHECK_CUDA(cudaGetLastError());
-    return GEFEN_B200_OK;
+    return count;
 }
 
 int gefen_b200_lloyd_accumulate(const void* grad_flat, int grad_dtype, int64_t numel, int64_t period,

@@ -64,10 +64,7 @@ def largest_divisor_at_most(value: int, limit: int) -> int:
         raise ValueError("Expected limit to be positive, got {}".format(limit))
     if value <= limit:
         return value
-    found = partitioning.divisors(value, max_divisor=limit)
-    if not found:
-        raise ValueError("Could not find a positive divisor for value {}".format(value))
-    return found[-1]
+    return next(d for d in range(limit, 0, -1) if value % d == 0)
 
 
 def _local(tensor, what: str) -> torch.Tensor:
@@ -236,16 +233,14 @@ class Gefen(torch.optim.Optimizer):
         """todo: list of (name, param, grad). Scores every tensor's candidate periods on the GPU,
         then fetches all scores with one copy and applies the integer rule (reference :765-828 and
         partitioning.py:225-347, without the per-divisor synchronisation)."""
-        launched = []
         for name, p, grad in todo:
             if grad.device.type != "cuda":
                 raise ValueError("gefen_b200 needs CUDA gradients, got device {} for {}".format(grad.device, name))
-            launched.append(partitioning.launch_period_scores(grad, input_is_squared=False))
-        stats = [s for _, _, s, _ in launched if s is not None]
-        host = torch.cat(stats, dim=0).cpu() if stats else None
+        found, stats = partitioning.launch_period_scores_many([grad for _, _, grad in todo])
+        host = torch.cat([s.cpu() for s in stats], dim=0) if stats else None
         periods, cursor = [], 0
-        for n, cand, s, _ in launched:
-            if s is None:
+        for n, cand in found:
+            if not cand:
                 periods.append(1)
                 continue
             periods.append(partitioning.decide_period(n, cand, host[cursor:cursor + len(cand)]))

@@ -81,6 +81,49 @@ def period_scan_async(flat: torch.Tensor, periods, *, input_is_squared: bool, ep
     return stats
 
 
+# Scratch of one many-tensor scan, in doubles (1 GiB): larger sets of tensors are scanned in several calls.
+SCAN_SCRATCH_DOUBLES = 1 << 27
+
+
+def period_scan_many_async(flats, periods, *, input_is_squared: bool, epsilon: float):
+    """The scores of many tensors: flats[t] (contiguous) with the candidates periods[t]. Enqueues a handful of launches
+    per SCAN_SCRATCH_DOUBLES of scratch; returns device tensors [candidates, 2] as period_scan_async does, whose rows
+    follow the tensors' order, without synchronising."""
+    lib = _lib.load()
+    cost = {}   # scratch of a tensor by (length, candidates)
+    parts, begin, used = [], 0, 0
+    for t, (flat, cand) in enumerate(zip(flats, periods)):
+        key = (flat.numel(), tuple(cand))
+        if key not in cost:
+            host = np.asarray(cand, dtype=np.int64)
+            cost[key] = lib.gefen_b200_period_scan_scratch_doubles(flat.numel(), host.ctypes.data, host.size)
+        if t > begin and (used + cost[key] > SCAN_SCRATCH_DOUBLES or flat.device != flats[begin].device):
+            parts.append((begin, t))
+            begin, used = t, 0
+        used += cost[key]
+    if flats:
+        parts.append((begin, len(flats)))
+    out = []
+    for first, end in parts:
+        run, device = flats[first:end], flats[first].device
+        numels = np.array([f.numel() for f in run], dtype=np.int64)
+        values = np.array([f.data_ptr() for f in run], dtype=np.uint64)
+        dtypes = np.array([_lib.dtype_tag(f.dtype) for f in run], dtype=np.int32)
+        offsets = np.concatenate([[0], np.cumsum([len(c) for c in periods[first:end]])]).astype(np.int32)
+        flat_periods = np.concatenate([np.asarray(c, dtype=np.int64) for c in periods[first:end]])
+        stats = torch.empty((int(offsets[-1]), 2), dtype=torch.float64, device=device)
+        need = lib.gefen_b200_period_scan_many_scratch_doubles(len(run), numels.ctypes.data, offsets.ctypes.data,
+                                                               flat_periods.ctypes.data)
+        scratch = torch.empty(need, dtype=torch.float64, device=device)
+        with _lib.device_guard(device):
+            _lib.check(lib.gefen_b200_period_scan_many(
+                len(run), values.ctypes.data, dtypes.ctypes.data, numels.ctypes.data, offsets.ctypes.data,
+                flat_periods.ctypes.data, int(bool(input_is_squared)), float(epsilon), _lib.ptr(stats), _lib.ptr(scratch),
+                _lib.current_stream(device)))
+        out.append(stats)
+    return out
+
+
 def scores_from_stats(stats_host: torch.Tensor):
     """Applies the reference's error rule (period_variance_kernel.cu:392-394) to fetched stats."""
     if stats_host.numel() and bool((stats_host[:, 1] > 0).any()):

@@ -40,6 +40,20 @@ def divisors(n: int, max_divisor: Optional[int] = None) -> List[int]:
     return small + large
 
 
+def native_divisors(n: int) -> List[int]:
+    """All divisors of n > 1, ascending (`divisors` without a limit), from the library: the trial divisions of a large
+    tensor's length take milliseconds in Python."""
+    import numpy as np
+
+    from . import _lib
+
+    out = np.empty(16384, dtype=np.int64)   # (no 64-bit length that fits a GPU has as many)
+    count = _lib.load().gefen_b200_divisors(int(n), out.ctypes.data, out.size)
+    if count < 0:
+        return divisors(n)
+    return out[:count].tolist()
+
+
 def candidate_periods(n: int, max_period: Optional[int] = None, min_num_blocks: int = DMNB) -> List[int]:
     return [p for p in divisors(n, max_period) if n // p >= min_num_blocks]
 
@@ -76,8 +90,8 @@ def _finalize_period_results(list_periods_and_scores: Sequence[Tuple[int, float]
             raise ValueError("Expected finite best score, got {}.".format(best[0]))
         best_period = best[1]
     if best_period > PERIOD_CAP:
-        best_period = min(q for q in divisors(flattened_length)
-                          if PERIOD_CAP < q <= best_period and best_period % q == 0)
+        # (its divisors divide the length as well)
+        best_period = min(q for q in divisors(best_period) if PERIOD_CAP < q)
     if print_results:
         print("Flattened length: {}".format(flattened_length))
         for idx, (p, score) in enumerate(ps):
@@ -104,6 +118,24 @@ def launch_period_scores(values: torch.Tensor, *, input_is_squared: bool, max_pe
         return n, [], None, bool(cands)
     stats = period_scan_async(flat, periods, input_is_squared=input_is_squared, epsilon=epsilon)
     return n, periods, stats, True
+
+
+def launch_period_scores_many(grads, epsilon: float = 1e-12, min_num_blocks: int = DMNB):
+    """launch_period_scores(input_is_squared=False) for many gradients in the same launches. Returns ([(length, periods)],
+    [device stats]): the stats of the tensors that have periods, one after the other."""
+    from .kernels.period_variance import period_scan_many_async
+
+    by_length, found, flats = {}, [], []
+    for grad in grads:
+        flat = grad.detach().reshape(-1)
+        n = flat.numel()
+        if n not in by_length:
+            by_length[n] = decision_periods([p for p in native_divisors(n) if n // p >= min_num_blocks]) if n > 1 else []
+        found.append((n, by_length[n]))
+        if by_length[n]:
+            flats.append(flat if flat.is_contiguous() else flat.contiguous())
+    stats = period_scan_many_async(flats, [p for _, p in found if p], input_is_squared=False, epsilon=epsilon)
+    return found, stats
 
 
 def decide_period(n: int, periods: Sequence[int], stats_host: Optional[torch.Tensor], print_results: bool = False) -> int:

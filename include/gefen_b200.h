@@ -245,9 +245,9 @@ int gefen_b200_average_adjacent_log_block_mean_difference(const void* values, in
                                                           void* stream);
 
 /* All candidate periods of one tensor in one call with no host synchronisation in between
- * (replaces the per-divisor launch + .item() loop of partitioning.py:259-268). The logarithm is
- * taken ONCE per element: block sums are formed at the gcd of the candidate periods and every
- * candidate's sums are regrouped from those of its largest already-computed divisor. stats holds
+ * (replaces the per-divisor launch + .item() loop of partitioning.py:259-268). Candidates that no
+ * other candidate divides read the tensor (one logarithm per block, of the product of its elements);
+ * the sums of all others are regrouped from those of a candidate that divides them. stats holds
  * 2 * n_periods doubles: stats[2*i] = score of host_periods[i], stats[2*i+1] = the number of
  * elements whose log input was <= 0. `scratch` must hold
  * gefen_b200_period_scan_scratch_doubles(numel, host_periods, n_periods) doubles. */
@@ -256,6 +256,16 @@ int64_t gefen_b200_period_scan_scratch_doubles(int64_t numel, const int64_t* hos
 int gefen_b200_period_scan(const void* values, int dtype, int64_t numel, int input_is_squared,
                            double epsilon, const int64_t* host_periods, int n_periods,
                            double* stats, double* scratch, void* stream);
+/* The same for many tensors in the same launches: tensor t has the candidates periods[offsets[t]] to
+ * periods[offsets[t + 1] - 1] (offsets: n_tensors + 1 numbers from 0), values[t] its device address, dtypes[t] its tag;
+ * stats[2*i], stats[2*i+1] belong to periods[i]. All arrays but values' targets, stats and scratch are host memory. */
+int64_t gefen_b200_period_scan_many_scratch_doubles(int n_tensors, const int64_t* numels, const int32_t* offsets,
+                                                    const int64_t* periods);
+int gefen_b200_period_scan_many(int n_tensors, const uint64_t* values, const int32_t* dtypes, const int64_t* numels,
+                                const int32_t* offsets, const int64_t* periods, int input_is_squared, double epsilon,
+                                double* stats, double* scratch, void* stream);
+/* The divisors of n, ascending; returns how many there are, -1 if `capacity` is too small. */
+int gefen_b200_divisors(int64_t n, int64_t* out, int capacity);
 
 /* Replace gefen_lloyd_accumulate_cuda and gefen_lloyd_mse_cuda (gefen_cuda_binding.cpp:90-105;
  * lloyd_max_fused_kernel.cu:244-356). */
