@@ -10,7 +10,7 @@
 //   code' = nearest codebook entry of m_i / mag'   (IEEE divide by the un-rounded fp32 mag')
 //   p_i  -= cb[code'_i] * mag' * step * lr,   step = (1/bc1) / (sqrt(v/bc2) + eps)
 //
-// Two kernels:
+// Three kernels:
 //  * step_vec_kernel  - the fast path: one warp owns one block, or several blocks when they are not longer than 1024
 //    elements (see lanes_shift). Codes and gradients are read once in chunks of eight elements (four, two or one
 //    where the block length or a pointer is a multiple of no more), the updated momenta wait in the warp's slice of
@@ -25,9 +25,10 @@
 //    bounds tests); blocks of 512 0.275 -> 0.230 ms, of 128 0.455 -> 0.315 ms; fp32 of 768 / 2048 0.193 -> 0.192 /
 //    0.182 -> 0.183 ms (67 M elements). Rows that are no multiples of eight, which the generic kernel used to take:
 //    120 M bf16 elements in blocks of 300 1.87 -> 0.37 ms, 135 M of 1500 2.26 -> 0.32 ms, 59 M of 147 0.98 -> 0.46 ms.
-//  * step_generic_kernel - blocks of more than 8192 elements, fp64, period-1 tensors and
+//  * step_vector_kernel - period-1 tensors, one warp per magnitude, everything in registers.
+//  * step_generic_kernel - blocks of more than 8192 elements, fp64 and
 //    4-bit packed codes: two passes with scalar accesses, the second pass re-reading from L1/L2.
-// Both take their tensors from a descriptor table (one launch for many tensors); a single-tensor
+// All take their tensors from a descriptor table (one launch for many tensors); a single-tensor
 // call passes a one-row table inside the kernel parameters. For data-parallel ranks whose buffers
 // are mapped into each other's address space the kernels can also store every updated parameter
 // to the peers' copies (the all-gather) and average the gradients over the peers' copies while
@@ -80,6 +81,8 @@ struct StepLaunch {
     long long param_mc_delta;
     // iteration limit of the wait for the staged tables (g_stage_spin_limit on the host)
     unsigned int spin_limit;
+    // host only: the launch before this one belongs to the same step (see let_successor_in)
+    int follows;
 };
 
 // Set (never cleared by a kernel) when a bounded wait ran out and the CTA left without doing its
@@ -168,6 +171,26 @@ __device__ __forceinline__ int find_tensor(const gefen_b200_step_tensor_t* table
     }
     return lo;
 }
+// The same by a whole warp for one gb: 32 probes at a time, so that a table of 148 rows takes two dependent loads
+// instead of eight.
+__device__ __forceinline__ int find_tensor_warp(const gefen_b200_step_tensor_t* table, int n, long long gb) {
+    int lo = 0, count = n;   // the row lies in [lo, lo + count)
+    while (count > 1) {
+        const int step = (count + 31) >> 5;
+        const int probe = static_cast<int>(threadIdx.x & 31) * step;
+        const unsigned votes = __ballot_sync(0xffffffffu, probe < count && table[lo + probe].first_block <= gb);
+        const int last = 31 - __clz(votes);   // (lane 0 always votes: the rows before lo are out)
+        lo += last * step;
+        count = count - last * step < step ? count - last * step : step;
+    }
+    return lo;
+}
+
+// The launches of one step follow each other without waiting (programmatic dependent launch): they work on different
+// tensors. A kernel lets its successor in at its start, and waits for its predecessor at its end, so that whatever
+// follows the last of them follows all of them.
+__device__ __forceinline__ void let_successor_in() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // --------------------------------------------------------------------------- vector IO
 // A "chunk" is 8 consecutive elements: 8 code bytes, 16 B of bf16/f16 or 32 B of fp32. Everything is
@@ -1102,11 +1125,13 @@ template <typename S, int V, int GSRC, bool FULL>
 __global__ void __launch_bounds__(kVecThreads, 1) step_vec_kernel(const __grid_constant__ StepLaunch L,
                                                                   const __grid_constant__ gefen_b200_step_tensor_t single) {
     SmemView s;
+    let_successor_in();
     if (smem_u32(g_smem) > kFixed) {   // (static variables have outgrown their share: nothing is done, the status says so)
         if (threadIdx.x == 0) atomicOr(&g_step_status, 2);
+        wait_for_predecessor();
         return;
     }
-    if (!stage_tables(L.ws, fast_smem(kWsAt), s, L.spin_limit)) return;
+    if (!stage_tables(L.ws, fast_smem(kWsAt), s, L.spin_limit)) { wait_for_predecessor(); return; }
     const gefen_b200_step_tensor_t* table = L.table != nullptr ? L.table : &single;
 
     const int lane = threadIdx.x & 31;
@@ -1123,7 +1148,7 @@ __global__ void __launch_bounds__(kVecThreads, 1) step_vec_kernel(const __grid_c
     long long t_first = 0, t_units = 0;
     for (long long gb = warp_global; gb < L.total_blocks; gb += warp_stride) {
         if (gb < t_first || gb >= t_first + t_units) {
-            const gefen_b200_step_tensor_t* found = table + find_tensor(table, L.n_tensors, gb);
+            const gefen_b200_step_tensor_t* found = table + find_tensor_warp(table, L.n_tensors, gb);
             if (lane == 0) t.load(found, V);
             __syncwarp();
             t_first = t.first;
@@ -1143,6 +1168,7 @@ __global__ void __launch_bounds__(kVecThreads, 1) step_vec_kernel(const __grid_c
         }
         warp_block_step<S, V, GSRC, FULL>(t, unit, L, tables, stage, lane);
     }
+    wait_for_predecessor();
 }
 
 // One gradient element as the step sees it: the local value, or the rounded average over the
@@ -1166,7 +1192,8 @@ __global__ void __launch_bounds__(kThreads) step_generic_kernel(const __grid_con
     __shared__ float red_max[kWarps];
     __shared__ float red_sum[kWarps];
     SmemView s;
-    if (!stage_tables(L.ws, g_smem, s, L.spin_limit)) return;
+    let_successor_in();
+    if (!stage_tables(L.ws, g_smem, s, L.spin_limit)) { wait_for_predecessor(); return; }
     const gefen_b200_step_tensor_t* table = L.table != nullptr ? L.table : &single;
 
     const int lane = threadIdx.x & 31;
@@ -1314,6 +1341,80 @@ __global__ void __launch_bounds__(kThreads) step_generic_kernel(const __grid_con
         }
         }
     }
+    wait_for_predecessor();
+}
+
+// --------------------------------------------------------------------------- vectors
+// Period-1 tensors (biases, norm weights): a second moment per element, one magnitude per `period` <= 256 elements
+// (reference: automatic_gefen_fused_kernel.cu:320-407). One warp takes one run of that many elements, at most eight per
+// lane, with all loads issued at once: such launches are a few hundred warps and take as long as their chain of
+// dependent loads (98 vectors of GPT-2: 21 us with the generic kernel's loops).
+constexpr int kVectorMost = 256;
+constexpr int kVectorThreads = 128;
+template <typename S>
+__global__ void __launch_bounds__(kVectorThreads) step_vector_kernel(const __grid_constant__ StepLaunch L,
+                                                                     const __grid_constant__ gefen_b200_step_tensor_t single) {
+    constexpr int E = kVectorMost / 32;
+    let_successor_in();
+    const gefen_b200_step_tensor_t* table = L.table != nullptr ? L.table : &single;
+    const int lane = threadIdx.x & 31;
+    const long long gb = static_cast<long long>(blockIdx.x) * (kVectorThreads / 32) + (threadIdx.x >> 5);
+    const bool active = gb < L.total_blocks;
+    const gefen_b200_step_tensor_t* tp = table + find_tensor_warp(table, L.n_tensors, active ? gb : 0);
+    const long long b = gb - tp->first_block;
+    const int period = active ? static_cast<int>(tp->period) : 0;
+    const long long start = b * period;
+    const S* g = static_cast<const S*>(tp->g) + start;
+    S* prm = static_cast<S*>(tp->p) + start;
+    uint8_t* codes = tp->codes + start;
+    void* const v_ptr = tp->v;
+    void* const mag_ptr = tp->mag;
+    const int mag_dtype = tp->mag_dtype, v_dtype = tp->v_dtype;
+    const float beta1 = tp->beta1, beta2 = tp->beta2, lr = tp->lr, bc1 = tp->bc1, bc2 = tp->bc2, eps = tp->eps, wd_mul = tp->wd_mul;
+    const bool wd = (tp->flags & GEFEN_B200_STEP_WEIGHT_DECAY) != 0;
+    float gi[E], vi[E], pi[E];
+    uint32_t code[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int i = lane + 32 * e;
+        if (i < period) {
+            gi[e] = ScalarIO<S>::load(g + i);
+            vi[e] = load_state(v_ptr, start + i, v_dtype);
+            pi[e] = ScalarIO<S>::load(prm + i);
+            code[e] = codes[i];
+        }
+    }
+    const float old_mag = active ? load_state(mag_ptr, b, mag_dtype) : 0.0f;
+    SmemView s;
+    if (!stage_tables(L.ws, g_smem, s, L.spin_limit)) { wait_for_predecessor(); return; }
+    if (active) {
+        const float omb1 = 1.0f - beta1, omb2 = 1.0f - beta2;
+        float u[E];
+        float absmax = 0.0f;   // NaN-ignoring, as the reference's `>` test
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            if (lane + 32 * e < period) {
+                vi[e] = store_state(v_ptr, start + lane + 32 * e, v_dtype, fmaf(beta2, vi[e], (omb2 * gi[e]) * gi[e]));
+                u[e] = ema_update_period1(beta1, old_mag * s.cb[code[e]], omb1, gi[e]);
+                absmax = fmaxf(absmax, fabsf(u[e]));
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) absmax = fmaxf(absmax, __shfl_xor_sync(0xffffffffu, absmax, o));
+        if (lane == 0) store_state(mag_ptr, b, mag_dtype, absmax);   // (the shuffles are behind every lane's read of the old one)
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const int i = lane + 32 * e;
+            if (i < period) {
+                const float x = absmax > 0.0f ? u[e] / absmax : 0.0f;
+                const uint32_t c = static_cast<uint32_t>(entry_exact(x, s.thr, s.cb, s.k));
+                codes[i] = static_cast<uint8_t>(c);
+                const float p0 = wd ? ScalarIO<S>::round(pi[e] * wd_mul) : pi[e];
+                ScalarIO<S>::store(prm + i, fmaf(-((s.cb[c] * absmax) * adam_step_size(vi[e], bc1, bc2, eps)), lr, p0));
+            }
+        }
+    }
+    wait_for_predecessor();
 }
 
 // --------------------------------------------------------------------------- vmean only
@@ -1455,6 +1556,25 @@ static int warps_override() {
 constexpr unsigned int kDefaultStageSpinLimit = 4000000u;
 static unsigned int g_stage_spin_limit = kDefaultStageSpinLimit;
 
+template <typename K>
+static int launch_step(K kernel, int grid, int threads, int smem, const StepLaunch& L, const gefen_b200_step_tensor_t& single,
+                       cudaStream_t stream) {
+    cudaLaunchConfig_t config = {};
+    config.gridDim = dim3(static_cast<unsigned>(grid));
+    config.blockDim = dim3(static_cast<unsigned>(threads));
+    config.dynamicSmemBytes = static_cast<size_t>(smem);
+    config.stream = stream;
+    cudaLaunchAttribute overlap = {};
+    overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    overlap.val.programmaticStreamSerializationAllowed = 1;
+    if (L.follows) {
+        config.attrs = &overlap;
+        config.numAttrs = 1;
+    }
+    GEFEN_CHECK_CUDA(cudaLaunchKernelEx(&config, kernel, L, single));
+    return GEFEN_B200_OK;
+}
+
 template <typename S, int V, int GSRC, bool FULL>
 static int launch_vec_variant(StepLaunch L, const gefen_b200_step_tensor_t& single, long long max_unit, cudaStream_t stream) {
     static bool configured[kMaxDevices];
@@ -1484,9 +1604,7 @@ static int launch_vec_variant(StepLaunch L, const gefen_b200_step_tensor_t& sing
     if (ctas_per_sm < 1) ctas_per_sm = 1;
     L.stage_floats = static_cast<int>(stage_bytes / 4);
     const int grid = grid_for(L.total_blocks, warps, ctas_per_sm);
-    kernel<<<grid, warps * 32, smem, stream>>>(L, single);
-    GEFEN_CHECK_CUDA(cudaGetLastError());
-    return GEFEN_B200_OK;
+    return launch_step(kernel, grid, warps * 32, smem, L, single, stream);
 }
 
 template <typename S>
@@ -1494,6 +1612,10 @@ static int launch_vec(int cls, StepLaunch L, const gefen_b200_step_tensor_t& sin
     if (cls == 3) return launch_vec_variant<S, 4, 0, false>(L, single, max_unit, stream);
     if (cls == 4) return launch_vec_variant<S, 2, 0, false>(L, single, max_unit, stream);
     if (cls == 5) return launch_vec_variant<S, 1, 0, false>(L, single, max_unit, stream);
+    if (cls == 6) {
+        constexpr int kPer = kVectorThreads / 32;
+        return launch_step(step_vector_kernel<S>, static_cast<int>((L.total_blocks + kPer - 1) / kPer), kVectorThreads, kSmemWs, L, single, stream);
+    }
     if (cls == 1) {
         if (L.grad_mc_delta != 0) return launch_vec_variant<S, 8, 2, true>(L, single, max_unit, stream);
         if (L.n_grad_srcs > 0) return launch_vec_variant<S, 8, 1, true>(L, single, max_unit, stream);
@@ -1521,23 +1643,20 @@ static int launch_generic(bool cta_per_block, const StepLaunch& L, const gefen_b
         }
     }
     if (cta_per_block) {
-        const int grid = grid_for(L.total_blocks, 1, 3);
-        step_generic_kernel<S, 256><<<grid, kThreads, smem, stream>>>(L, single);
-    } else {
-        const int grid = grid_for(L.total_blocks, kWarps, 3);
-        step_generic_kernel<S, 32><<<grid, kThreads, smem, stream>>>(L, single);
+        return launch_step(step_generic_kernel<S, 256>, grid_for(L.total_blocks, 1, 3), kThreads, smem, L, single, stream);
     }
-    GEFEN_CHECK_CUDA(cudaGetLastError());
-    return GEFEN_B200_OK;
+    return launch_step(step_generic_kernel<S, 32>, grid_for(L.total_blocks, kWarps, 3), kThreads, smem, L, single, stream);
 }
 
 // Class of a tensor: 1 = staged path in chunks of eight with whole-warp blocks, 2 = the same with several blocks
 // per warp pass (blocks of up to 1024 elements), 3 / 4 / 5 = staged path in chunks of four, two, one (the most that
-// divides the block length and the alignment of all pointers), 0 = generic warp per block, -1 = generic CTA per block.
+// divides the block length and the alignment of all pointers), 6 = vectors (period 1, runs of up to 256 elements), 0 =
+// generic warp per block, -1 = generic CTA per block.
 static int generic_class(const gefen_b200_step_tensor_t& t) { return t.period > 2048 ? -1 : 0; }
 static int class_chunk(int cls) { return cls <= 2 ? 8 : (cls == 3 ? 4 : (cls == 4 ? 2 : 1)); }
 static int tensor_class(const gefen_b200_step_tensor_t& t, int dtype) {
     const bool vec_dtype = dtype == GEFEN_B200_F32 || dtype == GEFEN_B200_BF16 || dtype == GEFEN_B200_F16;
+    if (vec_dtype && (t.flags & GEFEN_B200_STEP_PERIOD1) != 0 && t.period <= kVectorMost && t.num_blocks < (1 << 28)) return 6;
     if (!vec_dtype || (t.flags & (GEFEN_B200_STEP_PERIOD1 | GEFEN_B200_STEP_PACKED)) != 0 || t.period > kFastMaxPeriod) return generic_class(t);
     const uintptr_t ptrs = reinterpret_cast<uintptr_t>(t.g) | reinterpret_cast<uintptr_t>(t.p);
     for (int cls = 2; cls <= 5; ++cls) {
@@ -1551,7 +1670,7 @@ static int tensor_class(const gefen_b200_step_tensor_t& t, int dtype) {
 // Units of a tensor in its launch's index space: passes of a warp on the staged path, blocks elsewhere.
 // (4-bit codes with an odd period: a pair of blocks is one unit, see step_generic_kernel)
 static long long class_units(const gefen_b200_step_tensor_t& t, int cls, int dtype) {
-    if (cls >= 1) return vec_units(t.num_blocks, t.period, class_chunk(cls), dtype_size(dtype));
+    if (cls >= 1 && cls <= 5) return vec_units(t.num_blocks, t.period, class_chunk(cls), dtype_size(dtype));
     const bool paired = (t.flags & GEFEN_B200_STEP_PACKED) != 0 && (t.period & 1) != 0;
     return paired ? (t.num_blocks + 1) / 2 : t.num_blocks;
 }
@@ -1606,7 +1725,8 @@ static int run_single(gefen_b200_step_tensor_t& t, int param_dtype, const float*
     L.grad_mc_delta = 0;
     L.param_mc_delta = 0;
     L.spin_limit = g_stage_spin_limit;
-    return launch_class(cls, param_dtype, L, t, cls >= 1 ? unit_floats(t.period, class_chunk(cls), dtype_size(param_dtype)) : t.period, stream);
+    L.follows = 0;
+    return launch_class(cls, param_dtype, L, t, cls >= 1 && cls <= 5 ? unit_floats(t.period, class_chunk(cls), dtype_size(param_dtype)) : t.period, stream);
 }
 
 }  // namespace gefen
@@ -1945,6 +2065,7 @@ int gefen_b200_multi_tensor_step_multicast(gefen_b200_step_tensor_t* host_table,
     }
     GEFEN_CHECK_CUDA(cudaMemcpyAsync(device_table, host_table, sizeof(gefen_b200_step_tensor_t) * n_tensors,
                                      cudaMemcpyHostToDevice, stream));
+    bool launched = false;
     for (int begin = 0; begin < n_tensors;) {
         const int run = host_table[begin].reserved_[1];
         const gefen_b200_step_tensor_t& last = host_table[begin + run - 1];
@@ -1952,7 +2073,7 @@ int gefen_b200_multi_tensor_step_multicast(gefen_b200_step_tensor_t* host_table,
         long long max_period = 0;   // largest staging need of a warp: the elements of one unit on the staged path
         for (int i = begin; i < begin + run; ++i) {
             const int cls = host_table[begin].reserved_[0];
-            const long long need = cls >= 1 ? unit_floats(host_table[i].period, class_chunk(cls), dtype_size(param_dtype)) : host_table[i].period;
+            const long long need = cls >= 1 && cls <= 5 ? unit_floats(host_table[i].period, class_chunk(cls), dtype_size(param_dtype)) : host_table[i].period;
             max_period = need > max_period ? need : max_period;
         }
         if (total > 0) {
@@ -1971,6 +2092,8 @@ int gefen_b200_multi_tensor_step_multicast(gefen_b200_step_tensor_t* host_table,
             L.grad_mc_delta = grad_multicast_delta;
             L.param_mc_delta = param_multicast_delta;
             L.spin_limit = g_stage_spin_limit;
+            L.follows = launched && n_peers == 0 && n_grad_srcs == 0;
+            launched = true;
             const int rc = launch_class(host_table[begin].reserved_[0], param_dtype, L, host_table[begin], max_period, stream);
             if (rc != GEFEN_B200_OK) return rc;
         }

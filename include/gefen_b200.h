@@ -196,7 +196,7 @@ int gefen_b200_step_tensor_size(void);
  * 0 = any other block of up to 2048 elements, -1 = any other longer block. */
 int gefen_b200_step_tensor_class(const gefen_b200_step_tensor_t* host_entry, int param_dtype);
 /* The launch a table entry goes to: 1 and 2 as above, 3 / 4 / 5 = staged path in chunks of four, two, one
- * element (blocks and pointers that are multiples of no more than that), 0 / -1 = generic kernels. Rows
+ * element (blocks and pointers that are multiples of no more than that), 6 = period-1 vectors, 0 / -1 = generic. Rows
  * of equal launch class that are adjacent in the table share one launch. */
 int gefen_b200_step_launch_class(const gefen_b200_step_tensor_t* host_entry, int param_dtype);
 
