@@ -759,6 +759,7 @@ typedef gefen_b200_ns_matrix_t NsMatrix;
 constexpr int kNormParts = 64;      // CTAs per matrix of the norm
 constexpr int kElemThreads = 256;
 constexpr int kTile = 64;           // transposing tile
+constexpr int kTilePitch = 72;      // its rows start on 16 bytes
 
 __device__ __forceinline__ bool ns_tall(const NsMatrix& m) { return m.rows > m.cols; }
 __device__ __forceinline__ int ns_wide_rows(const NsMatrix& m) { return (static_cast<int>(m.rows < m.cols ? m.rows : m.cols) + 7) / 8 * 8; }
@@ -800,7 +801,7 @@ __global__ void __launch_bounds__(kElemThreads) ns_norm_kernel(const NsMatrix* _
 // x.div_(x.norm().clamp(min=eps)) on a bf16 tensor rounds them (reference: gefen_muon.py:38).
 template <typename S>
 __global__ void __launch_bounds__(kElemThreads) ns_normalise_kernel(const NsMatrix* __restrict__ table, const float* __restrict__ parts, float eps) {
-    __shared__ __nv_bfloat16 tile[kTile][kTile + 2];
+    __shared__ __align__(16) __nv_bfloat16 tile[kTile][kTilePitch];
     __shared__ float norm_shared;
     const NsMatrix& m = table[blockIdx.y];
     if (threadIdx.x < 32) {
@@ -841,14 +842,32 @@ __global__ void __launch_bounds__(kElemThreads) ns_normalise_kernel(const NsMatr
         const int r0 = t / tiles_c * kTile, c0 = t % tiles_c * kTile;
         if (ns_tall(m)) {
             __syncthreads();
-            for (int y = y0; y < kTile; y += kElemThreads / kTile) {   // source row c0 + y, column r0 + x
-                float f = 0.0f;
-                if (c0 + y < rows && r0 + x < cols) f = as_bf16(src + static_cast<long long>(c0 + y) * cols + r0 + x) / norm;
-                tile[y][x] = __float2bfloat16_rn(f);
+            // a thread reads eight columns of source row c0 + x (16 or 32 bytes where rows start on 16) and leaves them
+            // in the tile transposed: neighbouring threads write neighbouring elements
+            const bool vec = cols % 8 == 0;
+            for (int piece = y0; piece < kTile / 8; piece += kElemThreads / kTile) {
+                float f[8];
+                const int row = c0 + x, col = r0 + 8 * piece;
+                const S* from = src + static_cast<long long>(row) * cols + col;
+                if (vec && row < rows && col < cols) {
+                    alignas(16) S v[8];
+#pragma unroll
+                    for (int q = 0; q < static_cast<int>(sizeof(S)) / 2; ++q) reinterpret_cast<uint4*>(v)[q] = reinterpret_cast<const uint4*>(from)[q];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) f[e] = as_bf16(v + e) / norm;
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) f[e] = row < rows && col + e < cols ? as_bf16(from + e) / norm : 0.0f;
+                }
+#pragma unroll
+                for (int e = 0; e < 8; ++e) tile[8 * piece + e][x] = __float2bfloat16_rn(f[e]);
             }
             __syncthreads();
-            for (int y = y0; y < kTile; y += kElemThreads / kTile)
-                if (r0 + y < wr && c0 + x < wc) dst[static_cast<long long>(r0 + y) * wc + c0 + x] = tile[x][y];
+            for (int i = threadIdx.x; i < kTile * kTile / 8; i += kElemThreads) {   // (wide columns come in eights)
+                const int y = i / (kTile / 8), c = c0 + i % (kTile / 8) * 8;
+                if (r0 + y < wr && c < wc)
+                    *reinterpret_cast<uint4*>(dst + static_cast<long long>(r0 + y) * wc + c) = *reinterpret_cast<const uint4*>(&tile[y][c - c0]);
+            }
         } else {
             for (int y = y0; y < kTile; y += kElemThreads / kTile) {
                 if (r0 + y >= wr || c0 + x >= wc) continue;
@@ -869,7 +888,7 @@ struct ApplyPeers {
 // muon_apply_kernel does for one matrix (reference: gefen_muon.py:326-329), peer stores included.
 template <typename S>
 __global__ void __launch_bounds__(kElemThreads) ns_apply_kernel(const NsMatrix* __restrict__ table, int in_x1, const __grid_constant__ ApplyPeers peers) {
-    __shared__ __nv_bfloat16 tile[kTile][kTile + 2];
+    __shared__ __align__(16) __nv_bfloat16 tile[kTile][kTilePitch];
     const NsMatrix& m = table[blockIdx.y];
     const __nv_bfloat16* u = static_cast<const __nv_bfloat16*>(in_x1 ? m.x1 : m.x0);
     S* p = static_cast<S*>(m.p);
@@ -911,13 +930,38 @@ __global__ void __launch_bounds__(kElemThreads) ns_apply_kernel(const NsMatrix* 
         const int r0 = t / tiles_c * kTile, c0 = t % tiles_c * kTile;
         if (ns_tall(m)) {
             __syncthreads();
-            for (int y = y0; y < kTile; y += kElemThreads / kTile)   // u row c0 + y, column r0 + x
-                if (c0 + y < wr && r0 + x < wc) tile[y][x] = u[static_cast<long long>(c0 + y) * wc + r0 + x];
+            for (int piece = y0; piece < kTile / 8; piece += kElemThreads / kTile) {   // eight columns of u row c0 + x
+                const int row = c0 + x, col = r0 + 8 * piece;
+                alignas(16) __nv_bfloat16 v[8] = {};
+                if (row < wr && col < wc) *reinterpret_cast<uint4*>(v) = *reinterpret_cast<const uint4*>(u + static_cast<long long>(row) * wc + col);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) tile[8 * piece + e][x] = v[e];
+            }
             __syncthreads();
-            for (int y = y0; y < kTile; y += kElemThreads / kTile) {
-                if (r0 + y >= rows || c0 + x >= cols) continue;
-                const long long at = static_cast<long long>(r0 + y) * cols + c0 + x;
-                put(at, update(ScalarIO<S>::load(p + at), __bfloat162float(tile[x][y])));
+            if (cols % 8 == 0 && (reinterpret_cast<uintptr_t>(p) & 15u) == 0) {
+                for (int i = threadIdx.x; i < kTile * kTile / 8; i += kElemThreads) {
+                    const int y = i / (kTile / 8), c = c0 + i % (kTile / 8) * 8;
+                    if (r0 + y >= rows || c >= cols) continue;
+                    constexpr int kWide = static_cast<int>(sizeof(S)) / 2;
+                    S* at = p + static_cast<long long>(r0 + y) * cols + c;
+                    alignas(16) S v[8];
+#pragma unroll
+                    for (int q = 0; q < kWide; ++q) reinterpret_cast<uint4*>(v)[q] = reinterpret_cast<const uint4*>(at)[q];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) ScalarIO<S>::store(v + e, update(ScalarIO<S>::load(v + e), __bfloat162float(tile[y][c - c0 + e])));
+#pragma unroll
+                    for (int q = 0; q < kWide; ++q) {
+                        reinterpret_cast<uint4*>(at)[q] = reinterpret_cast<uint4*>(v)[q];
+                        for (int r = 0; r < peers.n; ++r)
+                            reinterpret_cast<uint4*>(reinterpret_cast<uintptr_t>(at) + peers.delta[r])[q] = reinterpret_cast<uint4*>(v)[q];
+                    }
+                }
+            } else {
+                for (int y = y0; y < kTile; y += kElemThreads / kTile) {
+                    if (r0 + y >= rows || c0 + x >= cols) continue;
+                    const long long at = static_cast<long long>(r0 + y) * cols + c0 + x;
+                    put(at, update(ScalarIO<S>::load(p + at), __bfloat162float(tile[y][x])));
+                }
             }
         } else {
             for (int y = y0; y < kTile; y += kElemThreads / kTile) {
