@@ -46,25 +46,27 @@ int sm_count() {
     return cached[dev];
 }
 
-// One CTA of 256 threads. Thread i < k-1 bisects threshold i; then all threads fill the cells.
-__global__ void __launch_bounds__(256) codebook_prepare_kernel(const float* __restrict__ codebook, int k,
-                                                               unsigned char* __restrict__ ws) {
-    __shared__ float cb[kMaxCodebook];
+// Fills a workspace from a codebook in shared memory (256 entries, the tail padded with the last); one CTA of
+// kPrepareThreads threads. Thread i < k-1 bisects threshold i; then all threads fill the cells.
+constexpr int kPrepareThreads = 1024;
+__device__ __forceinline__ void build_workspace(const float* cb, int k, unsigned char* ws) {
     __shared__ float thr[kMaxCodebook];
     __shared__ int tcell[kMaxCodebook];
     __shared__ int any_slow;
     const int t = threadIdx.x;
     if (t == 0) any_slow = 0;
-    cb[t] = codebook[t < k ? t : k - 1];
-    __syncthreads();
-    thr[t] = (t < k - 1) ? entry_threshold(t, cb, k) : INFINITY;
-    tcell[t] = lut_threshold_cell(thr[t]);
+    if (t < kMaxCodebook) {
+        thr[t] = (t < k - 1) ? entry_threshold(t, cb, k) : INFINITY;
+        tcell[t] = lut_threshold_cell(thr[t]);
+    }
     __syncthreads();
     float* ws_cb = reinterpret_cast<float*>(ws + kWsCodebookOff);
     float* ws_thr = reinterpret_cast<float*>(ws + kWsThresholdOff);
     uint32_t* ws_lut = reinterpret_cast<uint32_t*>(ws + kWsLutOff);
-    ws_cb[t] = cb[t];
-    ws_thr[t] = thr[t];
+    if (t < kMaxCodebook) {
+        ws_cb[t] = cb[t];
+        ws_thr[t] = thr[t];
+    }
     int slow = 0;
     for (int cell = t; cell < kLutBytes / 8; cell += blockDim.x) {
         uint32_t w0 = 0x7f800000u, w1 = 0u;  // padding entries: +inf threshold, nothing below
@@ -84,8 +86,60 @@ __global__ void __launch_bounds__(256) codebook_prepare_kernel(const float* __re
     }
 }
 
+__global__ void __launch_bounds__(kPrepareThreads) codebook_prepare_kernel(const float* __restrict__ codebook, int k,
+                                                                           unsigned char* __restrict__ ws) {
+    __shared__ float cb[kMaxCodebook];
+    if (threadIdx.x < kMaxCodebook) cb[threadIdx.x] = codebook[static_cast<int>(threadIdx.x) < k ? threadIdx.x : k - 1];
+    __syncthreads();
+    build_workspace(cb, k, ws);
+}
+
+// The M-step of the Lloyd-Max fit in one launch: entry <- sum / count where there are values, the ends pinned when asked,
+// sorted; the sums and counts go back to zero and the workspace of the new codebook is built. (As a dozen small torch
+// kernels and the table build it took longer than the pass over 33 M values.)
+__global__ void __launch_bounds__(kPrepareThreads) lloyd_update_kernel(float* __restrict__ codebook, float* __restrict__ sums,
+                                                                       unsigned long long* __restrict__ counts, int k, int force,
+                                                                       unsigned char* __restrict__ ws) {
+    __shared__ uint32_t keys[kMaxCodebook];
+    __shared__ float cb[kMaxCodebook];
+    const int t = threadIdx.x;
+    if (t < kMaxCodebook) {
+        uint32_t key = 0xFFFFFFFFu;   // behind every entry, NaN included
+        if (t < k) {
+            const unsigned long long n = counts[t];
+            float v = codebook[t];
+            if (n > 0) v = sums[t] / static_cast<float>(n);
+            if (force && t == 0) v = -1.0f;
+            if (force && t == k - 1) v = 1.0f;
+            key = float_to_ordered(v);
+            sums[t] = 0.0f;
+            counts[t] = 0ull;
+        }
+        keys[t] = key;
+    }
+    __syncthreads();
+    for (int size = 2; size <= kMaxCodebook; size <<= 1) {
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            const int other = t ^ stride;
+            if (t < kMaxCodebook && other > t) {
+                const uint32_t a = keys[t], b = keys[other];
+                const bool ascending = (t & size) == 0;
+                if ((a > b) == ascending) { keys[t] = b; keys[other] = a; }
+            }
+            __syncthreads();
+        }
+    }
+    if (t < kMaxCodebook) {
+        const float v = ordered_to_float(keys[t < k ? t : k - 1]);
+        cb[t] = v;
+        if (t < k) codebook[t] = v;
+    }
+    __syncthreads();
+    build_workspace(cb, k, ws);
+}
+
 static int launch_prepare(const float* codebook, int k, void* ws, cudaStream_t stream) {
-    codebook_prepare_kernel<<<1, 256, 0, stream>>>(codebook, k, static_cast<unsigned char*>(ws));
+    codebook_prepare_kernel<<<1, kPrepareThreads, 0, stream>>>(codebook, k, static_cast<unsigned char*>(ws));
     GEFEN_CHECK_CUDA(cudaGetLastError());
     return GEFEN_B200_OK;
 }
@@ -141,6 +195,20 @@ int gefen_b200_codebook_prepare(const float* codebook, int codebook_size, void* 
                     "Expected codebook to have between 1 and 256 entries, got %d.", codebook_size);
     GEFEN_CHECK_ARG(aligned16(workspace), "Expected workspace to be 16-byte aligned.");
     return launch_prepare(codebook, codebook_size, workspace, static_cast<cudaStream_t>(stream));
+}
+
+int gefen_b200_lloyd_update(float* codebook, int codebook_size, int force_endpoints, float* sums, int64_t* counts, void* workspace,
+                            void* stream) {
+    using namespace gefen;
+    GEFEN_CHECK_ARG(codebook && sums && counts && workspace, "Expected non-null arguments.");
+    GEFEN_CHECK_ARG(codebook_size >= 1 && codebook_size <= kMaxCodebook,
+                    "Expected codebook to have between 1 and 256 entries, got %d.", codebook_size);
+    GEFEN_CHECK_ARG(aligned16(workspace), "Expected workspace to be 16-byte aligned.");
+    lloyd_update_kernel<<<1, kPrepareThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+        codebook, sums, reinterpret_cast<unsigned long long*>(counts), codebook_size, force_endpoints ? 1 : 0,
+        static_cast<unsigned char*>(workspace));
+    GEFEN_CHECK_CUDA(cudaGetLastError());
+    return GEFEN_B200_OK;
 }
 
 }  // extern "C"

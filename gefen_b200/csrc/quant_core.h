@@ -66,6 +66,14 @@ GEFEN_HD float entry_threshold(int i, const float* cb, int k) {
     uint32_t lo = float_to_ordered(-INFINITY);   // entry(-inf) == 0 <= i always
     uint32_t hi = float_to_ordered(cb[k - 1]);
     if (nearest_entry_reference(cb[k - 1], cb, k) <= i) return INFINITY;
+    // the threshold is within a few floats of the midpoint: where that holds, two evaluations replace most of the steps
+    const float mid_point = 0.5f * (cb[i] + cb[i + 1 < k ? i + 1 : i]);
+    if (mid_point == mid_point) {
+        const uint32_t at = float_to_ordered(mid_point);
+        const uint32_t below = at - 4u, above = at + 4u;
+        if (below > lo && below < hi && nearest_entry_reference(ordered_to_float(below), cb, k) <= i) lo = below;
+        if (above > lo && above < hi && nearest_entry_reference(ordered_to_float(above), cb, k) > i) hi = above;
+    }
     while (hi - lo > 1u) {
         const uint32_t mid = lo + ((hi - lo) >> 1);
         if (nearest_entry_reference(ordered_to_float(mid), cb, k) <= i) lo = mid; else hi = mid;

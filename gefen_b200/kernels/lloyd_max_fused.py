@@ -27,6 +27,10 @@ def _check_flat_and_codebook(grad_flat, codebook, period):
 
 def gefen_lloyd_accumulate_cuda(grad_flat, codebook, period: int, sums, counts) -> None:
     """sums[e] += sum of normalised values nearest to entry e; counts[e] += their number."""
+    _accumulate(grad_flat, codebook, None, period, sums, counts)
+
+
+def _accumulate(grad_flat, codebook, workspace, period: int, sums, counts) -> None:
     require_cuda_tensors({"grad_flat": grad_flat, "codebook": codebook, "sums": sums, "counts": counts})
     _check_flat_and_codebook(grad_flat, codebook, period)
     if sums.dim() != 1 or sums.numel() != codebook.numel():
@@ -39,10 +43,12 @@ def gefen_lloyd_accumulate_cuda(grad_flat, codebook, period: int, sums, counts) 
         raise ValueError("Expected counts to be int64, got {}".format(counts.dtype))
     grad_flat = grad_flat.contiguous()
     codebook = codebook.contiguous()
+    if workspace is None:
+        workspace = _lib.codebook_workspace(codebook)
     with _lib.device_guard(grad_flat.device):
         _lib.check(_lib.load().gefen_b200_lloyd_accumulate(
             _lib.ptr(grad_flat), _lib.dtype_tag(grad_flat.dtype), grad_flat.numel(), int(period),
-            _lib.ptr(codebook), codebook.numel(), _lib.ptr(_lib.codebook_workspace(codebook)), _lib.ptr(sums),
+            _lib.ptr(codebook), codebook.numel(), _lib.ptr(workspace), _lib.ptr(sums),
             _lib.ptr(counts), _lib.current_stream(grad_flat.device)))
 
 
@@ -77,15 +83,19 @@ def lloyd_max_fit(grads_and_periods, codebook: torch.Tensor, iterations: int = 1
     entries pinned to -1 and +1 when force_endpoints, then re-sorted. Returns a new codebook."""
     cb = codebook.detach().clone().float().contiguous()
     k = cb.numel()
-    for _ in range(iterations):
-        sums = torch.zeros(k, dtype=torch.float32, device=cb.device)
-        counts = torch.zeros(k, dtype=torch.int64, device=cb.device)
-        for flat, period in grads_and_periods:
-            gefen_lloyd_accumulate_cuda(flat, cb, period, sums, counts)
-        filled = counts > 0
-        new_cb = torch.where(filled, sums / counts.clamp(min=1).float(), cb)
-        if force_endpoints:
-            new_cb[0] = -1.0
-            new_cb[-1] = 1.0
-        cb = new_cb.sort().values.contiguous()
+    if iterations <= 0:
+        return cb
+    require_cuda_tensors({"codebook": cb})
+    lib = _lib.load()
+    sums = torch.zeros(k, dtype=torch.float32, device=cb.device)
+    counts = torch.zeros(k, dtype=torch.int64, device=cb.device)
+    workspace = torch.empty(_lib.CODEBOOK_WS_BYTES, dtype=torch.uint8, device=cb.device)
+    with _lib.device_guard(cb.device):
+        stream = _lib.current_stream(cb.device)
+        _lib.check(lib.gefen_b200_codebook_prepare(_lib.ptr(cb), k, _lib.ptr(workspace), stream))
+        for _ in range(iterations):
+            for flat, period in grads_and_periods:
+                _accumulate(flat, cb, workspace, period, sums, counts)
+            _lib.check(lib.gefen_b200_lloyd_update(_lib.ptr(cb), k, int(bool(force_endpoints)), _lib.ptr(sums),
+                                                   _lib.ptr(counts), _lib.ptr(workspace), stream))
     return cb

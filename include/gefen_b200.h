@@ -273,6 +273,11 @@ int gefen_b200_lloyd_accumulate(const void* grad_flat, int grad_dtype, int64_t n
                                 int64_t period, const float* codebook, int codebook_size,
                                 const void* codebook_ws, float* sums, int64_t* counts,
                                 void* stream);
+/* The update that follows (no counterpart: the reference ships the two kernels only): codebook[e] <- sums[e] / counts[e]
+ * where counts[e] > 0, the ends set to -1 and +1 with force_endpoints, sorted, all in place; sums and counts go back to
+ * zero and `workspace` is built for the new codebook (see gefen_b200_codebook_prepare). */
+int gefen_b200_lloyd_update(float* codebook, int codebook_size, int force_endpoints, float* sums,
+                            int64_t* counts, void* workspace, void* stream);
 int gefen_b200_lloyd_mse(const void* grad_flat, int grad_dtype, int64_t numel, int64_t period,
                          const float* old_codebook, const float* new_codebook, int codebook_size,
                          const void* old_codebook_ws, float* mse_normalized_sum,
