@@ -101,6 +101,8 @@ def _declare(lib):
         "gefen_b200_divisors": (i32, [i64, vp, i32]),
         "gefen_b200_lloyd_accumulate": (i32, [vp, i32, i64, i64, vp, i32, vp, vp, vp, vp]),
         "gefen_b200_lloyd_update": (i32, [vp, i32, i32, vp, vp, vp, vp]),
+        "gefen_b200_exact_histogram_many": (i32, [i32, vp, vp, vp, vp, vp, vp, i32, vp, vp]),
+        "gefen_b200_exact_histogram_many_table_bytes": (i64, [i32]),
         "gefen_b200_lloyd_mse": (i32, [vp, i32, i64, i64, vp, vp, i32, vp, vp, vp, vp]),
         "gefen_b200_exact_dp_scratch_bytes": (i64, [i32, i32]),
         "gefen_b200_exact_dp": (i32, [vp, vp, vp, i32, i32, i32, vp, vp, vp]),

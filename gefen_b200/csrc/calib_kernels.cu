@@ -201,6 +201,111 @@ __global__ void __launch_bounds__(kThreads) histogram_kernel(const S* __restrict
     }
 }
 
+// The histograms of many tensors in one launch, and their float32 sum in the tensors' order. A unit of work is a run of
+// blocks of one tensor (about 256 k elements, whose counts are then added to the tensor's row).
+struct HistEntry {
+    const void* values;
+    long long period, nb;
+    long long first_unit;
+    int dtype, vec;
+};
+__host__ __device__ inline long long hist_unit_blocks(long long period) {
+    const long long blocks = (1 << 18) / period;
+    return blocks < kWarps ? (period > 8192 ? 1 : kWarps) : blocks;
+}
+template <typename S>
+__device__ __forceinline__ void hist_unit(const HistEntry& e, long long unit, int bins, bool pow2, unsigned int* hist, float* red) {
+    const float scale = 0.5f * static_cast<float>(bins);
+    const int last_bin = bins - 1;
+    const S* values = static_cast<const S*>(e.values);
+    const long long per = hist_unit_blocks(e.period), first = unit * per;
+    const long long end = first + per < e.nb ? first + per : e.nb;
+    const int lane = threadIdx.x & 31;
+    auto count_scalar = [&](const S* gb, float absmax, int index, int stride) {
+        for (long long i = index; i < e.period; i += stride) {
+            const float v = ScalarIO<S>::load(gb + i);
+            float x = 0.0f;
+            if (absmax > 0.0f) x = v / absmax;
+            int bin = static_cast<int>(floorf((x + 1.0f) * scale));
+            bin = bin < 0 ? 0 : (bin > last_bin ? last_bin : bin);
+            atomicAdd(&hist[bin], 1u);
+        }
+    };
+    if (e.period > 8192) {   // the whole CTA on one block at a time
+        for (long long b = first; b < end; ++b) {
+            const S* gb = values + b * e.period;
+            const float absmax = block_absmax<S, kThreads>(gb, e.period, threadIdx.x, red);
+            count_scalar(gb, absmax, threadIdx.x, kThreads);
+        }
+        return;
+    }
+    for (long long b = first + (threadIdx.x >> 5); b < end; b += kWarps) {
+        const S* gb = values + b * e.period;
+        if (!e.vec) {
+            count_scalar(gb, block_absmax<S, 32>(gb, e.period, lane, red), lane, 32);
+            continue;
+        }
+        if constexpr (sizeof(S) < 8) {   // as histogram_kernel's vector form
+            const int nchunks = static_cast<int>(e.period >> 3);
+            float m = 0.0f;
+            for (int c = lane; c < nchunks; c += 32) m = absmax8<S>(gb + 8 * c, m);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+            const BlockDivider divide(m);
+            auto second_look = [&](auto quotient) {
+                for (int c = lane; c < nchunks; c += 32) {
+                    float f[8];
+                    load8<S>(gb + 8 * c, f);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const float x = quotient(f[i]);
+                        const float y = pow2 ? fmaf(x, scale, scale) : (x + 1.0f) * scale;
+                        atomicAdd(&hist[__float2uint_rz(y)], 1u);
+                    }
+                }
+            };
+            if (divide.fast) second_look([&](float v) { return divide.quick(v); });
+            else second_look([&](float v) { return divide.careful(v); });
+        }
+    }
+}
+__global__ void __launch_bounds__(kThreads) histogram_many_kernel(const HistEntry* __restrict__ table, int n, long long units, int bins,
+                                                                  unsigned long long* __restrict__ rows) {
+    __shared__ unsigned int hist[4096 + 1];
+    __shared__ float red[kWarps];
+    const bool pow2 = (bins & (bins - 1)) == 0 && bins >= 2;
+    for (long long u = blockIdx.x; u < units; u += gridDim.x) {
+        int lo = 0, hi = n - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (table[mid].first_unit <= u) lo = mid; else hi = mid - 1;
+        }
+        const HistEntry& e = table[lo];
+        for (int i = threadIdx.x; i <= bins; i += kThreads) hist[i] = 0u;
+        __syncthreads();
+        switch (e.dtype) {
+            case GEFEN_B200_F32: hist_unit<float>(e, u - e.first_unit, bins, pow2, hist, red); break;
+            case GEFEN_B200_F16: hist_unit<__half>(e, u - e.first_unit, bins, pow2, hist, red); break;
+            case GEFEN_B200_BF16: hist_unit<__nv_bfloat16>(e, u - e.first_unit, bins, pow2, hist, red); break;
+            default: hist_unit<double>(e, u - e.first_unit, bins, pow2, hist, red); break;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) { hist[bins - 1] += hist[bins]; hist[bins] = 0u; }   // x == 1, see histogram_kernel
+        __syncthreads();
+        unsigned long long* row = rows + static_cast<long long>(lo) * bins;
+        for (int i = threadIdx.x; i < bins; i += kThreads)
+            if (hist[i]) atomicAdd(&row[i], static_cast<unsigned long long>(hist[i]));
+        __syncthreads();
+    }
+}
+__global__ void __launch_bounds__(kThreads) histogram_total_kernel(const long long* __restrict__ rows, int n, int bins, float* __restrict__ total) {
+    const int i = blockIdx.x * kThreads + threadIdx.x;
+    if (i >= bins) return;
+    float t = 0.0f;
+    for (int r = 0; r < n; ++r) t += static_cast<float>(rows[static_cast<long long>(r) * bins + i]);
+    total[i] = t;
+}
+
 // ------------------------------------------------------------------------------- period scores
 // Sum over one block of log(x + eps) in fp64, x = v*v in fp64 unless the input is already squared
 // (reference: period_variance_kernel.cu:124-139). `invalid` counts non-positive log inputs.
@@ -968,6 +1073,50 @@ int gefen_b200_exact_histogram(const void* grad_flat, int grad_dtype, int64_t nu
     }
     GEFEN_CHECK_CUDA(cudaGetLastError());
     return GEFEN_B200_OK;
+}
+
+int64_t gefen_b200_exact_histogram_many_table_bytes(int n_tensors) {
+    return n_tensors > 0 ? static_cast<int64_t>(n_tensors) * static_cast<int64_t>(sizeof(HistEntry)) : 0;
+}
+
+int gefen_b200_exact_histogram_many(int n_tensors, const uint64_t* values, const int32_t* dtypes, const int64_t* numels,
+                                    const int64_t* periods, int64_t* rows, float* total, int histogram_bins, void* device_table,
+                                    void* stream_) {
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+    GEFEN_CHECK_ARG(n_tensors >= 1 && values && dtypes && numels && periods && rows && total && device_table, "Expected non-null arguments.");
+    GEFEN_CHECK_ARG(histogram_bins >= 1 && histogram_bins <= 4096, "Expected histogram size in [1, 4096].");
+    GEFEN_CHECK_ARG(aligned16(device_table), "Expected a 16-byte aligned table.");
+    try {
+        std::vector<HistEntry> table(n_tensors);
+        int64_t units = 0;
+        for (int t = 0; t < n_tensors; ++t) {
+            HistEntry& e = table[t];
+            e.values = reinterpret_cast<const void*>(static_cast<uintptr_t>(values[t]));
+            const int rc = check_flat(e.values, dtypes[t], numels[t], periods[t]);
+            if (rc != GEFEN_B200_OK) return rc;
+            e.period = periods[t];
+            e.nb = numels[t] / periods[t];
+            e.dtype = dtypes[t];
+            e.vec = e.period % 8 == 0 && aligned16(e.values) && e.dtype != GEFEN_B200_F64;
+            e.first_unit = units;
+            units += (e.nb + hist_unit_blocks(e.period) - 1) / hist_unit_blocks(e.period);
+            GEFEN_CHECK_ARG(e.period <= 0x7fffffffll, "Period %lld is too large.", static_cast<long long>(e.period));
+        }
+        GEFEN_CHECK_CUDA(cudaMemsetAsync(rows, 0, sizeof(int64_t) * histogram_bins * n_tensors, stream));
+        GEFEN_CHECK_CUDA(cudaMemcpyAsync(device_table, table.data(), sizeof(HistEntry) * n_tensors, cudaMemcpyHostToDevice, stream));
+        if (units > 0) {
+            const int grid = static_cast<int>(std::min<int64_t>(units, static_cast<int64_t>(sm_count()) * 6));
+            histogram_many_kernel<<<grid, kThreads, 0, stream>>>(static_cast<const HistEntry*>(device_table), n_tensors, units, histogram_bins,
+                                                                 reinterpret_cast<unsigned long long*>(rows));
+            GEFEN_CHECK_CUDA(cudaGetLastError());
+        }
+        histogram_total_kernel<<<(histogram_bins + kThreads - 1) / kThreads, kThreads, 0, stream>>>(
+            reinterpret_cast<const long long*>(rows), n_tensors, histogram_bins, total);
+        GEFEN_CHECK_CUDA(cudaGetLastError());
+        return GEFEN_B200_OK;
+    } catch (const std::bad_alloc&) {
+        return fail(GEFEN_B200_ERUNTIME, "Out of host memory for the histogram table.");
+    }
 }
 
 int gefen_b200_average_within_block_variance(const void* values, int dtype, int64_t numel, int64_t period,

@@ -84,23 +84,16 @@ def learn_gefen_exact_codebook_from_grad_periods(*, grad_periods, codebook_devic
     """One global codebook from the gradients of all tensors (reference :305-419).
 
     Each tensor's exact int64 histogram is produced on the GPU into its own row; the rows are
-    fetched with one copy and accumulated on the host in float32 in parameter order, which is the
-    reference's arithmetic (:331, :347). The codebook is then the exact-DP fit of the active bins.
+    added up there in float32 in parameter order, which is the reference's arithmetic (:331, :347). The codebook is then the exact-DP fit of the active bins.
     """
     items = [(flat, period) for _, flat, period, _ in grad_periods]
     if not items:
         return None
-    from .kernels.exact_histogram_fused import gefen_exact_histogram_cuda
+    from .kernels.exact_histogram_fused import gefen_exact_histogram_many_cuda
 
     bins = num_codebooks * 16
     device = items[0][0].device
-    rows = torch.zeros((len(items), bins), dtype=torch.int64, device=device)
-    for row, (flat, period) in zip(rows, items):
-        gefen_exact_histogram_cuda(flat, period, row)
-    rows_host = rows.cpu()
-    bin_counts = torch.zeros(bins, dtype=torch.float32)
-    for row in rows_host:
-        bin_counts.add_(row.to(torch.float32))
+    bin_counts = gefen_exact_histogram_many_cuda([flat for flat, _ in items], [period for _, period in items], bins).cpu()
 
     edges = torch.linspace(-1.0, 1.0, steps=bins + 1, dtype=torch.float32)
     centers = 0.5 * (edges[:-1] + edges[1:])

@@ -2,6 +2,7 @@
 (reference: kernels/exact_histogram_fused.py:10-58)."""
 from __future__ import annotations
 
+import numpy as np
 import torch
 
 from .. import _lib
@@ -31,3 +32,28 @@ def gefen_exact_histogram_cuda(grad_flat: torch.Tensor, period: int, bin_counts:
         _lib.check(_lib.load().gefen_b200_exact_histogram(
             _lib.ptr(grad_flat), _lib.dtype_tag(grad_flat.dtype), grad_flat.numel(), int(period),
             _lib.ptr(bin_counts), bin_counts.numel(), _lib.current_stream(grad_flat.device)))
+
+
+def gefen_exact_histogram_many_cuda(grads_flat, periods, histogram_bins: int) -> torch.Tensor:
+    """The float32 sum, in the given order, of the histograms of many contiguous 1-D gradients on one device, each
+    converted to float32 first: one launch for all of them. Device tensor [histogram_bins]."""
+    device = grads_flat[0].device
+    require_cuda_tensors({"grad_flat {}".format(i): g for i, g in enumerate(grads_flat)})
+    for g, period in zip(grads_flat, periods):
+        if period <= 0 or g.numel() % period != 0:
+            raise ValueError("Expected grad_flat.numel()={} to be divisible by period={}.".format(g.numel(), period))
+    n = len(grads_flat)
+    grads_flat = [g.contiguous() for g in grads_flat]
+    lib = _lib.load()
+    values = np.array([g.data_ptr() for g in grads_flat], dtype=np.uint64)
+    dtypes = np.array([_lib.dtype_tag(g.dtype) for g in grads_flat], dtype=np.int32)
+    numels = np.array([g.numel() for g in grads_flat], dtype=np.int64)
+    lengths = np.array(periods, dtype=np.int64)
+    rows = torch.empty((n, histogram_bins), dtype=torch.int64, device=device)
+    total = torch.empty(histogram_bins, dtype=torch.float32, device=device)
+    table = torch.empty(lib.gefen_b200_exact_histogram_many_table_bytes(n), dtype=torch.uint8, device=device)
+    with _lib.device_guard(device):
+        _lib.check(lib.gefen_b200_exact_histogram_many(
+            n, values.ctypes.data, dtypes.ctypes.data, numels.ctypes.data, lengths.ctypes.data, _lib.ptr(rows),
+            _lib.ptr(total), int(histogram_bins), _lib.ptr(table), _lib.current_stream(device)))
+    return total

@@ -217,6 +217,14 @@ int gefen_b200_debug_set_stage_spin_limit(int64_t limit);
 int gefen_b200_exact_histogram(const void* grad_flat, int grad_dtype, int64_t numel,
                                int64_t period, int64_t* bin_counts, int histogram_bins,
                                void* stream);
+/* The histograms of many tensors in one launch: rows[t * bins + b] = counts of tensor t (set, not added to), total[b] =
+ * float32 sum of the rows in the order of the tensors, each converted to float32 first (the reference's accumulation,
+ * gefen.py:331, :347). values, dtypes, numels, periods: host arrays; rows, total: device; device_table: table_bytes
+ * bytes of device scratch. */
+int64_t gefen_b200_exact_histogram_many_table_bytes(int n_tensors);
+int gefen_b200_exact_histogram_many(int n_tensors, const uint64_t* values, const int32_t* dtypes,
+                                    const int64_t* numels, const int64_t* periods, int64_t* rows,
+                                    float* total, int histogram_bins, void* device_table, void* stream);
 
 /* Replace average_within_block_variance_cuda, average_within_block_coefficient_of_variation_cuda
  * and average_adjacent_log_block_mean_difference_cuda (gefen_cuda_binding.cpp:71-88;
