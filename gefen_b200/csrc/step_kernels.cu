@@ -37,6 +37,7 @@
 
 #include <mutex>
 #include <stdlib.h>
+#include <string.h>
 
 namespace gefen {
 
@@ -54,7 +55,7 @@ __device__ __forceinline__ float ema_update_period1(float beta, float cur, float
 }
 
 struct StepLaunch {
-    const gefen_b200_step_tensor_t* table;  // device table, or nullptr: the row in the kernel params
+    const gefen_b200_step_tensor_t* table;  // device table, or nullptr: the rows in the kernel params
     int n_tensors;
     int stage_floats;                       // fast path: floats of staging per warp (>= max period)
     long long total_blocks;
@@ -84,6 +85,14 @@ struct StepLaunch {
     // host only: the launch before this one belongs to the same step (see let_successor_in)
     int follows;
 };
+
+// Descriptors that travel with the launch itself: a call of up to this many tensors needs no copy of its table to the
+// device (kernel parameters hold 4 KB; the copy costs the host about 5 us and the GPU a launch gap).
+constexpr int kParamRows = 24;
+struct StepRows {
+    gefen_b200_step_tensor_t row[kParamRows];
+};
+static_assert(sizeof(StepRows) + sizeof(StepLaunch) <= 4096, "kernel parameter space");
 
 // Set (never cleared by a kernel) when a bounded wait ran out and the CTA left without doing its
 // share of the step: bit 0 = the table staging of a step kernel, bit 1 = its shared-memory layout does not fit. Read and cleared by
@@ -1123,7 +1132,7 @@ constexpr int kVecThreads = 512;
 // its own loop structure.
 template <typename S, int V, int GSRC, bool FULL>
 __global__ void __launch_bounds__(kVecThreads, 1) step_vec_kernel(const __grid_constant__ StepLaunch L,
-                                                                  const __grid_constant__ gefen_b200_step_tensor_t single) {
+                                                                  const __grid_constant__ StepRows rows) {
     SmemView s;
     let_successor_in();
     if (smem_u32(g_smem) > kFixed) {   // (static variables have outgrown their share: nothing is done, the status says so)
@@ -1132,7 +1141,7 @@ __global__ void __launch_bounds__(kVecThreads, 1) step_vec_kernel(const __grid_c
         return;
     }
     if (!stage_tables(L.ws, fast_smem(kWsAt), s, L.spin_limit)) { wait_for_predecessor(); return; }
-    const gefen_b200_step_tensor_t* table = L.table != nullptr ? L.table : &single;
+    const gefen_b200_step_tensor_t* table = L.table != nullptr ? L.table : rows.row;
 
     const int lane = threadIdx.x & 31;
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
@@ -1188,13 +1197,13 @@ constexpr int kWarps = kThreads / 32;
 
 template <typename S, int GROUP>
 __global__ void __launch_bounds__(kThreads) step_generic_kernel(const __grid_constant__ StepLaunch L,
-                                                                const __grid_constant__ gefen_b200_step_tensor_t single) {
+                                                                const __grid_constant__ StepRows rows) {
     __shared__ float red_max[kWarps];
     __shared__ float red_sum[kWarps];
     SmemView s;
     let_successor_in();
     if (!stage_tables(L.ws, g_smem, s, L.spin_limit)) { wait_for_predecessor(); return; }
-    const gefen_b200_step_tensor_t* table = L.table != nullptr ? L.table : &single;
+    const gefen_b200_step_tensor_t* table = L.table != nullptr ? L.table : rows.row;
 
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -1353,10 +1362,10 @@ constexpr int kVectorMost = 256;
 constexpr int kVectorThreads = 128;
 template <typename S>
 __global__ void __launch_bounds__(kVectorThreads) step_vector_kernel(const __grid_constant__ StepLaunch L,
-                                                                     const __grid_constant__ gefen_b200_step_tensor_t single) {
+                                                                     const __grid_constant__ StepRows rows) {
     constexpr int E = kVectorMost / 32;
     let_successor_in();
-    const gefen_b200_step_tensor_t* table = L.table != nullptr ? L.table : &single;
+    const gefen_b200_step_tensor_t* table = L.table != nullptr ? L.table : rows.row;
     const int lane = threadIdx.x & 31;
     const long long gb = static_cast<long long>(blockIdx.x) * (kVectorThreads / 32) + (threadIdx.x >> 5);
     const bool active = gb < L.total_blocks;
@@ -1557,7 +1566,7 @@ constexpr unsigned int kDefaultStageSpinLimit = 4000000u;
 static unsigned int g_stage_spin_limit = kDefaultStageSpinLimit;
 
 template <typename K>
-static int launch_step(K kernel, int grid, int threads, int smem, const StepLaunch& L, const gefen_b200_step_tensor_t& single,
+static int launch_step(K kernel, int grid, int threads, int smem, const StepLaunch& L, const StepRows& rows,
                        cudaStream_t stream) {
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3(static_cast<unsigned>(grid));
@@ -1571,12 +1580,12 @@ static int launch_step(K kernel, int grid, int threads, int smem, const StepLaun
         config.attrs = &overlap;
         config.numAttrs = 1;
     }
-    GEFEN_CHECK_CUDA(cudaLaunchKernelEx(&config, kernel, L, single));
+    GEFEN_CHECK_CUDA(cudaLaunchKernelEx(&config, kernel, L, rows));
     return GEFEN_B200_OK;
 }
 
 template <typename S, int V, int GSRC, bool FULL>
-static int launch_vec_variant(StepLaunch L, const gefen_b200_step_tensor_t& single, long long max_unit, cudaStream_t stream) {
+static int launch_vec_variant(StepLaunch L, const StepRows& rows, long long max_unit, cudaStream_t stream) {
     static bool configured[kMaxDevices];
     auto kernel = step_vec_kernel<S, V, GSRC, FULL>;
     {
@@ -1604,30 +1613,30 @@ static int launch_vec_variant(StepLaunch L, const gefen_b200_step_tensor_t& sing
     if (ctas_per_sm < 1) ctas_per_sm = 1;
     L.stage_floats = static_cast<int>(stage_bytes / 4);
     const int grid = grid_for(L.total_blocks, warps, ctas_per_sm);
-    return launch_step(kernel, grid, warps * 32, smem, L, single, stream);
+    return launch_step(kernel, grid, warps * 32, smem, L, rows, stream);
 }
 
 template <typename S>
-static int launch_vec(int cls, StepLaunch L, const gefen_b200_step_tensor_t& single, long long max_unit, cudaStream_t stream) {
-    if (cls == 3) return launch_vec_variant<S, 4, 0, false>(L, single, max_unit, stream);
-    if (cls == 4) return launch_vec_variant<S, 2, 0, false>(L, single, max_unit, stream);
-    if (cls == 5) return launch_vec_variant<S, 1, 0, false>(L, single, max_unit, stream);
+static int launch_vec(int cls, StepLaunch L, const StepRows& rows, long long max_unit, cudaStream_t stream) {
+    if (cls == 3) return launch_vec_variant<S, 4, 0, false>(L, rows, max_unit, stream);
+    if (cls == 4) return launch_vec_variant<S, 2, 0, false>(L, rows, max_unit, stream);
+    if (cls == 5) return launch_vec_variant<S, 1, 0, false>(L, rows, max_unit, stream);
     if (cls == 6) {
         constexpr int kPer = kVectorThreads / 32;
-        return launch_step(step_vector_kernel<S>, static_cast<int>((L.total_blocks + kPer - 1) / kPer), kVectorThreads, kSmemWs, L, single, stream);
+        return launch_step(step_vector_kernel<S>, static_cast<int>((L.total_blocks + kPer - 1) / kPer), kVectorThreads, kSmemWs, L, rows, stream);
     }
     if (cls == 1) {
-        if (L.grad_mc_delta != 0) return launch_vec_variant<S, 8, 2, true>(L, single, max_unit, stream);
-        if (L.n_grad_srcs > 0) return launch_vec_variant<S, 8, 1, true>(L, single, max_unit, stream);
-        return launch_vec_variant<S, 8, 0, true>(L, single, max_unit, stream);
+        if (L.grad_mc_delta != 0) return launch_vec_variant<S, 8, 2, true>(L, rows, max_unit, stream);
+        if (L.n_grad_srcs > 0) return launch_vec_variant<S, 8, 1, true>(L, rows, max_unit, stream);
+        return launch_vec_variant<S, 8, 0, true>(L, rows, max_unit, stream);
     }
-    if (L.grad_mc_delta != 0) return launch_vec_variant<S, 8, 2, false>(L, single, max_unit, stream);
-    if (L.n_grad_srcs > 0) return launch_vec_variant<S, 8, 1, false>(L, single, max_unit, stream);
-    return launch_vec_variant<S, 8, 0, false>(L, single, max_unit, stream);
+    if (L.grad_mc_delta != 0) return launch_vec_variant<S, 8, 2, false>(L, rows, max_unit, stream);
+    if (L.n_grad_srcs > 0) return launch_vec_variant<S, 8, 1, false>(L, rows, max_unit, stream);
+    return launch_vec_variant<S, 8, 0, false>(L, rows, max_unit, stream);
 }
 
 template <typename S>
-static int launch_generic(bool cta_per_block, const StepLaunch& L, const gefen_b200_step_tensor_t& single,
+static int launch_generic(bool cta_per_block, const StepLaunch& L, const StepRows& rows,
                           cudaStream_t stream) {
     constexpr int smem = kSmemWs;
     static bool configured[kMaxDevices];
@@ -1643,9 +1652,9 @@ static int launch_generic(bool cta_per_block, const StepLaunch& L, const gefen_b
         }
     }
     if (cta_per_block) {
-        return launch_step(step_generic_kernel<S, 256>, grid_for(L.total_blocks, 1, 3), kThreads, smem, L, single, stream);
+        return launch_step(step_generic_kernel<S, 256>, grid_for(L.total_blocks, 1, 3), kThreads, smem, L, rows, stream);
     }
-    return launch_step(step_generic_kernel<S, 32>, grid_for(L.total_blocks, kWarps, 3), kThreads, smem, L, single, stream);
+    return launch_step(step_generic_kernel<S, 32>, grid_for(L.total_blocks, kWarps, 3), kThreads, smem, L, rows, stream);
 }
 
 // Class of a tensor: 1 = staged path in chunks of eight with whole-warp blocks, 2 = the same with several blocks
@@ -1675,19 +1684,19 @@ static long long class_units(const gefen_b200_step_tensor_t& t, int cls, int dty
     return paired ? (t.num_blocks + 1) / 2 : t.num_blocks;
 }
 
-static int launch_class(int cls, int dtype, const StepLaunch& L, const gefen_b200_step_tensor_t& single,
+static int launch_class(int cls, int dtype, const StepLaunch& L, const StepRows& rows,
                         long long max_unit, cudaStream_t stream) {
     if (cls >= 1) {
-        if (dtype == GEFEN_B200_BF16) return launch_vec<__nv_bfloat16>(cls, L, single, max_unit, stream);
-        if (dtype == GEFEN_B200_F16) return launch_vec<__half>(cls, L, single, max_unit, stream);
-        return launch_vec<float>(cls, L, single, max_unit, stream);
+        if (dtype == GEFEN_B200_BF16) return launch_vec<__nv_bfloat16>(cls, L, rows, max_unit, stream);
+        if (dtype == GEFEN_B200_F16) return launch_vec<__half>(cls, L, rows, max_unit, stream);
+        return launch_vec<float>(cls, L, rows, max_unit, stream);
     }
     const bool cta = cls < 0;
     switch (dtype) {
-        case GEFEN_B200_F32: return launch_generic<float>(cta, L, single, stream);
-        case GEFEN_B200_F16: return launch_generic<__half>(cta, L, single, stream);
-        case GEFEN_B200_BF16: return launch_generic<__nv_bfloat16>(cta, L, single, stream);
-        case GEFEN_B200_F64: return launch_generic<double>(cta, L, single, stream);
+        case GEFEN_B200_F32: return launch_generic<float>(cta, L, rows, stream);
+        case GEFEN_B200_F16: return launch_generic<__half>(cta, L, rows, stream);
+        case GEFEN_B200_BF16: return launch_generic<__nv_bfloat16>(cta, L, rows, stream);
+        case GEFEN_B200_F64: return launch_generic<double>(cta, L, rows, stream);
     }
     return fail(GEFEN_B200_EINVAL, "Unsupported parameter dtype tag %d.", dtype);
 }
@@ -1726,7 +1735,9 @@ static int run_single(gefen_b200_step_tensor_t& t, int param_dtype, const float*
     L.param_mc_delta = 0;
     L.spin_limit = g_stage_spin_limit;
     L.follows = 0;
-    return launch_class(cls, param_dtype, L, t, cls >= 1 && cls <= 5 ? unit_floats(t.period, class_chunk(cls), dtype_size(param_dtype)) : t.period, stream);
+    StepRows rows = {};
+    rows.row[0] = t;
+    return launch_class(cls, param_dtype, L, rows, cls >= 1 && cls <= 5 ? unit_floats(t.period, class_chunk(cls), dtype_size(param_dtype)) : t.period, stream);
 }
 
 }  // namespace gefen
@@ -2063,8 +2074,15 @@ int gefen_b200_multi_tensor_step_multicast(gefen_b200_step_tensor_t* host_table,
         host_table[begin].reserved_[1] = end - begin;  // run length, read back below
         begin = end;
     }
-    GEFEN_CHECK_CUDA(cudaMemcpyAsync(device_table, host_table, sizeof(gefen_b200_step_tensor_t) * n_tensors,
-                                     cudaMemcpyHostToDevice, stream));
+    // Few tensors: their descriptors go with the launches. Not while the stream is being captured: a replay of the graph
+    // reads the host table again, as it did before.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    GEFEN_CHECK_CUDA(cudaStreamIsCapturing(stream, &capture));
+    const bool in_params = n_tensors <= kParamRows && capture == cudaStreamCaptureStatusNone;
+    if (!in_params)
+        GEFEN_CHECK_CUDA(cudaMemcpyAsync(device_table, host_table, sizeof(gefen_b200_step_tensor_t) * n_tensors,
+                                         cudaMemcpyHostToDevice, stream));
+    StepRows rows = {};
     bool launched = false;
     for (int begin = 0; begin < n_tensors;) {
         const int run = host_table[begin].reserved_[1];
@@ -2078,7 +2096,8 @@ int gefen_b200_multi_tensor_step_multicast(gefen_b200_step_tensor_t* host_table,
         }
         if (total > 0) {
             StepLaunch L;
-            L.table = static_cast<const gefen_b200_step_tensor_t*>(device_table) + begin;
+            L.table = in_params ? nullptr : static_cast<const gefen_b200_step_tensor_t*>(device_table) + begin;
+            if (in_params) memcpy(rows.row, host_table + begin, sizeof(gefen_b200_step_tensor_t) * run);
             L.n_tensors = run;
             L.stage_floats = 0;
             L.total_blocks = total;
@@ -2094,7 +2113,7 @@ int gefen_b200_multi_tensor_step_multicast(gefen_b200_step_tensor_t* host_table,
             L.spin_limit = g_stage_spin_limit;
             L.follows = launched && n_peers == 0 && n_grad_srcs == 0;
             launched = true;
-            const int rc = launch_class(host_table[begin].reserved_[0], param_dtype, L, host_table[begin], max_period, stream);
+            const int rc = launch_class(host_table[begin].reserved_[0], param_dtype, L, rows, max_period, stream);
             if (rc != GEFEN_B200_OK) return rc;
         }
         begin += run;
