@@ -141,16 +141,16 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
 
 // Tile t of the persistent schedule: row-major over the tiles that are computed (all of them, or for
 // a symmetric result those that reach the upper triangle: n0 + bn > m0).
-__host__ __device__ inline bool tile_coords(int M, int N, int bn, int symmetric, long long t, int* m0, int* n0) {
-    const int tiles_m = (M + kBM - 1) / kBM, tiles_n = (N + bn - 1) / bn;
+__host__ __device__ inline bool tile_coords(int M, int N, int bm, int bn, int symmetric, long long t, int* m0, int* n0) {
+    const int tiles_m = (M + bm - 1) / bm, tiles_n = (N + bn - 1) / bn;
     if (!symmetric) {
         if (t >= static_cast<long long>(tiles_m) * tiles_n) return false;
-        *m0 = static_cast<int>(t / tiles_n) * kBM;
+        *m0 = static_cast<int>(t / tiles_n) * bm;
         *n0 = static_cast<int>(t % tiles_n) * bn;
         return true;
     }
     for (int mi = 0; mi < tiles_m; ++mi) {
-        const int row0 = mi * kBM;
+        const int row0 = mi * bm;
         const int first = row0 >= bn ? (row0 - bn) / bn + 1 : 0;
         const int cnt = tiles_n - first;
         if (t < cnt) {
@@ -179,6 +179,136 @@ struct TileView {
     int M, N, K, m0, n0;
     long long ldc, ldd;
 };
+// Stores one accumulator of 128 rows from row m0 and BN columns from column t.n0: alpha, beta * C, bf16, and the mirror
+// image of a symmetric result. Four warps; warp w owns TMEM lanes (rows) 32w .. 32w+31. `wait` returns when the
+// accumulator is complete (false: given up).
+template <int BN, typename Wait>
+__device__ __forceinline__ bool epilogue_tile(const GemmArgs& args, const TileView& t, int m0, uint32_t tmem_acc, int warp, int lane, Wait wait) {
+    const int n0 = t.n0;
+        const int row = m0 + warp * 32 + lane;
+        const bool row_ok = row < t.M;
+        // C does not depend on the accumulators: the first chunk's row segment is fetched while the main
+        // loop runs, and chunk j+1's while chunk j is converted and stored.
+        const bool use_c = row_ok && args.beta != 0.0f;
+        const __nv_bfloat16* crow_base = use_c ? t.c + static_cast<long long>(row) * t.ldc : nullptr;
+        const bool c_vec = use_c && ((reinterpret_cast<uintptr_t>(crow_base) & 15u) == 0) && (t.ldc % 8 == 0) && (n0 % 8 == 0);
+        uint4 cnext[4];
+        auto fetch_c = [&](int j) {
+            const int col0 = n0 + j * 32;
+            if (c_vec && col0 + 32 <= t.N) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) cnext[q] = reinterpret_cast<const uint4*>(crow_base + col0)[q];
+            }
+        };
+        fetch_c(0);
+        const bool ok = wait();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (!ok) return false;
+        {
+#pragma unroll 2
+            for (int j = 0; j < BN / 32; ++j) {
+                uint32_t r[32];
+                const uint32_t taddr = tmem_acc + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(j * 32);
+                asm volatile(
+                    "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+                    "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+                    "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+                    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                      "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+                      "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+                      "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+                    : "r"(taddr)
+                    : "memory");
+                uint4 ccur[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) ccur[q] = cnext[q];
+                if (j + 1 < BN / 32) fetch_c(j + 1);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                const int col0 = n0 + j * 32;
+                if (col0 >= t.N) continue;
+                const bool full_cols = col0 + 32 <= t.N;
+                float v[32];
+#pragma unroll
+                for (int i = 0; i < 32; ++i) v[i] = args.alpha * __uint_as_float(r[i]);
+                if (use_c) {
+                    const __nv_bfloat16* crow = crow_base + col0;
+                    if (full_cols && c_vec) {
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const uint4 raw = ccur[q];
+                            const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                v[q * 8 + 2 * e] = fmaf(args.beta, __uint_as_float(w[e] << 16), v[q * 8 + 2 * e]);
+                                v[q * 8 + 2 * e + 1] = fmaf(args.beta, __uint_as_float(w[e] & 0xFFFF0000u), v[q * 8 + 2 * e + 1]);
+                            }
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i)
+                            if (col0 + i < t.N) v[i] = fmaf(args.beta, __bfloat162float(crow[i]), v[i]);
+                    }
+                }
+                if (row_ok) {
+                    __nv_bfloat16* drow = t.d + static_cast<long long>(row) * t.ldd + col0;
+                    if (args.symmetric && col0 < row) {
+                        // chunk crosses or lies left of the diagonal: only the elements with column >= row
+#pragma unroll
+                        for (int i = 0; i < 32; ++i)
+                            if (col0 + i < t.N && col0 + i >= row) drow[i] = __float2bfloat16_rn(v[i]);
+                    } else if (full_cols && ((reinterpret_cast<uintptr_t>(drow) & 15u) == 0)) {
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            uint32_t w[4];
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                const __nv_bfloat162 h = __floats2bfloat162_rn(v[q * 8 + 2 * e], v[q * 8 + 2 * e + 1]);
+                                w[e] = *reinterpret_cast<const uint32_t*>(&h);
+                            }
+                            reinterpret_cast<uint4*>(drow)[q] = make_uint4(w[0], w[1], w[2], w[3]);
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i)
+                            if (col0 + i < t.N) drow[i] = __float2bfloat16_rn(v[i]);
+                    }
+                    if (args.dt != nullptr) {
+                        // transposed copy: for a fixed column the lanes of a warp write consecutive addresses
+#pragma unroll
+                        for (int i = 0; i < 32; ++i)
+                            if (col0 + i < t.N)
+                                args.dt[static_cast<long long>(col0 + i) * args.lddt + row] = __float2bfloat16_rn(v[i]);
+                    }
+                }
+                if (args.symmetric) {
+                    // mirror: element (row, c) with c > row also goes to (c, row)
+                    const int warp_row0 = m0 + warp * 32;
+                    if (col0 > warp_row0 + 31 && warp_row0 + 31 < t.M && full_cols) {
+                        // the whole chunk is right of every row of this warp (warp-uniform): lanes pair up so
+                        // that each store carries two consecutive rows of one column (4 bytes)
+                        const bool odd = (lane & 1) != 0;
+#pragma unroll
+                        for (int i = 0; i < 32; i += 2) {
+                            const float send = odd ? v[i] : v[i + 1];
+                            const float recv = __shfl_xor_sync(0xffffffffu, send, 1);
+                            const float lo = odd ? recv : v[i];          // value of the even row
+                            const float hi = odd ? v[i + 1] : recv;      // value of the odd row
+                            const int c = col0 + i + (odd ? 1 : 0);
+                            const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+                            *reinterpret_cast<__nv_bfloat162*>(t.d + static_cast<long long>(c) * t.ldd + (row & ~1)) = h;
+                        }
+                    } else if (row_ok && col0 + 31 > row) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i)
+                            if (col0 + i < t.N && col0 + i > row)
+                                t.d[static_cast<long long>(col0 + i) * t.ldd + row] = __float2bfloat16_rn(v[i]);
+                    }
+                }
+            }
+        }
+    return true;
+}
+
 template <int BN, int STAGES, bool A_MN, bool B_MN, bool PERSIST, bool GROUP = false>
 __global__ void __launch_bounds__(kGemmThreads, (STAGES * (kBM + BN) * kBK * 2 <= 96 * 1024) ? 2 : 1) ns_gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a,
                                                                      const __grid_constant__ CUtensorMap map_b,
@@ -227,7 +357,7 @@ __global__ void __launch_bounds__(kGemmThreads, (STAGES * (kBM + BN) * kBK * 2 <
             t.n0 = blockIdx.x * BN;
             return li == 0;
         }
-        return index < args.n_tiles && tile_coords(args.M, args.N, BN, args.symmetric, index, &t.m0, &t.n0);
+        return index < args.n_tiles && tile_coords(args.M, args.N, kBM, BN, args.symmetric, index, &t.m0, &t.n0);
     };
 
     if (threadIdx.x == 0) {
@@ -333,129 +463,11 @@ __global__ void __launch_bounds__(kGemmThreads, (STAGES * (kBM + BN) * kBK * 2 <
         // ---------------- epilogue: warp w owns TMEM lanes (rows) 32w .. 32w+31
         TileView t;
         for (int li = 0; my_tile(li, t); ++li) {
-        const int m0 = t.m0, n0 = t.n0;
         const int buf = PERSIST ? (li & 1) : 0;
-        const int row = m0 + warp * 32 + lane;
-        const bool row_ok = row < t.M;
-        // C does not depend on the accumulators: the first chunk's row segment is fetched while the main
-        // loop runs, and chunk j+1's while chunk j is converted and stored.
-        const bool use_c = row_ok && args.beta != 0.0f;
-        const __nv_bfloat16* crow_base = use_c ? t.c + static_cast<long long>(row) * t.ldc : nullptr;
-        const bool c_vec = use_c && ((reinterpret_cast<uintptr_t>(crow_base) & 15u) == 0) && (t.ldc % 8 == 0) && (n0 % 8 == 0);
-        uint4 cnext[4];
-        auto fetch_c = [&](int j) {
-            const int col0 = n0 + j * 32;
-            if (c_vec && col0 + 32 <= t.N) {
-#pragma unroll
-                for (int q = 0; q < 4; ++q) cnext[q] = reinterpret_cast<const uint4*>(crow_base + col0)[q];
-            }
-        };
-        fetch_c(0);
-        const bool ok = wait_or_abort(&acc_full[buf], PERSIST ? ((li >> 1) & 1) : 0, &abort_flag);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (!ok || abort_flag) break;
-        {
-#pragma unroll 2
-            for (int j = 0; j < BN / 32; ++j) {
-                uint32_t r[32];
-                const uint32_t taddr = tmem_base + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(buf * BN + j * 32);
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                    "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-                    "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-                    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                      "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-                      "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-                      "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-                    : "r"(taddr)
-                    : "memory");
-                uint4 ccur[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) ccur[q] = cnext[q];
-                if (j + 1 < BN / 32) fetch_c(j + 1);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                const int col0 = n0 + j * 32;
-                if (col0 >= t.N) continue;
-                const bool full_cols = col0 + 32 <= t.N;
-                float v[32];
-#pragma unroll
-                for (int i = 0; i < 32; ++i) v[i] = args.alpha * __uint_as_float(r[i]);
-                if (use_c) {
-                    const __nv_bfloat16* crow = crow_base + col0;
-                    if (full_cols && c_vec) {
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            const uint4 raw = ccur[q];
-                            const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                v[q * 8 + 2 * e] = fmaf(args.beta, __uint_as_float(w[e] << 16), v[q * 8 + 2 * e]);
-                                v[q * 8 + 2 * e + 1] = fmaf(args.beta, __uint_as_float(w[e] & 0xFFFF0000u), v[q * 8 + 2 * e + 1]);
-                            }
-                        }
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            if (col0 + i < t.N) v[i] = fmaf(args.beta, __bfloat162float(crow[i]), v[i]);
-                    }
-                }
-                if (row_ok) {
-                    __nv_bfloat16* drow = t.d + static_cast<long long>(row) * t.ldd + col0;
-                    if (args.symmetric && col0 < row) {
-                        // chunk crosses or lies left of the diagonal: only the elements with column >= row
-#pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            if (col0 + i < t.N && col0 + i >= row) drow[i] = __float2bfloat16_rn(v[i]);
-                    } else if (full_cols && ((reinterpret_cast<uintptr_t>(drow) & 15u) == 0)) {
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            uint32_t w[4];
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                const __nv_bfloat162 h = __floats2bfloat162_rn(v[q * 8 + 2 * e], v[q * 8 + 2 * e + 1]);
-                                w[e] = *reinterpret_cast<const uint32_t*>(&h);
-                            }
-                            reinterpret_cast<uint4*>(drow)[q] = make_uint4(w[0], w[1], w[2], w[3]);
-                        }
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            if (col0 + i < t.N) drow[i] = __float2bfloat16_rn(v[i]);
-                    }
-                    if (args.dt != nullptr) {
-                        // transposed copy: for a fixed column the lanes of a warp write consecutive addresses
-#pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            if (col0 + i < t.N)
-                                args.dt[static_cast<long long>(col0 + i) * args.lddt + row] = __float2bfloat16_rn(v[i]);
-                    }
-                }
-                if (args.symmetric) {
-                    // mirror: element (row, c) with c > row also goes to (c, row)
-                    const int warp_row0 = m0 + warp * 32;
-                    if (col0 > warp_row0 + 31 && warp_row0 + 31 < t.M && full_cols) {
-                        // the whole chunk is right of every row of this warp (warp-uniform): lanes pair up so
-                        // that each store carries two consecutive rows of one column (4 bytes)
-                        const bool odd = (lane & 1) != 0;
-#pragma unroll
-                        for (int i = 0; i < 32; i += 2) {
-                            const float send = odd ? v[i] : v[i + 1];
-                            const float recv = __shfl_xor_sync(0xffffffffu, send, 1);
-                            const float lo = odd ? recv : v[i];          // value of the even row
-                            const float hi = odd ? v[i + 1] : recv;      // value of the odd row
-                            const int c = col0 + i + (odd ? 1 : 0);
-                            const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
-                            *reinterpret_cast<__nv_bfloat162*>(t.d + static_cast<long long>(c) * t.ldd + (row & ~1)) = h;
-                        }
-                    } else if (row_ok && col0 + 31 > row) {
-#pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            if (col0 + i < t.N && col0 + i > row)
-                                t.d[static_cast<long long>(col0 + i) * t.ldd + row] = __float2bfloat16_rn(v[i]);
-                    }
-                }
-            }
-        }
+        const bool ok = epilogue_tile<BN>(args, t, t.m0, tmem_base + static_cast<uint32_t>(buf * BN), warp, lane, [&]() {
+            return wait_or_abort(&acc_full[buf], PERSIST ? ((li >> 1) & 1) : 0, &abort_flag) && !abort_flag;
+        });
+        if (!ok) break;
         if (PERSIST) {   // this warp has read its rows of the buffer: one arrival per warp
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
@@ -470,6 +482,326 @@ __global__ void __launch_bounds__(kGemmThreads, (STAGES * (kBM + BN) * kBK * 2 <
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
     }
     if (threadIdx.x == 0 && abort_flag && args.status != nullptr) atomicExch(args.status, 1);
+}
+
+// --------------------------------------------------------------------------- pairs of CTAs
+// The grouped products on pairs of SMs: tcgen05.mma.cta_group::2 on tiles of 256 x 256. Each CTA stages its 128 rows of A
+// and its half of B's 256 columns (32 KB per 64 k instead of 48 KB for the 128 x 256 tile of a single CTA, whose
+// operand stream the L2 cannot feed at the tensor cores' rate) and holds its 128 rows of the accumulator in its own TMEM.
+// The first CTA's thread issues the products and the commits; "slot full" barriers live in the first CTA (both CTAs'
+// copies complete on them), "slot free" and "accumulator full" arrive in both, "accumulator drained" in the first.
+// Products of 28 Qwen3-1.7B-shaped matrices (6.83 TFLOP): 6.43 ms with 128 x 256 tiles, 6.04 on pairs, 5.55 with the
+// epilogue through shared memory = 1230 TFLOP/s, 0.88 of the measured sustained rate; what is left is the tensor
+// cores at the clock that the power limit leaves. 24 matrices of a 768-wide transformer: 0.85 -> 0.74 ms.
+// Every wait gives up after kPairWaitCycles; the roles then leave, a grace period lets copies in flight land, and the
+// CTAs part at a cluster barrier that all their threads reach.
+constexpr int kPairStages = 6;
+constexpr int kPairBN = 256;
+constexpr long long kPairWaitCycles = 1000000000ll;   // about half a second
+
+__device__ __forceinline__ uint32_t cluster_address(const void* local, uint32_t rank) {
+    uint32_t out;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(smem_u32(local)), "r"(rank));
+    return out;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ bool pair_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+    const uint32_t addr = smem_u32(bar);
+    const long long begin = clock64();
+    for (uint32_t it = 1;; ++it) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(addr), "r"(parity)
+            : "memory");
+        if (done) return true;
+        if ((it & 15u) == 0u && (*abort_flag || clock64() - begin > kPairWaitCycles)) break;
+    }
+    *abort_flag = 1;
+    return false;
+}
+__device__ __forceinline__ void pair_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+            smem_u32(dst)),
+        "l"(map), "r"(x), "r"(y), "r"(bar)
+        : "memory");
+}
+__device__ __forceinline__ void pair_commit(uint64_t* bar) {   // arrives on this barrier of both CTAs
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+                 "h"(static_cast<uint16_t>(3))
+                 : "memory");
+}
+
+// The same through shared memory, 64 columns at a time: a row of the accumulator belongs to a lane, so that direct loads
+// of C and stores of D touch 32 rows with 16 bytes each per instruction, which costs the memory pipe as much time as a
+// product of 2048 k takes; here an instruction moves four rows of 128 bytes. `stage`: this warp's 32 rows of
+// kStagePitch elements. C and D: 16-byte aligned rows, N a multiple of 8 (groups guarantee both).
+constexpr int kStagePitch = 72;
+__device__ __forceinline__ void tmem_load32(uint32_t taddr, uint32_t* r) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr)
+        : "memory");
+}
+template <int BN, typename Wait>
+__device__ __forceinline__ bool epilogue_tile_staged(const GemmArgs& args, const TileView& t, int m0, uint32_t tmem_acc, int warp, int lane,
+                                                     __nv_bfloat16* stage, Wait wait) {
+    const int row0 = m0 + warp * 32, row = row0 + lane;
+    const bool use_c = args.beta != 0.0f;
+    const int piece_row = lane >> 3, piece_col = (lane & 7) * 8;   // of the coalesced accesses: four rows of 128 bytes each
+    uint4 cnext[8];
+    auto fetch_c = [&](int col0) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int r = row0 + 4 * q + piece_row, c = col0 + piece_col;
+            if (r < t.M && c < t.N) cnext[q] = *reinterpret_cast<const uint4*>(t.c + static_cast<long long>(r) * t.ldc + c);
+        }
+    };
+    if (use_c) fetch_c(t.n0);
+    if (!wait()) return false;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    __nv_bfloat16* const own = stage + lane * kStagePitch;
+    for (int j = 0; j < BN / 64; ++j) {
+        const int col0 = t.n0 + 64 * j;
+        if (col0 >= t.N) break;
+        uint32_t r[64];
+        const uint32_t taddr = tmem_acc + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(j * 64);
+        tmem_load32(taddr, r);
+        tmem_load32(taddr + 32, r + 32);
+        if (use_c) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) *reinterpret_cast<uint4*>(stage + (4 * q + piece_row) * kStagePitch + piece_col) = cnext[q];
+            if (j + 1 < BN / 64) fetch_c(col0 + 64);
+            __syncwarp();
+        }
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        float v[64];
+#pragma unroll
+        for (int i = 0; i < 64; ++i) v[i] = args.alpha * __uint_as_float(r[i]);
+        if (use_c) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const uint4 raw = *reinterpret_cast<const uint4*>(own + 8 * q);
+                const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    v[q * 8 + 2 * e] = fmaf(args.beta, __uint_as_float(w[e] << 16), v[q * 8 + 2 * e]);
+                    v[q * 8 + 2 * e + 1] = fmaf(args.beta, __uint_as_float(w[e] & 0xFFFF0000u), v[q * 8 + 2 * e + 1]);
+                }
+            }
+        }
+        // (a lane overwrites its own row of C only: no other lane reads it any more)
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            uint32_t w[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const __nv_bfloat162 h = __floats2bfloat162_rn(v[q * 8 + 2 * e], v[q * 8 + 2 * e + 1]);
+                w[e] = *reinterpret_cast<const uint32_t*>(&h);
+            }
+            *reinterpret_cast<uint4*>(own + 8 * q) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int rr = row0 + 4 * q + piece_row, c = col0 + piece_col;
+            if (rr >= t.M || c >= t.N) continue;
+            const __nv_bfloat16* from = stage + (4 * q + piece_row) * kStagePitch + piece_col;
+            __nv_bfloat16* to = t.d + static_cast<long long>(rr) * t.ldd + c;
+            if (!args.symmetric || c >= rr) {
+                *reinterpret_cast<uint4*>(to) = *reinterpret_cast<const uint4*>(from);
+            } else {   // crosses or lies left of the diagonal: only the elements with column >= row
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                    if (c + e >= rr) to[e] = from[e];
+            }
+        }
+        if (args.symmetric) {
+            // mirror: element (row, c) with c > row also goes to (c, row)
+            if (col0 > row0 + 31 && row0 + 31 < t.M && col0 + 64 <= t.N) {
+                // the whole chunk is right of every row of this warp (warp-uniform): lanes pair up so that each store
+                // carries two consecutive rows of one column (4 bytes)
+                const bool odd = (lane & 1) != 0;
+#pragma unroll
+                for (int i = 0; i < 64; i += 2) {
+                    const float send = odd ? v[i] : v[i + 1];
+                    const float recv = __shfl_xor_sync(0xffffffffu, send, 1);
+                    const float lo = odd ? recv : v[i];          // value of the even row
+                    const float hi = odd ? v[i + 1] : recv;      // value of the odd row
+                    const int c = col0 + i + (odd ? 1 : 0);
+                    const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+                    *reinterpret_cast<__nv_bfloat162*>(t.d + static_cast<long long>(c) * t.ldd + (row & ~1)) = h;
+                }
+            } else if (row < t.M && col0 + 63 > row) {
+#pragma unroll
+                for (int i = 0; i < 64; ++i)
+                    if (col0 + i < t.N && col0 + i > row) t.d[static_cast<long long>(col0 + i) * t.ldd + row] = __float2bfloat16_rn(v[i]);
+            }
+        }
+        __syncwarp();   // the stage is free for the next 64 columns
+    }
+    return true;
+}
+
+template <bool B_MN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1) ns_gemm_pair_kernel(const __grid_constant__ GemmArgs args) {
+    constexpr int kABytes = kBM * kBK * 2;            // this CTA's rows of A
+    constexpr int kBBytes = kPairBN / 2 * kBK * 2;    // and its half of B
+    constexpr int kStageBytes = kABytes + kBBytes;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+    __shared__ uint64_t full_bar[kPairStages];    // first CTA: operands of both CTAs have arrived
+    __shared__ uint64_t empty_bar[kPairStages];   // each CTA: its slot has been read
+    __shared__ uint64_t acc_full[2];              // each CTA: accumulator complete
+    __shared__ uint64_t acc_empty[2];             // first CTA: drained by the eight epilogue warps of the pair
+    __shared__ uint32_t tmem_slot;
+    __shared__ int abort_flag;
+
+    // (behind the ring of slots: the epilogue warps' stages)
+    __nv_bfloat16* const stages = reinterpret_cast<__nv_bfloat16*>(smem + kPairStages * kStageBytes);
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    uint32_t rank;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    const int pair_index = static_cast<int>(blockIdx.x >> 1), pairs = static_cast<int>(gridDim.x >> 1);
+    auto my_tile = [&](int li, TileView& t) -> bool {
+        const long long index = static_cast<long long>(pair_index) + static_cast<long long>(li) * pairs;
+        if (index >= args.n_tiles) return false;
+        const GroupTile g = args.tiles[index];
+        const GroupEntry* e = args.entries + g.entry;
+        t.map_a = &e->a;
+        t.map_b = &e->b;
+        t.c = e->c;
+        t.d = e->d;
+        t.M = e->M; t.N = e->N; t.K = e->K;
+        t.ldc = e->ldc; t.ldd = e->ldd;
+        t.m0 = g.m0; t.n0 = g.n0;
+        return true;
+    };
+
+    if (threadIdx.x == 0) {
+        abort_flag = 0;
+        for (int s = 0; s < kPairStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 8); }
+        fence_mbar_init();
+    }
+    if (warp == 5) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(2 * kPairBN) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    cluster_sync_all();   // both CTAs' barriers exist before either signals the other's
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem_base = tmem_slot;
+
+    if (warp == 4) {
+        // ---------------- producer of this CTA's operands
+        if (lane == 0) {
+            uint32_t it = 0;
+            bool ok = true;
+            TileView t;
+            for (int li = 0; ok && my_tile(li, t); ++li) {
+                const int m0 = t.m0 + static_cast<int>(rank) * kBM, n0 = t.n0 + static_cast<int>(rank) * (kPairBN / 2);
+                const int k_blocks = (t.K + kBK - 1) / kBK;
+                asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(t.map_a) : "memory");
+                asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(t.map_b) : "memory");
+                for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+                    const int s = it % kPairStages;
+                    if (!pair_wait(&empty_bar[s], ((it / kPairStages) & 1) ^ 1, &abort_flag)) { ok = false; break; }
+                    if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * kStageBytes);
+                    const uint32_t bar = cluster_address(&full_bar[s], 0);
+                    unsigned char* a_dst = smem + s * kStageBytes;
+                    pair_load_2d(a_dst, t.map_a, kb * kBK, m0, bar);
+                    if (!B_MN) {
+                        pair_load_2d(a_dst + kABytes, t.map_b, kb * kBK, n0, bar);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < kPairBN / 2 / 64; ++j)   // 64 K-rows x 64 N-columns per box
+                            pair_load_2d(a_dst + kABytes + j * (kBK * 128), t.map_b, n0 + 64 * j, kb * kBK, bar);
+                    }
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == 5) {
+        // ---------------- MMA issuer of the pair
+        if (lane == 0 && rank == 0) {
+            constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (B_MN ? (1u << 16) : 0u) |
+                                       (static_cast<uint32_t>(kPairBN >> 3) << 17) | (static_cast<uint32_t>(2 * kBM >> 4) << 24);
+            bool ok = true;
+            uint32_t it = 0;
+            TileView t;
+            for (int li = 0; ok && my_tile(li, t); ++li) {
+                const int k_blocks = (t.K + kBK - 1) / kBK;
+                const int buf = li & 1;
+                const uint32_t tmem_acc = tmem_base + static_cast<uint32_t>(buf * kPairBN);
+                ok = pair_wait(&acc_empty[buf], ((li >> 1) & 1) ^ 1, &abort_flag);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+                    const int s = it % kPairStages;
+                    ok = pair_wait(&full_bar[s], (it / kPairStages) & 1, &abort_flag);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t a_addr = smem_u32(smem + s * kStageBytes);
+                    const uint64_t desc_a = umma_desc_k_major_sw128(a_addr);
+                    const uint64_t desc_b = B_MN ? umma_desc_mn_major_sw128(a_addr + kABytes, kBK * 128) : umma_desc_k_major_sw128(a_addr + kABytes);
+#pragma unroll
+                    for (int k = 0; k < kBK / 16; ++k) {
+                        asm volatile(
+                            "{\n\t.reg .pred p;\n\t"
+                            "setp.ne.b32 p, %4, 0;\n\t"
+                            "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                            ::"r"(tmem_acc), "l"(desc_a + 2 * k), "l"(desc_b + (B_MN ? 128 : 2) * k), "r"(idesc), "r"((kb > 0 || k > 0) ? 1u : 0u)
+                            : "memory");
+                    }
+                    pair_commit(&empty_bar[s]);   // the slot is free in both CTAs once these products have read it
+                }
+                if (ok) pair_commit(&acc_full[buf]);
+            }
+        }
+        __syncwarp();
+    } else {
+        // ---------------- epilogue of this CTA's rows
+        TileView t;
+        for (int li = 0; my_tile(li, t); ++li) {
+            const int buf = li & 1;
+            const bool ok = epilogue_tile_staged<kPairBN>(args, t, t.m0 + static_cast<int>(rank) * kBM, tmem_base + static_cast<uint32_t>(buf * kPairBN),
+                                                          warp, lane, stages + warp * 32 * kStagePitch,
+                                                          [&]() { return pair_wait(&acc_full[buf], (li >> 1) & 1, &abort_flag); });
+            if (!ok) break;
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_address(&acc_empty[buf], 0)) : "memory");
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    }
+    __syncthreads();
+    if (abort_flag) {   // given up: copies and products in flight get time to end before their memory goes
+        const long long begin = clock64();
+        while (clock64() - begin < 4000000ll) __nanosleep(1000);
+    }
+    cluster_sync_all();
+    if (warp == 5) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * kPairBN) : "memory");
+    }
+    if (threadIdx.x == 0 && abort_flag && args.status != nullptr) atomicExch(args.status, 1);
+    cluster_sync_all();   // (neither CTA's TMEM permits or shared memory go before the other is done with the pair)
 }
 
 // ------------------------------------------------------------------------------- host side
@@ -507,12 +839,12 @@ static int make_map(CUtensorMap* map, const void* base, long long rows, long lon
 }
 
 // Tiles a launch computes (see tile_coords).
-static int count_tiles(int M, int N, int bn, int symmetric) {
-    const int tiles_m = (M + kBM - 1) / kBM, tiles_n = (N + bn - 1) / bn;
+static int count_tiles(int M, int N, int bm, int bn, int symmetric) {
+    const int tiles_m = (M + bm - 1) / bm, tiles_n = (N + bn - 1) / bn;
     if (!symmetric) return tiles_m * tiles_n;
     int total = 0;
     for (int mi = 0; mi < tiles_m; ++mi) {
-        const int row0 = mi * kBM;
+        const int row0 = mi * bm;
         total += tiles_n - (row0 >= bn ? (row0 - bn) / bn + 1 : 0);
     }
     return total;
@@ -529,7 +861,7 @@ static int launch_gemm_variant(const CUtensorMap& ma, const CUtensorMap& mb, Gem
         GEFEN_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         configured[dev] = true;
     }
-    if (!GROUP) args.n_tiles = count_tiles(args.M, args.N, BN, args.symmetric);
+    if (!GROUP) args.n_tiles = count_tiles(args.M, args.N, kBM, BN, args.symmetric);
     dim3 grid(GROUP ? 1 : (args.N + BN - 1) / BN, GROUP ? 1 : (args.M + kBM - 1) / kBM);
     if (PERSIST) grid = dim3(args.n_tiles < sm_count() ? args.n_tiles : sm_count(), 1);
     kernel<<<grid, kGemmThreads, smem, stream>>>(ma, mb, args);
@@ -547,7 +879,7 @@ static int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const GemmA
         const char* e = getenv("GEFEN_B200_NS_PERSIST");
         forced = e == nullptr ? -1 : (e[0] == '0' ? 0 : 1);
     }
-    bool persist = count_tiles(args.M, args.N, BN, args.symmetric) > sm_count();
+    bool persist = count_tiles(args.M, args.N, kBM, BN, args.symmetric) > sm_count();
     if (forced >= 0) persist = forced == 1;
     if constexpr (STAGES * (kBM + BN) * kBK * 2 > 96 * 1024) {   // the two-CTAs-per-SM variants stay one tile per CTA
         if (persist) return launch_gemm_variant<BN, STAGES, A_MN, B_MN, true>(ma, mb, args, stream);
@@ -749,7 +1081,7 @@ extern "C" int gefen_b200_ns_gemm_tt(const void* a, const void* b, const void* c
 // the last wave is paid once per product instead of once per matrix and product, and so that the host enqueues
 // 3 * steps + 3 launches instead of that many per matrix. Measured, whole GefenMuon steps: 24 matrices of a 768-wide
 // transformer 3.86 -> 1.25 ms, four matrices of 64 to 1026 rows 0.61 -> 0.27 ms, 28 Qwen3-1.7B-shaped matrices
-// 9.5 -> 8.3 ms (there the products themselves, 1060 TFLOP/s, are what is left). Tall matrices enter transposed (Y^T Y = X X^T for X = Y^T), so
+// 9.5 -> 8.3 ms (7.6 ms on pairs of CTAs). Tall matrices enter transposed (Y^T Y = X X^T for X = Y^T), so
 // every product has one of two forms: A * B^T with both operands K-major, or A * B with B MN-major.
 namespace gefen {
 
@@ -976,7 +1308,7 @@ __global__ void __launch_bounds__(kElemThreads) ns_apply_kernel(const NsMatrix* 
 // The plan of a group: five lists of products (Gram matrix of x0 / of x1, polynomial, update x0 -> x1 / x1 -> x0) and
 // two lists of tiles (of the symmetric m x m results, of the m x k results).
 struct GroupShape {
-    int bn;
+    int bm, bn;            // 256 x 256: pairs of CTAs
     int64_t gram_tiles, update_tiles, entries_bytes, bytes;
 };
 static void wide_dims(const NsMatrix& m, int* wr, int* wc) {
@@ -986,16 +1318,20 @@ static void wide_dims(const NsMatrix& m, int* wr, int* wc) {
 }
 static GroupShape group_shape(const NsMatrix* mats, int n) {
     GroupShape g;
-    for (g.bn = 256;; g.bn = 128) {
+    // Tiles of 256 x 256 on pairs of CTAs have the best ratio of operand bytes to work, 128 x 256 the next; where a
+    // kind does not fill the GPU the next smaller one is taken (measurements: see launch_group)
+    static const int kinds[3][2] = {{256, 256}, {128, 256}, {128, 128}};
+    for (int kind = 0; kind < 3; ++kind) {
+        g.bm = kinds[kind][0];
+        g.bn = kinds[kind][1];
         g.gram_tiles = g.update_tiles = 0;
         for (int i = 0; i < n; ++i) {
             int m, k;
             wide_dims(mats[i], &m, &k);
-            g.gram_tiles += count_tiles(m, m, g.bn, 1);
-            g.update_tiles += count_tiles(m, k, g.bn, 0);
+            g.gram_tiles += count_tiles(m, m, g.bm, g.bn, 1);
+            g.update_tiles += count_tiles(m, k, g.bm, g.bn, 0);
         }
-        // tiles of 128 x 256 have the better ratio of operand bytes to work; where they do not fill the SMs, 128 x 128
-        if (g.bn == 128 || g.gram_tiles >= sm_count()) break;
+        if (g.gram_tiles * (g.bm / kBM) >= sm_count()) break;
     }
     g.entries_bytes = static_cast<int64_t>(5) * n * static_cast<int64_t>(sizeof(GroupEntry));
     g.bytes = g.entries_bytes + (g.gram_tiles + g.update_tiles) * static_cast<int64_t>(sizeof(GroupTile));
@@ -1052,14 +1388,30 @@ static int build_group_plan(const NsMatrix* mats, int n, const GroupShape& g, st
         fill(3, poly, x_mn[0], mat.x0, mat.x1, k, m);
         fill(4, poly, x_mn[1], mat.x1, mat.x0, k, m);
         int m0, n0;
-        for (int64_t t = 0; tile_coords(m, m, g.bn, 1, t, &m0, &n0); ++t) gram_tiles[gt++] = {i, m0, n0, 0};
-        for (int64_t t = 0; tile_coords(m, k, g.bn, 0, t, &m0, &n0); ++t) update_tiles[ut++] = {i, m0, n0, 0};
+        for (int64_t t = 0; tile_coords(m, m, g.bm, g.bn, 1, t, &m0, &n0); ++t) gram_tiles[gt++] = {i, m0, n0, 0};
+        for (int64_t t = 0; tile_coords(m, k, g.bm, g.bn, 0, t, &m0, &n0); ++t) update_tiles[ut++] = {i, m0, n0, 0};
     }
     return GEFEN_B200_OK;
 }
 
 template <bool B_MN>
 static int launch_group(const GroupShape& g, GemmArgs args, cudaStream_t stream) {
+    if (g.bm == 256) {
+        constexpr int smem = kPairStages * (kBM + kPairBN / 2) * kBK * 2 + 4 * 32 * kStagePitch * 2 + 1024;
+        static std::once_flag configured[64];
+        int dev = 0;
+        GEFEN_CHECK_CUDA(cudaGetDevice(&dev));
+        GEFEN_CHECK_ARG(dev >= 0 && dev < 64, "Unsupported device ordinal %d.", dev);
+        cudaError_t err = cudaSuccess;
+        std::call_once(configured[dev], [&] {
+            err = cudaFuncSetAttribute(ns_gemm_pair_kernel<B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        });
+        GEFEN_CHECK_CUDA(err);
+        const int pairs = std::min(args.n_tiles, sm_count() / 2);
+        ns_gemm_pair_kernel<B_MN><<<2 * pairs, kGemmThreads, smem, stream>>>(args);
+        GEFEN_CHECK_CUDA(cudaGetLastError());
+        return GEFEN_B200_OK;
+    }
     const CUtensorMap none = {};
     if (g.bn == 256) return launch_gemm_variant<256, 4, false, B_MN, true, true>(none, none, args, stream);
     return launch_gemm_variant<128, 6, false, B_MN, true, true>(none, none, args, stream);

@@ -52,3 +52,31 @@ def test_runs_of_a_group():
     assert ns.group_runs("aab", [1, 2, 3]) == [(0, 2), (2, 3)]
     assert ns.group_runs("aaaa", [cap, 1, cap - 1, 1]) == [(0, 1), (1, 3), (3, 4)]
     assert ns.group_runs("aa", [2 * cap, 2 * cap]) == [(0, 1), (1, 2)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shapes", [
+    [(2048, 2304), (2048, 2048), (2056, 2120)],                                   # 256 x 256 tiles on pairs, ragged edges
+    [(768, 3072)] * 5 + [(3072, 768)] * 5 + [(768, 768), (776, 1000), (200, 900), (8, 16)] * 2,
+])
+def test_groups_that_fill_the_gpu(cuda_device, shapes):
+    """Enough tiles for pairs of CTAs: every matrix against torch's chain and, up to a bf16 rounding of a few elements
+    whose sums are added up in another order, against the same matrix alone (smaller tiles, single CTAs)."""
+    from gefen_b200 import newton_schulz as ns
+
+    gen = torch.Generator(device=cuda_device).manual_seed(7)
+    grads = [(torch.randn(s, generator=gen, device=cuda_device) * 1e-3).bfloat16() for s in shapes]
+    group = ns.MatrixGroup(shapes, torch.full((ns.group_scratch_elements(shapes),), float("nan"), dtype=torch.bfloat16, device=cuda_device))
+    group.run(grads, NS, 5, 1e-7)
+    ns.check_status(cuda_device)
+    for i, g in enumerate(grads):
+        got = group.result(i).float()
+        x = g / g.norm().clamp(min=1e-7)
+        x = x.T if g.shape[0] > g.shape[1] else x
+        for _ in range(5):
+            gram = x @ x.T
+            x = torch.addmm(x, torch.addmm(gram, gram, gram, beta=NS[1], alpha=NS[2]), x, beta=NS[0])
+        want = (x.T if g.shape[0] > g.shape[1] else x).float()
+        assert float((got - want).norm() / want.norm()) <= 2e-2, shapes[i]
+        alone = ns.zeropower_via_newtonschulz(g, NS, 5, 1e-7).float()
+        assert float((got - alone).norm() / alone.norm()) <= 1e-2, shapes[i]
