@@ -439,7 +439,7 @@ def run_gpu_arm(args, cfg, rank, world, local_rank):
                           "unit": "GB/s", "frac": achieved / peak,
                           "traffic": ratio * vec_bytes if ratio is not None else None,
                           "algorithmic_bytes_per_launch": vec_bytes, "launch_ms": vec_ms}
-    result["launches_per_step"] = len(set(cls))
+    result["launches_per_step"] = len({lib.gefen_b200_step_launch_class(rows[r:r + 1].ctypes.data, table["tag"]) for r in range(len(rows))})
 
     # ---- end to end through the public API with HOST buffers: gradients come from pinned host
     # memory every step and the updated parameters go back to pinned host memory
@@ -535,6 +535,22 @@ def ns_flops(shape, steps=5):
     return steps * (4 * m * m * n + 2 * m ** 3)
 
 
+def muon_launches(numels) -> int:
+    """Launches of this library's kernels in one GefenMuon step: per chunk of the momentum scratch two step kernels (its
+    two kinds of blocks), per group of matrices norm, normalisation, three products per iteration and the update."""
+    from gefen_b200 import gefen_muon, newton_schulz as ns
+
+    chunks, cur, total = [], [], 0
+    for n in numels:
+        if cur and total + n > gefen_muon.MOMENTUM_CHUNK_ELEMENTS:
+            chunks.append(cur)
+            cur, total = [], 0
+        cur.append(n)
+        total += n
+    chunks += [cur] if cur else []
+    return sum(2 + (3 * 5 + 3) * len(ns.group_runs([0] * len(c), c)) for c in chunks)
+
+
 def run_muon_sharded_arm(args, cfg, rank, world, local_rank):
     """GefenMuon with whole matrices assigned to the ranks (Zero1GefenMuon): reduce-scatter of the
     gradients, GefenMuon on the owned matrices, all-gather of the parameters."""
@@ -578,7 +594,7 @@ def run_muon_sharded_arm(args, cfg, rank, world, local_rank):
                    "weight_decay": cfg["wd"], "matrices": len(shapes), "elements": elems,
                    "parallelism": "zero1-dp{} (whole matrices per rank)".format(world)},
         "calibration_first_step_ms": calibration_ms, "clocks": clocks, "breakdown_ms": breakdown, "n_vs_1": n_vs_1,
-        "gpu_launches": args.steps * (owned * 15 + 8),
+        "gpu_launches": args.steps * muon_launches([elems // max(1, len(shapes))] * owned),   # (matrices of average size)
     }))
 
 
@@ -637,7 +653,7 @@ def measure_muon(cfg, steps: int, warmup: int):
     peak = json.loads(peak_file.read_text())["bf16_tflops_sustained"] if peak_file.exists() else 1400.0
     achieved = total_flops / results["tcgen05"] / 1e9
     elems = sum(workloads.numel(s) for _, s in shapes)
-    roofline = {"bound": "tensor", "kernel": "ns_gemm_tn_kernel", "achieved": achieved, "peak": peak,
+    roofline = {"bound": "tensor", "kernel": "ns_gemm_pair_kernel", "achieved": achieved, "peak": peak,
                 "peak_kind": "measured cuBLAS bf16, sustained", "unit": "TFLOP/s", "frac": achieved / peak,
                 "traffic": None, "algorithmic_flops_per_step": total_flops,
                 "newton_schulz_ms": results["tcgen05"],
@@ -661,7 +677,7 @@ def run_muon_arm(args, cfg):
                    "weight_decay": cfg["wd"], "matrices": len(m["shapes"]), "elements": m["elements"]},
         "calibration_first_step_ms": m["calibration_ms"], "clocks": m["clocks"],
         "roofline": m["roofline"],
-        "gpu_launches": args.steps * (len(m["shapes"]) * 15 + 8),
+        "gpu_launches": args.steps * muon_launches([workloads.numel(s) for _, s in m["shapes"]]),
     }
     print(json.dumps(line))
 
