@@ -25,6 +25,7 @@ import torch.nn as nn
 from . import _lib
 from . import partitioning
 from . import quantization
+from .kernels._common import require_one_device
 
 F_FP32 = False              # force fp32 optimizer state regardless of the gradient dtype (reference :18, :53-69)
 NUM_CODEBOOK_ENTRIES = 256  # reference :937
@@ -229,6 +230,7 @@ class Gefen(torch.optim.Optimizer):
         for name, p, grad in todo:
             if grad.device.type != "cuda":
                 raise ValueError("gefen_b200 needs CUDA gradients, got device {} for {}".format(grad.device, name))
+        require_one_device("the gradients of one optimizer", [grad for _, _, grad in todo])
         found, stats = partitioning.launch_period_scores_many([grad for _, _, grad in todo])
         host = torch.cat([s.cpu() for s in stats], dim=0) if stats else None
         periods, cursor = [], 0

@@ -14,6 +14,13 @@ def require_cuda_tensors(tensors: dict) -> None:
             raise ValueError("Expected {} to be on CUDA, got device {}.".format(name, tensor.device))
 
 
+def require_one_device(what: str, tensors) -> None:
+    """A kernel reads all of them through plain pointers on the device of the first."""
+    devices = sorted({str(t.device) for t in tensors})
+    if len(devices) > 1:
+        raise ValueError("Expected {} to be on one device, got {}.".format(what, ", ".join(devices)))
+
+
 def require_contiguous(tensors: dict) -> None:
     for name, tensor in tensors.items():
         if not tensor.is_contiguous():

@@ -6,12 +6,13 @@ import numpy as np
 import torch
 
 from .. import _lib
-from ._common import require_cuda_tensors
+from ._common import require_cuda_tensors, require_one_device
 
 
 def gefen_exact_histogram_cuda(grad_flat: torch.Tensor, period: int, bin_counts: torch.Tensor) -> None:
     """bin_counts[b] += number of elements whose g/absmax(block) falls in bin b; int64, added to."""
     require_cuda_tensors({"grad_flat": grad_flat, "bin_counts": bin_counts})
+    require_one_device("grad_flat and bin_counts", (grad_flat, bin_counts))
     if grad_flat.dim() != 1:
         raise ValueError("Expected grad_flat to be 1D, got dim={}".format(grad_flat.dim()))
     if bin_counts.dim() != 1:
@@ -38,6 +39,7 @@ def gefen_exact_histogram_many_cuda(grads_flat, periods, histogram_bins: int) ->
     """The float32 sum, in the given order, of the histograms of many contiguous 1-D gradients on one device, each
     converted to float32 first: one launch for all of them. Device tensor [histogram_bins]."""
     device = grads_flat[0].device
+    require_one_device("the gradients of one histogram", grads_flat)
     require_cuda_tensors({"grad_flat {}".format(i): g for i, g in enumerate(grads_flat)})
     for g, period in zip(grads_flat, periods):
         if period <= 0 or g.numel() % period != 0:

@@ -200,3 +200,18 @@ def test_kernel_class_of_a_table_row():
     assert cls(2048, flags=_lib.STEP_PACKED) == 0
     assert cls(2048, p=0x10008) == 0 and cls(2048, g=0x20002) == 0 and cls(2048, codes=0x30004) == 0
     assert cls(2048, _lib.F64) == 0
+
+
+def test_tensors_of_two_devices_are_refused():
+    """One launch reads all tensors of a calibration through plain pointers: gradients on two devices raise on the host,
+    before any launch. (Stand-ins with a device and a size: nothing here touches a GPU.)"""
+    from types import SimpleNamespace
+
+    from gefen_b200 import Gefen
+    from gefen_b200.kernels.exact_histogram_fused import gefen_exact_histogram_many_cuda
+
+    grads = [SimpleNamespace(device=torch.device("cuda", i), numel=lambda: 64) for i in (0, 1)]
+    with pytest.raises(ValueError, match="one device"):
+        gefen_exact_histogram_many_cuda(grads, [8, 8], 4096)
+    with pytest.raises(ValueError, match="one device"):
+        Gefen._predict_periods(None, [("a", None, grads[0]), ("b", None, grads[1])])
