@@ -395,9 +395,11 @@ __global__ void adjacent_diff_final_kernel(const double* __restrict__ partial, i
 // factors neither overflow nor underflow, other values take their own logarithm). One rounding of 2^-53 per factor is
 // less than what adding up logarithms of about -25 costs (2^-49 per term). Two double-precision operations per
 // element remain, and the tensor is read once per base instead of a double per element written and read back.
-struct LogProduct {
+// An element moves the exponent by at most 128: 32 bits (E = int) hold it for blocks below kCtaPeriod, the longer blocks
+// count in 64 (zeros in fp32 with eps = 1e-12 leave 32 bits at 430 M elements per block).
+template <typename E> struct LogProduct {
     double mantissa, slow;
-    int exponent;
+    E exponent;
     __device__ __forceinline__ LogProduct() : mantissa(1.0), slow(0.0), exponent(0) {}
     __device__ __forceinline__ void split() {
         const int hi = __double2hiint(mantissa);
@@ -467,6 +469,7 @@ constexpr int kGroupPeriod = 512;       // shorter ones: eight lanes each; longe
                                         // whole warps spent most of their time on the warp's reduction and logarithm:
                                         // the scan of 383 M bf16 elements 2.06 -> 1.63 ms),
 constexpr int kCtaPeriod = 16384;       // from here on one CTA
+static_assert(128ll * kCtaPeriod < (1ll << 31), "a 32-bit exponent holds the product of a shorter block");
 // Blocks of one unit of work (a CTA's turn).
 __host__ __device__ inline long long base_unit_blocks(long long period) {
     if (period < kThreadPeriod) return 2 * kThreads;
@@ -477,9 +480,9 @@ __host__ __device__ inline long long base_unit_blocks(long long period) {
 template <typename S> __device__ __forceinline__ float scan_value(const S* p) { return ScalarIO<S>::load(p); }
 
 // The product over elements first, first + stride, ... (stride counted in elements; VEC: runs of eight) of one block.
-template <typename S, bool SQUARED>
+template <typename S, bool SQUARED, typename E>
 __device__ __forceinline__ void block_product(const S* v, long long period, int index, int count, bool vec, double eps, bool eps_ok,
-                                              LogProduct& p, unsigned long long& invalid) {
+                                              LogProduct<E>& p, unsigned long long& invalid) {
     if constexpr (sizeof(S) == 8) {
         for (long long i = index; i < period; i += count) p.slow += log_term<S, SQUARED>(v + i, eps, invalid);
     } else {
@@ -510,7 +513,7 @@ __device__ __forceinline__ void scan_base_unit(const ScanBase& b, long long unit
         for (int r = 0; r < 2; ++r) {
             const long long j = first + r * kThreads + threadIdx.x;
             if (j >= b.nb) return;
-            LogProduct p;
+            LogProduct<int> p;
             block_product<S, SQUARED>(values + j * period, period, 0, 1, b.vec != 0, eps, eps_ok, p, invalid);
             sums[j] = p.value();
         }
@@ -518,7 +521,7 @@ __device__ __forceinline__ void scan_base_unit(const ScanBase& b, long long unit
         const long long end = first + base_unit_blocks(period) < b.nb ? first + base_unit_blocks(period) : b.nb;
         for (long long j0 = first; j0 < end; j0 += kThreads / 8) {   // uniform over the CTA: the groups shuffle together
             const long long j = j0 + (threadIdx.x >> 3);
-            LogProduct p;
+            LogProduct<int> p;
             if (j < end) block_product<S, SQUARED>(values + j * period, period, threadIdx.x & 7, 8, b.vec != 0, eps, eps_ok, p, invalid);
             p.template combine<8>();
             if (j < end && (threadIdx.x & 7) == 0) sums[j] = p.value();
@@ -527,14 +530,14 @@ __device__ __forceinline__ void scan_base_unit(const ScanBase& b, long long unit
         const int lane = threadIdx.x & 31;
         const long long end = first + base_unit_blocks(period) < b.nb ? first + base_unit_blocks(period) : b.nb;
         for (long long j = first + (threadIdx.x >> 5); j < end; j += kWarps) {
-            LogProduct p;
+            LogProduct<int> p;
             block_product<S, SQUARED>(values + j * period, period, lane, 32, b.vec != 0, eps, eps_ok, p, invalid);
             p.template combine<32>();
             if (lane == 0) sums[j] = p.value();
         }
     } else {
         __shared__ double red[kWarps];
-        LogProduct p;
+        LogProduct<long long> p;
         block_product<S, SQUARED>(values + first * period, period, threadIdx.x, kThreads, b.vec != 0, eps, eps_ok, p, invalid);
         p.template combine<32>();
         __syncthreads();   // the previous unit's sum has been read

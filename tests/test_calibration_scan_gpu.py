@@ -63,6 +63,21 @@ def test_scan_counts_invalid_inputs_and_follows_nan(cuda_device):
     assert bool(torch.isfinite(tiny).all())
 
 
+@pytest.mark.gpu
+def test_blocks_whose_logarithms_leave_32_bits(cuda_device):
+    """Two blocks of 2^29 + 2^20 elements, zeros and ones: the binary exponent of the first block's product is -40 times
+    its length, about five times what 32 bits hold."""
+    from gefen_b200.kernels.period_variance import period_scan_async
+
+    period = (1 << 29) + (1 << 20)
+    x = torch.zeros(2 * period, dtype=torch.bfloat16, device=cuda_device)
+    x[period:] = 1.0
+    want = math.log(1.0 + 1e-12) - math.log(1e-12)
+    got = float(period_scan_async(x, [period], input_is_squared=False, epsilon=1e-12).cpu()[0, 0])
+    # one rounding of 2^-53 per factor (relative), and the logarithm itself
+    assert abs(got - want) <= 1e-12 * want
+
+
 def test_native_divisors():
     from gefen_b200 import partitioning
 
