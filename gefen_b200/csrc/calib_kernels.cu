@@ -391,8 +391,8 @@ __global__ void adjacent_diff_final_kernel(const double* __restrict__ partial, i
 // of 768 x 2304 elements) read the tensor themselves.
 //
 // A base takes one logarithm per block, not per element: the sum of log x_i is the logarithm of the product, which is
-// kept as a mantissa in [1, 2) and an exponent (split off every eight factors; with eps >= 2^-120 and |g| < 2^63 eight
-// factors neither overflow nor underflow, other values take their own logarithm). One rounding of 2^-53 per factor is
+// kept as a mantissa in [1, 2) and an exponent (split off every eight factors; with 2^-120 <= eps <= 2^100 and
+// |g| < 2^63 eight factors neither overflow nor underflow, other values take their own logarithm). One rounding of 2^-53 per factor is
 // less than what adding up logarithms of about -25 costs (2^-49 per term). Two double-precision operations per
 // element remain, and the tensor is read once per base instead of a double per element written and read back.
 // An element moves the exponent by at most 128: 32 bits (E = int) hold it for blocks below kCtaPeriod, the longer blocks
@@ -565,7 +565,8 @@ template <bool SQUARED>
 __global__ void __launch_bounds__(kThreads) scan_base_kernel(double* __restrict__ scratch, const ScanBase* __restrict__ table, int n,
                                                              long long units, double eps, unsigned long long* __restrict__ invalid_out) {
     // 2^-120; squared inputs: 2^-70 (zeros and subnormal values count as up to 2^-126 themselves, not squared)
-    const bool eps_ok = eps >= (SQUARED ? 8.470329472543003e-22 : 7.52316384526264e-37);
+    // up to 2^100: a factor stays below 2^127, eight of them and the mantissa below 2^1017
+    const bool eps_ok = eps >= (SQUARED ? 8.470329472543003e-22 : 7.52316384526264e-37) && eps <= 1.2676506002282294e30;
     for (long long u = blockIdx.x; u < units; u += gridDim.x) {
         const ScanBase& b = table[find_entry(table, n, u, [](const ScanBase& e) { return e.first_unit; })];
         const long long unit = u - b.first_unit;

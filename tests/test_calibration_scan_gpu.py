@@ -64,6 +64,20 @@ def test_scan_counts_invalid_inputs_and_follows_nan(cuda_device):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("squared", [False, True])
+@pytest.mark.parametrize("eps", [2.0 ** -121, 2.0 ** -119, 2.0 ** -71, 2.0 ** -69, 1.0, 2.0 ** 99, 2.0 ** 101, 2.0 ** 130, 1e300])
+def test_epsilon_on_both_sides_of_the_product_form(cuda_device, squared, eps):
+    from gefen_b200.kernels.period_variance import period_scan_async
+
+    gen = torch.Generator(device=cuda_device).manual_seed(1)
+    x = torch.exp2(torch.rand(64 * 96, generator=gen, device=cuda_device) * 122.5 - 60)
+    got = period_scan_async(x, [8, 64, 512], input_is_squared=squared, epsilon=eps).cpu()
+    for want, row in zip(_scores(x, [8, 64, 512], squared, eps), got):
+        # means of logarithms of up to 700: 2^-53 of those per term
+        assert abs(float(row[0]) - want) <= 1e-12 * (1 + abs(want)), (want, float(row[0]))
+
+
+@pytest.mark.gpu
 def test_blocks_whose_logarithms_leave_32_bits(cuda_device):
     """Two blocks of 2^29 + 2^20 elements, zeros and ones: the binary exponent of the first block's product is -40 times
     its length, about five times what 32 bits hold."""
