@@ -1338,7 +1338,8 @@ static GroupShape group_shape(const NsMatrix* mats, int n) {
     return g;
 }
 static int check_group(const NsMatrix* mats, int n) {
-    GEFEN_CHECK_ARG(n >= 1 && n <= 4096 && mats != nullptr, "Expected between 1 and 4096 matrices, got %d.", n);
+    GEFEN_CHECK_ARG(n >= 1 && n <= GEFEN_B200_NS_GROUP_MATRICES && mats != nullptr, "Expected between 1 and %d matrices, got %d.",
+                    GEFEN_B200_NS_GROUP_MATRICES, n);
     for (int i = 0; i < n; ++i) {
         GEFEN_CHECK_ARG(mats[i].rows > 0 && mats[i].cols > 0 && mats[i].rows <= (1 << 24) && mats[i].cols <= (1 << 24),
                         "Matrix %d has bad dimensions.", i);

@@ -25,6 +25,8 @@ _STATUS = {}
 # Elements of all matrices that go through the iteration together: enough tiles for several waves of the GPU's SMs
 # (two layers of a 1.7 B model), and a bound on the iterates' memory (4 bytes per element, the Gram matrices on top).
 GROUP_ELEMENTS = 1 << 27
+# Matrices that one group may hold (GEFEN_B200_NS_GROUP_MATRICES of the library).
+GROUP_MATRICES = 4096
 
 
 def _status(device) -> torch.Tensor:
@@ -197,10 +199,11 @@ def zeropower_via_newtonschulz(grad: torch.Tensor, ns_coefficients: Tuple[float,
 
 
 def group_runs(keys: Sequence, numels: Sequence[int]) -> List[Tuple[int, int]]:
-    """Cuts a sequence of matrices into runs of equal keys and at most GROUP_ELEMENTS elements (one at least)."""
+    """Cuts a sequence of matrices into runs of equal keys, at most GROUP_MATRICES matrices and GROUP_ELEMENTS elements
+    (one matrix at least)."""
     runs, begin, total = [], 0, 0
     for i, (key, n) in enumerate(zip(keys, numels)):
-        if i > begin and (key != keys[begin] or total + n > GROUP_ELEMENTS):
+        if i > begin and (key != keys[begin] or total + n > GROUP_ELEMENTS or i - begin == GROUP_MATRICES):
             runs.append((begin, i))
             begin, total = i, 0
         total += n

@@ -349,6 +349,8 @@ typedef struct gefen_b200_ns_matrix {
     int32_t decay, reserved_;
 } gefen_b200_ns_matrix_t;
 int gefen_b200_ns_matrix_size(void);
+/* Matrices that one group may hold. */
+#define GEFEN_B200_NS_GROUP_MATRICES 4096
 /* The plan depends on the shapes and buffers only: plan_bytes bytes, filled on the host by ns_group_plan, copied by the
  * caller to a 64-byte aligned device buffer before ns_group runs. 0 bytes: bad arguments. */
 int64_t gefen_b200_ns_group_plan_bytes(const gefen_b200_ns_matrix_t* mats, int n);

@@ -52,6 +52,22 @@ def test_runs_of_a_group():
     assert ns.group_runs("aab", [1, 2, 3]) == [(0, 2), (2, 3)]
     assert ns.group_runs("aaaa", [cap, 1, cap - 1, 1]) == [(0, 1), (1, 3), (3, 4)]
     assert ns.group_runs("aa", [2 * cap, 2 * cap]) == [(0, 1), (1, 2)]
+    most = ns.GROUP_MATRICES
+    assert ns.group_runs("a" * (2 * most + 1), [8] * (2 * most + 1)) == [(0, most), (most, 2 * most), (2 * most, 2 * most + 1)]
+
+
+def test_largest_group_is_what_the_library_takes():
+    import numpy as np
+
+    from gefen_b200 import _lib, newton_schulz as ns
+
+    mats = np.zeros(ns.GROUP_MATRICES + 1, dtype=_lib.NS_MATRIX_DTYPE)
+    mats["rows"], mats["cols"] = 8, 16
+    for field in ("x0", "x1", "gram", "poly"):
+        mats[field] = 4096   # (sizes only: nothing is read)
+    plan_bytes = _lib.load().gefen_b200_ns_group_plan_bytes
+    assert plan_bytes(mats.ctypes.data, ns.GROUP_MATRICES) > 0
+    assert plan_bytes(mats.ctypes.data, ns.GROUP_MATRICES + 1) == 0
 
 
 @pytest.mark.gpu
