@@ -1341,7 +1341,7 @@ static int check_group(const NsMatrix* mats, int n) {
     GEFEN_CHECK_ARG(n >= 1 && n <= GEFEN_B200_NS_GROUP_MATRICES && mats != nullptr, "Expected between 1 and %d matrices, got %d.",
                     GEFEN_B200_NS_GROUP_MATRICES, n);
     for (int i = 0; i < n; ++i) {
-        GEFEN_CHECK_ARG(mats[i].rows > 0 && mats[i].cols > 0 && mats[i].rows <= (1 << 24) && mats[i].cols <= (1 << 24),
+        GEFEN_CHECK_ARG(mats[i].rows > 0 && mats[i].cols > 0 && mats[i].rows <= (1 << 30) && mats[i].cols <= (1 << 30),
                         "Matrix %d has bad dimensions.", i);
         GEFEN_CHECK_ARG(mats[i].x0 && mats[i].x1 && mats[i].gram && mats[i].poly, "Matrix %d has a null buffer.", i);
         GEFEN_CHECK_ARG(aligned16(mats[i].x0) && aligned16(mats[i].x1) && aligned16(mats[i].gram) && aligned16(mats[i].poly),

@@ -68,6 +68,9 @@ def test_largest_group_is_what_the_library_takes():
     plan_bytes = _lib.load().gefen_b200_ns_group_plan_bytes
     assert plan_bytes(mats.ctypes.data, ns.GROUP_MATRICES) > 0
     assert plan_bytes(mats.ctypes.data, ns.GROUP_MATRICES + 1) == 0
+    for rows, cols in ((1 << 25, 4), (4, 3 << 24), (1 << 30, 8)):   # long and thin ones
+        mats["rows"], mats["cols"] = rows, cols
+        assert plan_bytes(mats.ctypes.data, 1) > 0
 
 
 @pytest.mark.gpu
