@@ -1153,11 +1153,9 @@ __global__ void __launch_bounds__(kElemThreads) ns_normalise_kernel(const NsMatr
         for (long long c = static_cast<long long>(blockIdx.x) * kElemThreads + threadIdx.x; c < chunks; c += static_cast<long long>(gridDim.x) * kElemThreads) {
             uint32_t w[4];
             alignas(16) S v[8];
-            if constexpr (sizeof(S) == 2) *reinterpret_cast<uint4*>(v) = reinterpret_cast<const uint4*>(src)[c];
-            else {
-                reinterpret_cast<uint4*>(v)[0] = reinterpret_cast<const uint4*>(src)[2 * c];
-                reinterpret_cast<uint4*>(v)[1] = reinterpret_cast<const uint4*>(src)[2 * c + 1];
-            }
+            constexpr int kWide = static_cast<int>(sizeof(S)) / 2;   // 16-byte pieces of eight values
+#pragma unroll
+            for (int q = 0; q < kWide; ++q) reinterpret_cast<uint4*>(v)[q] = reinterpret_cast<const uint4*>(src)[kWide * c + q];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const __nv_bfloat162 h = __floats2bfloat162_rn(as_bf16(v + 2 * e) / norm, as_bf16(v + 2 * e + 1) / norm);

@@ -210,7 +210,9 @@ class GefenMuon(Gefen):
         if any(min(shape) == 0 for shape in shapes):
             return
         matrices = self._matrix_group(shapes, device)
-        together = all(local_p.is_contiguous() for group, name, p, local_p, grad in run)
+        # the update kernel takes contiguous parameters of these types; torch updates the others
+        together = updates[0].dtype in (torch.float32, torch.float16, torch.bfloat16) and all(
+            local_p.is_contiguous() for group, name, p, local_p, grad in run)
         if together:
             matrices.update_of([local_p for group, name, p, local_p, grad in run], wd_muls, alphas)
         matrices.run(updates, first["ns_coefficients"], first["ns_steps"], first["eps"])

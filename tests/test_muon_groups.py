@@ -44,6 +44,50 @@ def test_group_equals_single_runs_and_the_torch_update(cuda_device, dtype, steps
         assert torch.equal(got, p), SHAPES[i]
 
 
+@pytest.mark.gpu
+def test_float64_sources(cuda_device):
+    """Wide, tall, padded and square sources in float64 give what their float32 values give."""
+    from gefen_b200 import newton_schulz as ns
+
+    gen = torch.Generator(device=cuda_device).manual_seed(2)
+    grads = [torch.randn(s, generator=gen, device=cuda_device) * 0.1 for s in SHAPES]
+    results = []
+    for dtype in (torch.float32, torch.float64):
+        scratch = torch.full((ns.group_scratch_elements(SHAPES),), float("nan"), dtype=torch.bfloat16, device=cuda_device)
+        group = ns.MatrixGroup(SHAPES, scratch)
+        group.run([g.to(dtype) for g in grads], NS, 5, 1e-7)
+        results.append([group.result(i).clone() for i in range(len(SHAPES))])
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.gpu
+def test_step_of_float64_parameters(cuda_device, monkeypatch):
+    """GefenMuon on float64 parameters (fp32 state): the update is torch's, on the orthogonalised momentum."""
+    import gefen_b200.gefen as gefen
+    from gefen_b200 import GefenMuon, newton_schulz as ns
+
+    monkeypatch.setattr(gefen, "F_FP32", True)
+    gen = torch.Generator(device=cuda_device).manual_seed(4)
+    shapes = [(64, 128), (256, 64), (48, 36)]
+    params = [torch.nn.Parameter((torch.randn(s, generator=gen, device=cuda_device) * 0.02).double()) for s in shapes]
+    opt = GefenMuon(params, lr=0.02, weight_decay=0.1, nesterov=False)
+    for _ in range(2):
+        for p in params:
+            p.grad = (torch.randn(p.shape, generator=gen, device=cuda_device) * 1e-3).double()
+        before = [p.detach().clone() for p in params]
+        opt.step()
+        for p, old in zip(params, before):
+            st = opt.state[p]
+            period = st["automatic_period"]
+            block = opt._period_one_divisor_from_state(st, p.numel()) if period == 1 else period
+            codes = st["m_codebook"].reshape(-1, block).long()
+            momentum = (opt._gefen_codebook[codes] * st["m_magnitude"].float()).reshape(p.shape)
+            ortho = ns.zeropower_via_newtonschulz(momentum, NS, 5, 1e-7)
+            want = old.mul_(1 - 0.02 * 0.1).add_(ortho, alpha=-0.02 * max(1, p.shape[0] / p.shape[1]) ** 0.5)
+            assert torch.equal(p.detach(), want)
+
+
 def test_runs_of_a_group():
     from gefen_b200 import newton_schulz as ns
 
