@@ -1139,8 +1139,10 @@ __global__ void __launch_bounds__(kElemThreads) ns_normalise_kernel(const NsMatr
     if (threadIdx.x < 32) {
         float t = parts[blockIdx.y * kNormParts + threadIdx.x] + parts[blockIdx.y * kNormParts + 32 + threadIdx.x];
         t = warp_sum(t);
-        if (threadIdx.x == 0)
-            norm_shared = fmaxf(__bfloat162float(__float2bfloat16_rn(sqrtf(t))), __bfloat162float(__float2bfloat16_rn(eps)));
+        if (threadIdx.x == 0) {
+            const float n = __bfloat162float(__float2bfloat16_rn(sqrtf(t))), least = __bfloat162float(__float2bfloat16_rn(eps));
+            norm_shared = n < least ? least : n;   // (a NaN norm stays one, as torch's clamp leaves it)
+        }
     }
     __syncthreads();
     const float norm = norm_shared;

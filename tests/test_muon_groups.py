@@ -45,6 +45,25 @@ def test_group_equals_single_runs_and_the_torch_update(cuda_device, dtype, steps
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("steps", [0, 1])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_values_that_are_not_finite(cuda_device, steps, bad):
+    """As torch's x / x.norm().clamp(min=eps): a NaN makes the whole matrix NaN, an infinity leaves zeros and a NaN."""
+    from gefen_b200 import newton_schulz as ns
+
+    for shape in [(16, 64), (64, 16), (20, 33)]:
+        g = torch.ones(shape, device=cuda_device)
+        g[3, 5] = bad
+        x = g.bfloat16()
+        want = x / x.norm().clamp(min=1e-7)
+        if steps:
+            assert bool(want.isnan().any())
+            want = torch.full_like(want, float("nan"))   # the Gram matrix of a row with a NaN, twice
+        got = ns.zeropower_via_newtonschulz(g, NS, steps, 1e-7)
+        assert torch.equal(torch.nan_to_num(got.float(), nan=7.0), torch.nan_to_num(want.float(), nan=7.0)), shape
+
+
+@pytest.mark.gpu
 def test_float64_sources(cuda_device):
     """Wide, tall, padded and square sources in float64 give what their float32 values give."""
     from gefen_b200 import newton_schulz as ns
