@@ -710,7 +710,7 @@ __device__ __forceinline__ void first_pass_group(const S* g_blk, const uint8_t* 
 template <typename S, int NSRC, bool EXACT = false>
 __device__ __forceinline__ void reduce_pass(const StepLaunch& L, const S* g_blk, const uint8_t* codes_in, float* stage, int half,
                                             const LaneTables& t, int lane, int LANES, int nchunks,
-                                            float old_mag, float beta1, float omb1, float& absmax, float& sumsq) {
+                                            float old_mag, float beta1, float omb1, float& absmax, f32x2& sumsq2) {
     constexpr int kSlots = sizeof(S) == 2 ? 4 : 2;
     constexpr int BS = NSRC < kSlots ? NSRC : kSlots;
     constexpr int U = kSlots / BS;
@@ -766,8 +766,9 @@ __device__ __forceinline__ void reduce_pass(const StepLaunch& L, const S* g_blk,
                     const float cur = old_mag * t.value(t.row_of_byte(craw[u].w[i >> 2], i & 3));
                     m[i] = ema_update(beta1, cur, omb1, g[i]);
                     absmax = max_abs_nan(absmax, m[i]);
-                    sumsq = fmaf(g[i], g[i], sumsq);
                 }
+#pragma unroll
+                for (int i = 0; i < 8; i += 2) sumsq2 = fma2(pair(g[i], g[i + 1]), pair(g[i], g[i + 1]), sumsq2);   // as first_pass_group
                 stage_store<8>(stage, half, c, m);
             }
         }
@@ -956,7 +957,7 @@ __device__ __forceinline__ void warp_block_step(const TensorSlot<S>& t, long lon
         // as a reduce-scatter into that dtype would leave it.
         if constexpr (GSRC == 1) {
             const int n_src = L.n_grad_srcs;
-#define GEFEN_REDUCE_PASS(...) reduce_pass<S, __VA_ARGS__>(L, g_blk, codes, stage, half, tables, lane, LANES, nchunks, old_mag, beta1, omb1, absmax, sumsq)
+#define GEFEN_REDUCE_PASS(...) reduce_pass<S, __VA_ARGS__>(L, g_blk, codes, stage, half, tables, lane, LANES, nchunks, old_mag, beta1, omb1, absmax, sumsq2)
             if (n_src == 2) GEFEN_REDUCE_PASS(2, true);
             else if (n_src < 2) GEFEN_REDUCE_PASS(2);
             else if (n_src == 4) GEFEN_REDUCE_PASS(4, true);
@@ -981,6 +982,8 @@ __device__ __forceinline__ void warp_block_step(const TensorSlot<S>& t, long lon
         for (; c0 < chunks; c0 += LANES * U)
             first_pass_group<S, V, U, true, SUMMED>(g_src, codes, stage, half, tables, c0 + lane, LANES, nchunks, mag2, beta2_, omb2_,
                                                     scale, absmax, sumsq2);
+    }
+    {   // (the same two partial sums wherever the gradients come from: a rank's second moments are a single process's)
         float even, odd;
         unpair(sumsq2, even, odd);
         sumsq = even + odd;
