@@ -775,6 +775,70 @@ __device__ __forceinline__ void reduce_pass(const StepLaunch& L, const S* g_blk,
     }
 }
 
+// The same in chunks of V < 8 elements, for any number of sources (none: this GPU's buffer). Four chunks per lane are in
+// flight for one source at a time; the sums are formed in the order of first_pass_group.
+template <typename S, int V>
+__device__ __forceinline__ void reduce_pass_small(const StepLaunch& L, const S* g_blk, const uint8_t* codes_in, float* stage, int half,
+                                                  const LaneTables& t, int lane, int LANES, int nchunks, float old_mag, float beta1,
+                                                  float omb1, float& absmax, f32x2& sumsq2) {
+    constexpr int U = 4;
+    const int n_src = L.n_grad_srcs;
+    for (int c0 = lane; c0 < nchunks; c0 += LANES * U) {
+        CodeChunk<V> craw[U];
+        Chunk<S, V> graw[U];
+        float acc[U][V];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+#pragma unroll
+            for (int i = 0; i < V; ++i) acc[u][i] = 0.0f;
+            if (c0 + LANES * u < nchunks) {
+                craw[u].load(codes_in, c0 + LANES * u);
+                if (n_src == 0) graw[u].load(g_blk, c0 + LANES * u);
+            }
+        }
+        for (int r = 0; r < n_src; ++r) {
+            const S* const src = peer_ptr(g_blk, L.grad_delta[r]);
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (c0 + LANES * u < nchunks) graw[u].load(src, c0 + LANES * u);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (c0 + LANES * u < nchunks) {
+                    float part[V];
+                    graw[u].unpack(part);
+#pragma unroll
+                    for (int i = 0; i < V; ++i) acc[u][i] += part[i];
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int c = c0 + LANES * u;
+            if (c < nchunks) {
+                if (n_src > 0) {
+#pragma unroll
+                    for (int i = 0; i < V; ++i) acc[u][i] *= L.grad_scale;
+                    graw[u].pack(acc[u]);
+                }
+                float g[V], m[V];
+                graw[u].unpack(g);
+#pragma unroll
+                for (int i = 0; i < V; ++i) {
+                    const float cur = old_mag * t.value(t.row_of_byte(craw[u].w[0], i));
+                    m[i] = ema_update(beta1, cur, omb1, g[i]);
+                    absmax = max_abs_nan(absmax, m[i]);
+                }
+#pragma unroll
+                for (int i = 0; i < V; i += 2) {
+                    const f32x2 g2 = V == 1 ? pair(g[0], 0.0f) : pair_at(g, i);
+                    sumsq2 = fma2(g2, g2, sumsq2);
+                }
+                stage_store<V>(stage, half, c, m);
+            }
+        }
+    }
+}
+
 // One chunk of the re-encode and update of the common case (finite block, Gefen update of the parameters) with
 // everything that is fixed per launch or per tensor decided at compile time: WD = the decoupled weight decay of the
 // reference's separate multiply, STORE = 0 this GPU's copy only, 1 peer stores as well, 2 one multicast store, ONE =
@@ -904,13 +968,14 @@ __device__ __forceinline__ void second_pass_muon(const LaneTables& t, const floa
 // each (a power of two, uniform over the warp; FULL fixes it to 32 at compile
 // time, for blocks of more than 1024 elements). A block's slice of `stage` holds period floats (see stage_store).
 // GSRC: where the gradients come from: 0 = this GPU's buffer, 1 = averaged over the ranks' buffers with peer
-// loads, 2 = summed by the switch through the multicast mapping (StepLaunch::grad_mc_delta).
+// loads, 2 = summed by the switch through the multicast mapping (StepLaunch::grad_mc_delta). Chunks below eight elements
+// know 0 and 1 only: 1 is every launch with peers, gradients of this GPU's buffer (no sources) included.
 template <typename S, int V, int GSRC, bool FULL>
 __device__ __forceinline__ void warp_block_step(const TensorSlot<S>& t, long long unit, const StepLaunch& L, const LaneTables& tables,
                                                 float* stage, int warp_lane) {
     const float* const stepsize = L.stepsize;
-    const int n_peers = GSRC == 0 && V < 8 ? 0 : L.n_peers;            // (chunks below 8 serve this GPU's buffers only)
-    const long long param_mc = GSRC == 0 && V < 8 ? 0 : L.param_mc_delta;
+    const int n_peers = GSRC == 0 && V < 8 ? 0 : L.n_peers;            // (chunks below 8: GSRC == 1 wherever there are peers)
+    const long long param_mc = V < 8 ? 0 : L.param_mc_delta;           // (a multicast access moves 16 bytes)
     // (the shuffle tells the compiler that the period is the same in all lanes, which the loops' bounds profit from)
     const int period = __shfl_sync(0xffffffffu, t.period, 0);
     const int chunks = period / V;                     // of a block
@@ -955,7 +1020,9 @@ __device__ __forceinline__ void warp_block_step(const TensorSlot<S>& t, long lon
         // The gradient of this block is the average over the ranks' buffers (this GPU's and the
         // peers', read over NVLink), summed in fp32 in rank order and rounded to the gradient dtype,
         // as a reduce-scatter into that dtype would leave it.
-        if constexpr (GSRC == 1) {
+        if constexpr (GSRC == 1 && V < 8) {
+            reduce_pass_small<S, V>(L, g_blk, codes, stage, half, tables, lane, LANES, nchunks, old_mag, beta1, omb1, absmax, sumsq2);
+        } else if constexpr (GSRC == 1) {
             const int n_src = L.n_grad_srcs;
 #define GEFEN_REDUCE_PASS(...) reduce_pass<S, __VA_ARGS__>(L, g_blk, codes, stage, half, tables, lane, LANES, nchunks, old_mag, beta1, omb1, absmax, sumsq2)
             if (n_src == 2) GEFEN_REDUCE_PASS(2, true);
@@ -1050,7 +1117,8 @@ __device__ __forceinline__ void warp_block_step(const TensorSlot<S>& t, long lon
             } else if (store == 1) { if (wd) GEFEN_SECOND_PASS(true, 1, false); else GEFEN_SECOND_PASS(false, 1, false); }
             else { if (wd) GEFEN_SECOND_PASS(true, 2, false); else GEFEN_SECOND_PASS(false, 2, false); }
         } else {
-            if (wd) GEFEN_SECOND_PASS(true, 0, false); else GEFEN_SECOND_PASS(false, 0, false);
+            constexpr int kStore = GSRC == 0 ? 0 : 1;
+            if (wd) GEFEN_SECOND_PASS(true, kStore, false); else GEFEN_SECOND_PASS(false, kStore, false);
         }
 #undef GEFEN_SECOND_PASS
         __syncwarp();  // the staging slice is free for this warp's next block
@@ -1621,6 +1689,11 @@ static int launch_vec_variant(StepLaunch L, const StepRows& rows, long long max_
 
 template <typename S>
 static int launch_vec(int cls, StepLaunch L, const StepRows& rows, long long max_unit, cudaStream_t stream) {
+    if (cls >= 3 && cls <= 5 && (L.n_peers > 0 || L.n_grad_srcs > 0)) {
+        if (cls == 3) return launch_vec_variant<S, 4, 1, false>(L, rows, max_unit, stream);
+        if (cls == 4) return launch_vec_variant<S, 2, 1, false>(L, rows, max_unit, stream);
+        return launch_vec_variant<S, 1, 1, false>(L, rows, max_unit, stream);
+    }
     if (cls == 3) return launch_vec_variant<S, 4, 0, false>(L, rows, max_unit, stream);
     if (cls == 4) return launch_vec_variant<S, 2, 0, false>(L, rows, max_unit, stream);
     if (cls == 5) return launch_vec_variant<S, 1, 0, false>(L, rows, max_unit, stream);
@@ -2062,8 +2135,8 @@ int gefen_b200_multi_tensor_step_multicast(gefen_b200_step_tensor_t* host_table,
         GEFEN_CHECK_ARG(n_grad_srcs == 0 || !(t.flags & GEFEN_B200_STEP_MUON),
                         "Tensor %d: the momentum-only step does not average gradients over ranks.", i);
         int cls = tensor_class(t, param_dtype);
-        // chunks below eight serve this GPU's buffers only; with peers the generic kernels do (same order of rows)
-        if (cls >= 3 && (n_peers > 0 || n_grad_srcs > 0)) cls = generic_class(t);
+        // vectors with peers: the generic kernel (no sums of squares there, so the results are the same bits)
+        if (cls == 6 && (n_peers > 0 || n_grad_srcs > 0)) cls = generic_class(t);
         t.reserved_[0] = cls;
     }
     for (int begin = 0; begin < n_tensors;) {
