@@ -439,7 +439,7 @@ def run_gpu_arm(args, cfg, rank, world, local_rank):
                           "unit": "GB/s", "frac": achieved / peak,
                           "traffic": ratio * vec_bytes if ratio is not None else None,
                           "algorithmic_bytes_per_launch": vec_bytes, "launch_ms": vec_ms}
-    result["launches_per_step"] = len({lib.gefen_b200_step_launch_class(rows[r:r + 1].ctypes.data, table["tag"]) for r in range(len(rows))})
+    result["launches_per_step"] = len(set(_lib.step_classes(rows, table["tag"])[1]))
 
     # ---- end to end through the public API with HOST buffers: gradients come from pinned host
     # memory every step and the updated parameters go back to pinned host memory

@@ -87,6 +87,7 @@ def _declare(lib):
         "gefen_b200_step_tensor_size": (i32, []),
         "gefen_b200_step_tensor_class": (i32, [vp, i32]),
         "gefen_b200_step_launch_class": (i32, [vp, i32]),
+        "gefen_b200_step_classes": (i32, [vp, i32, i32, vp, vp]),
         "gefen_b200_step_status": (i32, [vp, i32]),
         "gefen_b200_debug_set_stage_spin_limit": (i32, [i64]),
         "gefen_b200_exact_histogram": (i32, [vp, i32, i64, i64, vp, i32, vp]),
@@ -159,6 +160,13 @@ def check(rc: int) -> None:
 
 def ptr(t):
     return None if t is None else ctypes.c_void_p(t.data_ptr())
+
+
+def step_classes(rows: np.ndarray, dtype_tag: int):
+    """(kernel class as `gefen_b200_step_tensor_class` gives it, launch class) of every row of a step table, as lists."""
+    classes = np.empty((2, len(rows)), dtype=np.int32)
+    check(load().gefen_b200_step_classes(rows.ctypes.data, len(rows), dtype_tag, classes[0].ctypes.data, classes[1].ctypes.data))
+    return classes.tolist()
 
 
 def step_status(device, clear: bool = True) -> int:

@@ -2008,6 +2008,17 @@ int gefen_b200_step_launch_class(const gefen_b200_step_tensor_t* host_entry, int
     return tensor_class(*host_entry, param_dtype);
 }
 
+int gefen_b200_step_classes(const gefen_b200_step_tensor_t* host_table, int n_tensors, int param_dtype, int32_t* tensor_classes,
+                            int32_t* launch_classes) {
+    GEFEN_CHECK_ARG(n_tensors >= 0 && (n_tensors == 0 || host_table != nullptr), "Expected a table of %d rows.", n_tensors);
+    for (int i = 0; i < n_tensors; ++i) {
+        const int cls = tensor_class(host_table[i], param_dtype);
+        if (launch_classes != nullptr) launch_classes[i] = cls;
+        if (tensor_classes != nullptr) tensor_classes[i] = cls >= 3 ? generic_class(host_table[i]) : cls;
+    }
+    return GEFEN_B200_OK;
+}
+
 int gefen_b200_multicast_sum(void* dst, const void* src_multicast, int dtype, int64_t numel, double scale, void* stream_) {
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
     GEFEN_CHECK_ARG(dst != nullptr && src_multicast != nullptr, "Expected non-null buffers.");

@@ -431,7 +431,6 @@ class Gefen(torch.optim.Optimizer):
         if len(self._plans) >= 512:   # callers that keep changing the set of tensors: start over
             self._plans.clear()
         plan = self._plans[key] = self._plan = _StepPlan()
-        lib = _lib.load()
         by_dtype = {}
         for idx, (group, name, p, local_p, grad) in enumerate(work):
             by_dtype.setdefault((grad.dtype, grad.device), []).append(idx)
@@ -471,8 +470,7 @@ class Gefen(torch.optim.Optimizer):
                 rows[r]["flags"] = flags
                 rows[r]["p"] = local_p.data_ptr() + b0 * block * local_p.element_size()
                 rows[r]["g"] = grad.data_ptr() + b0 * block * grad.element_size()
-            classes = [lib.gefen_b200_step_tensor_class(rows[r:r + 1].ctypes.data, tag) for r in range(len(idxs))]
-            launch = [lib.gefen_b200_step_launch_class(rows[r:r + 1].ctypes.data, tag) for r in range(len(idxs))]
+            classes, launch = _lib.step_classes(rows, tag)
             order = sorted(range(len(idxs)), key=lambda r: launch[r])
             rows = np.ascontiguousarray(rows[order])
             tables.append({

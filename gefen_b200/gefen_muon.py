@@ -130,8 +130,8 @@ class GefenMuon(Gefen):
             rows[r]["flags"] = flags
             state["step"] += 1
         tag = _lib.dtype_tag(chunk[0][4].dtype)
-        classes = [lib.gefen_b200_step_launch_class(rows[r:r + 1].ctypes.data, tag) for r in range(len(chunk))]
-        order = sorted(range(len(chunk)), key=lambda r: classes[r])
+        _, launch = _lib.step_classes(rows, tag)
+        order = sorted(range(len(chunk)), key=lambda r: launch[r])
         rows = np.ascontiguousarray(rows[order])
         device = chunk[0][4].device
         table = self._device_table(rows.nbytes, device)

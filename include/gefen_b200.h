@@ -199,6 +199,9 @@ int gefen_b200_step_tensor_class(const gefen_b200_step_tensor_t* host_entry, int
  * element (blocks and pointers that are multiples of no more than that), 6 = period-1 vectors, 0 / -1 = generic. Rows
  * of equal launch class that are adjacent in the table share one launch. */
 int gefen_b200_step_launch_class(const gefen_b200_step_tensor_t* host_entry, int param_dtype);
+/* Both classes of every row of a table (host arrays of n_tensors; either may be NULL). */
+int gefen_b200_step_classes(const gefen_b200_step_tensor_t* host_table, int n_tensors, int param_dtype,
+                            int32_t* tensor_classes, int32_t* launch_classes);
 
 /* Error status of the step kernels on the CURRENT device. Every wait inside them is bounded; a CTA
  * whose wait for its staged tables runs out leaves without doing its share of the step and raises

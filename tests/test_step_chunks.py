@@ -93,3 +93,20 @@ def test_launch_class_follows_length_and_alignment():
                 fits = [v for v in (8, 4, 2, 1) if period % v == 0 and shift * size % min(16, v * size) == 0 and shift % v == 0]
                 assert chunk[cls] == fits[0], (period, shift, size, cls)
                 assert cls != 1 or period > 1024
+
+
+def test_classes_of_a_whole_table():
+    import numpy as np
+
+    from gefen_b200 import _lib
+
+    lib = _lib.load()
+    rows = np.zeros(60, dtype=_lib.STEP_TENSOR_DTYPE)
+    rows["num_blocks"], rows["period"] = 3, [1 + 7 * i * i for i in range(60)]
+    rows["g"], rows["p"], rows["codes"] = 4096 + 4 * np.arange(60), 8192, 16384
+    rows["flags"] = np.where(np.arange(60) % 5 == 0, _lib.STEP_PERIOD1, 0)
+    for tag in (_lib.F32, _lib.BF16, _lib.F64):
+        tensor, launch = _lib.step_classes(rows, tag)
+        assert tensor == [lib.gefen_b200_step_tensor_class(rows[i:i + 1].ctypes.data, tag) for i in range(60)]
+        assert launch == [lib.gefen_b200_step_launch_class(rows[i:i + 1].ctypes.data, tag) for i in range(60)]
+    assert _lib.step_classes(rows[:0], _lib.F32) == [[], []]
