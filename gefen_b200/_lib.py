@@ -179,10 +179,14 @@ def step_status(device, clear: bool = True) -> int:
 
 
 def check_step_status(device) -> None:
-    """Raises GefenB200Error if a step kernel on `device` gave up a bounded wait (synchronises)."""
-    if step_status(device, clear=True) != 0:
-        raise GefenB200Error("a Gefen step kernel gave up waiting for its staged codebook tables; the optimizer "
-                             "state and parameters of that step are incomplete")
+    """Raises GefenB200Error if a step kernel on `device` left without doing its work (synchronises)."""
+    status = step_status(device, clear=True)
+    if status == 0:
+        return
+    reasons = [text for bit, text in ((1, "gave up waiting for its staged codebook tables"),
+                                      (2, "found its shared-memory tables out of place")) if status & bit]
+    raise GefenB200Error("a Gefen step kernel {}; the optimizer state and parameters of that step are incomplete".format(
+        " and ".join(reasons) or "reported status {}".format(status)))
 
 
 def current_stream(device) -> ctypes.c_void_p:

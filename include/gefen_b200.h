@@ -205,7 +205,8 @@ int gefen_b200_step_classes(const gefen_b200_step_tensor_t* host_table, int n_te
 
 /* Error status of the step kernels on the CURRENT device. Every wait inside them is bounded; a CTA
  * whose wait for its staged tables runs out leaves without doing its share of the step and raises
- * bit 0 of a status word. This call synchronises the device, writes the word to *host_status and,
+ * bit 0 of a status word; bit 1: the tables do not lie where the kernel was compiled to read them
+ * (its static shared memory has outgrown its share), nothing was done. This call synchronises the device, writes the word to *host_status and,
  * with clear != 0, resets it. Non-zero means that a step since the last clear was incomplete. The
  * reference has no counterpart: its kernels do not wait on anything (errors there are exceptions
  * from C10_CUDA_KERNEL_LAUNCH_CHECK). */

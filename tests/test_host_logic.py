@@ -215,3 +215,15 @@ def test_tensors_of_two_devices_are_refused():
         gefen_exact_histogram_many_cuda(grads, [8, 8], 4096)
     with pytest.raises(ValueError, match="one device"):
         Gefen._predict_periods(None, [("a", None, grads[0]), ("b", None, grads[1])])
+
+
+def test_status_word_names_its_cause(monkeypatch):
+    from gefen_b200 import _lib
+
+    for status, texts in ((1, ["waiting"]), (2, ["out of place"]), (3, ["waiting", "out of place"])):
+        monkeypatch.setattr(_lib, "step_status", lambda device, clear=True: status)
+        with pytest.raises(_lib.GefenB200Error) as error:
+            _lib.check_step_status(None)
+        assert all((text in str(error.value)) == (text in texts) for text in ("waiting", "out of place"))
+    monkeypatch.setattr(_lib, "step_status", lambda device, clear=True: 0)
+    _lib.check_step_status(None)
