@@ -109,6 +109,7 @@ def _declare(lib):
         "gefen_b200_exact_dp": (i32, [vp, vp, vp, i32, i32, i32, vp, vp, vp]),
         "gefen_b200_ns_gemm_tn": (i32, [vp, vp, vp, vp, vp, i32, i32, i32, i64, i64, i64, i64, i64, dbl, dbl, i32, vp, vp]),
         "gefen_b200_newton_schulz": (i32, [vp, vp, vp, vp, i32, i32, i32, dbl, dbl, dbl, vp, vp]),
+        "gefen_b200_upload": (i32, [vp, vp, i64, vp]),
         "gefen_b200_ns_matrix_size": (i32, []),
         "gefen_b200_ns_group_plan_bytes": (i64, [vp, i32]),
         "gefen_b200_ns_group_plan": (i32, [vp, i32, vp]),
@@ -191,6 +192,11 @@ def check_step_status(device) -> None:
 
 def current_stream(device) -> ctypes.c_void_p:
     return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+
+
+def upload(dst: torch.Tensor, host: np.ndarray) -> None:
+    """Copies a table to the device in stream order (see gefen_b200_upload). The current device is dst's."""
+    check(load().gefen_b200_upload(ptr(dst), host.ctypes.data, host.nbytes, current_stream(dst.device)))
 
 
 class device_guard:

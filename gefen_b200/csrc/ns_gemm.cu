@@ -1418,7 +1418,43 @@ static int launch_group(const GroupShape& g, GemmArgs args, cudaStream_t stream)
     return launch_gemm_variant<128, 6, false, B_MN, true, true>(none, none, args, stream);
 }
 
+// Tables travel as kernel parameters, one launch per kUploadBytes: no host memory that a copy reads later (a pageable
+// copy of more than 64 KB first waits for the stream), and a captured upload carries its bytes with it.
+constexpr int kUploadBytes = 4000;
+struct UploadPiece {
+    uint4 word[kUploadBytes / 16];
+};
+__global__ void __launch_bounds__(256) upload_kernel(uint4* __restrict__ dst, int words, const __grid_constant__ UploadPiece piece) {
+    if (static_cast<int>(threadIdx.x) < words) dst[threadIdx.x] = piece.word[threadIdx.x];
+    asm volatile("fence.proxy.tensormap::generic.release.gpu;" ::: "memory");   // (there may be tensor maps among the words)
+}
+static_assert(kUploadBytes % 16 == 0 && kUploadBytes / 16 <= 256 && sizeof(UploadPiece) + 16 <= 4096, "one word per thread, kernel parameter space");
+constexpr int64_t kMostUploadLaunches = 64;
+
 }  // namespace gefen
+
+extern "C" int gefen_b200_upload(void* dst, const void* src, int64_t bytes, void* stream_) {
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+    GEFEN_CHECK_ARG(bytes >= 0 && bytes % 16 == 0, "Expected a multiple of 16 bytes.");
+    if (bytes == 0) return GEFEN_B200_OK;
+    GEFEN_CHECK_ARG(dst != nullptr && src != nullptr && aligned16(dst), "Expected a source and a 16-byte aligned destination.");
+    if (bytes > kMostUploadLaunches * kUploadBytes) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        GEFEN_CHECK_CUDA(cudaStreamIsCapturing(stream, &capture));
+        if (capture == cudaStreamCaptureStatusNone) {
+            GEFEN_CHECK_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream));
+            return GEFEN_B200_OK;
+        }
+    }
+    UploadPiece piece;
+    for (int64_t done = 0; done < bytes; done += kUploadBytes) {
+        const int n = static_cast<int>(std::min<int64_t>(bytes - done, kUploadBytes));
+        memcpy(piece.word, static_cast<const unsigned char*>(src) + done, n);
+        upload_kernel<<<1, 256, 0, stream>>>(reinterpret_cast<uint4*>(static_cast<unsigned char*>(dst) + done), n / 16, piece);
+    }
+    GEFEN_CHECK_CUDA(cudaGetLastError());
+    return GEFEN_B200_OK;
+}
 
 extern "C" int gefen_b200_ns_matrix_size(void) { return static_cast<int>(sizeof(gefen_b200_ns_matrix_t)); }
 

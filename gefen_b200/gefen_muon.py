@@ -82,16 +82,23 @@ class GefenMuon(Gefen):
         self._scratch = None
         self._ns_scratch = None     # buffers of the Newton-Schulz groups, and the launch tables over them by shapes
         self._ns_groups = {}
+        self._captured_rows = []
 
     # ------------------------------------------------------------------ momentum
     def _momentum_scratch(self, numel: int, dtype, device) -> torch.Tensor:
+        """Dense momenta of a chunk, kept between steps (a captured step has its own, see _matrix_group)."""
+        if torch.cuda.is_current_stream_capturing():
+            return torch.empty(numel, dtype=dtype, device=device)
         if (self._scratch is None or self._scratch.numel() < numel or self._scratch.dtype != dtype
                 or self._scratch.device != device):
             self._scratch = torch.empty(numel, dtype=dtype, device=device)
         return self._scratch
 
     def _device_table(self, nbytes: int, device) -> torch.Tensor:
-        """Device copy of the launch table, kept between steps (work on one stream is ordered)."""
+        """Device copy of the launch table, kept between steps (work on one stream is ordered; a captured step has its
+        own, see _matrix_group)."""
+        if torch.cuda.is_current_stream_capturing():
+            return torch.empty(nbytes, dtype=torch.uint8, device=device)
         t = getattr(self, "_table", None)
         if t is None or t.numel() < nbytes or t.device != device:
             t = self._table = torch.empty(max(nbytes, 4096), dtype=torch.uint8, device=device)
@@ -135,6 +142,8 @@ class GefenMuon(Gefen):
         rows = np.ascontiguousarray(rows[order])
         device = chunk[0][4].device
         table = self._device_table(rows.nbytes, device)
+        if torch.cuda.is_current_stream_capturing():
+            self._captured_rows.append(rows)   # every replay of the graph copies the rows from here
         ws = _lib.codebook_workspace(self._gefen_codebook)
         with _lib.device_guard(device):
             _lib.check(lib.gefen_b200_multi_tensor_step(rows.ctypes.data, _lib.ptr(table), len(chunk), tag, _lib.ptr(ws),
@@ -182,8 +191,11 @@ class GefenMuon(Gefen):
 
     def _matrix_group(self, shapes, device) -> "newton_schulz.MatrixGroup":
         """Launch tables for matrices of these shapes, kept between steps over one scratch buffer that grows on demand
-        (work on one stream is ordered, so the groups of a step share it)."""
+        (work on one stream is ordered, so the groups of a step share it). A captured step has its own: the graph keeps
+        their addresses, and they are filled when it runs."""
         need = newton_schulz.group_scratch_elements(shapes)
+        if torch.cuda.is_current_stream_capturing():
+            return newton_schulz.MatrixGroup(shapes, torch.empty(need, dtype=torch.bfloat16, device=device))
         if self._ns_scratch is None or self._ns_scratch.numel() < need or self._ns_scratch.device != device:
             self._ns_scratch = torch.empty(need, dtype=torch.bfloat16, device=device)
             self._ns_groups.clear()

@@ -109,7 +109,8 @@ def group_scratch_elements(shapes: Sequence[Tuple[int, int]]) -> int:
 class MatrixGroup:
     """The launch tables of a group of matrices of given shapes over one scratch buffer (at least
     `group_scratch_elements` bf16 elements). It can be kept and run again as long as the shapes repeat; its work is
-    ordered by the stream it runs on."""
+    ordered by the stream it runs on. One that is made under stream capture belongs to that graph: its tables are written
+    when the graph runs."""
 
     def __init__(self, shapes: Sequence[Tuple[int, int]], scratch: torch.Tensor):
         lib = _lib.load()
@@ -127,10 +128,11 @@ class MatrixGroup:
                 offset += n
         if offset > scratch.numel():
             raise ValueError("Expected {} elements of scratch for the group, got {}".format(offset, scratch.numel()))
-        nbytes = lib.gefen_b200_ns_group_plan_bytes(self.mats.ctypes.data, len(shapes))
-        host = torch.empty(max(nbytes, 1), dtype=torch.uint8)
-        _lib.check(lib.gefen_b200_ns_group_plan(self.mats.ctypes.data, len(shapes), _lib.ptr(host)))
-        self.plan = host.to(self.device)
+        host = np.empty(lib.gefen_b200_ns_group_plan_bytes(self.mats.ctypes.data, len(shapes)), dtype=np.uint8)
+        _lib.check(lib.gefen_b200_ns_group_plan(self.mats.ctypes.data, len(shapes), host.ctypes.data))
+        self.plan = torch.empty(host.nbytes, dtype=torch.uint8, device=self.device)
+        with _lib.device_guard(self.device):
+            _lib.upload(self.plan, host)
         self.table = torch.empty(self.mats.nbytes, dtype=torch.uint8, device=self.device)
         self.partials = torch.empty(64 * len(shapes), dtype=torch.float32, device=self.device)
         self.steps = 0
@@ -140,9 +142,9 @@ class MatrixGroup:
         scalars of `apply` beforehand, if that follows."""
         a, b, c = ns_coefficients
         self.mats["src"] = [t.data_ptr() for t in sources]
-        self.table.copy_(torch.from_numpy(self.mats.view(np.uint8)), non_blocking=True)
         self.steps = int(ns_steps)
         with _lib.device_guard(self.device):
+            _lib.upload(self.table, self.mats)
             _lib.check(_lib.load().gefen_b200_ns_group(
                 self.mats.ctypes.data, len(self.mats), _lib.ptr(self.table), _lib.ptr(self.plan), _lib.ptr(self.partials),
                 _lib.dtype_tag(sources[0].dtype), self.steps, float(a), float(b), float(c), float(eps),

@@ -355,8 +355,12 @@ typedef struct gefen_b200_ns_matrix {
 int gefen_b200_ns_matrix_size(void);
 /* Matrices that one group may hold. */
 #define GEFEN_B200_NS_GROUP_MATRICES 4096
+/* Copies a small table from any host memory to the device, in stream order, without waiting and without reading the host
+ * memory after the call; may be captured (a replay writes the same bytes again). bytes: a multiple of 16; dst: 16-byte
+ * aligned. */
+int gefen_b200_upload(void* dst, const void* src, int64_t bytes, void* stream);
 /* The plan depends on the shapes and buffers only: plan_bytes bytes, filled on the host by ns_group_plan, copied by the
- * caller to a 64-byte aligned device buffer before ns_group runs. 0 bytes: bad arguments. */
+ * caller to a 64-byte aligned device buffer before ns_group runs (gefen_b200_upload). 0 bytes: bad arguments. */
 int64_t gefen_b200_ns_group_plan_bytes(const gefen_b200_ns_matrix_t* mats, int n);
 int gefen_b200_ns_group_plan(const gefen_b200_ns_matrix_t* mats, int n, void* host_plan);
 /* Normalises every matrix and runs `steps` iterations; the results lie in x0 (even number of steps) or x1. device_mats:
