@@ -28,10 +28,8 @@
 
 #include <cuda.h>
 #include <algorithm>
-#include <map>
 #include <mutex>
 #include <new>
-#include <tuple>
 #include <vector>
 
 namespace gefen {
@@ -163,14 +161,7 @@ __host__ __device__ inline bool tile_coords(int M, int N, int bm, int bn, int sy
     return false;
 }
 
-// B_MN = false: B is [N, K] row-major (K-major operand). B_MN = true: B is [K, N] row-major
-// (MN-major operand), i.e. D = alpha * A * B + beta * C without any transposed copy of B.
-// A_MN: likewise A given as [K, M] row-major (D = alpha * A^T * B ...), used for the Gram matrix of a
-// tall matrix, Y^T Y, without transposing Y.
-// Variants whose ring is at most 96 KB run two CTAs per SM: the epilogue of one overlaps the main
-// loop of the other (each holds BN <= 256 of the 512 TMEM columns).
-// GROUP (a persistent variant): the launch computes the products of many matrices; a tile names its product, whose
-// tensor maps and sizes come from global memory (the host has copied them there before the launch).
+// A tile of a launch: its operands, its product's sizes and its place.
 struct TileView {
     const CUtensorMap* map_a;
     const CUtensorMap* map_b;
@@ -309,6 +300,14 @@ __device__ __forceinline__ bool epilogue_tile(const GemmArgs& args, const TileVi
     return true;
 }
 
+// B_MN = false: B is [N, K] row-major (K-major operand). B_MN = true: B is [K, N] row-major
+// (MN-major operand), i.e. D = alpha * A * B + beta * C without any transposed copy of B.
+// A_MN: likewise A given as [K, M] row-major (D = alpha * A^T * B ...), used for the Gram matrix of a
+// tall matrix, Y^T Y, without transposing Y.
+// Variants whose ring is at most 96 KB run two CTAs per SM: the epilogue of one overlaps the main
+// loop of the other (each holds BN <= 256 of the 512 TMEM columns).
+// GROUP (a persistent variant): the launch computes the products of many matrices; a tile names its product, whose
+// tensor maps and sizes come from global memory (the host has copied them there before the launch).
 template <int BN, int STAGES, bool A_MN, bool B_MN, bool PERSIST, bool GROUP = false>
 __global__ void __launch_bounds__(kGemmThreads, (STAGES * (kBM + BN) * kBK * 2 <= 96 * 1024) ? 2 : 1) ns_gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a,
                                                                      const __grid_constant__ CUtensorMap map_b,
@@ -951,8 +950,8 @@ static int ns_gemm(const void* a, bool a_is_km, const void* b, bool b_is_kn, con
     return launch_gemm<128, 6, false, false>(ma, mb, args, stream);
 }
 
-// The whole Newton-Schulz iteration of one matrix, enqueued from native code (fifteen GEMM launches
-// for five steps) so that the host cost per product is a tensor-map encode and a launch.
+// The Newton-Schulz iteration of one already normalised matrix in the caller's buffers, for callers of the C interface
+// (the package itself runs groups, see below): fifteen GEMM launches for five steps, a tall matrix as it lies (Y^T Y, Y B).
 static int enqueue_newton_schulz(void* x0, void* x1, void* gram, void* poly, int rows, int cols, int steps, double a,
                                  double b, double c, int* status, void* stream) {
     const int m = rows < cols ? rows : cols;
@@ -982,79 +981,12 @@ static int enqueue_newton_schulz(void* x0, void* x1, void* gram, void* poly, int
     return GEFEN_B200_OK;
 }
 
-// The chain is the same fifteen launches whenever buffers, shape and coefficients repeat (an optimizer
-// calls it for every matrix of a shape with the same scratch buffers, every step): from the second
-// identical call on it is replayed as one CUDA graph, which shortens the gaps between the dependent
-// launches. The first call runs eagerly (it also configures the kernels); the capture happens on a
-// private stream in thread-local mode, and the graph is launched into the caller's stream.
-// GEFEN_B200_NS_GRAPH=0 keeps every call eager.
-namespace {
-struct ChainKey {
-    int dev, rows, cols, steps;
-    void *x0, *x1, *gram, *poly, *status;
-    double a, b, c;
-    bool operator<(const ChainKey& o) const {
-        return std::tie(dev, rows, cols, steps, x0, x1, gram, poly, status, a, b, c) <
-               std::tie(o.dev, o.rows, o.cols, o.steps, o.x0, o.x1, o.gram, o.poly, o.status, o.a, o.b, o.c);
-    }
-};
-std::mutex g_chain_mutex;
-std::map<ChainKey, cudaGraphExec_t> g_chain_graphs;   // nullptr: seen once, not captured yet
-cudaStream_t g_capture_stream[64];
-constexpr size_t kMaxChainGraphs = 64;
-}  // namespace
-
 extern "C" int gefen_b200_newton_schulz(void* x0, void* x1, void* gram, void* poly, int rows, int cols, int steps,
                                         double a, double b, double c, int* status, void* stream) {
     GEFEN_CHECK_ARG(x0 && x1 && gram && poly, "Expected non-null buffers.");
     GEFEN_CHECK_ARG(rows > 0 && cols > 0 && rows % 8 == 0 && cols % 8 == 0, "Expected dimensions that are multiples of 8.");
     GEFEN_CHECK_ARG(steps >= 0 && steps < 100, "Number of steps must be less than 100.");
-    static int use_graphs = -1;
-    if (use_graphs < 0) {
-        const char* e = getenv("GEFEN_B200_NS_GRAPH");
-        use_graphs = (e != nullptr && e[0] == '0') ? 0 : 1;
-    }
-    int dev = 0;
-    GEFEN_CHECK_CUDA(cudaGetDevice(&dev));
-    if (!use_graphs || steps == 0 || dev < 0 || dev >= 64)
-        return enqueue_newton_schulz(x0, x1, gram, poly, rows, cols, steps, a, b, c, status, stream);
-
-    const ChainKey key{dev, rows, cols, steps, x0, x1, gram, poly, status, a, b, c};
-    std::lock_guard<std::mutex> lock(g_chain_mutex);
-    auto it = g_chain_graphs.find(key);
-    if (it == g_chain_graphs.end()) {
-        if (g_chain_graphs.size() >= kMaxChainGraphs) {   // callers whose buffers keep moving: start over
-            for (auto& kv : g_chain_graphs)
-                if (kv.second != nullptr) cudaGraphExecDestroy(kv.second);
-            g_chain_graphs.clear();
-        }
-        g_chain_graphs[key] = nullptr;
-        return enqueue_newton_schulz(x0, x1, gram, poly, rows, cols, steps, a, b, c, status, stream);
-    }
-    if (it->second == nullptr) {
-        if (g_capture_stream[dev] == nullptr)
-            GEFEN_CHECK_CUDA(cudaStreamCreateWithFlags(&g_capture_stream[dev], cudaStreamNonBlocking));
-        cudaStream_t cs = g_capture_stream[dev];
-        cudaGraph_t graph = nullptr;
-        cudaGraphExec_t exec = nullptr;
-        bool ok = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
-        if (ok) {
-            const int rc = enqueue_newton_schulz(x0, x1, gram, poly, rows, cols, steps, a, b, c, status, cs);
-            const cudaError_t end = cudaStreamEndCapture(cs, &graph);
-            ok = rc == GEFEN_B200_OK && end == cudaSuccess && graph != nullptr;
-        }
-        if (ok) ok = cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
-        if (graph != nullptr) cudaGraphDestroy(graph);
-        if (!ok) {   // leave this chain eager for good
-            cudaGetLastError();
-            g_chain_graphs.erase(it);
-            use_graphs = 0;
-            return enqueue_newton_schulz(x0, x1, gram, poly, rows, cols, steps, a, b, c, status, stream);
-        }
-        it->second = exec;
-    }
-    GEFEN_CHECK_CUDA(cudaGraphLaunch(it->second, static_cast<cudaStream_t>(stream)));
-    return GEFEN_B200_OK;
+    return enqueue_newton_schulz(x0, x1, gram, poly, rows, cols, steps, a, b, c, status, stream);
 }
 
 extern "C" int gefen_b200_ns_gemm_tn(const void* a, const void* b, const void* c, void* d, void* dt, int M, int N, int K,

@@ -107,6 +107,32 @@ def test_step_of_float64_parameters(cuda_device, monkeypatch):
             assert torch.equal(p.detach(), want)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(64, 200), (200, 64), (768, 768), (1032, 264), (256, 2304)])
+@pytest.mark.parametrize("steps", [1, 4, 5])
+def test_single_matrix_entry_of_the_c_interface(cuda_device, shape, steps):
+    """gefen_b200_newton_schulz on a normalised matrix in the caller's buffers, wide and tall."""
+    from gefen_b200 import _lib, newton_schulz as ns
+
+    gen = torch.Generator(device=cuda_device).manual_seed(steps)
+    x = torch.randn(shape, generator=gen, device=cuda_device).bfloat16()
+    x = x / x.norm()
+    m = min(shape)
+    x0, x1 = x.clone(), torch.full_like(x, float("nan"))
+    gram, poly = (torch.full((m, m), float("nan"), dtype=torch.bfloat16, device=cuda_device) for _ in range(2))
+    _lib.check(_lib.load().gefen_b200_newton_schulz(
+        _lib.ptr(x0), _lib.ptr(x1), _lib.ptr(gram), _lib.ptr(poly), shape[0], shape[1], steps, *NS,
+        _lib.ptr(ns._status(cuda_device)), _lib.current_stream(cuda_device)))
+    got = (x1 if steps % 2 else x0).float()
+    ns.check_status(cuda_device)
+    want = x.T if shape[0] > shape[1] else x
+    for _ in range(steps):
+        g = want @ want.T
+        want = torch.addmm(want, torch.addmm(g, g, g, beta=NS[1], alpha=NS[2]), want, beta=NS[0])
+    want = (want.T if shape[0] > shape[1] else want).float()
+    assert float((got - want).norm() / want.norm()) <= 2e-2
+
+
 def test_runs_of_a_group():
     from gefen_b200 import newton_schulz as ns
 
