@@ -65,7 +65,9 @@ def largest_divisor_at_most(value: int, limit: int) -> int:
         raise ValueError("Expected limit to be positive, got {}".format(limit))
     if value <= limit:
         return value
-    return next(d for d in range(limit, 0, -1) if value % d == 0)
+    if limit <= 4096:   # (fewer trial divisions than all divisors would take)
+        return next(d for d in range(limit, 0, -1) if value % d == 0)
+    return partitioning.divisors(value, max_divisor=limit)[-1]
 
 
 def _local(tensor, what: str) -> torch.Tensor:

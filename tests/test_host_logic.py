@@ -227,3 +227,15 @@ def test_status_word_names_its_cause(monkeypatch):
         assert all((text in str(error.value)) == (text in texts) for text in ("waiting", "out of place"))
     monkeypatch.setattr(_lib, "step_status", lambda device, clear=True: 0)
     _lib.check_step_status(None)
+
+
+def test_largest_divisor_below_a_large_limit():
+    """The work is bounded by the square root of the value, whatever the limit."""
+    from gefen_b200.gefen import largest_divisor_at_most
+
+    assert largest_divisor_at_most(10 ** 12 + 39, 10 ** 11) == 1          # a prime
+    assert largest_divisor_at_most(3 * 999999937, 10 ** 9) == 999999937   # its larger factor
+    for value in list(range(1, 300)) + [768 * 50257, 4096 * 4097]:
+        for limit in (1, 2, 7, 255, 256, 4096, 4097, 10 ** 6):
+            want = value if value <= limit else max(d for d in range(1, limit + 1) if value % d == 0)
+            assert largest_divisor_at_most(value, limit) == want
