@@ -168,8 +168,8 @@ def test_largest_group_is_what_the_library_takes():
     [(768, 3072)] * 5 + [(3072, 768)] * 5 + [(768, 768), (776, 1000), (200, 900), (8, 16)] * 2,
 ])
 def test_groups_that_fill_the_gpu(cuda_device, shapes):
-    """Enough tiles for pairs of CTAs: every matrix against torch's chain and, up to a bf16 rounding of a few elements
-    whose sums are added up in another order, against the same matrix alone (smaller tiles, single CTAs)."""
+    """Enough tiles for pairs of CTAs: every matrix against torch's chain and, bit for bit, against the same matrix alone
+    (smaller tiles, single CTAs): a sharded run groups the matrices otherwise than one process and has to give the same."""
     from gefen_b200 import newton_schulz as ns
 
     gen = torch.Generator(device=cuda_device).manual_seed(7)
@@ -186,5 +186,41 @@ def test_groups_that_fill_the_gpu(cuda_device, shapes):
             x = torch.addmm(x, torch.addmm(gram, gram, gram, beta=NS[1], alpha=NS[2]), x, beta=NS[0])
         want = (x.T if g.shape[0] > g.shape[1] else x).float()
         assert float((got - want).norm() / want.norm()) <= 2e-2, shapes[i]
-        alone = ns.zeropower_via_newtonschulz(g, NS, 5, 1e-7).float()
-        assert float((got - alone).norm() / alone.norm()) <= 1e-2, shapes[i]
+        assert torch.equal(group.result(i), ns.zeropower_via_newtonschulz(g, NS, 5, 1e-7)), shapes[i]
+
+
+@pytest.mark.gpu
+def test_mixed_settings_and_strides_in_one_step(cuda_device):
+    """Parameter groups with iterations of their own, and parameters that are not contiguous (torch updates their run):
+    every matrix moves by the orthogonalisation of its own momentum."""
+    from gefen_b200 import GefenMuon, newton_schulz as ns
+
+    gen = torch.Generator(device=cuda_device).manual_seed(6)
+    shapes = [(64, 128), (96, 64), (48, 36), (128, 128), (40, 200), (72, 24)]
+    settings = [dict(ns_steps=5, eps=1e-7), dict(ns_steps=3, eps=1e-7), dict(ns_steps=5, eps=1e-3)]
+    params = []
+    for i, s in enumerate(shapes):
+        t = torch.randn((s[1], s[0]) if i in (1, 4) else s, generator=gen, device=cuda_device) * 0.02
+        params.append(torch.nn.Parameter(t.t() if i in (1, 4) else t))
+    assert not params[1].is_contiguous() and not params[4].is_contiguous()
+    opt = GefenMuon(params, lr=0.02, weight_decay=0.1, nesterov=False)
+    by_param = {}
+    for group in opt.param_groups:   # (one per parameter)
+        for p in group["params"]:
+            i = next(k for k, q in enumerate(params) if q is p)
+            group.update(settings[(i // 2) % 3])
+            by_param[i] = group
+    for step in range(2):
+        for p in params:
+            p.grad = torch.randn(p.shape, generator=gen, device=cuda_device) * 1e-3
+        before = [p.detach().clone() for p in params]
+        opt.step()
+        for i, (p, old) in enumerate(zip(params, before)):
+            st = opt.state[p]
+            period = st["automatic_period"]
+            block = opt._period_one_divisor_from_state(st, p.numel()) if period == 1 else period
+            momentum = opt._gefen_codebook[st["m_codebook"].reshape(-1, block).long()] * st["m_magnitude"]
+            group = by_param[i]
+            ortho = ns.zeropower_via_newtonschulz(momentum.reshape(p.shape), NS, group["ns_steps"], group["eps"])
+            want = old.mul_(1 - 0.02 * 0.1).add_(ortho, alpha=-0.02 * max(1, p.shape[0] / p.shape[1]) ** 0.5)
+            assert torch.equal(p.detach(), want), (step, i)
