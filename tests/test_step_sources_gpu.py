@@ -30,7 +30,8 @@ def _step(device, dtype, nb, period, sources, copies, steps=2, wd=0.1):
     peers = np.array([(r + 1) * pad * params.element_size() for r in range(copies)], dtype=np.int64)
     grads = np.zeros(max(sources, 1), dtype=np.int64)
     for step in range(steps):
-        g = make_grad((nb, period), period, 0, step, dtype).to(device)
+        # 8 significant bits (fp16: 11): the sum of up to eight equal values takes three more, exact in fp32
+        g = make_grad((nb, period), period, 0, step, dtype if dtype == torch.float16 else torch.bfloat16).to(dtype).to(device)
         rows["p"], rows["g"], rows["codes"], rows["mag"], rows["v"] = (t.data_ptr() for t in (params, g, codes, mag, v))
         rows["num_blocks"], rows["period"], rows["mag_dtype"], rows["v_dtype"] = nb, period, _lib.F32, _lib.F32
         rows["flags"] = _lib.STEP_FUSE_VMEAN | (_lib.STEP_WEIGHT_DECAY if wd else 0)
