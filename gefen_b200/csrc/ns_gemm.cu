@@ -1239,8 +1239,11 @@ __global__ void __launch_bounds__(kElemThreads) ns_apply_kernel(const NsMatrix* 
 
 // The plan of a group: five lists of products (Gram matrix of x0 / of x1, polynomial, update x0 -> x1 / x1 -> x0) and
 // two lists of tiles (of the symmetric m x m results, of the m x k results).
-struct GroupShape {
+struct TileKind {
     int bm, bn;            // 256 x 256: pairs of CTAs
+};
+struct GroupShape {
+    TileKind gram, update;
     int64_t gram_tiles, update_tiles, entries_bytes, bytes;
 };
 static void wide_dims(const NsMatrix& m, int* wr, int* wc) {
@@ -1248,23 +1251,39 @@ static void wide_dims(const NsMatrix& m, int* wr, int* wc) {
     *wr = static_cast<int>(std::min(a, b));
     *wc = static_cast<int>(std::max(a, b));
 }
+// Kind of tiles for a list of products: the fewest rounds of the persistent CTAs, weighed with what a round of the kind
+// takes (all kinds give the same bits). Chosen for the symmetric products and the updates apart. Five iterations of
+// single matrices and groups, us, with the symmetric products forced to 256 x 256 / 128 x 256 / 128 x 128, then the updates:
+//   768 x 2304        312 / 302 / 261     280 / 281 / 262        2048 x 6144      652 / 646 / 608     616 / 622 / 754
+//   2048 x 2048       402 / 382 / 360     358 / 352 / 391        2560 x 2560      524 / 513 / 616     522 / 534 / 571
+//   4096 x 4096       1357 / 1378 / 1787  1318 / 1420 / 1718     8 of 1024 x 4096 862 / 879 / 785     821 / 867 / 966
+// (One kind for all products, the first whose symmetric tiles fill the GPU, took 797 us for 2048 x 6144 and 436 for
+// 2048 x 2048 where this rule takes 620 and 355.)
+static TileKind choose_tiles(const NsMatrix* mats, int n, bool symmetric, int64_t* tiles) {
+    static const struct { TileKind kind; double round; } kinds[3] = {{{256, 256}, 1.0}, {{128, 256}, 1.15}, {{128, 128}, 0.88}};
+    TileKind best = {};
+    double least = 0.0;
+    for (const auto& k : kinds) {
+        int64_t count = 0;
+        for (int i = 0; i < n; ++i) {
+            int m, c;
+            wide_dims(mats[i], &m, &c);
+            count += count_tiles(m, symmetric ? m : c, k.kind.bm, k.kind.bn, symmetric);
+        }
+        const int64_t at_once = k.kind.bm == 256 ? sm_count() / 2 : sm_count();
+        const double cost = static_cast<double>((count + at_once - 1) / at_once) * k.round;
+        if (best.bm == 0 || cost < least) {
+            best = k.kind;
+            least = cost;
+            *tiles = count;
+        }
+    }
+    return best;
+}
 static GroupShape group_shape(const NsMatrix* mats, int n) {
     GroupShape g;
-    // Tiles of 256 x 256 on pairs of CTAs have the best ratio of operand bytes to work, 128 x 256 the next; where a
-    // kind does not fill the GPU the next smaller one is taken (measurements: see launch_group)
-    static const int kinds[3][2] = {{256, 256}, {128, 256}, {128, 128}};
-    for (int kind = 0; kind < 3; ++kind) {
-        g.bm = kinds[kind][0];
-        g.bn = kinds[kind][1];
-        g.gram_tiles = g.update_tiles = 0;
-        for (int i = 0; i < n; ++i) {
-            int m, k;
-            wide_dims(mats[i], &m, &k);
-            g.gram_tiles += count_tiles(m, m, g.bm, g.bn, 1);
-            g.update_tiles += count_tiles(m, k, g.bm, g.bn, 0);
-        }
-        if (g.gram_tiles * (g.bm / kBM) >= sm_count()) break;
-    }
+    g.gram = choose_tiles(mats, n, true, &g.gram_tiles);
+    g.update = choose_tiles(mats, n, false, &g.update_tiles);
     g.entries_bytes = static_cast<int64_t>(5) * n * static_cast<int64_t>(sizeof(GroupEntry));
     g.bytes = g.entries_bytes + (g.gram_tiles + g.update_tiles) * static_cast<int64_t>(sizeof(GroupTile));
     return g;
@@ -1321,15 +1340,15 @@ static int build_group_plan(const NsMatrix* mats, int n, const GroupShape& g, st
         fill(3, poly, x_mn[0], mat.x0, mat.x1, k, m);
         fill(4, poly, x_mn[1], mat.x1, mat.x0, k, m);
         int m0, n0;
-        for (int64_t t = 0; tile_coords(m, m, g.bm, g.bn, 1, t, &m0, &n0); ++t) gram_tiles[gt++] = {i, m0, n0, 0};
-        for (int64_t t = 0; tile_coords(m, k, g.bm, g.bn, 0, t, &m0, &n0); ++t) update_tiles[ut++] = {i, m0, n0, 0};
+        for (int64_t t = 0; tile_coords(m, m, g.gram.bm, g.gram.bn, 1, t, &m0, &n0); ++t) gram_tiles[gt++] = {i, m0, n0, 0};
+        for (int64_t t = 0; tile_coords(m, k, g.update.bm, g.update.bn, 0, t, &m0, &n0); ++t) update_tiles[ut++] = {i, m0, n0, 0};
     }
     return GEFEN_B200_OK;
 }
 
 template <bool B_MN>
-static int launch_group(const GroupShape& g, GemmArgs args, cudaStream_t stream) {
-    if (g.bm == 256) {
+static int launch_group(const TileKind& kind, GemmArgs args, cudaStream_t stream) {
+    if (kind.bm == 256) {
         constexpr int smem = kPairStages * (kBM + kPairBN / 2) * kBK * 2 + 4 * 32 * kStagePitch * 2 + 1024;
         static std::once_flag configured[64];
         int dev = 0;
@@ -1346,7 +1365,7 @@ static int launch_group(const GroupShape& g, GemmArgs args, cudaStream_t stream)
         return GEFEN_B200_OK;
     }
     const CUtensorMap none = {};
-    if (g.bn == 256) return launch_gemm_variant<256, 4, false, B_MN, true, true>(none, none, args, stream);
+    if (kind.bn == 256) return launch_gemm_variant<256, 4, false, B_MN, true, true>(none, none, args, stream);
     return launch_gemm_variant<128, 6, false, B_MN, true, true>(none, none, args, stream);
 }
 
@@ -1451,18 +1470,18 @@ extern "C" int gefen_b200_ns_group(const gefen_b200_ns_matrix_t* mats, int n, co
         args.entries = entries + (it & 1) * n;
         args.alpha = 1.0f;
         args.beta = 0.0f;
-        if ((rc = launch_group<false>(g, args, stream)) != GEFEN_B200_OK) return rc;
+        if ((rc = launch_group<false>(g.gram, args, stream)) != GEFEN_B200_OK) return rc;
         args.entries = entries + 2 * n;
         args.alpha = static_cast<float>(c);
         args.beta = static_cast<float>(b);
-        if ((rc = launch_group<false>(g, args, stream)) != GEFEN_B200_OK) return rc;
+        if ((rc = launch_group<false>(g.gram, args, stream)) != GEFEN_B200_OK) return rc;
         args.tiles = tiles + g.gram_tiles;
         args.n_tiles = static_cast<int>(g.update_tiles);
         args.symmetric = 0;
         args.entries = entries + (3 + (it & 1)) * n;
         args.alpha = 1.0f;
         args.beta = static_cast<float>(a);
-        if ((rc = launch_group<true>(g, args, stream)) != GEFEN_B200_OK) return rc;
+        if ((rc = launch_group<true>(g.update, args, stream)) != GEFEN_B200_OK) return rc;
     }
     return GEFEN_B200_OK;
 }
