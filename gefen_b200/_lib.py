@@ -194,11 +194,6 @@ def current_stream(device) -> ctypes.c_void_p:
     return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
 
 
-def upload(dst: torch.Tensor, host: np.ndarray) -> None:
-    """Copies a table to the device in stream order (see gefen_b200_upload). The current device is dst's."""
-    check(load().gefen_b200_upload(ptr(dst), host.ctypes.data, host.nbytes, current_stream(dst.device)))
-
-
 class device_guard:
     """Makes `device` current for the duration of a call (reference: c10::cuda::CUDAGuard)."""
 

@@ -128,13 +128,19 @@ class MatrixGroup:
                 offset += n
         if offset > scratch.numel():
             raise ValueError("Expected {} elements of scratch for the group, got {}".format(offset, scratch.numel()))
-        host = np.empty(lib.gefen_b200_ns_group_plan_bytes(self.mats.ctypes.data, len(shapes)), dtype=np.uint8)
-        _lib.check(lib.gefen_b200_ns_group_plan(self.mats.ctypes.data, len(shapes), host.ctypes.data))
-        self.plan = torch.empty(host.nbytes, dtype=torch.uint8, device=self.device)
-        with _lib.device_guard(self.device):
-            _lib.upload(self.plan, host)
-        self.table = torch.empty(self.mats.nbytes, dtype=torch.uint8, device=self.device)
-        self.partials = torch.empty(64 * len(shapes), dtype=torch.float32, device=self.device)
+        # one device buffer: plan, matrix table, partial norms; the first two come from one host buffer
+        n = len(shapes)
+        plan_bytes = lib.gefen_b200_ns_group_plan_bytes(self.mats.ctypes.data, n)
+        place = (plan_bytes + 63) // 64 * 64
+        self._host = np.zeros(place + self.mats.nbytes, dtype=np.uint8)
+        _lib.check(lib.gefen_b200_ns_group_plan(self.mats.ctypes.data, n, self._host.ctypes.data))
+        self._host[place:] = self.mats.view(np.uint8)
+        self.mats = self._host[place:].view(_lib.NS_MATRIX_DTYPE)
+        self._address = self._host.ctypes.data
+        self._place, self._uploaded = place, 0      # bytes of the host buffer that the device has for good
+        parts = (place + self.mats.nbytes + 15) // 16 * 16
+        self.tables = torch.empty(parts + 256 * n, dtype=torch.uint8, device=self.device)
+        self._partials = parts
         self.steps = 0
 
     def run(self, sources: Sequence[torch.Tensor], ns_coefficients, ns_steps: int, eps: float) -> None:
@@ -143,12 +149,15 @@ class MatrixGroup:
         a, b, c = ns_coefficients
         self.mats["src"] = [t.data_ptr() for t in sources]
         self.steps = int(ns_steps)
+        lib, tables, mats, sent = _lib.load(), self.tables.data_ptr(), self._address + self._place, self._uploaded
         with _lib.device_guard(self.device):
-            _lib.upload(self.table, self.mats)
-            _lib.check(_lib.load().gefen_b200_ns_group(
-                self.mats.ctypes.data, len(self.mats), _lib.ptr(self.table), _lib.ptr(self.plan), _lib.ptr(self.partials),
-                _lib.dtype_tag(sources[0].dtype), self.steps, float(a), float(b), float(c), float(eps),
-                _lib.ptr(_status(self.device)), _lib.current_stream(self.device)))
+            stream = _lib.current_stream(self.device)
+            _lib.check(lib.gefen_b200_upload(tables + sent, self._address + sent, self._host.nbytes - sent, stream))
+            if not sent and not torch.cuda.is_current_stream_capturing():
+                self._uploaded = self._place
+            _lib.check(lib.gefen_b200_ns_group(
+                mats, len(self.mats), tables + self._place, tables, tables + self._partials, _lib.dtype_tag(sources[0].dtype),
+                self.steps, float(a), float(b), float(c), float(eps), _lib.ptr(_status(self.device)), stream))
 
     def update_of(self, params: Sequence[torch.Tensor], wd_muls, alphas) -> None:
         self.mats["p"] = [p.data_ptr() for p in params]
@@ -160,7 +169,7 @@ class MatrixGroup:
         n_peers = 0 if peers is None else len(peers)
         with _lib.device_guard(self.device):
             _lib.check(_lib.load().gefen_b200_ns_group_apply(
-                self.mats.ctypes.data, len(self.mats), _lib.ptr(self.table), _lib.dtype_tag(dtype), self.steps,
+                self._address + self._place, len(self.mats), self.tables.data_ptr() + self._place, _lib.dtype_tag(dtype), self.steps,
                 peers.ctypes.data if n_peers else None, n_peers, _lib.current_stream(self.device)))
 
     def result(self, i: int) -> torch.Tensor:

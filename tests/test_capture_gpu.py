@@ -17,17 +17,21 @@ def test_upload(cuda_device, nbytes, captured):
     host = np.random.default_rng(nbytes).integers(0, 256, nbytes, dtype=np.uint8)
     want = torch.from_numpy(host.copy())
     dst = torch.zeros(nbytes + 16, dtype=torch.uint8, device=cuda_device)
+
+    def upload():
+        _lib.check(_lib.load().gefen_b200_upload(_lib.ptr(dst), host.ctypes.data, nbytes, _lib.current_stream(cuda_device)))
+
     stream = torch.cuda.Stream()
     stream.wait_stream(torch.cuda.current_stream())
     with torch.cuda.stream(stream):
         if captured:
             graph = torch.cuda.CUDAGraph()
             with torch.cuda.graph(graph, stream=stream):
-                _lib.upload(dst, host)
+                upload()
             host[:] = 0
             graph.replay()
         else:
-            _lib.upload(dst, host)
+            upload()
             host[:] = 0
     stream.synchronize()
     assert torch.equal(dst[:nbytes].cpu(), want) and not bool(dst[nbytes:].any())
