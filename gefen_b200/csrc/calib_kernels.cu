@@ -265,6 +265,8 @@ __device__ __forceinline__ void hist_unit(const HistEntry& e, long long unit, in
                     }
                 }
             };
+            // (once per block in every type: here fp32 gains too, 134 M values in blocks of 64 / 768 / 2048 0.587 / 0.163 /
+            // 0.159 ms against 0.726 / 0.185 / 0.179 with a choice per element)
             if (divide.fast) second_look([&](float v) { return divide.quick(v); });
             else second_look([&](float v) { return divide.careful(v); });
         }
