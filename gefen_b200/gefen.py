@@ -421,6 +421,13 @@ class Gefen(torch.optim.Optimizer):
                 work.append((group, name, p, local_p, grad))
         return work
 
+    def _require_codebook_beside(self, work) -> None:
+        """The kernels read the codebook's tables through a plain pointer on the tensors' device."""
+        for group, name, p, local_p, grad in work:
+            if grad.device != self._gefen_codebook.device:
+                raise ValueError("Expected {} on the device of the Gefen codebook, {}, got {}.".format(
+                    name, self._gefen_codebook.device, grad.device))
+
     def _step_tables(self, work, muon: bool = False, ranges=None):
         """Builds (or reuses) the launch tables for `work`. Static columns are cached; the pointer
         and scalar columns are refreshed by the caller every step. ranges: {id(param): (first block, end
@@ -508,6 +515,7 @@ class Gefen(torch.optim.Optimizer):
             return
         if self._gefen_codebook is None:
             raise ValueError("Expected Gefen codebook to be initialized before fused update.")
+        self._require_codebook_beside(work)
         copies = []
         for i, (group, name, p, local_p, grad) in enumerate(work):
             self._ensure_state(name, p, local_p, grad)

@@ -157,6 +157,7 @@ class GefenMuon(Gefen):
             return
         if self._gefen_codebook is None:
             raise ValueError("Expected Gefen codebook to be initialized before fused GefenMuon update.")
+        self._require_codebook_beside(work)
         for i, (group, name, p, local_p, grad) in enumerate(work):
             if torch.is_complex(local_p):
                 raise RuntimeError("GefenMuon does not support complex parameters")

@@ -213,6 +213,11 @@ def test_tensors_of_two_devices_are_refused():
     grads = [SimpleNamespace(device=torch.device("cuda", i), numel=lambda: 64) for i in (0, 1)]
     with pytest.raises(ValueError, match="one device"):
         gefen_exact_histogram_many_cuda(grads, [8, 8], 4096)
+    # a step with a restored codebook, parameters on two devices
+    restored = SimpleNamespace(_gefen_codebook=grads[0])
+    Gefen._require_codebook_beside(restored, [(None, "a", None, None, grads[0])])
+    with pytest.raises(ValueError, match="device of the Gefen codebook"):
+        Gefen._require_codebook_beside(restored, [(None, n, None, None, g) for n, g in zip("ab", grads)])
     with pytest.raises(ValueError, match="one device"):
         Gefen._predict_periods(None, [("a", None, grads[0]), ("b", None, grads[1])])
 
