@@ -285,6 +285,14 @@ template <typename S, int V> struct Chunk {
             w[0] = __ldcs(reinterpret_cast<const unsigned short*>(p));
         }
     }
+    __device__ __forceinline__ void load_again_later(const void* base, long long chunk) {   // (V = 8; no streaming hint)
+        const uint4* p = reinterpret_cast<const uint4*>(static_cast<const char*>(base) + chunk * kBytes);
+#pragma unroll
+        for (int q = 0; q < kBytes / 16; ++q) {
+            const uint4 v = p[q];
+            w[4 * q] = v.x; w[4 * q + 1] = v.y; w[4 * q + 2] = v.z; w[4 * q + 3] = v.w;
+        }
+    }
     __device__ __forceinline__ void store(void* base, long long chunk) const {
         char* p = static_cast<char*>(base) + chunk * kBytes;
         if constexpr (kBytes >= 16) {
@@ -351,6 +359,10 @@ template <int V> struct CodeChunk {
         } else if constexpr (V == 4) w[0] = __ldcs(reinterpret_cast<const unsigned int*>(base) + chunk);
         else if constexpr (V == 2) w[0] = __ldcs(reinterpret_cast<const unsigned short*>(base) + chunk);
         else w[0] = __ldcs(base + chunk);
+    }
+    __device__ __forceinline__ void load_again_later(const uint8_t* base, long long chunk) {   // (V = 8; no streaming hint)
+        const uint2 v = reinterpret_cast<const uint2*>(base)[chunk];
+        w[0] = v.x; w[1] = v.y;
     }
     __device__ __forceinline__ void store(uint8_t* base, long long chunk) const {
         if constexpr (V == 8) reinterpret_cast<uint2*>(base)[chunk] = make_uint2(w[0], w[1]);
@@ -652,7 +664,7 @@ template <typename S> struct alignas(8) TensorSlot {
 // moment update, the running absmax and sum of squares, and the staging of the updated momenta.
 // SUMMED: g_blk is the multicast address of the block's gradients; a load returns the sum over the ranks,
 // which is scaled by `scale` and rounded to the gradient dtype as a reduce-scatter into it would leave it.
-template <typename S, int V, int U, bool GUARD, bool SUMMED>
+template <typename S, int V, int U, bool GUARD, bool SUMMED, bool STAGED = true>
 __device__ __forceinline__ void first_pass_group(const S* g_blk, const uint8_t* codes_in, float* stage, int half,
                                                  const LaneTables& t, int c0, int LANES, int nchunks, f32x2 mag2,
                                                  f32x2 beta2_, f32x2 omb2_, float scale, float& absmax, f32x2& sumsq2) {
@@ -662,9 +674,11 @@ __device__ __forceinline__ void first_pass_group(const S* g_blk, const uint8_t* 
     for (int u = 0; u < U; ++u) {
         const int c = c0 + LANES * u;
         if (!GUARD || c < nchunks) {
-            craw[u].load(codes_in, c);
+            if constexpr (STAGED) craw[u].load(codes_in, c);
+            else craw[u].load_again_later(codes_in, c);
             if (SUMMED) graw[u].load_sum(g_blk, c);
-            else graw[u].load(g_blk, c);
+            else if constexpr (STAGED) graw[u].load(g_blk, c);
+            else graw[u].load_again_later(g_blk, c);
         }
     }
 #pragma unroll
@@ -698,7 +712,7 @@ __device__ __forceinline__ void first_pass_group(const S* g_blk, const uint8_t* 
                     sumsq2 = fma2(g2, g2, sumsq2);
                 }
             }
-            stage_store<V>(stage, half, c, m);
+            if (STAGED) stage_store<V>(stage, half, c, m);
         }
     }
 }
@@ -839,6 +853,43 @@ __device__ __forceinline__ void reduce_pass_small(const StepLaunch& L, const S* 
     }
 }
 
+// Where the second pass takes a chunk's updated momenta from: the warp's staging slice, or, for blocks whose slices
+// would leave too few warps (see long_class), computed once more from codes and gradients, which L2 still holds; the
+// next chunk's are requested while this one is worked on. Both walk the chunks of a lane in order.
+template <typename S, int V, bool STAGED> struct Momenta {   // STAGED
+    const float* const stage;
+    const int half;
+    __device__ __forceinline__ Momenta(const float* s, int h, const uint8_t*, const S*, const LaneTables&, float, float, float)
+        : stage(s), half(h) {}
+    __device__ __forceinline__ void start(int, int, int) {}
+    __device__ __forceinline__ void take(int c, int, int, float (&m)[V]) { stage_load<V>(stage, half, c, m); }
+};
+template <typename S, int V> struct Momenta<S, V, false> {
+    const uint8_t* const codes;
+    const S* const g;
+    const LaneTables& t;
+    const f32x2 mag2, beta2_, omb2_;
+    CodeChunk<V> craw;
+    Chunk<S, V> graw;
+    __device__ __forceinline__ Momenta(const float*, int, const uint8_t* c, const S* gradients, const LaneTables& tables, float old_mag,
+                                       float beta1, float omb1)
+        : codes(c), g(gradients), t(tables), mag2(pair(old_mag, old_mag)), beta2_(pair(beta1, beta1)), omb2_(pair(omb1, omb1)) {}
+    __device__ __forceinline__ void start(int lane, int, int nchunks) {
+        if (lane < nchunks) { craw.load(codes, lane); graw.load(g, lane); }
+    }
+    __device__ __forceinline__ void take(int c, int LANES, int nchunks, float (&m)[V]) {
+        const CodeChunk<V> code = craw;
+        float gv[V];
+        graw.unpack(gv);
+        if (c + LANES < nchunks) { craw.load(codes, c + LANES); graw.load(g, c + LANES); }
+#pragma unroll
+        for (int i = 0; i < V; i += 2) {
+            const f32x2 cur = mul2(mag2, pair(t.value(t.row_of_byte(code.w[i >> 2], i & 3)), t.value(t.row_of_byte(code.w[i >> 2], (i & 3) + 1))));
+            unpair(fma2(beta2_, cur, mul2(omb2_, pair(gv[i], gv[i + 1]))), m[i], m[i + 1]);   // as first_pass_group
+        }
+    }
+};
+
 // One chunk of the re-encode and update of the common case (finite block, Gefen update of the parameters) with
 // everything that is fixed per launch or per tensor decided at compile time: WD = the decoupled weight decay of the
 // reference's separate multiply, STORE = 0 this GPU's copy only, 1 peer stores as well, 2 one multicast store, ONE =
@@ -846,11 +897,11 @@ __device__ __forceinline__ void reduce_pass_small(const StepLaunch& L, const S* 
 struct BlockScalars {
     f32x2 neg_absmax2, rinv2, step2, lr2, wd2;
 };
-template <typename S, int V, bool WD, int STORE, bool ONE>
-__device__ __forceinline__ void update_chunk(const StepLaunch& L, const LaneTables& t, const float* stage, int half,
+template <typename S, int V, bool WD, int STORE, bool ONE, typename M>
+__device__ __forceinline__ void update_chunk(const StepLaunch& L, const LaneTables& t, M& momenta, int LANES, int nchunks,
                                              uint8_t* codes, S* p_blk, Chunk<S, V> praw, int c, const BlockScalars& b) {
     float m[V];
-    stage_load<V>(stage, half, c, m);
+    momenta.take(c, LANES, nchunks, m);
     uint32_t row[V];
     encode<V, ONE>(m, b.neg_absmax2, b.rinv2, t, row);
     row_codes<V>(row).store(codes, c);
@@ -898,9 +949,8 @@ template <typename S, int V> struct Ahead {
 };
 // The chunks of one block: `full` rounds in which every lane of the warp has one, then the guarded rest. The
 // parameters of the next chunks are fetched while this one is encoded.
-template <typename S, int V, bool WD, int STORE, bool ONE>
-__device__ __forceinline__ void second_pass_common(const StepLaunch& L, const LaneTables& t, const float* stage,
-                                                   int half, uint8_t* codes, S* p_blk, Ahead<S, V>& ahead, int lane, int LANES,
+template <typename S, int V, bool WD, int STORE, bool ONE, typename M>
+__device__ __forceinline__ void second_pass_common(const StepLaunch& L, const LaneTables& t, M& momenta, uint8_t* codes, S* p_blk, Ahead<S, V>& ahead, int lane, int LANES,
                                                    int nchunks, int full, int rounds_all, const BlockScalars& b) {
     constexpr int D = Ahead<S, V>::kDepth;
     int c = lane;
@@ -908,7 +958,7 @@ __device__ __forceinline__ void second_pass_common(const StepLaunch& L, const La
     if constexpr (D == 1) {
         for (; it < full; ++it, c += LANES) {
             const Chunk<S, V> praw = ahead.take(0, p_blk, c, LANES, nchunks);
-            update_chunk<S, V, WD, STORE, ONE>(L, t, stage, half, codes, p_blk, praw, c, b);
+            update_chunk<S, V, WD, STORE, ONE>(L, t, momenta, LANES, nchunks, codes, p_blk, praw, c, b);
         }
     }
     for (; it < rounds_all; it += D, c += D * LANES) {
@@ -916,7 +966,7 @@ __device__ __forceinline__ void second_pass_common(const StepLaunch& L, const La
         for (int u = 0; u < D; ++u) {
             if (c + u * LANES < nchunks) {
                 const Chunk<S, V> praw = ahead.take(u, p_blk, c + u * LANES, LANES, nchunks);
-                update_chunk<S, V, WD, STORE, ONE>(L, t, stage, half, codes, p_blk, praw, c + u * LANES, b);
+                update_chunk<S, V, WD, STORE, ONE>(L, t, momenta, LANES, nchunks, codes, p_blk, praw, c + u * LANES, b);
             }
         }
     }
@@ -926,8 +976,8 @@ __device__ __forceinline__ void second_pass_common(const StepLaunch& L, const La
 // with the gradient when asked (torch: m.mul_(momentum).add_(g, alpha=1-momentum) on the rounded momentum,
 // reference gefen_muon.py:312-314; alpha travels in the descriptor's beta2), goes where the Gefen step keeps
 // the parameters. The gradient chunk of the next iteration is requested while this one is encoded.
-template <typename S, int V, bool NESTEROV>
-__device__ __forceinline__ void second_pass_muon(const LaneTables& t, const float* stage, int half, uint8_t* codes,
+template <typename S, int V, bool NESTEROV, typename M>
+__device__ __forceinline__ void second_pass_muon(const LaneTables& t, M& momenta, uint8_t* codes,
                                                  const S* g_blk, S* out_blk, int lane, int LANES, int nchunks, float absmax,
                                                  f32x2 neg_absmax2, f32x2 rinv2, float beta1, float alpha) {
     constexpr int D = Ahead<S, V>::kDepth;
@@ -941,7 +991,7 @@ __device__ __forceinline__ void second_pass_muon(const LaneTables& t, const floa
         Chunk<S, V> graw;
         if (NESTEROV) graw = ahead.take(u, g_blk, c, LANES, nchunks);
         float m[V];
-        stage_load<V>(stage, half, c, m);
+        momenta.take(c, LANES, nchunks, m);
         uint32_t row[V];
         encode<V, false>(m, neg_absmax2, rinv2, t, row);
         row_codes<V>(row).store(codes, c);
@@ -970,7 +1020,7 @@ __device__ __forceinline__ void second_pass_muon(const LaneTables& t, const floa
 // GSRC: where the gradients come from: 0 = this GPU's buffer, 1 = averaged over the ranks' buffers with peer
 // loads, 2 = summed by the switch through the multicast mapping (StepLaunch::grad_mc_delta). Chunks below eight elements
 // know 0 and 1 only: 1 is every launch with peers, gradients of this GPU's buffer (no sources) included.
-template <typename S, int V, int GSRC, bool FULL>
+template <typename S, int V, int GSRC, bool FULL, bool STAGED>
 __device__ __forceinline__ void warp_block_step(const TensorSlot<S>& t, long long unit, const StepLaunch& L, const LaneTables& tables,
                                                 float* stage, int warp_lane) {
     const float* const stepsize = L.stepsize;
@@ -1043,11 +1093,11 @@ __device__ __forceinline__ void warp_block_step(const TensorSlot<S>& t, long lon
         int c0 = 0;
         if (all_valid && sizeof(S) == 2) {   // (fp32: the second copy of the loop costs registers; measured slower)
             for (; c0 + LANES * U <= chunks; c0 += LANES * U)
-                first_pass_group<S, V, U, false, SUMMED>(g_src, codes, stage, half, tables, c0 + lane, LANES, nchunks, mag2, beta2_, omb2_,
+                first_pass_group<S, V, U, false, SUMMED, STAGED>(g_src, codes, stage, half, tables, c0 + lane, LANES, nchunks, mag2, beta2_, omb2_,
                                                          scale, absmax, sumsq2);
         }
         for (; c0 < chunks; c0 += LANES * U)
-            first_pass_group<S, V, U, true, SUMMED>(g_src, codes, stage, half, tables, c0 + lane, LANES, nchunks, mag2, beta2_, omb2_,
+            first_pass_group<S, V, U, true, SUMMED, STAGED>(g_src, codes, stage, half, tables, c0 + lane, LANES, nchunks, mag2, beta2_, omb2_,
                                                     scale, absmax, sumsq2);
     }
     {   // (the same two partial sums wherever the gradients come from: a rank's second moments are a single process's)
@@ -1075,15 +1125,17 @@ __device__ __forceinline__ void warp_block_step(const TensorSlot<S>& t, long lon
         }
     }
     __syncwarp();  // staged momenta are visible to the whole warp; every lane has read the old magnitude
+    Momenta<S, V, STAGED> momenta(stage, half, codes, g_blk, tables, old_mag, beta1, omb1);
 
     // ---- rare: a NaN or Inf in the block. The reference's max ignores NaN; redo it that way and
     // let the exact (threshold) quantiser handle non-finite quotients.
     bool exact_path = false;
     if (__any_sync(0xffffffffu, !(absmax <= 3.0e38f))) {   // warp-uniform: the reduction below shuffles
         float mx = 0.0f;
+        momenta.start(lane, LANES, nchunks);
         for (int c = lane; c < nchunks; c += LANES) {
             float m[V];
-            stage_load<V>(stage, half, c, m);
+            momenta.take(c, LANES, nchunks, m);
 #pragma unroll
             for (int i = 0; i < V; ++i) mx = fmaxf(mx, fabsf(m[i]));
         }
@@ -1102,12 +1154,13 @@ __device__ __forceinline__ void warp_block_step(const TensorSlot<S>& t, long lon
 
     // ---- re-encode and update; the parameters of the next chunk are fetched while this one is encoded
     if (!kEarlyParams && load_p) ahead.start(p_blk, lane, LANES, nchunks);
+    momenta.start(lane, LANES, nchunks);
     // The common case takes the loop that was compiled for it (the conditions are uniform over the warp: they
     // come from the launch and the tensor's descriptor, and a warp's blocks go one way together).
     if (__all_sync(0xffffffffu, fastdiv || !valid) && !muon && do_update) {
         const int rounds_all = (chunks + LANES - 1) >> shift, full = all_valid ? chunks >> shift : 0;
 #define GEFEN_SECOND_PASS(WD_, STORE_, ONE_)                                                                                       \
-    second_pass_common<S, V, WD_, STORE_, ONE_>(L, tables, stage, half, codes, p_blk, ahead, lane, LANES, nchunks, full,        \
+    second_pass_common<S, V, WD_, STORE_, ONE_>(L, tables, momenta, codes, p_blk, ahead, lane, LANES, nchunks, full,             \
                                                 rounds_all, bs)
         if constexpr (V == 8) {
             const int store = param_mc != 0 ? 2 : (n_peers > 0 ? 1 : 0);
@@ -1125,9 +1178,9 @@ __device__ __forceinline__ void warp_block_step(const TensorSlot<S>& t, long lon
         return;
     }
     if (GSRC == 0 && muon && __all_sync(0xffffffffu, fastdiv || !valid)) {
-        if (nesterov) second_pass_muon<S, V, true>(tables, stage, half, codes, g_blk, p_blk, lane, LANES, nchunks, absmax,
+        if (nesterov) second_pass_muon<S, V, true>(tables, momenta, codes, g_blk, p_blk, lane, LANES, nchunks, absmax,
                                                    bs.neg_absmax2, bs.rinv2, beta1, t.beta2);
-        else second_pass_muon<S, V, false>(tables, stage, half, codes, g_blk, p_blk, lane, LANES, nchunks, absmax, bs.neg_absmax2,
+        else second_pass_muon<S, V, false>(tables, momenta, codes, g_blk, p_blk, lane, LANES, nchunks, absmax, bs.neg_absmax2,
                                            bs.rinv2, beta1, t.beta2);
         __syncwarp();  // the staging slice is free for this warp's next block
         return;
@@ -1138,7 +1191,7 @@ __device__ __forceinline__ void warp_block_step(const TensorSlot<S>& t, long lon
         Chunk<S, V> praw;
         if (load_p) praw.load(p_blk, c);
         float m[V];
-        stage_load<V>(stage, half, c, m);
+        momenta.take(c, LANES, nchunks, m);
         uint32_t row[V];
         float q[V];
         if (fastdiv) {
@@ -1200,8 +1253,8 @@ constexpr int kVecThreads = 512;
 
 // GSRC: see warp_block_step. FULL: every tensor of the launch has whole-warp blocks (32 lanes per block);
 // otherwise none has. The kinds are separate kernels so that each is compiled (registers, code size) for
-// its own loop structure.
-template <typename S, int V, int GSRC, bool FULL>
+// its own loop structure. STAGED: see Momenta.
+template <typename S, int V, int GSRC, bool FULL, bool STAGED = true>
 __global__ void __launch_bounds__(kVecThreads, 1) step_vec_kernel(const __grid_constant__ StepLaunch L,
                                                                   const __grid_constant__ StepRows rows) {
     SmemView s;
@@ -1246,7 +1299,7 @@ __global__ void __launch_bounds__(kVecThreads, 1) step_vec_kernel(const __grid_c
                 if (!(t.flags & GEFEN_B200_STEP_MUON) && unit_elems * static_cast<int>(sizeof(S)) < 8192) prefetch_l2_range(t.p + elem0, unit_elems * sizeof(S));
             }
         }
-        warp_block_step<S, V, GSRC, FULL>(t, unit, L, tables, stage, lane);
+        warp_block_step<S, V, GSRC, FULL, STAGED>(t, unit, L, tables, stage, lane);
     }
     wait_for_predecessor();
 }
@@ -1655,10 +1708,10 @@ static int launch_step(K kernel, int grid, int threads, int smem, const StepLaun
     return GEFEN_B200_OK;
 }
 
-template <typename S, int V, int GSRC, bool FULL>
+template <typename S, int V, int GSRC, bool FULL, bool STAGED = true>
 static int launch_vec_variant(StepLaunch L, const StepRows& rows, long long max_unit, cudaStream_t stream) {
     static bool configured[kMaxDevices];
-    auto kernel = step_vec_kernel<S, V, GSRC, FULL>;
+    auto kernel = step_vec_kernel<S, V, GSRC, FULL, STAGED>;
     {
         int dev = 0;
         const int rc = current_device(&dev);
@@ -1671,7 +1724,7 @@ static int launch_vec_variant(StepLaunch L, const StepRows& rows, long long max_
     }
     // a warp stages one unit: one long block, or the 32 / lanes shorter blocks that share the warp
     // (max_unit: the largest need of the launch, see unit_floats; a slice starts on 16 bytes)
-    const long long stage_bytes = ((max_unit > 256 ? max_unit : 256) * 4 + 15) / 16 * 16;
+    const long long stage_bytes = ((STAGED && max_unit > 256 ? max_unit : 256) * 4 + 15) / 16 * 16;   // (256: build_lane_tables)
     int max_warps = kVecThreads / 32;
     if (warps_override() > 0 && warps_override() < max_warps) max_warps = warps_override();
     int warps = static_cast<int>((kMaxSmem - kStaticSmemSlack - kSmemTables) / stage_bytes);
@@ -1687,6 +1740,16 @@ static int launch_vec_variant(StepLaunch L, const StepRows& rows, long long max_
     return launch_step(kernel, grid, warps * 32, smem, L, rows, stream);
 }
 
+// Blocks of more than 2048 elements (fp32: 3072) in chunks of eight, this GPU's buffers only: their slices of shared
+// memory would leave fifteen warps and fewer (four for 8192 elements), so the second pass forms the momenta once more
+// instead (Momenta; launch class 1 to callers). 134 M bf16 / 67 M fp32 elements, ms, staged against computed: blocks of
+// 2056 0.299 / 0.220 and 0.289 / 0.212, 2560 0.259 / 0.201 and 0.249 / 0.202, 3072 0.282 / 0.212 and 0.263 / 0.218, 4096
+// 0.381 / 0.235 and 0.267 / 0.226, 8192 0.626 / 0.371 and 0.304 / 0.243.
+constexpr int kLongClass = 7;
+static int long_class(int cls, long long period, int dtype) {
+    return cls == 1 && period > (dtype_size(dtype) == 2 ? 2048 : 3072) ? kLongClass : cls;
+}
+
 template <typename S>
 static int launch_vec(int cls, StepLaunch L, const StepRows& rows, long long max_unit, cudaStream_t stream) {
     if (cls >= 3 && cls <= 5 && (L.n_peers > 0 || L.n_grad_srcs > 0)) {
@@ -1697,6 +1760,7 @@ static int launch_vec(int cls, StepLaunch L, const StepRows& rows, long long max
     if (cls == 3) return launch_vec_variant<S, 4, 0, false>(L, rows, max_unit, stream);
     if (cls == 4) return launch_vec_variant<S, 2, 0, false>(L, rows, max_unit, stream);
     if (cls == 5) return launch_vec_variant<S, 1, 0, false>(L, rows, max_unit, stream);
+    if (cls == kLongClass) return launch_vec_variant<S, 8, 0, true, false>(L, rows, max_unit, stream);
     if (cls == 6) {
         constexpr int kPer = kVectorThreads / 32;
         return launch_step(step_vector_kernel<S>, static_cast<int>((L.total_blocks + kPer - 1) / kPer), kVectorThreads, kSmemWs, L, rows, stream);
@@ -1738,7 +1802,8 @@ static int launch_generic(bool cta_per_block, const StepLaunch& L, const StepRow
 // divides the block length and the alignment of all pointers), 6 = vectors (period 1, runs of up to 256 elements), 0 =
 // generic warp per block, -1 = generic CTA per block.
 static int generic_class(const gefen_b200_step_tensor_t& t) { return t.period > 2048 ? -1 : 0; }
-static int class_chunk(int cls) { return cls <= 2 ? 8 : (cls == 3 ? 4 : (cls == 4 ? 2 : 1)); }
+static int class_chunk(int cls) { return cls <= 2 || cls == kLongClass ? 8 : (cls == 3 ? 4 : (cls == 4 ? 2 : 1)); }
+static bool staged_class(int cls) { return (cls >= 1 && cls <= 5) || cls == kLongClass; }
 static int tensor_class(const gefen_b200_step_tensor_t& t, int dtype) {
     const bool vec_dtype = dtype == GEFEN_B200_F32 || dtype == GEFEN_B200_BF16 || dtype == GEFEN_B200_F16;
     if (vec_dtype && (t.flags & GEFEN_B200_STEP_PERIOD1) != 0 && t.period <= kVectorMost && t.num_blocks < (1 << 28)) return 6;
@@ -1755,7 +1820,7 @@ static int tensor_class(const gefen_b200_step_tensor_t& t, int dtype) {
 // Units of a tensor in its launch's index space: passes of a warp on the staged path, blocks elsewhere.
 // (4-bit codes with an odd period: a pair of blocks is one unit, see step_generic_kernel)
 static long long class_units(const gefen_b200_step_tensor_t& t, int cls, int dtype) {
-    if (cls >= 1 && cls <= 5) return vec_units(t.num_blocks, t.period, class_chunk(cls), dtype_size(dtype));
+    if (staged_class(cls)) return vec_units(t.num_blocks, t.period, class_chunk(cls), dtype_size(dtype));
     const bool paired = (t.flags & GEFEN_B200_STEP_PACKED) != 0 && (t.period & 1) != 0;
     return paired ? (t.num_blocks + 1) / 2 : t.num_blocks;
 }
@@ -1800,7 +1865,7 @@ static int run_single(gefen_b200_step_tensor_t& t, int param_dtype, const float*
     L.table = nullptr;
     L.n_tensors = 1;
     L.stage_floats = 0;
-    const int cls = tensor_class(t, param_dtype);
+    const int cls = long_class(tensor_class(t, param_dtype), t.period, param_dtype);
     L.total_blocks = class_units(t, cls, param_dtype);
     L.ws = static_cast<const unsigned char*>(ws);
     L.stepsize = stepsize;
@@ -1813,7 +1878,7 @@ static int run_single(gefen_b200_step_tensor_t& t, int param_dtype, const float*
     L.follows = 0;
     StepRows rows = {};
     rows.row[0] = t;
-    return launch_class(cls, param_dtype, L, rows, cls >= 1 && cls <= 5 ? unit_floats(t.period, class_chunk(cls), dtype_size(param_dtype)) : t.period, stream);
+    return launch_class(cls, param_dtype, L, rows, staged_class(cls) ? unit_floats(t.period, class_chunk(cls), dtype_size(param_dtype)) : t.period, stream);
 }
 
 }  // namespace gefen
@@ -2148,6 +2213,7 @@ int gefen_b200_multi_tensor_step_multicast(gefen_b200_step_tensor_t* host_table,
         int cls = tensor_class(t, param_dtype);
         // vectors with peers: the generic kernel (no sums of squares there, so the results are the same bits)
         if (cls == 6 && (n_peers > 0 || n_grad_srcs > 0)) cls = generic_class(t);
+        if (n_peers == 0 && n_grad_srcs == 0) cls = long_class(cls, t.period, param_dtype);
         t.reserved_[0] = cls;
     }
     for (int begin = 0; begin < n_tensors;) {
@@ -2178,7 +2244,7 @@ int gefen_b200_multi_tensor_step_multicast(gefen_b200_step_tensor_t* host_table,
         long long max_period = 0;   // largest staging need of a warp: the elements of one unit on the staged path
         for (int i = begin; i < begin + run; ++i) {
             const int cls = host_table[begin].reserved_[0];
-            const long long need = cls >= 1 && cls <= 5 ? unit_floats(host_table[i].period, class_chunk(cls), dtype_size(param_dtype)) : host_table[i].period;
+            const long long need = staged_class(cls) ? unit_floats(host_table[i].period, class_chunk(cls), dtype_size(param_dtype)) : host_table[i].period;
             max_period = need > max_period ? need : max_period;
         }
         if (total > 0) {

@@ -48,7 +48,7 @@ def _step(device, dtype, nb, period, sources, copies, steps=2, wd=0.1):
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("nb,period", [(6, 2048), (37, 512), (65, 64), (5, 1664),
                                        (9, 300), (5, 1500), (33, 12), (11, 514), (33, 18), (21, 147), (50, 27), (3, 2047),
-                                       (2, 8188), (2, 8191)])
+                                       (2, 8188), (2, 8191), (3, 4096), (2, 8192)])
 def test_averaged_gradients_and_copies(cuda_device, dtype, nb, period):
     plain = _step(cuda_device, dtype, nb, period, 0, 0)
     # powers of two: the average of equal gradients is the gradient itself
