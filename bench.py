@@ -363,8 +363,9 @@ def run_sharded_arm(args, cfg, rank, world, local_rank):
 
 
 # DRAM bytes (read + write) per algorithmic byte of one launch of the staged step kernel, from an ncu
-# capture of a 134 M-element launch of the same kernel (traffic grows in proportion to the elements).
-STEP_KERNEL_DRAM_BYTES_PER_ALGORITHMIC_BYTE = {2: 0.967}
+# capture of a 134 M-element launch of the same kernel, fused second moment and weight decay as in this step (traffic
+# grows in proportion to the elements; part of the writes is still in L2 when the launch ends).
+STEP_KERNEL_DRAM_BYTES_PER_ALGORITHMIC_BYTE = {2: 0.949}
 
 
 def run_gpu_arm(args, cfg, rank, world, local_rank):
@@ -637,7 +638,7 @@ def measure_muon(cfg, steps: int, warmup: int):
     total_flops = sum(ns_flops(s) for _, s in shapes)
     coeffs = (3.4445, -4.7750, 2.0315)
 
-    def ns_ours():   # the optimizer's own path: the chains of two matrices side by side
+    def ns_ours():   # the optimizer's own path: groups of matrices
         ns.orthogonalize_all([(g, coeffs, 5, 1e-7) for g in grads], lambda i, ortho: None)
 
     def ns_torch():

@@ -14,8 +14,9 @@
 //  * step_vec_kernel  - the fast path: one warp owns one block, or several blocks when they are not longer than 1024
 //    elements (see lanes_shift). Codes and gradients are read once in chunks of eight elements (four, two or one
 //    where the block length or a pointer is a multiple of no more), the updated momenta wait in the warp's slice of
-//    shared memory while the block's absmax is reduced with shuffles, then they are re-encoded and the parameters
-//    updated: codes, gradients and params cross HBM exactly once (8 B/element in bf16, 14 B/element in fp32).
+//    shared memory while the block's absmax is reduced with shuffles (long blocks: are formed again, see long_class), then
+//    they are re-encoded and the parameters updated: codes, gradients and params cross HBM exactly once (8 B/element in
+//    bf16, 14 B/element in fp32).
 //    Codebook and thresholds arrive by one bulk (TMA) copy per CTA, which turns them into tables with a copy per
 //    lane (see LaneTables). No __syncthreads after set-up; the loops are short so the code stays in
 //    the instruction cache.
@@ -26,8 +27,8 @@
 //    0.182 -> 0.183 ms (67 M elements). Rows that are no multiples of eight, which the generic kernel used to take:
 //    120 M bf16 elements in blocks of 300 1.87 -> 0.37 ms, 135 M of 1500 2.26 -> 0.32 ms, 59 M of 147 0.98 -> 0.46 ms.
 //  * step_vector_kernel - period-1 tensors, one warp per magnitude, everything in registers.
-//  * step_generic_kernel - blocks of more than 8192 elements, fp64 and
-//    4-bit packed codes: two passes with scalar accesses, the second pass re-reading from L1/L2.
+//  * step_generic_kernel - blocks of more than 8192 elements, fp64, 4-bit packed codes, and vectors of ranks with peers:
+//    two passes with scalar accesses, the second pass re-reading from L1/L2.
 // All take their tensors from a descriptor table (one launch for many tensors); a single-tensor
 // call passes a one-row table inside the kernel parameters. For data-parallel ranks whose buffers
 // are mapped into each other's address space the kernels can also store every updated parameter

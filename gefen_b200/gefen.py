@@ -489,6 +489,7 @@ class Gefen(torch.optim.Optimizer):
                 "static_flags": rows["flags"].copy(),
                 "entries": [idxs[r] for r in order],
                 "classes": [classes[r] for r in order],
+                "launch": [launch[r] for r in order],
                 # byte offset of each row's first element in its tensor (0 unless a block range was given)
                 "offsets": [int((ranges or {}).get(id(work[idxs[r]][2]), (0, 0))[0]) * int(rows[i]["period"])
                             for i, r in enumerate(order)],

@@ -689,7 +689,9 @@ class Zero1Gefen:
         m = self._events
         launches = 0
         if self.local is not None and getattr(self.local, "_plan", None) is not None:
-            launches = sum(len(set(t.get("classes", [1]))) for t in (self.local._plan.tables or []))
+            # (one launch per launch class; vectors (6) join the generic kernel (0) where the ranks' buffers are mapped)
+            mapped = self._peer_deltas is not None or self._grad_deltas is not None or self._recv is not None
+            launches = sum(len({0 if mapped and c == 6 else c for c in t.get("launch", [1])}) for t in (self.local._plan.tables or []))
         return {"reduce_scatter": m[0].elapsed_time(m[1]), "local_step": m[1].elapsed_time(m[2]),
                 "all_gather": m[2].elapsed_time(m[3]), "kernel_launches_per_step": launches}
 
@@ -963,12 +965,13 @@ class Zero1Gefen:
 class Zero1GefenMuon(Zero1Gefen):
     """GefenMuon over ZeRO-1 sharded state. Newton-Schulz needs whole matrices, so whole tensors are
     assigned to ranks (`WholeTensorLayout`); the step is NCCL's reduce-scatter of the gradients, then
-    GefenMuon on the owned matrices, whose last kernel per matrix (decay + update,
-    `gefen_b200_muon_apply`) also stores the new matrix into every peer's parameter buffer: the
-    all-gather rides on those stores, under the other matrices' Newton-Schulz products (plain peer
+    GefenMuon on the owned matrices, whose last kernel per group of matrices (decay + update,
+    `gefen_b200_ns_group_apply`) also stores the new matrices into every peer's parameter buffer: the
+    all-gather rides on those stores (plain peer
     stores; the multicast form would only add the loop back through the switch here, since nothing flows
     the other way at the same time). N ranks reproduce one rank bit for bit: every matrix is processed
-    whole by the same kernels, and the codebook is fitted from the gathered histogram."""
+    whole, the kinds of tiles that groups of different sizes choose give the same bits, and the codebook is fitted from
+    the gathered histogram."""
 
     def __init__(self, named_params, lr=1e-3, weight_decay=0.1, momentum=0.95, nesterov=True,
                  ns_coefficients=(3.4445, -4.7750, 2.0315), eps=1e-7, ns_steps=5, adjust_lr_fn=None, *, group=None,

@@ -118,7 +118,9 @@ int gefen_b200_automatic_gefen_muon_momentum(
 
 /* One launch for many tensors (no counterpart in the reference, which launches 2-3 kernels per
  * tensor from Python, gefen.py:1208-1333). The host table is copied into `device_table`
- * (n_tensors * sizeof(gefen_b200_step_tensor_t) bytes, caller-owned) on `stream`. Keep
+ * (n_tensors * sizeof(gefen_b200_step_tensor_t) bytes, caller-owned) on `stream`, except that the rows of
+ * a call of up to 24 tensors travel as kernel parameters and `device_table` is not written, unless the
+ * stream is being captured: then every replay copies the host table as it is at that time, so keep it. Keep
  * host_table in pageable memory, or do not touch a pinned one until the copy has run: the
  * library writes first_block and reserved_ into it and the copy reads it later. All tensors of
  * one call share param_dtype. Fuses the vmean update, the weight-decay pre-multiply and the
@@ -174,7 +176,7 @@ int gefen_b200_multi_tensor_step_peers(gefen_b200_step_tensor_t* host_table, voi
  *    switch adds the ranks' copies, fp32 accumulation, one rounding to the gradient dtype), scales by
  *    grad_scale and rounds, instead of n_grad_srcs peer loads: 1/N of the ingress of the unicast
  *    reduce-scatter. The order of the switch's additions is not the rank order of the peer-load path.
- * The kernels for short, odd or unaligned blocks keep using the per-rank offsets, which must therefore be
+ * Blocks that the staged kernel takes in chunks below eight elements, and the generic kernels, use the per-rank offsets, which must therefore be
  * given as well. Ordering between ranks is the caller's, as for gefen_b200_multi_tensor_step_peers. No
  * counterpart in the reference. */
 int gefen_b200_multi_tensor_step_multicast(gefen_b200_step_tensor_t* host_table, void* device_table,
@@ -372,7 +374,8 @@ int gefen_b200_ns_group(const gefen_b200_ns_matrix_t* mats, int n, const void* d
 int gefen_b200_ns_group_apply(const gefen_b200_ns_matrix_t* mats, int n, const void* device_mats, int dtype, int steps,
                               const int64_t* peer_deltas, int n_peers, void* stream);
 
-/* `steps` Newton-Schulz iterations (reference: gefen_muon.py:38-47) of one already normalised bf16
+/* For callers of this interface (the package runs groups): `steps` Newton-Schulz iterations (reference:
+ * gefen_muon.py:38-47) of one already normalised bf16
  * matrix [rows, cols] (row-major, contiguous, dimensions multiples of 8), enqueued as 3 * steps
  * GEMMs: G = X X^T, B = b G + c G G, X <- a X + B X on the wide orientation, or the mirrored form
  * (Y^T Y, Y B) for rows > cols, so no transpose is ever materialised. x0 holds the input; the
