@@ -35,7 +35,6 @@ NVCC_FLAGS = [
     "-gencode",
     "arch=compute_100a,code=sm_100a",
     "-lineinfo",
-    "-split-compile=0",
     "-Xcompiler",
     "-fPIC",
 ]

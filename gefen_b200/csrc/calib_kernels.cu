@@ -8,7 +8,7 @@
 //
 // All of them are one read of the gradient from HBM (the reference reads it twice per kernel and,
 // for the adjacent-log score, twice per candidate period; here once per candidate that no other one
-// divides, two to four per tensor). A warp owns a block; the second look at
+// divides, one to six per tensor). A warp owns a block; the second look at
 // a block's elements, where one is needed, comes from L1.
 #include "common.cuh"
 
