@@ -10,22 +10,17 @@
 //   code' = nearest codebook entry of m_i / mag'   (IEEE divide by the un-rounded fp32 mag')
 //   p_i  -= cb[code'_i] * mag' * step * lr,   step = (1/bc1) / (sqrt(v/bc2) + eps)
 //
-// Three kernels:
-//  * step_vec_kernel  - the fast path: one warp owns one block, or several blocks when they are not longer than 1024
-//    elements (see lanes_shift). Codes and gradients are read once in chunks of eight elements (four, two or one
-//    where the block length or a pointer is a multiple of no more), the updated momenta wait in the warp's slice of
-//    shared memory while the block's absmax is reduced with shuffles (long blocks: are formed again, see long_class), then
-//    they are re-encoded and the parameters updated: codes, gradients and params cross HBM exactly once (8 B/element in
-//    bf16, 14 B/element in fp32).
-//    Codebook and thresholds arrive by one bulk (TMA) copy per CTA, which turns them into tables with a copy per
-//    lane (see LaneTables). No __syncthreads after set-up; the loops are short so the code stays in
-//    the instruction cache.
-//    What bounds it: for two-byte types the issue of instructions (31 per element) together with the latency that
-//    sixteen warps per SM can cover, for fp32 HBM. 134 M elements in blocks of 2048 bf16: 0.259 -> 0.221 ms = 0.75 of
-//    the measured copy bandwidth (the tables without bank conflicts, arithmetic on pairs, loops without per-lane
-//    bounds tests); blocks of 512 0.275 -> 0.230 ms, of 128 0.455 -> 0.315 ms; fp32 of 768 / 2048 0.193 -> 0.192 /
-//    0.182 -> 0.183 ms (67 M elements). Rows that are no multiples of eight, which the generic kernel used to take:
-//    120 M bf16 elements in blocks of 300 1.87 -> 0.37 ms, 135 M of 1500 2.26 -> 0.32 ms, 59 M of 147 0.98 -> 0.46 ms.
+// Four kernels:
+//  * step_ring_kernel - what every usual tensor takes: one warp owns one block, or several blocks when they are not longer
+//    than 1024 elements (see lanes_shift). Codes and gradients come through shared memory by bulk (TMA) copies one unit
+//    ahead, in chunks of eight elements (four, two or one where the block length or a pointer is a multiple of no more);
+//    the updated momenta wait in tensor memory while the block's absmax is reduced with shuffles, then they are re-encoded
+//    and the parameters updated: codes, gradients and parameters cross HBM exactly once (8 B/element in bf16, 14 in fp32).
+//    The codebook arrives by one bulk copy per CTA, which turns it into tables with a copy per lane (see LaneTables). No
+//    __syncthreads after set-up; the loops are short so the code stays in the instruction cache. What bounds it and what it
+//    measured stands at the kernel.
+//  * step_vec_kernel - the same without the ring: gradients averaged over ranks, chunks below eight with peer stores, and
+//    blocks too long for the buffers (see route); momenta in shared memory or formed twice (see Momenta).
 //  * step_vector_kernel - period-1 tensors, one warp per magnitude, everything in registers.
 //  * step_generic_kernel - blocks of more than 8192 elements, fp64, 4-bit packed codes, and vectors of ranks with peers:
 //    two passes with scalar accesses, the second pass re-reading from L1/L2.
@@ -58,7 +53,9 @@ __device__ __forceinline__ float ema_update_period1(float beta, float cur, float
 struct StepLaunch {
     const gefen_b200_step_tensor_t* table;  // device table, or nullptr: the rows in the kernel params
     int n_tensors;
-    int stage_floats;                       // fast path: floats of staging per warp (>= max period)
+    int stage_floats;                       // staged kernel: floats of staging per warp (>= max period)
+    int ring_g, ring_codes;                 // ring kernel: bytes of a warp's buffers for one unit's gradients and codes
+    int hold_columns, tmem_columns;         // ring kernel: tensor-memory columns of a warp and of the CTA
     long long total_blocks;
     const unsigned char* ws;                // codebook workspace
     const float* stepsize;                  // optional precomputed per-block step (single tensor only)
@@ -294,6 +291,16 @@ template <typename S, int V> struct Chunk {
             w[4 * q] = v.x; w[4 * q + 1] = v.y; w[4 * q + 2] = v.z; w[4 * q + 3] = v.w;
         }
     }
+    __device__ __forceinline__ void load_shared(uint32_t at) {
+        if constexpr (kBytes >= 16) {
+#pragma unroll
+            for (int q = 0; q < kBytes / 16; ++q)
+                asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                             : "=r"(w[4 * q]), "=r"(w[4 * q + 1]), "=r"(w[4 * q + 2]), "=r"(w[4 * q + 3]) : "r"(at + 16 * q));
+        } else if constexpr (kBytes == 8) asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(w[0]), "=r"(w[1]) : "r"(at));
+        else if constexpr (kBytes == 4) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[0]) : "r"(at));
+        else asm volatile("ld.shared.u16 %0, [%1];" : "=r"(w[0]) : "r"(at));
+    }
     __device__ __forceinline__ void store(void* base, long long chunk) const {
         char* p = static_cast<char*>(base) + chunk * kBytes;
         if constexpr (kBytes >= 16) {
@@ -365,6 +372,12 @@ template <int V> struct CodeChunk {
         const uint2 v = reinterpret_cast<const uint2*>(base)[chunk];
         w[0] = v.x; w[1] = v.y;
     }
+    __device__ __forceinline__ void load_shared(uint32_t at) {
+        if constexpr (V == 8) asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(w[0]), "=r"(w[1]) : "r"(at));
+        else if constexpr (V == 4) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[0]) : "r"(at));
+        else if constexpr (V == 2) asm volatile("ld.shared.u16 %0, [%1];" : "=r"(w[0]) : "r"(at));
+        else asm volatile("ld.shared.u8 %0, [%1];" : "=r"(w[0]) : "r"(at));
+    }
     __device__ __forceinline__ void store(uint8_t* base, long long chunk) const {
         if constexpr (V == 8) reinterpret_cast<uint2*>(base)[chunk] = make_uint2(w[0], w[1]);
         else if constexpr (V == 4) reinterpret_cast<uint32_t*>(base)[chunk] = w[0];
@@ -405,6 +418,33 @@ template <int V> __device__ __forceinline__ void stage_load(const float* stage, 
         const float2 a = *reinterpret_cast<const float2*>(stage + 2 * c);
         m[0] = a.x; m[1] = a.y;
     } else m[0] = stage[c];
+}
+
+// The same in tensor memory: each lane keeps V floats of its own per round, in V consecutive columns. Both are
+// executed by the whole warp.
+template <int V> __device__ __forceinline__ void hold_store(uint32_t at, const float (&m)[V]) {
+    if constexpr (V == 8)
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(at), "f"(m[0]), "f"(m[1]),
+                     "f"(m[2]), "f"(m[3]), "f"(m[4]), "f"(m[5]), "f"(m[6]), "f"(m[7]) : "memory");
+    else if constexpr (V == 4)
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "f"(m[0]), "f"(m[1]), "f"(m[2]), "f"(m[3]) : "memory");
+    else if constexpr (V == 2)
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x2.b32 [%0], {%1, %2};" ::"r"(at), "f"(m[0]), "f"(m[1]) : "memory");
+    else
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(at), "f"(m[0]) : "memory");
+}
+__device__ __forceinline__ void hold_stores_done() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+template <int V> __device__ __forceinline__ void hold_load(uint32_t at, float (&m)[V]) {
+    if constexpr (V == 8)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\ttcgen05.wait::ld.sync.aligned;"
+                     : "=f"(m[0]), "=f"(m[1]), "=f"(m[2]), "=f"(m[3]), "=f"(m[4]), "=f"(m[5]), "=f"(m[6]), "=f"(m[7]) : "r"(at) : "memory");
+    else if constexpr (V == 4)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];\n\ttcgen05.wait::ld.sync.aligned;"
+                     : "=f"(m[0]), "=f"(m[1]), "=f"(m[2]), "=f"(m[3]) : "r"(at) : "memory");
+    else if constexpr (V == 2)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];\n\ttcgen05.wait::ld.sync.aligned;" : "=f"(m[0]), "=f"(m[1]) : "r"(at) : "memory");
+    else
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];\n\ttcgen05.wait::ld.sync.aligned;" : "=f"(m[0]) : "r"(at) : "memory");
 }
 
 // --------------------------------------------------------------------------- fast path
@@ -576,35 +616,35 @@ template <int V> __device__ __forceinline__ CodeChunk<V> row_codes(const uint32_
 // several chunks of its block, which keeps as many loads in flight and shares the per-block work (reductions,
 // step size, reciprocal) between more elements: about eight chunks of eight elements per lane for blocks of more
 // than 256 elements, as in a 2048-element block (8 lanes for 512 elements, 16 for 1024, all 32 from 1032 on), up to
-// four below that (134 M bf16 elements in blocks of 128 / 64 / 32: 0.315 / 0.331 / 0.332 ms, with up to two chunks
-// per lane 0.46 / 0.47 / 0.50; fp32 keeps two for blocks of 64 and less, whose lanes would otherwise each read
-// 128 bytes of their own: 67 M elements 0.233 against 0.427 ms).
-__host__ __device__ __forceinline__ int lanes_shift(long long nchunks, int v, int es) {   // log2 of the lanes; chunks of v elements of es bytes
+// four down to blocks of 72 elements, two below that (the blocks of a warp lie side by side in its buffer, so lanes with
+// four chunks of their own would read the same banks: 134 M bf16 elements in blocks of 64 / 32 0.60 / 0.58 ms with four,
+// 0.345 / 0.338 with two; before the buffers 0.349 / 0.357).
+__host__ __device__ __forceinline__ int lanes_shift(long long nchunks, int v) {   // log2 of the lanes; chunks of v elements
     if (v < 8) {   // smaller chunks: about sixteen per lane, eight of them in flight
         int shift = 0;
         while (shift < 5 && (16 << shift) < nchunks) ++shift;
         return shift;
     }
-    const long long want = nchunks > 32 ? (nchunks + 7) >> 3 : ((es == 4 && nchunks <= 8) ? (nchunks + 1) >> 1 : (nchunks + 3) >> 2);
+    const long long want = nchunks > 32 ? (nchunks + 7) >> 3 : (nchunks <= 8 ? (nchunks + 1) >> 1 : (nchunks + 3) >> 2);
     int shift = 0;
     while (shift < 5 && (1 << shift) < want) ++shift;
     return shift;
 }
 // Elements of one work unit of a tensor (what a warp stages at a time), blocks of nchunks chunks of v elements.
-__host__ __device__ __forceinline__ long long unit_elements(long long period, int v, int es) { return period << (5 - lanes_shift(period / v, v, es)); }
+__host__ __device__ __forceinline__ long long unit_elements(long long period, int v) { return period << (5 - lanes_shift(period / v, v)); }
 // Floats from one block's staged momenta to the next one's in a warp's slice. Eight lanes make one 128-byte access;
 // where they belong to several blocks (fewer than eight lanes per block), the blocks' slices start on different banks.
 __host__ __device__ __forceinline__ int slice_stride(int period, int shift, int v) {
     return v < 8 || shift >= 3 ? period : ((period + 31) & ~31) + (4 << shift);
 }
 // Floats that a warp stages for one unit.
-__host__ __device__ __forceinline__ long long unit_floats(long long period, int v, int es) {
-    const int shift = lanes_shift(period / v, v, es);
+__host__ __device__ __forceinline__ long long unit_floats(long long period, int v) {
+    const int shift = lanes_shift(period / v, v);
     return static_cast<long long>(slice_stride(static_cast<int>(period), shift, v)) << (5 - shift);
 }
 // Work units (one warp pass each) of a tensor on the fast path.
-__host__ __device__ __forceinline__ long long vec_units(long long num_blocks, long long period, int v, int es) {
-    const int shift = 5 - lanes_shift(period / v, v, es);
+__host__ __device__ __forceinline__ long long vec_units(long long num_blocks, long long period, int v) {
+    const int shift = 5 - lanes_shift(period / v, v);
     return (num_blocks + (1 << shift) - 1) >> shift;
 }
 
@@ -648,7 +688,7 @@ template <typename S> struct alignas(8) TensorSlot {
         num_blocks = t->num_blocks;
         period = static_cast<int>(t->period);   // at most kFastMaxPeriod
         flags = t->flags;
-        units = vec_units(num_blocks, period, v_elems, sizeof(S));
+        units = vec_units(num_blocks, period, v_elems);
         mag_dtype = t->mag_dtype;
         v_dtype = t->v_dtype;
         beta1 = t->beta1;
@@ -715,6 +755,52 @@ __device__ __forceinline__ void first_pass_group(const S* g_blk, const uint8_t* 
             }
             if (STAGED) stage_store<V>(stage, half, c, m);
         }
+    }
+}
+
+// The same over U chunks of a unit whose inputs a bulk copy has brought to shared memory (g_at, codes_at: the lane's
+// block); the updated momenta go to tensor memory, V columns per round. The whole warp calls it.
+template <typename S, int V, int U, bool GUARD>
+__device__ __forceinline__ void first_pass_ring(uint32_t g_at, uint32_t codes_at, uint32_t hold, const LaneTables& t, int c0, int LANES,
+                                                int nchunks, f32x2 mag2, f32x2 beta2_, f32x2 omb2_, float& absmax, f32x2& sumsq2) {
+    CodeChunk<V> craw[U];
+    Chunk<S, V> graw[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int c = c0 + LANES * u;
+        if (!GUARD || c < nchunks) {
+            craw[u].load_shared(codes_at + c * V);
+            graw[u].load_shared(g_at + c * Chunk<S, V>::kBytes);
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        float m[V];
+#pragma unroll
+        for (int i = 0; i < V; ++i) m[i] = 0.0f;
+        if (!GUARD || c0 + LANES * u < nchunks) {
+            float g[V];
+            graw[u].unpack(g);
+            if constexpr (V == 1) {
+                const float cur = t.value(t.row_of_byte(craw[u].w[0], 0));
+                float spare;
+                unpair(fma2(beta2_, mul2(mag2, pair(cur, cur)), mul2(omb2_, pair(g[0], g[0]))), m[0], spare);
+                absmax = max_abs_nan(absmax, m[0]);
+                sumsq2 = fma2(pair(g[0], 0.0f), pair(g[0], 0.0f), sumsq2);
+            } else {
+#pragma unroll
+                for (int i = 0; i < V; i += 2) {
+                    const f32x2 g2 = pair(g[i], g[i + 1]);
+                    const f32x2 cur = mul2(mag2, pair(t.value(t.row_of_byte(craw[u].w[i >> 2], i & 3)),
+                                                      t.value(t.row_of_byte(craw[u].w[i >> 2], (i & 3) + 1))));
+                    unpair(fma2(beta2_, cur, mul2(omb2_, g2)), m[i], m[i + 1]);   // ema_update
+                    absmax = max_abs_nan(max_abs_nan(absmax, m[i]), m[i + 1]);
+                    sumsq2 = fma2(g2, g2, sumsq2);
+                }
+            }
+        }
+        if (GUARD) __syncwarp();
+        hold_store<V>(hold + u * V, m);
     }
 }
 
@@ -854,31 +940,49 @@ __device__ __forceinline__ void reduce_pass_small(const StepLaunch& L, const S* 
     }
 }
 
-// Where the second pass takes a chunk's updated momenta from: the warp's staging slice, or, for blocks whose slices
-// would leave too few warps (see long_class), computed once more from codes and gradients, which L2 still holds; the
-// next chunk's are requested while this one is worked on. Both walk the chunks of a lane in order.
-template <typename S, int V, bool STAGED> struct Momenta {   // STAGED
+// Where the second pass takes a chunk's updated momenta from:
+//   kShared  the warp's slice of shared memory (gradients of several ranks, and what route() leaves);
+//   kTwice   computed once more from codes and gradients, which L2 still holds (blocks too long for the other two, see
+//            route); the next chunk's are requested while this one is worked on;
+//   kTensor  the warp's columns of tensor memory (step_ring_kernel).
+// All walk the chunks of a lane in order; the whole warp calls take() (round `it`, chunk c of the lane; ALL: every lane
+// has one).
+enum Hold { kShared, kTwice, kTensor };
+template <typename S, int V, int HOLD> struct Momenta {   // kShared
     const float* const stage;
     const int half;
-    __device__ __forceinline__ Momenta(const float* s, int h, const uint8_t*, const S*, const LaneTables&, float, float, float)
+    __device__ __forceinline__ Momenta(const float* s, int h, uint32_t, const uint8_t*, const S*, const LaneTables&, float, float, float)
         : stage(s), half(h) {}
     __device__ __forceinline__ void start(int, int, int) {}
-    __device__ __forceinline__ void take(int c, int, int, float (&m)[V]) { stage_load<V>(stage, half, c, m); }
+    template <bool ALL> __device__ __forceinline__ void take(int, int c, int, int nchunks, float (&m)[V]) {
+        if (ALL || c < nchunks) stage_load<V>(stage, half, c, m);
+    }
 };
-template <typename S, int V> struct Momenta<S, V, false> {
+template <typename S, int V> struct Momenta<S, V, kTensor> {
+    const uint32_t hold;
+    __device__ __forceinline__ Momenta(const float*, int, uint32_t h, const uint8_t*, const S*, const LaneTables&, float, float, float)
+        : hold(h) {}
+    __device__ __forceinline__ void start(int, int, int) {}
+    template <bool ALL> __device__ __forceinline__ void take(int it, int, int, int, float (&m)[V]) {
+        if (!ALL) __syncwarp();
+        hold_load<V>(hold + it * V, m);
+    }
+};
+template <typename S, int V> struct Momenta<S, V, kTwice> {
     const uint8_t* const codes;
     const S* const g;
     const LaneTables& t;
     const f32x2 mag2, beta2_, omb2_;
     CodeChunk<V> craw;
     Chunk<S, V> graw;
-    __device__ __forceinline__ Momenta(const float*, int, const uint8_t* c, const S* gradients, const LaneTables& tables, float old_mag,
-                                       float beta1, float omb1)
+    __device__ __forceinline__ Momenta(const float*, int, uint32_t, const uint8_t* c, const S* gradients, const LaneTables& tables,
+                                       float old_mag, float beta1, float omb1)
         : codes(c), g(gradients), t(tables), mag2(pair(old_mag, old_mag)), beta2_(pair(beta1, beta1)), omb2_(pair(omb1, omb1)) {}
     __device__ __forceinline__ void start(int lane, int, int nchunks) {
         if (lane < nchunks) { craw.load(codes, lane); graw.load(g, lane); }
     }
-    __device__ __forceinline__ void take(int c, int LANES, int nchunks, float (&m)[V]) {
+    template <bool ALL> __device__ __forceinline__ void take(int, int c, int LANES, int nchunks, float (&m)[V]) {
+        if (!ALL && c >= nchunks) return;
         const CodeChunk<V> code = craw;
         float gv[V];
         graw.unpack(gv);
@@ -898,11 +1002,9 @@ template <typename S, int V> struct Momenta<S, V, false> {
 struct BlockScalars {
     f32x2 neg_absmax2, rinv2, step2, lr2, wd2;
 };
-template <typename S, int V, bool WD, int STORE, bool ONE, typename M>
-__device__ __forceinline__ void update_chunk(const StepLaunch& L, const LaneTables& t, M& momenta, int LANES, int nchunks,
-                                             uint8_t* codes, S* p_blk, Chunk<S, V> praw, int c, const BlockScalars& b) {
-    float m[V];
-    momenta.take(c, LANES, nchunks, m);
+template <typename S, int V, bool WD, int STORE, bool ONE>
+__device__ __forceinline__ void update_chunk(const StepLaunch& L, const LaneTables& t, const float (&m)[V], uint8_t* codes, S* p_blk,
+                                             Chunk<S, V> praw, int c, const BlockScalars& b) {
     uint32_t row[V];
     encode<V, ONE>(m, b.neg_absmax2, b.rinv2, t, row);
     row_codes<V>(row).store(codes, c);
@@ -932,9 +1034,11 @@ __device__ __forceinline__ void update_chunk(const StepLaunch& L, const LaneTabl
     }
 }
 // Parameters (GefenMuon: gradients) of a lane's chunks that are requested ahead of the re-encoding: the next chunk of
-// eight elements, the next eight of the smaller chunks, whose work is too short to cover the latency of a load.
-template <typename S, int V> struct Ahead {
-    static constexpr int kDepth = V < 8 ? (V * sizeof(S) > 8 ? 4 : 8) : 1;
+// eight elements (two in the ring kernel, which has the registers for them: 134 M bf16 elements in blocks of 1120 0.322 ->
+// 0.227 ms, of 2048 0.208 -> 0.197), the next four to eight of the smaller chunks, whose work is too short to cover the
+// latency of a load.
+template <typename S, int V, int HOLD> struct Ahead {
+    static constexpr int kDepth = V < 8 ? (V * sizeof(S) > 8 || (V == 4 && HOLD == kTensor) ? 4 : 8) : (HOLD == kTensor ? 2 : 1);
     Chunk<S, V> slot[kDepth];
     __device__ __forceinline__ void start(const S* blk, int lane, int LANES, int nchunks) {
 #pragma unroll
@@ -950,24 +1054,34 @@ template <typename S, int V> struct Ahead {
 };
 // The chunks of one block: `full` rounds in which every lane of the warp has one, then the guarded rest. The
 // parameters of the next chunks are fetched while this one is encoded.
-template <typename S, int V, bool WD, int STORE, bool ONE, typename M>
-__device__ __forceinline__ void second_pass_common(const StepLaunch& L, const LaneTables& t, M& momenta, uint8_t* codes, S* p_blk, Ahead<S, V>& ahead, int lane, int LANES,
-                                                   int nchunks, int full, int rounds_all, const BlockScalars& b) {
-    constexpr int D = Ahead<S, V>::kDepth;
+template <typename S, int V, int HOLD, bool WD, int STORE, bool ONE>
+__device__ __forceinline__ void second_pass_common(const StepLaunch& L, const LaneTables& t, Momenta<S, V, HOLD>& momenta, uint8_t* codes, S* p_blk,
+                                                   Ahead<S, V, HOLD>& ahead, int lane, int LANES, int nchunks, int full, int rounds_all,
+                                                   const BlockScalars& b) {
+    constexpr int D = Ahead<S, V, HOLD>::kDepth;
     int c = lane;
     int it = 0;
-    if constexpr (D == 1) {
-        for (; it < full; ++it, c += LANES) {
-            const Chunk<S, V> praw = ahead.take(0, p_blk, c, LANES, nchunks);
-            update_chunk<S, V, WD, STORE, ONE>(L, t, momenta, LANES, nchunks, codes, p_blk, praw, c, b);
+    if constexpr (V == 8) {
+        for (; it + D <= full; it += D) {
+#pragma unroll
+            for (int u = 0; u < D; ++u, c += LANES) {
+                float m[V];
+                momenta.template take<true>(it + u, c, LANES, nchunks, m);
+                const Chunk<S, V> praw = ahead.take(u, p_blk, c, LANES, nchunks);
+                update_chunk<S, V, WD, STORE, ONE>(L, t, m, codes, p_blk, praw, c, b);
+            }
         }
     }
-    for (; it < rounds_all; it += D, c += D * LANES) {
+    for (; it < rounds_all; it += D) {
 #pragma unroll
-        for (int u = 0; u < D; ++u) {
-            if (c + u * LANES < nchunks) {
-                const Chunk<S, V> praw = ahead.take(u, p_blk, c + u * LANES, LANES, nchunks);
-                update_chunk<S, V, WD, STORE, ONE>(L, t, momenta, LANES, nchunks, codes, p_blk, praw, c + u * LANES, b);
+        for (int u = 0; u < D; ++u, c += LANES) {
+            if (it + u < rounds_all) {
+                float m[V];
+                momenta.template take<false>(it + u, c, LANES, nchunks, m);
+                if (c < nchunks) {
+                    const Chunk<S, V> praw = ahead.take(u, p_blk, c, LANES, nchunks);
+                    update_chunk<S, V, WD, STORE, ONE>(L, t, m, codes, p_blk, praw, c, b);
+                }
             }
         }
     }
@@ -977,40 +1091,44 @@ __device__ __forceinline__ void second_pass_common(const StepLaunch& L, const La
 // with the gradient when asked (torch: m.mul_(momentum).add_(g, alpha=1-momentum) on the rounded momentum,
 // reference gefen_muon.py:312-314; alpha travels in the descriptor's beta2), goes where the Gefen step keeps
 // the parameters. The gradient chunk of the next iteration is requested while this one is encoded.
-template <typename S, int V, bool NESTEROV, typename M>
-__device__ __forceinline__ void second_pass_muon(const LaneTables& t, M& momenta, uint8_t* codes,
-                                                 const S* g_blk, S* out_blk, int lane, int LANES, int nchunks, float absmax,
-                                                 f32x2 neg_absmax2, f32x2 rinv2, float beta1, float alpha) {
-    constexpr int D = Ahead<S, V>::kDepth;
-    Ahead<S, V> ahead;
+template <typename S, int V, int HOLD, bool NESTEROV, bool ONE>
+__device__ __forceinline__ void second_pass_muon(const LaneTables& t, Momenta<S, V, HOLD>& momenta, uint8_t* codes, const S* g_blk, S* out_blk,
+                                                 int lane, int LANES, int nchunks, int rounds_all, float absmax, f32x2 neg_absmax2, f32x2 rinv2,
+                                                 float beta1, float alpha) {
+    constexpr int D = Ahead<S, V, HOLD>::kDepth;
+    Ahead<S, V, HOLD> ahead;
     if (NESTEROV) ahead.start(g_blk, lane, LANES, nchunks);
-    for (int c0 = lane; c0 < nchunks; c0 += D * LANES) {
+    int c = lane;
+    for (int it = 0; it < rounds_all; it += D) {
 #pragma unroll
-        for (int u = 0; u < D; ++u) {
-        const int c = c0 + u * LANES;
-        if (c >= nchunks) break;
-        Chunk<S, V> graw;
-        if (NESTEROV) graw = ahead.take(u, g_blk, c, LANES, nchunks);
-        float m[V];
-        momenta.take(c, LANES, nchunks, m);
-        uint32_t row[V];
-        encode<V, false>(m, neg_absmax2, rinv2, t, row);
-        row_codes<V>(row).store(codes, c);
-        float q[V];
+        for (int u = 0; u < D; ++u, c += LANES) {
+            if (it + u >= rounds_all) break;
+            float m[V];
+            momenta.template take<false>(it + u, c, LANES, nchunks, m);
+            if (c >= nchunks) continue;
+            Chunk<S, V> graw;
+            if (NESTEROV) graw = ahead.take(u, g_blk, c, LANES, nchunks);
+            uint32_t row[V];
+            encode<V, ONE>(m, neg_absmax2, rinv2, t, row);
+            row_codes<V>(row).store(codes, c);
+            float q[V];
 #pragma unroll
-        for (int i = 0; i < V; ++i) q[i] = t.value(row[i]) * absmax;
-        if (NESTEROV) {
-            float g[V];
-            graw.unpack(g);
+            for (int i = 0; i < V; ++i) q[i] = t.value(row[i]) * absmax;
+            Chunk<S, V> out;
+            if (NESTEROV) {
+                float g[V];
+                graw.unpack(g);
+                out.pack(q);
+                out.unpack(q);
 #pragma unroll
-            for (int i = 0; i < V; ++i) {
-                const float m1 = ScalarIO<S>::round(ScalarIO<S>::round(q[i]) * beta1);
-                q[i] = fmaf(alpha, g[i], m1);
+                for (int i = 0; i < V; ++i) q[i] *= beta1;
+                out.pack(q);
+                out.unpack(q);
+#pragma unroll
+                for (int i = 0; i < V; ++i) q[i] = fmaf(alpha, g[i], q[i]);
             }
-        }
-        Chunk<S, V> out;
-        out.pack(q);
-        out.store(out_blk, c);
+            out.pack(q);
+            out.store(out_blk, c);
         }
     }
 }
@@ -1021,16 +1139,19 @@ __device__ __forceinline__ void second_pass_muon(const LaneTables& t, M& momenta
 // GSRC: where the gradients come from: 0 = this GPU's buffer, 1 = averaged over the ranks' buffers with peer
 // loads, 2 = summed by the switch through the multicast mapping (StepLaunch::grad_mc_delta). Chunks below eight elements
 // know 0 and 1 only: 1 is every launch with peers, gradients of this GPU's buffer (no sources) included.
-template <typename S, int V, int GSRC, bool FULL, bool STAGED>
-__device__ __forceinline__ void warp_block_step(const TensorSlot<S>& t, long long unit, const StepLaunch& L, const LaneTables& tables,
-                                                float* stage, int warp_lane) {
+// In: how the unit's inputs arrive (RingInputs; DirectInputs: they are loaded here). False: a bounded wait for the inputs
+// ran out and nothing was done.
+template <typename S, int V, int GSRC, bool FULL, int HOLD, typename In>
+__device__ __forceinline__ bool warp_block_step(const TensorSlot<S>& t, long long unit, const StepLaunch& L, const LaneTables& tables,
+                                                float* stage, In& in, int warp_lane) {
+    constexpr bool STAGED = HOLD == kShared;
     const float* const stepsize = L.stepsize;
     const int n_peers = GSRC == 0 && V < 8 ? 0 : L.n_peers;            // (chunks below 8: GSRC == 1 wherever there are peers)
     const long long param_mc = V < 8 ? 0 : L.param_mc_delta;           // (a multicast access moves 16 bytes)
     // (the shuffle tells the compiler that the period is the same in all lanes, which the loops' bounds profit from)
     const int period = __shfl_sync(0xffffffffu, t.period, 0);
     const int chunks = period / V;                     // of a block
-    const int shift = FULL ? 5 : lanes_shift(chunks, V, sizeof(S));
+    const int shift = FULL ? 5 : lanes_shift(chunks, V);
     const int LANES = 1 << shift;
     const int lane = warp_lane & (LANES - 1);          // lane within the block's group
     const int member = warp_lane >> shift;             // which block of the unit
@@ -1049,20 +1170,24 @@ __device__ __forceinline__ void warp_block_step(const TensorSlot<S>& t, long lon
 
     const float beta1 = t.beta1;
     const float omb1 = 1.0f - beta1;
-    const float old_mag = valid ? load_state(t.mag, b, t.mag_dtype) : 0.0f;
+    float old_mag = 0.0f;
+    if constexpr (HOLD == kTensor) old_mag = in.mag;
+    else if (valid) old_mag = load_state(t.mag, b, t.mag_dtype);
 
     // Everything the block needs from HBM besides codes and gradients is requested now, so that its
-    // latency overlaps the first pass: the second moment and, where the registers allow it (2-byte
-    // types), the first chunk of parameters.
-    constexpr bool kEarlyParams = sizeof(S) == 2;
+    // latency overlaps the first pass: the second moment (the ring kernel has it already) and, where the registers
+    // allow it (2-byte types, ring kernel), the first chunks of parameters.
+    constexpr bool kEarlyParams = sizeof(S) == 2 || HOLD == kTensor;
     const float lr = t.lr;
     const bool do_update = muon || lr != 0.0f;
     const bool load_p = !muon && do_update;
     float v_in = 1.0f;
-    if (!muon && valid) v_in = stepsize != nullptr ? stepsize[b] : load_state(t.v, b, t.v_dtype);
-    Ahead<S, V> ahead;
+    if constexpr (HOLD == kTensor) v_in = in.v;
+    else if (!muon && valid) v_in = stepsize != nullptr ? stepsize[b] : load_state(t.v, b, t.v_dtype);
+    Ahead<S, V, HOLD> ahead;
     if (kEarlyParams && load_p) ahead.start(p_blk, lane, LANES, nchunks);
 
+    const int rounds_all = (chunks + LANES - 1) >> shift, full = all_valid ? chunks >> shift : 0;
     // ---- pass over codes and gradients (the only read of both)
     float absmax = 0.0f;
     float sumsq = 0.0f;
@@ -1083,6 +1208,23 @@ __device__ __forceinline__ void warp_block_step(const TensorSlot<S>& t, long lon
             else GEFEN_REDUCE_PASS(8);
 #undef GEFEN_REDUCE_PASS
         }
+    } else if constexpr (HOLD == kTensor) {
+        constexpr int U = 2;
+        const long long unit0 = (unit << (5 - shift)) * period;
+        const uint32_t g_at = in.g_at(t.g + unit0) + static_cast<uint32_t>(member * period) * static_cast<uint32_t>(sizeof(S));
+        const uint32_t codes_at = in.codes_at(t.codes + unit0) + static_cast<uint32_t>(member * period);
+        const f32x2 mag2 = pair(old_mag, old_mag), beta2_ = pair(beta1, beta1), omb2_ = pair(omb1, omb1);
+        if (!in.arrived(L.spin_limit)) return false;
+        int it = 0;
+        for (; it + U <= full; it += U)
+            first_pass_ring<S, V, U, false>(g_at, codes_at, in.hold + it * V, tables, lane + it * LANES, LANES, nchunks, mag2, beta2_, omb2_,
+                                            absmax, sumsq2);
+        for (; it < rounds_all; ++it)
+            first_pass_ring<S, V, 1, true>(g_at, codes_at, in.hold + it * V, tables, lane + it * LANES, LANES, nchunks, mag2, beta2_, omb2_,
+                                           absmax, sumsq2);
+        hold_stores_done();
+        __syncwarp();   // the whole warp has read the buffers
+        in.request_next();
     } else {
         // Up to four chunks in flight per lane; complete groups of four in every lane without bounds tests, which
         // cost four instructions each and sit on the one path that every element takes.
@@ -1126,7 +1268,9 @@ __device__ __forceinline__ void warp_block_step(const TensorSlot<S>& t, long lon
         }
     }
     __syncwarp();  // staged momenta are visible to the whole warp; every lane has read the old magnitude
-    Momenta<S, V, STAGED> momenta(stage, half, codes, g_blk, tables, old_mag, beta1, omb1);
+    uint32_t hold = 0;
+    if constexpr (HOLD == kTensor) hold = in.hold;
+    Momenta<S, V, HOLD> momenta(stage, half, hold, codes, g_blk, tables, old_mag, beta1, omb1);
 
     // ---- rare: a NaN or Inf in the block. The reference's max ignores NaN; redo it that way and
     // let the exact (threshold) quantiser handle non-finite quotients.
@@ -1134,9 +1278,10 @@ __device__ __forceinline__ void warp_block_step(const TensorSlot<S>& t, long lon
     if (__any_sync(0xffffffffu, !(absmax <= 3.0e38f))) {   // warp-uniform: the reduction below shuffles
         float mx = 0.0f;
         momenta.start(lane, LANES, nchunks);
-        for (int c = lane; c < nchunks; c += LANES) {
+        for (int it = 0, c = lane; it < rounds_all; ++it, c += LANES) {
             float m[V];
-            momenta.take(c, LANES, nchunks, m);
+            momenta.template take<false>(it, c, LANES, nchunks, m);
+            if (c >= nchunks) continue;
 #pragma unroll
             for (int i = 0; i < V; ++i) mx = fmaxf(mx, fabsf(m[i]));
         }
@@ -1159,9 +1304,8 @@ __device__ __forceinline__ void warp_block_step(const TensorSlot<S>& t, long lon
     // The common case takes the loop that was compiled for it (the conditions are uniform over the warp: they
     // come from the launch and the tensor's descriptor, and a warp's blocks go one way together).
     if (__all_sync(0xffffffffu, fastdiv || !valid) && !muon && do_update) {
-        const int rounds_all = (chunks + LANES - 1) >> shift, full = all_valid ? chunks >> shift : 0;
 #define GEFEN_SECOND_PASS(WD_, STORE_, ONE_)                                                                                       \
-    second_pass_common<S, V, WD_, STORE_, ONE_>(L, tables, momenta, codes, p_blk, ahead, lane, LANES, nchunks, full,             \
+    second_pass_common<S, V, HOLD, WD_, STORE_, ONE_>(L, tables, momenta, codes, p_blk, ahead, lane, LANES, nchunks, full,             \
                                                 rounds_all, bs)
         if constexpr (V == 8) {
             const int store = param_mc != 0 ? 2 : (n_peers > 0 ? 1 : 0);
@@ -1176,23 +1320,27 @@ __device__ __forceinline__ void warp_block_step(const TensorSlot<S>& t, long lon
         }
 #undef GEFEN_SECOND_PASS
         __syncwarp();  // the staging slice is free for this warp's next block
-        return;
+        return true;
     }
     if (GSRC == 0 && muon && __all_sync(0xffffffffu, fastdiv || !valid)) {
-        if (nesterov) second_pass_muon<S, V, true>(tables, momenta, codes, g_blk, p_blk, lane, LANES, nchunks, absmax,
-                                                   bs.neg_absmax2, bs.rinv2, beta1, t.beta2);
-        else second_pass_muon<S, V, false>(tables, momenta, codes, g_blk, p_blk, lane, LANES, nchunks, absmax, bs.neg_absmax2,
-                                           bs.rinv2, beta1, t.beta2);
+#define GEFEN_SECOND_PASS(NESTEROV_, ONE_)                                                                                         \
+    second_pass_muon<S, V, HOLD, NESTEROV_, ONE_>(tables, momenta, codes, g_blk, p_blk, lane, LANES, nchunks, rounds_all, absmax,   \
+                                                  bs.neg_absmax2, bs.rinv2, beta1, t.beta2)
+        if (nesterov && tables.rounds == 1) GEFEN_SECOND_PASS(true, true);
+        else if (nesterov) GEFEN_SECOND_PASS(true, false);
+        else GEFEN_SECOND_PASS(false, false);
+#undef GEFEN_SECOND_PASS
         __syncwarp();  // the staging slice is free for this warp's next block
-        return;
+        return true;
     }
     // Everything else (lr == 0, blocks that are all zero or hold NaN or Inf, magnitudes outside the range of the
     // reciprocal, GefenMuon's momentum over averaged gradients): the general loop.
-    for (int c = lane; c < nchunks; c += LANES) {
+    for (int it = 0, c = lane; it < rounds_all; ++it, c += LANES) {
+        float m[V];
+        momenta.template take<false>(it, c, LANES, nchunks, m);
+        if (c >= nchunks) continue;
         Chunk<S, V> praw;
         if (load_p) praw.load(p_blk, c);
-        float m[V];
-        momenta.take(c, LANES, nchunks, m);
         uint32_t row[V];
         float q[V];
         if (fastdiv) {
@@ -1247,15 +1395,17 @@ __device__ __forceinline__ void warp_block_step(const TensorSlot<S>& t, long lon
         }
     }
     __syncwarp();  // the staging slice is free for this warp's next block
+    return true;
 }
 
 // Threads per CTA: sixteen warps of 128 registers; the tables leave room for sixteen staging slices of 2048 elements.
 constexpr int kVecThreads = 512;
+struct DirectInputs {};
 
 // GSRC: see warp_block_step. FULL: every tensor of the launch has whole-warp blocks (32 lanes per block);
 // otherwise none has. The kinds are separate kernels so that each is compiled (registers, code size) for
-// its own loop structure. STAGED: see Momenta.
-template <typename S, int V, int GSRC, bool FULL, bool STAGED = true>
+// its own loop structure. HOLD: see Momenta.
+template <typename S, int V, int GSRC, bool FULL, int HOLD = kShared>
 __global__ void __launch_bounds__(kVecThreads, 1) step_vec_kernel(const __grid_constant__ StepLaunch L,
                                                                   const __grid_constant__ StepRows rows) {
     SmemView s;
@@ -1279,6 +1429,7 @@ __global__ void __launch_bounds__(kVecThreads, 1) step_vec_kernel(const __grid_c
     // the warp's slot lies where the codebook was staged (build_lane_tables has consumed it)
     TensorSlot<S>& t = reinterpret_cast<TensorSlot<S>*>(fast_smem(kWsAt))[warp];
     static_assert(sizeof(TensorSlot<S>) * (kVecThreads / 32) <= kSmemWs, "a slot per warp");
+    DirectInputs in;
     long long t_first = 0, t_units = 0;
     for (long long gb = warp_global; gb < L.total_blocks; gb += warp_stride) {
         if (gb < t_first || gb >= t_first + t_units) {
@@ -1290,18 +1441,161 @@ __global__ void __launch_bounds__(kVecThreads, 1) step_vec_kernel(const __grid_c
         }
         const long long unit = gb - t_first;
         const long long next = unit + warp_stride;
-        // same tensor: hint the next block of this warp (measured: pays for 2-byte dtypes with long blocks only)
+        // same tensor: hint the next block of this warp
         if (GSRC == 0 && lane == 0 && next + 1 < t_units) {   // (not a ragged last unit)
-            const long long unit_elems = unit_elements(t.period, V, sizeof(S));
-            if (unit_elems >= 1024 || V < 8) {
-                const long long elem0 = next * unit_elems;
-                prefetch_l2_range(t.codes + elem0, unit_elems);
-                prefetch_l2_range(t.g + elem0, unit_elems * sizeof(S));
-                if (!(t.flags & GEFEN_B200_STEP_MUON) && unit_elems * static_cast<int>(sizeof(S)) < 8192) prefetch_l2_range(t.p + elem0, unit_elems * sizeof(S));
-            }
+            const long long unit_elems = unit_elements(t.period, V);
+            const long long elem0 = next * unit_elems;
+            prefetch_l2_range(t.codes + elem0, unit_elems);
+            prefetch_l2_range(t.g + elem0, unit_elems * sizeof(S));
+            if (!(t.flags & GEFEN_B200_STEP_MUON) && unit_elems * static_cast<int>(sizeof(S)) < 8192) prefetch_l2_range(t.p + elem0, unit_elems * sizeof(S));
         }
-        warp_block_step<S, V, GSRC, FULL, STAGED>(t, unit, L, tables, stage, lane);
+        warp_block_step<S, V, GSRC, FULL, HOLD>(t, unit, L, tables, stage, in, lane);
     }
+    wait_for_predecessor();
+}
+
+// --------------------------------------------------------------------------- ring kernel
+// The same step for every usual tensor: gradients in this GPU's buffer, units of up to kRingBytes of codes and gradients.
+// What is different:
+//  * The codes and gradients of a warp's next unit are on their way to shared memory (two bulk copies and one mbarrier
+//    per warp) from the moment that the first pass over the current unit is over, its magnitude and second moment to
+//    registers, its parameters to L2. The first pass waits for nothing.
+//  * The updated momenta of the unit wait in tensor memory (tcgen05.st / tcgen05.ld, four bytes exactly as they are),
+//    which leaves shared memory to those buffers and takes a quarter of the traffic off its data pipe.
+// Twenty warps of 96 registers (fp32: sixteen of 128) instead of sixteen of 128. Before, sixteen warps could not cover the
+// loads of the first pass (long scoreboard 2.06 of 7 cycles per issue, 56 % of the issue slots); now 70 % are used. 134 M
+// bf16 elements (67 M fp32) with second moment and decay, ms before and now: blocks of 2048 0.230 -> 0.199, 1664 0.242 ->
+// 0.188, 1120 0.293 -> 0.222, 512 0.238 -> 0.194, 128 0.333 -> 0.239; fp32 768 0.194 -> 0.166, 1152 0.186 -> 0.170; GefenMuon's
+// momentum, blocks of 2048, 0.242 -> 0.173; rows that are multiples of four only, 300 0.374 -> 0.243 (120 M), 1500 0.328 -> 0.246.
+template <typename S> constexpr int ring_threads() { return sizeof(S) == 2 ? 640 : 512; }
+
+// A warp's descriptors (the current unit's and the next one's) and the barrier of its buffers.
+template <typename S> struct alignas(16) RingWarp {
+    TensorSlot<S> slot[2];
+    uint64_t bar;
+};
+
+template <typename S, int V, bool FULL> struct RingInputs {
+    const StepLaunch& L;
+    const gefen_b200_step_tensor_t* const table;
+    RingWarp<S>& w;
+    const uint32_t buffer, hold;      // shared-memory address of the buffers, tensor-memory address of the warp's columns
+    const int lane;
+    const long long stride;
+    long long unit;                   // the unit that the buffers hold or wait for
+    long long first = 0, units = 0;   // of its tensor
+    int slot = 0;
+    uint32_t parity = 0;
+    float mag = 0.0f, v = 0.0f;       // of its blocks
+    __device__ __forceinline__ RingInputs(const StepLaunch& l, const gefen_b200_step_tensor_t* rows, RingWarp<S>& own, uint32_t buffers, uint32_t columns,
+                                          int lane_, long long unit0, long long stride_)
+        : L(l), table(rows), w(own), buffer(buffers), hold(columns), lane(lane_), stride(stride_), unit(unit0) {}
+    // the copies start on 16 bytes: where the unit's first byte lies in a buffer
+    __device__ __forceinline__ uint32_t g_at(const S* g) const { return buffer + (static_cast<uint32_t>(reinterpret_cast<uintptr_t>(g)) & 15u); }
+    __device__ __forceinline__ uint32_t codes_at(const uint8_t* codes) const {
+        return buffer + L.ring_g + (static_cast<uint32_t>(reinterpret_cast<uintptr_t>(codes)) & 15u);
+    }
+    // [p, p + bytes) widened to 16-byte boundaries: the bytes beside it lie in the same 16 bytes as bytes of the range, and
+    // nothing reads their copies.
+    static __device__ __forceinline__ uint32_t widened(const void* p, uint32_t bytes) {
+        return ((static_cast<uint32_t>(reinterpret_cast<uintptr_t>(p)) & 15u) + bytes + 15u) & ~15u;
+    }
+    static __device__ __forceinline__ void copy(uint32_t dst, const void* p, uint32_t bytes, uint64_t* bar) {
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                     "l"(reinterpret_cast<uintptr_t>(p) & ~static_cast<uintptr_t>(15)), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+    }
+    __device__ __forceinline__ void request() {
+        if (unit >= L.total_blocks) return;
+        if (unit < first || unit >= first + units) {
+            const gefen_b200_step_tensor_t* found = table + find_tensor_warp(table, L.n_tensors, unit);
+            slot ^= 1;
+            if (lane == 0) w.slot[slot].load(found, V);
+            __syncwarp();
+            first = w.slot[slot].first;
+            units = w.slot[slot].units;
+        }
+        const TensorSlot<S>& t = w.slot[slot];
+        const int period = t.period, shift = FULL ? 5 : lanes_shift(period / V, V);
+        const long long b0 = (unit - first) << (5 - shift), left = t.num_blocks - b0;
+        const int blocks = FULL ? 1 : (left < (1 << (5 - shift)) ? static_cast<int>(left) : 1 << (5 - shift));
+        const bool muon = (t.flags & GEFEN_B200_STEP_MUON) != 0;
+        if (lane == 0) {
+            const uint32_t elems = static_cast<uint32_t>(blocks * period);
+            const S* const g = t.g + b0 * period;
+            const uint8_t* const codes = t.codes + b0 * period;
+            const uint32_t g_bytes = widened(g, elems * static_cast<uint32_t>(sizeof(S))), code_bytes = widened(codes, elems);
+            mbar_expect_tx(&w.bar, g_bytes + code_bytes);
+            copy(buffer, g, g_bytes, &w.bar);
+            copy(buffer + L.ring_g, codes, code_bytes, &w.bar);
+            if (!muon) prefetch_l2_range(t.p + b0 * period, elems * static_cast<uint32_t>(sizeof(S)));
+        }
+        const long long b = b0 + (lane >> shift);
+        const bool valid = (lane >> shift) < blocks;
+        mag = valid ? load_state(t.mag, b, t.mag_dtype) : 0.0f;
+        v = valid && !muon ? (L.stepsize != nullptr ? L.stepsize[b] : load_state(t.v, b, t.v_dtype)) : 1.0f;
+    }
+    __device__ __forceinline__ void request_next() {
+        unit += stride;
+        request();
+    }
+    __device__ __forceinline__ bool arrived(uint32_t limit) {
+        const bool ok = mbar_wait_bounded(&w.bar, parity, limit);
+        parity ^= 1u;
+        return __all_sync(0xffffffffu, ok);
+    }
+};
+
+template <typename S, int V, bool FULL>
+__global__ void __launch_bounds__(ring_threads<S>(), 1) step_ring_kernel(const __grid_constant__ StepLaunch L,
+                                                                         const __grid_constant__ StepRows rows) {
+    __shared__ uint32_t tmem_base;
+    SmemView s;
+    let_successor_in();
+    if (smem_u32(g_smem) > kFixed) {   // (as in step_vec_kernel)
+        if (threadIdx.x == 0) atomicOr(&g_step_status, 2);
+        wait_for_predecessor();
+        return;
+    }
+    if (!stage_tables(L.ws, fast_smem(kWsAt), s, L.spin_limit)) { wait_for_predecessor(); return; }
+    const int lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+    const int warps = blockDim.x >> 5;
+    const LaneTables tables = build_lane_tables(s, fast_smem(kStageAt));
+    RingWarp<S>& own = reinterpret_cast<RingWarp<S>*>(fast_smem(kStageAt))[warp];
+    if (warp == 0) {   // (waits while another CTA of this SM holds the columns: that one ends by itself)
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)), "r"(L.tmem_columns) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (lane == 0) {
+        mbar_init(&own.bar, 1);
+        fence_mbar_init();
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // a warp reaches the 32 lanes of tensor memory that its place in its group of four gives it
+    const uint32_t hold = tmem_base + (static_cast<uint32_t>(warp & 3) << 21) + static_cast<uint32_t>((warp >> 2) * L.hold_columns);
+    const uint32_t buffer = kStageAt + static_cast<uint32_t>(sizeof(RingWarp<S>)) * warps + static_cast<uint32_t>(warp * (L.ring_g + L.ring_codes));
+    // Neighbouring units go to different SMs; where they share lines of memory (small chunks) and there are many, to
+    // the warps of one SM. (134 M bf16 elements in blocks of 1664 0.203 against 0.188 ms, of 128 0.256 / 0.236; with
+    // chunks of four, blocks of 2500, 0.234 / 0.261; chunks of one, blocks of 27, 0.540 / 0.612.)
+    const long long warp_stride = static_cast<long long>(gridDim.x) * warps;
+    const bool spread = V == 8 || L.total_blocks <= warp_stride;
+    const long long warp_global = spread ? static_cast<long long>(warp) * gridDim.x + blockIdx.x : static_cast<long long>(blockIdx.x) * warps + warp;
+    RingInputs<S, V, FULL> in(L, L.table != nullptr ? L.table : rows.row, own, buffer, hold, lane, warp_global, warp_stride);
+    in.request();
+    for (long long gb = warp_global; gb < L.total_blocks; gb += warp_stride) {
+        if (!warp_block_step<S, V, 0, FULL, kTensor>(own.slot[in.slot], gb - in.first, L, tables, nullptr, in, lane)) {
+            // the wait for the inputs ran out: this warp leaves its blocks as they are, but not before the copies have ended
+            if (lane == 0) atomicOr(&g_step_status, 1);
+            mbar_wait_bounded(&own.bar, in.parity ^ 1u, kStageDrainLimit);
+            break;
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(L.tmem_columns) : "memory");
     wait_for_predecessor();
 }
 
@@ -1709,10 +2003,10 @@ static int launch_step(K kernel, int grid, int threads, int smem, const StepLaun
     return GEFEN_B200_OK;
 }
 
-template <typename S, int V, int GSRC, bool FULL, bool STAGED = true>
+template <typename S, int V, int GSRC, bool FULL, int HOLD = kShared>
 static int launch_vec_variant(StepLaunch L, const StepRows& rows, long long max_unit, cudaStream_t stream) {
     static bool configured[kMaxDevices];
-    auto kernel = step_vec_kernel<S, V, GSRC, FULL, STAGED>;
+    auto kernel = step_vec_kernel<S, V, GSRC, FULL, HOLD>;
     {
         int dev = 0;
         const int rc = current_device(&dev);
@@ -1725,7 +2019,7 @@ static int launch_vec_variant(StepLaunch L, const StepRows& rows, long long max_
     }
     // a warp stages one unit: one long block, or the 32 / lanes shorter blocks that share the warp
     // (max_unit: the largest need of the launch, see unit_floats; a slice starts on 16 bytes)
-    const long long stage_bytes = ((STAGED && max_unit > 256 ? max_unit : 256) * 4 + 15) / 16 * 16;   // (256: build_lane_tables)
+    const long long stage_bytes = ((HOLD == kShared && max_unit > 256 ? max_unit : 256) * 4 + 15) / 16 * 16;   // (256: build_lane_tables)
     int max_warps = kVecThreads / 32;
     if (warps_override() > 0 && warps_override() < max_warps) max_warps = warps_override();
     int warps = static_cast<int>((kMaxSmem - kStaticSmemSlack - kSmemTables) / stage_bytes);
@@ -1741,39 +2035,86 @@ static int launch_vec_variant(StepLaunch L, const StepRows& rows, long long max_
     return launch_step(kernel, grid, warps * 32, smem, L, rows, stream);
 }
 
-// Blocks of more than 2048 elements (fp32: 3072) in chunks of eight, this GPU's buffers only: their slices of shared
-// memory would leave fifteen warps and fewer (four for 8192 elements), so the second pass forms the momenta once more
-// instead (Momenta; launch class 1 to callers). 134 M bf16 / 67 M fp32 elements, ms, staged against computed: blocks of
-// 2056 0.299 / 0.220 and 0.289 / 0.212, 2560 0.259 / 0.201 and 0.249 / 0.202, 3072 0.282 / 0.212 and 0.263 / 0.218, 4096
-// 0.381 / 0.235 and 0.267 / 0.226, 8192 0.626 / 0.371 and 0.304 / 0.243.
-constexpr int kLongClass = 7;
-static int long_class(int cls, long long period, int dtype) {
-    return cls == 1 && period > (dtype_size(dtype) == 2 ? 2048 : 3072) ? kLongClass : cls;
+// Kernels of the fast path beyond the classes of tensors: kRing + class = step_ring_kernel, kTwiceClass = long blocks
+// whose momenta are formed twice; a class by itself = step_vec_kernel with staged momenta.
+constexpr int kTwiceClass = 7, kRing = 16;
+// The most that the ring kernel's buffers of a unit may take (codes and gradients; this much leaves six warps). Blocks of
+// 4096 fp32 elements: 0.224 ms with the momenta formed twice (66 M elements), 0.186 here; bf16, 134 M: 4096 0.264 against
+// 0.225, 5120 0.277 / 0.239, 8192 (24 KB) 0.300 / 0.323.
+constexpr int kRingBytes = 20480;
+static int route(int cls, long long period, int dtype, int n_peers, int n_grad_srcs) {
+    if (cls < 1 || cls > 5 || n_grad_srcs > 0) return cls;   // (averaged gradients: the staged kernels)
+    if (cls >= 3 && n_peers > 0) return cls;                 // (small chunks with peer stores: staged)
+    const int v = cls <= 2 ? 8 : (cls == 3 ? 4 : (cls == 4 ? 2 : 1)), es = dtype_size(dtype);
+    // Small chunks with fewer than four lanes per block read the buffers from many blocks at once, on the same banks unless
+    // a block is an odd number of chunks.
+    const bool conflicts = v < 8 && lanes_shift(period / v, v) < 2 && (period / v) % 2 == 0;
+    if (!conflicts && unit_elements(period, v) * (es + 1) <= kRingBytes) return kRing + cls;
+    return cls == 1 && n_peers == 0 ? kTwiceClass : cls;
+}
+
+template <typename S, int V, bool FULL>
+static int launch_ring(StepLaunch L, const StepRows& rows, long long max_unit, cudaStream_t stream) {
+    static bool configured[kMaxDevices];
+    auto kernel = step_ring_kernel<S, V, FULL>;
+    constexpr int kMost = kMaxSmem - kStaticSmemSlack;
+    {
+        int dev = 0;
+        const int rc = current_device(&dev);
+        if (rc != GEFEN_B200_OK) return rc;
+        std::lock_guard<std::mutex> lock(g_config_mutex);
+        if (!configured[dev]) {
+            GEFEN_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost));
+            configured[dev] = true;
+        }
+    }
+    // (a copy of n bytes from any address covers at most n + 30 bytes when it is widened to 16-byte boundaries)
+    L.ring_g = static_cast<int>((max_unit * static_cast<int>(sizeof(S)) + 30) / 16 * 16);
+    L.ring_codes = static_cast<int>((max_unit + 30) / 16 * 16);
+    const int each = L.ring_g + L.ring_codes + static_cast<int>(sizeof(RingWarp<S>));
+    // a lane's momenta of one unit: whole rounds of chunks
+    L.hold_columns = static_cast<int>((max_unit + 31) / 32 + 7) / 8 * 8;
+    int warps = ring_threads<S>() / 32;
+    if (warps_override() > 0 && warps_override() < warps) warps = warps_override();
+    if (warps > (kMost - kSmemTables) / each) warps = (kMost - kSmemTables) / each;
+    if (warps > 512 / L.hold_columns * 4) warps = 512 / L.hold_columns * 4;
+    if (warps < 1) return fail(GEFEN_B200_EINVAL, "internal: unit of %lld elements too large for the ring", max_unit);
+    L.tmem_columns = 32;
+    while (L.tmem_columns < (warps + 3) / 4 * L.hold_columns) L.tmem_columns *= 2;
+    int smem = kSmemTables + each * warps;
+    if (smem < kSmemTables + 2048) smem = kSmemTables + 2048;   // (build_lane_tables)
+    return launch_step(kernel, grid_for(L.total_blocks, 1, 1), warps * 32, smem, L, rows, stream);
 }
 
 template <typename S>
 static int launch_vec(int cls, StepLaunch L, const StepRows& rows, long long max_unit, cudaStream_t stream) {
-    if (cls >= 3 && cls <= 5 && (L.n_peers > 0 || L.n_grad_srcs > 0)) {
+    switch (cls) {
+        case 6: {
+            constexpr int kPer = kVectorThreads / 32;
+            return launch_step(step_vector_kernel<S>, static_cast<int>((L.total_blocks + kPer - 1) / kPer), kVectorThreads, kSmemWs, L, rows, stream);
+        }
+        case kRing + 1: return launch_ring<S, 8, true>(L, rows, max_unit, stream);
+        case kRing + 2: return launch_ring<S, 8, false>(L, rows, max_unit, stream);
+        case kRing + 3: return launch_ring<S, 4, false>(L, rows, max_unit, stream);
+        case kRing + 4: return launch_ring<S, 2, false>(L, rows, max_unit, stream);
+        case kRing + 5: return launch_ring<S, 1, false>(L, rows, max_unit, stream);
+        case kTwiceClass: return launch_vec_variant<S, 8, 0, true, kTwice>(L, rows, max_unit, stream);
+        case 1:
+            if (L.grad_mc_delta != 0) return launch_vec_variant<S, 8, 2, true>(L, rows, max_unit, stream);
+            if (L.n_grad_srcs > 0) return launch_vec_variant<S, 8, 1, true>(L, rows, max_unit, stream);
+            return launch_vec_variant<S, 8, 0, true>(L, rows, max_unit, stream);
+        case 2:
+            if (L.grad_mc_delta != 0) return launch_vec_variant<S, 8, 2, false>(L, rows, max_unit, stream);
+            return launch_vec_variant<S, 8, 1, false>(L, rows, max_unit, stream);
+    }
+    if (L.n_peers > 0 || L.n_grad_srcs > 0) {
         if (cls == 3) return launch_vec_variant<S, 4, 1, false>(L, rows, max_unit, stream);
         if (cls == 4) return launch_vec_variant<S, 2, 1, false>(L, rows, max_unit, stream);
         return launch_vec_variant<S, 1, 1, false>(L, rows, max_unit, stream);
     }
     if (cls == 3) return launch_vec_variant<S, 4, 0, false>(L, rows, max_unit, stream);
     if (cls == 4) return launch_vec_variant<S, 2, 0, false>(L, rows, max_unit, stream);
-    if (cls == 5) return launch_vec_variant<S, 1, 0, false>(L, rows, max_unit, stream);
-    if (cls == kLongClass) return launch_vec_variant<S, 8, 0, true, false>(L, rows, max_unit, stream);
-    if (cls == 6) {
-        constexpr int kPer = kVectorThreads / 32;
-        return launch_step(step_vector_kernel<S>, static_cast<int>((L.total_blocks + kPer - 1) / kPer), kVectorThreads, kSmemWs, L, rows, stream);
-    }
-    if (cls == 1) {
-        if (L.grad_mc_delta != 0) return launch_vec_variant<S, 8, 2, true>(L, rows, max_unit, stream);
-        if (L.n_grad_srcs > 0) return launch_vec_variant<S, 8, 1, true>(L, rows, max_unit, stream);
-        return launch_vec_variant<S, 8, 0, true>(L, rows, max_unit, stream);
-    }
-    if (L.grad_mc_delta != 0) return launch_vec_variant<S, 8, 2, false>(L, rows, max_unit, stream);
-    if (L.n_grad_srcs > 0) return launch_vec_variant<S, 8, 1, false>(L, rows, max_unit, stream);
-    return launch_vec_variant<S, 8, 0, false>(L, rows, max_unit, stream);
+    return launch_vec_variant<S, 1, 0, false>(L, rows, max_unit, stream);
 }
 
 template <typename S>
@@ -1803,8 +2144,11 @@ static int launch_generic(bool cta_per_block, const StepLaunch& L, const StepRow
 // divides the block length and the alignment of all pointers), 6 = vectors (period 1, runs of up to 256 elements), 0 =
 // generic warp per block, -1 = generic CTA per block.
 static int generic_class(const gefen_b200_step_tensor_t& t) { return t.period > 2048 ? -1 : 0; }
-static int class_chunk(int cls) { return cls <= 2 || cls == kLongClass ? 8 : (cls == 3 ? 4 : (cls == 4 ? 2 : 1)); }
-static bool staged_class(int cls) { return (cls >= 1 && cls <= 5) || cls == kLongClass; }
+static int class_chunk(int cls) {
+    cls &= kRing - 1;
+    return cls <= 2 || cls == kTwiceClass ? 8 : (cls == 3 ? 4 : (cls == 4 ? 2 : 1));
+}
+static bool staged_class(int cls) { return cls >= 1 && cls != 6; }
 static int tensor_class(const gefen_b200_step_tensor_t& t, int dtype) {
     const bool vec_dtype = dtype == GEFEN_B200_F32 || dtype == GEFEN_B200_BF16 || dtype == GEFEN_B200_F16;
     if (vec_dtype && (t.flags & GEFEN_B200_STEP_PERIOD1) != 0 && t.period <= kVectorMost && t.num_blocks < (1 << 28)) return 6;
@@ -1814,14 +2158,14 @@ static int tensor_class(const gefen_b200_step_tensor_t& t, int dtype) {
         const int v = class_chunk(cls);
         const uintptr_t bytes = static_cast<uintptr_t>(v * dtype_size(dtype) < 16 ? v * dtype_size(dtype) : 16);
         if (t.period % v != 0 || ptrs % bytes != 0 || reinterpret_cast<uintptr_t>(t.codes) % v != 0) continue;
-        return cls == 2 && lanes_shift(t.period / 8, 8, dtype_size(dtype)) == 5 ? 1 : cls;
+        return cls == 2 && lanes_shift(t.period / 8, 8) == 5 ? 1 : cls;
     }
     return generic_class(t);   // (a pointer that is not aligned to its own type)
 }
 // Units of a tensor in its launch's index space: passes of a warp on the staged path, blocks elsewhere.
 // (4-bit codes with an odd period: a pair of blocks is one unit, see step_generic_kernel)
 static long long class_units(const gefen_b200_step_tensor_t& t, int cls, int dtype) {
-    if (staged_class(cls)) return vec_units(t.num_blocks, t.period, class_chunk(cls), dtype_size(dtype));
+    if (staged_class(cls)) return vec_units(t.num_blocks, t.period, class_chunk(cls));
     const bool paired = (t.flags & GEFEN_B200_STEP_PACKED) != 0 && (t.period & 1) != 0;
     return paired ? (t.num_blocks + 1) / 2 : t.num_blocks;
 }
@@ -1866,7 +2210,7 @@ static int run_single(gefen_b200_step_tensor_t& t, int param_dtype, const float*
     L.table = nullptr;
     L.n_tensors = 1;
     L.stage_floats = 0;
-    const int cls = long_class(tensor_class(t, param_dtype), t.period, param_dtype);
+    const int cls = route(tensor_class(t, param_dtype), t.period, param_dtype, 0, 0);
     L.total_blocks = class_units(t, cls, param_dtype);
     L.ws = static_cast<const unsigned char*>(ws);
     L.stepsize = stepsize;
@@ -1879,7 +2223,7 @@ static int run_single(gefen_b200_step_tensor_t& t, int param_dtype, const float*
     L.follows = 0;
     StepRows rows = {};
     rows.row[0] = t;
-    return launch_class(cls, param_dtype, L, rows, staged_class(cls) ? unit_floats(t.period, class_chunk(cls), dtype_size(param_dtype)) : t.period, stream);
+    return launch_class(cls, param_dtype, L, rows, staged_class(cls) ? unit_floats(t.period, class_chunk(cls)) : t.period, stream);
 }
 
 }  // namespace gefen
@@ -2214,8 +2558,7 @@ int gefen_b200_multi_tensor_step_multicast(gefen_b200_step_tensor_t* host_table,
         int cls = tensor_class(t, param_dtype);
         // vectors with peers: the generic kernel (no sums of squares there, so the results are the same bits)
         if (cls == 6 && (n_peers > 0 || n_grad_srcs > 0)) cls = generic_class(t);
-        if (n_peers == 0 && n_grad_srcs == 0) cls = long_class(cls, t.period, param_dtype);
-        t.reserved_[0] = cls;
+        t.reserved_[0] = route(cls, t.period, param_dtype, n_peers, n_grad_srcs);
     }
     for (int begin = 0; begin < n_tensors;) {
         int end = begin;
@@ -2245,7 +2588,7 @@ int gefen_b200_multi_tensor_step_multicast(gefen_b200_step_tensor_t* host_table,
         long long max_period = 0;   // largest staging need of a warp: the elements of one unit on the staged path
         for (int i = begin; i < begin + run; ++i) {
             const int cls = host_table[begin].reserved_[0];
-            const long long need = staged_class(cls) ? unit_floats(host_table[i].period, class_chunk(cls), dtype_size(param_dtype)) : host_table[i].period;
+            const long long need = staged_class(cls) ? unit_floats(host_table[i].period, class_chunk(cls)) : host_table[i].period;
             max_period = need > max_period ? need : max_period;
         }
         if (total > 0) {
