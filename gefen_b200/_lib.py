@@ -77,6 +77,8 @@ def _declare(lib):
             i32, [vp, vp, i32, vp, vp, i32, vp, vp, i32, vp, i32, i64, i64, dbl, dbl, vp]),
         "gefen_b200_automatic_gefen_period1_update": (
             i32, [vp, vp, i32, vp, vp, i32, vp, i32, vp, i32, vp, i64, i64, dbl, dbl, dbl, dbl, dbl, dbl, vp]),
+        "gefen_b200_automatic_gefen_step": (
+            i32, [vp, vp, i32, vp, vp, i32, vp, i32, vp, i32, vp, i64, i64, i32, dbl, dbl, dbl, dbl, dbl, dbl, dbl, vp]),
         "gefen_b200_automatic_gefen_muon_momentum": (
             i32, [vp, i32, vp, vp, i32, vp, i32, vp, vp, i32, i64, i64, dbl, vp]),
         "gefen_b200_multi_tensor_step": (i32, [vp, vp, i32, i32, vp, vp]),

@@ -2325,6 +2325,29 @@ int gefen_b200_automatic_gefen_period1_update(
     return run_single(t, param_dtype, nullptr, codebook, codebook_size, codebook_ws, static_cast<cudaStream_t>(stream));
 }
 
+int gefen_b200_automatic_gefen_step(
+    void* p, const void* grad, int param_dtype, uint8_t* m_sign, void* m_magnitude, int magnitude_dtype, void* vmean,
+    int vmean_dtype, const float* codebook, int codebook_size, const void* codebook_ws, int64_t num_blocks, int64_t period,
+    int period_one, double beta1, double beta2, double lr, double weight_decay_mul, double bias_correction_1,
+    double bias_correction_2, double eps, void* stream) {
+    int rc = check_common(grad, m_sign, m_magnitude, magnitude_dtype, param_dtype, 0, num_blocks, period);
+    if (rc != GEFEN_B200_OK) return rc;
+    GEFEN_CHECK_ARG(p != nullptr && vmean != nullptr, "Expected non-null p and vmean.");
+    GEFEN_CHECK_ARG(is_state_dtype(vmean_dtype), "Expected vmean to have dtype float32, float16, or bfloat16.");
+    GEFEN_CHECK_ARG(bias_correction_1 > 0.0, "Expected bias_correction_1 to be positive.");
+    GEFEN_CHECK_ARG(bias_correction_2 > 0.0, "Expected bias_correction_2 to be positive.");
+    GEFEN_CHECK_ARG(eps >= 0.0, "Expected eps to be non-negative.");
+    gefen_b200_step_tensor_t t = {};
+    t.p = p; t.g = grad; t.codes = m_sign; t.mag = m_magnitude; t.v = vmean;
+    t.num_blocks = num_blocks; t.period = period;
+    t.beta1 = static_cast<float>(beta1); t.beta2 = static_cast<float>(beta2); t.lr = static_cast<float>(lr);
+    t.bc1 = static_cast<float>(bias_correction_1); t.bc2 = static_cast<float>(bias_correction_2);
+    t.eps = static_cast<float>(eps); t.wd_mul = static_cast<float>(weight_decay_mul);
+    t.flags = (period_one ? GEFEN_B200_STEP_PERIOD1 : GEFEN_B200_STEP_FUSE_VMEAN) | (weight_decay_mul != 1.0 ? GEFEN_B200_STEP_WEIGHT_DECAY : 0u);
+    t.mag_dtype = magnitude_dtype; t.v_dtype = vmean_dtype;
+    return run_single(t, param_dtype, nullptr, codebook, codebook_size, codebook_ws, static_cast<cudaStream_t>(stream));
+}
+
 int gefen_b200_automatic_gefen_muon_momentum(
     const void* grad_view, int grad_dtype, uint8_t* m_sign, void* m_magnitude, int magnitude_dtype,
     const float* codebook, int codebook_size, const void* codebook_ws, void* momentum_update, int packed_indices,

@@ -142,6 +142,50 @@ def automatic_gefen_period1_update_cuda(p, grad_flat, m_sign, m_magnitude, vmean
             float(bias_correction_1), float(bias_correction_2), float(eps), _lib.current_stream(p.device)))
 
 
+def automatic_gefen_step_cuda(p, grad_view, m_sign, m_magnitude, vmean, codebook, period_one: bool, beta1: float,
+                              beta2: float, lr: float, weight_decay_mul: float, bias_correction_1: float,
+                              bias_correction_2: float, eps: float) -> None:
+    """The whole step of one tensor in one launch: second moment, decoupled weight decay (weight_decay_mul = 1 - lr * wd, or
+    1) and update. grad_view: [blocks, period]; period_one: [runs, elements of a run] with a second moment per element."""
+    require_cuda_tensors({"p": p, "grad_view": grad_view, "m_sign": m_sign, "m_magnitude": m_magnitude,
+                          "vmean": vmean, "codebook": codebook})
+    if grad_view.dim() != 2:
+        raise ValueError("Expected grad_view to be 2D, got dim={}".format(grad_view.dim()))
+    if grad_view.dtype != p.dtype:
+        raise ValueError("Expected grad_view dtype {} to match p dtype {}.".format(grad_view.dtype, p.dtype))
+    require_block_column("m_magnitude", m_magnitude)
+    require_block_column("vmean", vmean)
+    numel = grad_view.numel()
+    if grad_view.shape[0] != m_magnitude.shape[0]:
+        raise ValueError("Expected grad_view and m_magnitude to have the same number of blocks.")
+    if (numel if period_one else grad_view.shape[0]) != vmean.shape[0]:
+        raise ValueError("Expected vmean to have one row per {}.".format("element" if period_one else "block"))
+    require_state_dtype("m_magnitude", m_magnitude)
+    require_state_dtype("vmean", vmean)
+    require_codebook(codebook)
+    require_index_count(m_sign, numel, False)
+    if not 0.0 <= beta2 <= 1.0:
+        raise ValueError("Expected beta2 to be in [0, 1], got {}.".format(beta2))
+    if bias_correction_1 <= 0.0:
+        raise ValueError("Expected bias_correction_1 to be positive, got {}".format(bias_correction_1))
+    if bias_correction_2 <= 0.0:
+        raise ValueError("Expected bias_correction_2 to be positive, got {}".format(bias_correction_2))
+    if eps < 0.0:
+        raise ValueError("Expected eps to be non-negative, got {}".format(eps))
+    if p.numel() != numel:
+        raise ValueError("Expected p.numel() to match grad_view.numel().")
+    grad_view = grad_view.contiguous()
+    codebook = codebook.contiguous()
+    require_contiguous({"p": p, "m_sign": m_sign, "m_magnitude": m_magnitude, "vmean": vmean})
+    with _lib.device_guard(p.device):
+        _lib.check(_lib.load().gefen_b200_automatic_gefen_step(
+            _lib.ptr(p), _lib.ptr(grad_view), _lib.dtype_tag(p.dtype), _lib.ptr(m_sign), _lib.ptr(m_magnitude),
+            _lib.dtype_tag(m_magnitude.dtype), _lib.ptr(vmean), _lib.dtype_tag(vmean.dtype), _lib.ptr(codebook),
+            codebook.numel(), _ws(codebook), grad_view.shape[0], grad_view.shape[1], int(period_one), float(beta1),
+            float(beta2), float(lr), float(weight_decay_mul), float(bias_correction_1), float(bias_correction_2),
+            float(eps), _lib.current_stream(p.device)))
+
+
 def automatic_gefen_muon_momentum_cuda(grad_view, m_sign, m_magnitude, codebook, momentum_update,
                                        packed_indices: bool, beta1: float) -> None:
     """GefenMuon's quantised momentum: writes the dequantised new momentum into `momentum_update`

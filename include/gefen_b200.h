@@ -109,6 +109,15 @@ int gefen_b200_automatic_gefen_period1_update(
     double beta2, double lr, double bias_correction_1, double bias_correction_2, double eps,
     void* stream);
 
+/* The whole step of one tensor in one launch: the second moment (period_one: per element, num_blocks runs of `period`
+ * elements with a magnitude each; otherwise the mean square of each block), the decoupled weight decay p <- round(p *
+ * weight_decay_mul) and the update. What gefen_b200_multi_tensor_step does for a table of one row, without a table. */
+int gefen_b200_automatic_gefen_step(
+    void* p, const void* grad, int param_dtype, uint8_t* m_sign, void* m_magnitude, int magnitude_dtype, void* vmean,
+    int vmean_dtype, const float* codebook, int codebook_size, const void* codebook_ws, int64_t num_blocks,
+    int64_t period, int period_one, double beta1, double beta2, double lr, double weight_decay_mul,
+    double bias_correction_1, double bias_correction_2, double eps, void* stream);
+
 /* Replaces automatic_gefen_muon_momentum_cuda (gefen_cuda_binding.cpp:49-57;
  * automatic_gefen_fused_kernel.cu:1002-1103): momentum_update <- dequantised new momentum. */
 int gefen_b200_automatic_gefen_muon_momentum(

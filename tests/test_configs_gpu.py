@@ -161,3 +161,30 @@ def test_config4_llama_32b_layer_multi_tensor_equals_per_tensor(cuda_device):
         worst = max(worst, err)
         assert err <= 1e-4, "parameters differ by {:.3e} (relative L2)".format(err)
     assert periods & {1664, 1120, 3328, 2240, 6656, 8960, 17920} or max(periods) > 1024
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("wd", [0.0, 0.1])
+def test_step_of_one_tensor_in_one_call(cuda_device, dtype, wd):
+    """fused=False against fused=True on short, long, ragged and one-element tensors: the same bits."""
+    from gefen_b200 import Gefen
+
+    shapes = [(40, 512), (16, 9000), (50, 300), (1,), (77,), (24, 2056)]
+    gen = torch.Generator().manual_seed(3)
+    made = [torch.randn(s, generator=gen) * 0.02 for s in shapes]
+    opts = []
+    for fused in (True, False):
+        params = [("p%d" % i, torch.nn.Parameter(t.to(cuda_device, dtype))) for i, t in enumerate(made)]
+        opts.append((Gefen(params, lr=3e-4, weight_decay=wd, fused=fused), [p for _, p in params]))
+    for _ in range(3):
+        grads = [(torch.randn(s, generator=gen) * 1e-3).to(cuda_device, dtype) for s in shapes]
+        for opt, params in opts:
+            for p, g in zip(params, grads):
+                p.grad = g.clone()
+            opt.step()
+    for a, b in zip(opts[0][1], opts[1][1]):
+        assert torch.equal(a, b)
+        for k, v in opts[0][0].state[a].items():
+            w = opts[1][0].state[b][k]
+            assert torch.equal(v, w) if torch.is_tensor(v) else v == w
