@@ -234,7 +234,7 @@ class Gefen(torch.optim.Optimizer):
                 raise ValueError("gefen_b200 needs CUDA gradients, got device {} for {}".format(grad.device, name))
         require_one_device("the gradients of one optimizer", [grad for _, _, grad in todo])
         found, stats = partitioning.launch_period_scores_many([grad for _, _, grad in todo])
-        host = torch.cat([s.cpu() for s in stats], dim=0) if stats else None
+        host = torch.cat([s.cpu() for s in stats], dim=0).tolist() if stats else None
         periods, cursor = [], 0
         for n, cand in found:
             if not cand:
@@ -310,10 +310,11 @@ class Gefen(torch.optim.Optimizer):
             self._gefen_codebook = codebook.contiguous()
 
     # ------------------------------------------------------------------ state
-    def _init_gefen_state(self, state, grad_view: torch.Tensor) -> None:
-        """reference :1039-1062"""
+    def _init_gefen_state(self, state, grad_view: torch.Tensor, fresh: Optional[list] = None) -> None:
+        """reference :1039-1062. fresh: takes the new tensors unwritten, for the caller to zero together (see _zeroed)."""
+        make = torch.zeros if fresh is None else torch.empty
         state["m_codebook_shape"] = tuple(grad_view.shape)
-        state["m_codebook"] = torch.zeros(grad_view.shape, dtype=torch.uint8, device=grad_view.device)
+        state["m_codebook"] = make(grad_view.shape, dtype=torch.uint8, device=grad_view.device)
         state_dtype = gefen_state_dtype_from_grad(grad_view)
         if grad_view.shape[1] == 1:
             d = self._period_one_divisor_for_numel(grad_view.numel())
@@ -323,10 +324,23 @@ class Gefen(torch.optim.Optimizer):
             rows = grad_view.shape[0]
         else:
             raise ValueError("Expected grad_view second dimension to be positive, got {}".format(grad_view.shape[1]))
-        state["m_magnitude"] = torch.zeros((rows, 1), dtype=state_dtype, device=grad_view.device)
+        state["m_magnitude"] = make((rows, 1), dtype=state_dtype, device=grad_view.device)
+        if fresh is not None:
+            fresh += [state["m_codebook"], state["m_magnitude"]]
 
-    def _ensure_state(self, name: str, p, local_p: torch.Tensor, grad: torch.Tensor, with_vmean: bool = True):
-        """First visit of a parameter (reference :1232-1268)."""
+    @staticmethod
+    def _zeroed(fresh) -> None:
+        """Zeroes new state tensors, a few launches for each type. (A fill per tensor is three launches per parameter: the
+        first step of GPT-2 125M, 148 tensors, took 20.5 ms with them and takes 17.5 ms.)"""
+        by_type = {}
+        for t in fresh:
+            by_type.setdefault((t.dtype, t.device), []).append(t)
+        for tensors in by_type.values():
+            torch._foreach_zero_(tensors)
+
+    def _ensure_state(self, name: str, p, local_p: torch.Tensor, grad: torch.Tensor, with_vmean: bool = True,
+                      fresh: Optional[list] = None):
+        """First visit of a parameter (reference :1232-1268). fresh: see _init_gefen_state."""
         state = self.state[p]
         if "step" in state:
             return state
@@ -343,10 +357,12 @@ class Gefen(torch.optim.Optimizer):
         state["automatic_period"] = period
         state["step"] = 0
         grad_view = automatic_partition_view(grad.reshape(-1), period)
-        self._init_gefen_state(state, grad_view)
+        self._init_gefen_state(state, grad_view, fresh)
         if with_vmean:
-            state["vmean"] = torch.zeros((grad_view.shape[0], 1), dtype=gefen_state_dtype_from_grad(grad_view),
-                                         device=grad_view.device)
+            make = torch.zeros if fresh is None else torch.empty
+            state["vmean"] = make((grad_view.shape[0], 1), dtype=gefen_state_dtype_from_grad(grad_view), device=grad_view.device)
+            if fresh is not None:
+                fresh.append(state["vmean"])
         return state
 
     # ------------------------------------------------------------------ step, per-tensor launches
@@ -534,8 +550,13 @@ class Gefen(torch.optim.Optimizer):
             raise ValueError("Expected Gefen codebook to be initialized before fused update.")
         self._require_codebook_beside(work)
         copies = []
+        fresh = []
+        try:
+            for group, name, p, local_p, grad in work:
+                self._ensure_state(name, p, local_p, grad, fresh=fresh)
+        finally:   # (a refused parameter leaves the ones before it with a valid state)
+            self._zeroed(fresh)
         for i, (group, name, p, local_p, grad) in enumerate(work):
-            self._ensure_state(name, p, local_p, grad)
             fused_p = self._contiguous_param(p, local_p, name)
             if not grad.is_contiguous():
                 grad = grad.contiguous()

@@ -124,11 +124,12 @@ def period_scan_many_async(flats, periods, *, input_is_squared: bool, epsilon: f
     return out
 
 
-def scores_from_stats(stats_host: torch.Tensor):
-    """Applies the reference's error rule (period_variance_kernel.cu:392-394) to fetched stats."""
-    if stats_host.numel() and bool((stats_host[:, 1] > 0).any()):
+def scores_from_stats(stats_host):
+    """Applies the reference's error rule (period_variance_kernel.cu:392-394) to fetched stats (rows of a tensor, or lists)."""
+    rows = stats_host.tolist() if isinstance(stats_host, torch.Tensor) else stats_host
+    if any(invalid > 0 for _, invalid in rows):
         raise RuntimeError("Expected values plus epsilon to be positive before log transform.")
-    return [float(s) for s in stats_host[:, 0].tolist()]
+    return [score for score, _ in rows]
 
 
 def period_scan(flat: torch.Tensor, periods, *, input_is_squared: bool, epsilon: float):

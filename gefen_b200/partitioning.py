@@ -138,7 +138,8 @@ def launch_period_scores_many(grads, epsilon: float = 1e-12, min_num_blocks: int
     return found, stats
 
 
-def decide_period(n: int, periods: Sequence[int], stats_host: Optional[torch.Tensor], print_results: bool = False) -> int:
+def decide_period(n: int, periods: Sequence[int], stats_host, print_results: bool = False) -> int:
+    """stats_host: the fetched rows of (score, invalid count), a tensor or a list."""
     from .kernels.period_variance import scores_from_stats
 
     if not periods:
