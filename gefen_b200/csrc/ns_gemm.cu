@@ -1086,12 +1086,20 @@ __global__ void __launch_bounds__(kElemThreads) ns_norm_kernel(const NsMatrix* _
     const long long end = begin + per < n ? begin + per : n;
     float acc = 0.0f;
     long long i = begin + static_cast<long long>(threadIdx.x) * kVec;
-    for (; i + kVec <= end; i += kElemThreads * kVec) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(src + i);
+    auto take = [&](const uint4& raw) {
         const S* v = reinterpret_cast<const S*>(&raw);
 #pragma unroll
         for (int e = 0; e < kVec; ++e) { const float f = as_bf16(v + e); acc = fmaf(f, f, acc); }
+    };
+    constexpr int kAhead = 8;   // pieces in flight (28 matrices, 0.2 G bf16 elements: 102 -> 94 us)
+    for (; i + (kAhead - 1) * kElemThreads * kVec + kVec <= end; i += kAhead * kElemThreads * kVec) {
+        uint4 raw[kAhead];
+#pragma unroll
+        for (int q = 0; q < kAhead; ++q) raw[q] = *reinterpret_cast<const uint4*>(src + i + q * kElemThreads * kVec);
+#pragma unroll
+        for (int q = 0; q < kAhead; ++q) take(raw[q]);
     }
+    for (; i + kVec <= end; i += kElemThreads * kVec) take(*reinterpret_cast<const uint4*>(src + i));
     for (; i < end; ++i) { const float f = as_bf16(src + i); acc = fmaf(f, f, acc); }   // (at most one thread)
     acc = warp_sum(acc);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
@@ -1102,6 +1110,19 @@ __global__ void __launch_bounds__(kElemThreads) ns_norm_kernel(const NsMatrix* _
         parts[blockIdx.y * kNormParts + blockIdx.x] = t;
     }
 }
+
+// The IEEE quotient by the matrix's norm, through its reciprocal where that gives it (see div_by_block_constant; a value whose
+// remainder could underflow, zeros and a norm outside the range are divided). 28 matrices, 0.2 G bf16
+// elements: 204 -> 164 us; 24 fp32 matrices, 42 M elements: 59 -> 54.
+struct NormDivider {
+    float norm, rnorm, least;   // |v| above `least` takes the reciprocal
+    __device__ __forceinline__ explicit NormDivider(float n)
+        : norm(n), rnorm(1.0f / n), least(div_range_ok(n) ? 1e-18f * fmaxf(n, 1.0f) : INFINITY) {}
+    __device__ __forceinline__ float operator()(float v) const {
+        if (fabsf(v) > least) return div_by_block_constant(v, norm, rnorm);
+        return v / norm;
+    }
+};
 
 // x0 <- bf16(src) / max(norm, eps), wide and padded with zeros; norm and quotient rounded to bf16 as torch's
 // x.div_(x.norm().clamp(min=eps)) on a bf16 tensor rounds them (reference: gefen_muon.py:38).
@@ -1119,7 +1140,7 @@ __global__ void __launch_bounds__(kElemThreads) ns_normalise_kernel(const NsMatr
         }
     }
     __syncthreads();
-    const float norm = norm_shared;
+    const NormDivider quotient(norm_shared);
     const S* src = static_cast<const S*>(m.src);
     __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(m.x0);
     const int rows = static_cast<int>(m.rows), cols = static_cast<int>(m.cols);
@@ -1134,7 +1155,7 @@ __global__ void __launch_bounds__(kElemThreads) ns_normalise_kernel(const NsMatr
             for (int q = 0; q < kWide; ++q) reinterpret_cast<uint4*>(v)[q] = reinterpret_cast<const uint4*>(src)[kWide * c + q];
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                const __nv_bfloat162 h = __floats2bfloat162_rn(as_bf16(v + 2 * e) / norm, as_bf16(v + 2 * e + 1) / norm);
+                const __nv_bfloat162 h = __floats2bfloat162_rn(quotient(as_bf16(v + 2 * e)), quotient(as_bf16(v + 2 * e + 1)));
                 w[e] = *reinterpret_cast<const uint32_t*>(&h);
             }
             reinterpret_cast<uint4*>(dst)[c] = make_uint4(w[0], w[1], w[2], w[3]);
@@ -1160,10 +1181,10 @@ __global__ void __launch_bounds__(kElemThreads) ns_normalise_kernel(const NsMatr
 #pragma unroll
                     for (int q = 0; q < static_cast<int>(sizeof(S)) / 2; ++q) reinterpret_cast<uint4*>(v)[q] = reinterpret_cast<const uint4*>(from)[q];
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) f[e] = as_bf16(v + e) / norm;
+                    for (int e = 0; e < 8; ++e) f[e] = quotient(as_bf16(v + e));
                 } else {
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) f[e] = row < rows && col + e < cols ? as_bf16(from + e) / norm : 0.0f;
+                    for (int e = 0; e < 8; ++e) f[e] = row < rows && col + e < cols ? quotient(as_bf16(from + e)) : 0.0f;
                 }
 #pragma unroll
                 for (int e = 0; e < 8; ++e) tile[8 * piece + e][x] = __float2bfloat16_rn(f[e]);
@@ -1178,7 +1199,7 @@ __global__ void __launch_bounds__(kElemThreads) ns_normalise_kernel(const NsMatr
             for (int y = y0; y < kTile; y += kElemThreads / kTile) {
                 if (r0 + y >= wr || c0 + x >= wc) continue;
                 float f = 0.0f;
-                if (r0 + y < rows && c0 + x < cols) f = as_bf16(src + static_cast<long long>(r0 + y) * cols + c0 + x) / norm;
+                if (r0 + y < rows && c0 + x < cols) f = quotient(as_bf16(src + static_cast<long long>(r0 + y) * cols + c0 + x));
                 dst[static_cast<long long>(r0 + y) * wc + c0 + x] = __float2bfloat16_rn(f);
             }
         }
