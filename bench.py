@@ -362,10 +362,10 @@ def run_sharded_arm(args, cfg, rank, world, local_rank):
     return result, e2e
 
 
-# DRAM bytes (read + write) per algorithmic byte of one launch of the staged step kernel, from an ncu
+# DRAM bytes (read + write) per algorithmic byte of one launch of the step kernel (step_ring_kernel), from an ncu
 # capture of a 134 M-element launch of the same kernel, fused second moment and weight decay as in this step (traffic
 # grows in proportion to the elements; part of the writes is still in L2 when the launch ends).
-STEP_KERNEL_DRAM_BYTES_PER_ALGORITHMIC_BYTE = {2: 0.949}
+STEP_KERNEL_DRAM_BYTES_PER_ALGORITHMIC_BYTE = {2: 0.981}
 
 
 def run_gpu_arm(args, cfg, rank, world, local_rank):
@@ -403,7 +403,7 @@ def run_gpu_arm(args, cfg, rank, world, local_rank):
     result = {"ms": ms, "calibration_ms": calibration_ms, "clocks": clocks, "algo_bytes": algo_bytes,
               "total_elems": total_elems, "n_tensors": len(shapes), "periods": per_tensor, "shapes": shapes}
 
-    # ---- roofline of the dominant kernel: the staged vector step over all its tensors, one launch
+    # ---- roofline of the dominant kernel: the step over all its tensors of whole-warp or shared-warp blocks, one launch
     from gefen_b200 import _lib
 
     lib = _lib.load()
@@ -414,7 +414,7 @@ def run_gpu_arm(args, cfg, rank, world, local_rank):
     def row_bytes(r):
         return int(r["num_blocks"]) * int(r["period"]) * (3 * elem_bytes + 2) + int(r["num_blocks"]) * 4 * elem_bytes
 
-    # (the staged kernel comes in two kinds, one launch each: class 1 = one block per warp pass, class 2 = several
+    # (the kernel comes in two kinds, one launch each: class 1 = one block per warp pass, class 2 = several
     # blocks of up to 1024 elements per warp pass; the roofline is reported for the one that moves more bytes)
     by_class = {c: sum(row_bytes(rows[r]) for r, k in enumerate(cls) if k == c) for c in (1, 2)}
     top = 1 if by_class[1] >= by_class[2] else 2
@@ -433,7 +433,7 @@ def run_gpu_arm(args, cfg, rank, world, local_rank):
     peak, peak_kind = measured_peaks()
     achieved = vec_bytes / vec_ms / 1e6
     ratio = STEP_KERNEL_DRAM_BYTES_PER_ALGORITHMIC_BYTE.get(elem_bytes)
-    result["roofline"] = {"bound": "hbm", "kernel": "step_vec_kernel<{}, {}>".format(
+    result["roofline"] = {"bound": "hbm", "kernel": "step_ring_kernel<{}, {}>".format(
                               "bf16" if elem_bytes == 2 else "f32",
                               "one block per warp pass" if top == 1 else "several blocks per warp pass"),
                           "achieved": achieved, "peak": peak, "peak_kind": peak_kind + " copy bandwidth, burst",

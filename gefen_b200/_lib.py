@@ -186,7 +186,7 @@ def check_step_status(device) -> None:
     status = step_status(device, clear=True)
     if status == 0:
         return
-    reasons = [text for bit, text in ((1, "gave up waiting for its staged codebook tables"),
+    reasons = [text for bit, text in ((1, "gave up waiting for its staged codebook tables or inputs"),
                                       (2, "found its shared-memory tables out of place")) if status & bit]
     raise GefenB200Error("a Gefen step kernel {}; the optimizer state and parameters of that step are incomplete".format(
         " and ".join(reasons) or "reported status {}".format(status)))

@@ -178,7 +178,7 @@ int gefen_b200_multi_tensor_step_peers(gefen_b200_step_tensor_t* host_table, voi
 /* The same launch when the ranks' buffers are also bound to an NVLink multicast object (NVSwitch), as
  * symmetric-memory allocators provide it. *_multicast_delta = (multicast address of the buffer) -
  * (this GPU's address of it) in bytes, multiples of 16, 0 = not used:
- *  - param_multicast_delta: the staged kernel writes every updated parameter chunk with ONE multimem.st,
+ *  - param_multicast_delta: the kernels for chunks of eight write every updated parameter chunk with ONE multimem.st,
  *    which the switch delivers to every rank's copy (this GPU's included), instead of a local store plus
  *    n_peers peer stores: 1/N of the egress of the unicast all-gather;
  *  - grad_multicast_delta: the staged kernel reads every gradient chunk with ONE multimem.ld_reduce (the
@@ -215,8 +215,8 @@ int gefen_b200_step_classes(const gefen_b200_step_tensor_t* host_table, int n_te
                             int32_t* tensor_classes, int32_t* launch_classes);
 
 /* Error status of the step kernels on the CURRENT device. Every wait inside them is bounded; a CTA
- * whose wait for its staged tables runs out leaves without doing its share of the step and raises
- * bit 0 of a status word; bit 1: the tables do not lie where the kernel was compiled to read them
+ * whose wait for its staged tables, or a warp whose wait for its next inputs, runs out leaves without
+ * doing its share (the rest of its share) of the step and raises bit 0 of a status word; bit 1: the tables do not lie where the kernel was compiled to read them
  * (its static shared memory has outgrown its share), nothing was done. This call synchronises the device, writes the word to *host_status and,
  * with clear != 0, resets it. Non-zero means that a step since the last clear was incomplete. The
  * reference has no counterpart: its kernels do not wait on anything (errors there are exceptions

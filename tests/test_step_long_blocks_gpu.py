@@ -1,5 +1,4 @@
-"""Blocks of more than 2048 (fp32: 3072) elements, whose momenta the step forms twice instead of staging them: both sides
-of the line, the longest ones, every codebook density, values that are not finite, lr = 0 and GefenMuon's momentum, against the oracle
+"""Blocks of 2048 to 8192 elements (from 6832, fp32 4104, the step forms their momenta twice): the longest ones, every codebook density, values that are not finite, lr = 0 and GefenMuon's momentum, against the oracle
 bit for bit."""
 import pytest
 import torch

@@ -5,7 +5,8 @@ import numpy as np
 import pytest
 import torch
 
-from tests.test_step_chunks import _run
+from tests.test_step_chunks import _codebooks, _run
+from tests.test_step_kernels_gpu import _assert_codes, _state
 from tests.util import make_grad, make_param, reference_like_codebook
 
 pytestmark = pytest.mark.gpu
@@ -71,3 +72,28 @@ def test_tables_of_small_tensors(cuda_device, dtype, offset, periods):
     for a, b in zip(together, alone):
         for k in a:
             assert torch.equal(a[k], b[k]), k
+
+
+# blocks too long for the buffers, whose momenta are formed twice
+@pytest.mark.parametrize("name", sorted(_codebooks()))
+def test_codebooks_of_long_blocks(oracle, cuda_device, name):
+    _run(oracle, cuda_device, 5, 8184, torch.bfloat16, _codebooks()[name])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("period,lr", [(8192, 1e-3), (8192, 0.0), (512, 1e-3), (300, 1e-3), (300, 0.0)])
+def test_values_that_are_not_finite(oracle, cuda_device, dtype, period, lr):
+    from gefen_b200.kernels.automatic_gefen_fused import automatic_gefen_fused_update_from_vmean_cuda
+
+    cb = reference_like_codebook()
+    p, g, codes, mag, v = _state(6, period, dtype, dtype, seed=9)
+    g[1, 5], g[3, 7], g[4, 0], g[4, 9], g[5, period - 1] = (float(x) for x in ("nan", "inf", "-inf", "nan", "nan"))
+    g[2].zero_()
+    mag[2] = 0
+    dp, dg, dc, dm, dv = (t.to(cuda_device) for t in (p, g, codes, mag, v))
+    args = dict(beta1=0.9, lr=lr, bias_correction_1=0.1, bias_correction_2=0.001, eps=1e-8)
+    oracle.automatic_gefen_fused_update_from_vmean(p, g, codes, mag, v, cb, False, **args)
+    automatic_gefen_fused_update_from_vmean_cuda(dp, dg, dc, dm, dv, cb.to(cuda_device), False, **args)
+    _assert_codes(dc, codes)
+    assert torch.equal(dm.cpu(), mag)
+    assert torch.equal(torch.nan_to_num(dp.cpu(), nan=7.0), torch.nan_to_num(p, nan=7.0))
