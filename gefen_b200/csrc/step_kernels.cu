@@ -78,7 +78,7 @@ struct StepLaunch {
     // peer stores.
     long long grad_mc_delta;
     long long param_mc_delta;
-    // iteration limit of the wait for the staged tables (g_stage_spin_limit on the host)
+    // iteration limit of the waits for the staged tables and the ring's inputs (g_stage_spin_limit on the host)
     unsigned int spin_limit;
     // host only: the launch before this one belongs to the same step (see let_successor_in)
     int follows;
@@ -93,7 +93,7 @@ struct StepRows {
 static_assert(sizeof(StepRows) + sizeof(StepLaunch) <= 4096, "kernel parameter space");
 
 // Set (never cleared by a kernel) when a bounded wait ran out and the CTA left without doing its
-// share of the step: bit 0 = the table staging of a step kernel, bit 1 = its shared-memory layout does not fit. Read and cleared by
+// share of the step: bit 0 = the table staging or the inputs of a step kernel, bit 1 = its shared-memory layout does not fit. Read and cleared by
 // gefen_b200_step_status on the host.
 __device__ int g_step_status;
 
@@ -1466,7 +1466,7 @@ __global__ void __launch_bounds__(kVecThreads, 1) step_vec_kernel(const __grid_c
 // loads of the first pass (long scoreboard 2.06 of 7 cycles per issue, 56 % of the issue slots); now 70 % are used. 134 M
 // bf16 elements (67 M fp32) with second moment and decay, ms before and now: blocks of 2048 0.230 -> 0.199, 1664 0.242 ->
 // 0.188, 1120 0.293 -> 0.222, 512 0.238 -> 0.194, 128 0.333 -> 0.239; fp32 768 0.194 -> 0.166, 1152 0.186 -> 0.170; GefenMuon's
-// momentum, blocks of 2048, 0.242 -> 0.173; rows that are multiples of four only, 300 0.374 -> 0.243 (120 M), 1500 0.328 -> 0.246.
+// momentum, blocks of 2048, 0.242 -> 0.173; rows that are multiples of four only, 300 0.374 -> 0.254 (120 M), 1500 0.328 -> 0.250.
 template <typename S> constexpr int ring_threads() { return sizeof(S) == 2 ? 640 : 512; }
 
 // A warp's descriptors (the current unit's and the next one's) and the barrier of its buffers.
@@ -2083,7 +2083,10 @@ static int launch_ring(StepLaunch L, const StepRows& rows, long long max_unit, c
     while (L.tmem_columns < (warps + 3) / 4 * L.hold_columns) L.tmem_columns *= 2;
     int smem = kSmemTables + each * warps;
     if (smem < kSmemTables + 2048) smem = kSmemTables + 2048;   // (build_lane_tables)
-    return launch_step(kernel, grid_for(L.total_blocks, 1, 1), warps * 32, smem, L, rows, stream);
+    // Few units: eight to a CTA, which leaves SMs to the other launches of the step. A GefenMuon step of four small matrices
+    // (three launches) takes 219 us, with one unit to a CTA 231; 512 units alone take 15.0 us, with one to a CTA 11.7, with
+    // as many as there are warps 16.7.
+    return launch_step(kernel, grid_for(L.total_blocks, warps < 8 ? warps : 8, 1), warps * 32, smem, L, rows, stream);
 }
 
 template <typename S>
