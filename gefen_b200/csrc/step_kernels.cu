@@ -963,8 +963,10 @@ template <typename S, int V> struct Momenta<S, V, kTensor> {
     __device__ __forceinline__ Momenta(const float*, int, uint32_t h, const uint8_t*, const S*, const LaneTables&, float, float, float)
         : hold(h) {}
     __device__ __forceinline__ void start(int, int, int) {}
+    // (The work on the chunk before branches by lane: requests of the last rounds, the search of exact_row. tcgen05.ld
+    // wants the whole warp together.)
     template <bool ALL> __device__ __forceinline__ void take(int it, int, int, int, float (&m)[V]) {
-        if (!ALL) __syncwarp();
+        __syncwarp();
         hold_load<V>(hold + it * V, m);
     }
 };
@@ -1215,6 +1217,7 @@ __device__ __forceinline__ bool warp_block_step(const TensorSlot<S>& t, long lon
         const uint32_t codes_at = in.codes_at(t.codes + unit0) + static_cast<uint32_t>(member * period);
         const f32x2 mag2 = pair(old_mag, old_mag), beta2_ = pair(beta1, beta1), omb2_ = pair(omb1, omb1);
         if (!in.arrived(L.spin_limit)) return false;
+        __syncwarp();   // (the lanes leave the wait one by one, tcgen05.st wants them together)
         int it = 0;
         for (; it + U <= full; it += U)
             first_pass_ring<S, V, U, false>(g_at, codes_at, in.hold + it * V, tables, lane + it * LANES, LANES, nchunks, mag2, beta2_, omb2_,
