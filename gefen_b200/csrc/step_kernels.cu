@@ -80,8 +80,8 @@ struct StepLaunch {
     long long param_mc_delta;
     // iteration limit of the waits for the staged tables and the ring's inputs (g_stage_spin_limit on the host)
     unsigned int spin_limit;
-    // host only: the launch before this one belongs to the same step (see let_successor_in)
-    int follows;
+    // the launch before this one (host only) and the one after it belong to the same step (see let_successor_in)
+    int follows, leads;
 };
 
 // Descriptors that travel with the launch itself: a call of up to this many tensors needs no copy of its table to the
@@ -196,7 +196,12 @@ __device__ __forceinline__ int find_tensor_warp(const gefen_b200_step_tensor_t* 
 // The launches of one step follow each other without waiting (programmatic dependent launch): they work on different
 // tensors. A kernel lets its successor in at its start, and waits for its predecessor at its end, so that whatever
 // follows the last of them follows all of them.
-__device__ __forceinline__ void let_successor_in() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// The last one lets nobody in: what follows may be any kernel of the program that was launched programmatically, and one
+// that holds tensor memory while it waits for this one to end would keep a CTA of step_ring_kernel on its SM from ever
+// getting its columns. (A launch of this step gives its columns back before it waits for the one before it.)
+__device__ __forceinline__ void let_successor_in(const StepLaunch& L) {
+    if (L.leads) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 __device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // --------------------------------------------------------------------------- vector IO
@@ -1412,7 +1417,7 @@ template <typename S, int V, int GSRC, bool FULL, int HOLD = kShared>
 __global__ void __launch_bounds__(kVecThreads, 1) step_vec_kernel(const __grid_constant__ StepLaunch L,
                                                                   const __grid_constant__ StepRows rows) {
     SmemView s;
-    let_successor_in();
+    let_successor_in(L);
     if (smem_u32(g_smem) > kFixed) {   // (static variables have outgrown their share: nothing is done, the status says so)
         if (threadIdx.x == 0) atomicOr(&g_step_status, 2);
         wait_for_predecessor();
@@ -1553,7 +1558,7 @@ __global__ void __launch_bounds__(ring_threads<S>(), 1) step_ring_kernel(const _
                                                                          const __grid_constant__ StepRows rows) {
     __shared__ uint32_t tmem_base;
     SmemView s;
-    let_successor_in();
+    let_successor_in(L);
     if (smem_u32(g_smem) > kFixed) {   // (as in step_vec_kernel)
         if (threadIdx.x == 0) atomicOr(&g_step_status, 2);
         wait_for_predecessor();
@@ -1565,7 +1570,7 @@ __global__ void __launch_bounds__(ring_threads<S>(), 1) step_ring_kernel(const _
     const int warps = blockDim.x >> 5;
     const LaneTables tables = build_lane_tables(s, fast_smem(kStageAt));
     RingWarp<S>& own = reinterpret_cast<RingWarp<S>*>(fast_smem(kStageAt))[warp];
-    if (warp == 0) {   // (waits while another CTA of this SM holds the columns: that one ends by itself)
+    if (warp == 0) {   // (waits while another CTA of this SM holds the columns; that one does not wait for this launch, see let_successor_in)
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)), "r"(L.tmem_columns) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -1623,7 +1628,7 @@ __global__ void __launch_bounds__(kThreads) step_generic_kernel(const __grid_con
     __shared__ float red_max[kWarps];
     __shared__ float red_sum[kWarps];
     SmemView s;
-    let_successor_in();
+    let_successor_in(L);
     if (!stage_tables(L.ws, g_smem, s, L.spin_limit)) { wait_for_predecessor(); return; }
     const gefen_b200_step_tensor_t* table = L.table != nullptr ? L.table : rows.row;
 
@@ -1786,7 +1791,7 @@ template <typename S>
 __global__ void __launch_bounds__(kVectorThreads) step_vector_kernel(const __grid_constant__ StepLaunch L,
                                                                      const __grid_constant__ StepRows rows) {
     constexpr int E = kVectorMost / 32;
-    let_successor_in();
+    let_successor_in(L);
     const gefen_b200_step_tensor_t* table = L.table != nullptr ? L.table : rows.row;
     const int lane = threadIdx.x & 31;
     const long long gb = static_cast<long long>(blockIdx.x) * (kVectorThreads / 32) + (threadIdx.x >> 5);
@@ -2226,7 +2231,7 @@ static int run_single(gefen_b200_step_tensor_t& t, int param_dtype, const float*
     L.grad_mc_delta = 0;
     L.param_mc_delta = 0;
     L.spin_limit = g_stage_spin_limit;
-    L.follows = 0;
+    L.follows = L.leads = 0;
     StepRows rows = {};
     rows.row[0] = t;
     return launch_class(cls, param_dtype, L, rows, staged_class(cls) ? unit_floats(t.period, class_chunk(cls)) : t.period, stream);
@@ -2589,6 +2594,7 @@ int gefen_b200_multi_tensor_step_multicast(gefen_b200_step_tensor_t* host_table,
         if (cls == 6 && (n_peers > 0 || n_grad_srcs > 0)) cls = generic_class(t);
         t.reserved_[0] = route(cls, t.period, param_dtype, n_peers, n_grad_srcs);
     }
+    int last_run = 0;   // the first row of the last run with anything to do
     for (int begin = 0; begin < n_tensors;) {
         int end = begin;
         long long first = 0;
@@ -2598,6 +2604,7 @@ int gefen_b200_multi_tensor_step_multicast(gefen_b200_step_tensor_t* host_table,
             ++end;
         }
         host_table[begin].reserved_[1] = end - begin;  // run length, read back below
+        if (first > 0) last_run = begin;
         begin = end;
     }
     // Few tensors: their descriptors go with the launches. Not while the stream is being captured: a replay of the graph
@@ -2638,6 +2645,7 @@ int gefen_b200_multi_tensor_step_multicast(gefen_b200_step_tensor_t* host_table,
             L.param_mc_delta = param_multicast_delta;
             L.spin_limit = g_stage_spin_limit;
             L.follows = launched && n_peers == 0 && n_grad_srcs == 0;
+            L.leads = begin < last_run && n_peers == 0 && n_grad_srcs == 0;
             launched = true;
             const int rc = launch_class(host_table[begin].reserved_[0], param_dtype, L, rows, max_period, stream);
             if (rc != GEFEN_B200_OK) return rc;
