@@ -534,8 +534,9 @@ struct LaneTables {
     }
 };
 
-// Fills rows and cells from the staged codebook and thresholds; every thread of the CTA. `scratch`: 1028 bytes of
-// shared memory that are free until the next __syncthreads after the call.
+// Fills rows and cells from the staged codebook and thresholds; every thread of the CTA. `scratch`: kTableScratch bytes
+// of shared memory that are free until the next __syncthreads after the call.
+constexpr int kTableScratch = kCells + 16;
 __device__ __forceinline__ LaneTables build_lane_tables(const SmemView& s, unsigned char* scratch) {
     unsigned char* below = scratch;
     int* most = reinterpret_cast<int*>(scratch + kCells);
@@ -1476,6 +1477,10 @@ __global__ void __launch_bounds__(kVecThreads, 1) step_vec_kernel(const __grid_c
 // 0.188, 1120 0.293 -> 0.222, 512 0.238 -> 0.194, 128 0.333 -> 0.239; fp32 768 0.194 -> 0.166, 1152 0.186 -> 0.170; GefenMuon's
 // momentum, blocks of 2048, 0.242 -> 0.173; rows that are multiples of four only, 300 0.374 -> 0.254 (120 M), 1500 0.328 -> 0.250.
 template <typename S> constexpr int ring_threads() { return sizeof(S) == 2 ? 640 : 512; }
+// The warps' descriptors and buffers start behind the scratch of the tables: what the CTA has written there with ordinary
+// stores is not ordered before the bulk copies.
+constexpr int kRingAt = kStageAt + kTableScratch;
+constexpr int kSmemRing = kRingAt - 1024;       // dynamic shared memory up to them
 
 // A warp's descriptors (the current unit's and the next one's) and the barrier of its buffers.
 template <typename S> struct alignas(16) RingWarp {
@@ -1569,7 +1574,7 @@ __global__ void __launch_bounds__(ring_threads<S>(), 1) step_ring_kernel(const _
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
     const int warps = blockDim.x >> 5;
     const LaneTables tables = build_lane_tables(s, fast_smem(kStageAt));
-    RingWarp<S>& own = reinterpret_cast<RingWarp<S>*>(fast_smem(kStageAt))[warp];
+    RingWarp<S>& own = reinterpret_cast<RingWarp<S>*>(fast_smem(kRingAt))[warp];
     if (warp == 0) {   // (waits while another CTA of this SM holds the columns; that one does not wait for this launch, see let_successor_in)
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)), "r"(L.tmem_columns) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -1583,7 +1588,7 @@ __global__ void __launch_bounds__(ring_threads<S>(), 1) step_ring_kernel(const _
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     // a warp reaches the 32 lanes of tensor memory that its place in its group of four gives it
     const uint32_t hold = tmem_base + (static_cast<uint32_t>(warp & 3) << 21) + static_cast<uint32_t>((warp >> 2) * L.hold_columns);
-    const uint32_t buffer = kStageAt + static_cast<uint32_t>(sizeof(RingWarp<S>)) * warps + static_cast<uint32_t>(warp * (L.ring_g + L.ring_codes));
+    const uint32_t buffer = kRingAt + static_cast<uint32_t>(sizeof(RingWarp<S>)) * warps + static_cast<uint32_t>(warp * (L.ring_g + L.ring_codes));
     // Neighbouring units go to different SMs; where they share lines of memory (small chunks) and there are many, to
     // the warps of one SM. (134 M bf16 elements in blocks of 1664 0.203 against 0.188 ms, of 128 0.256 / 0.236; with
     // chunks of four, blocks of 2500, 0.234 / 0.261; chunks of one, blocks of 27, 0.540 / 0.612.)
@@ -2084,13 +2089,12 @@ static int launch_ring(StepLaunch L, const StepRows& rows, long long max_unit, c
     L.hold_columns = static_cast<int>((max_unit + 31) / 32 + 7) / 8 * 8;
     int warps = ring_threads<S>() / 32;
     if (warps_override() > 0 && warps_override() < warps) warps = warps_override();
-    if (warps > (kMost - kSmemTables) / each) warps = (kMost - kSmemTables) / each;
+    if (warps > (kMost - kSmemRing) / each) warps = (kMost - kSmemRing) / each;
     if (warps > 512 / L.hold_columns * 4) warps = 512 / L.hold_columns * 4;
     if (warps < 1) return fail(GEFEN_B200_EINVAL, "internal: unit of %lld elements too large for the ring", max_unit);
     L.tmem_columns = 32;
     while (L.tmem_columns < (warps + 3) / 4 * L.hold_columns) L.tmem_columns *= 2;
-    int smem = kSmemTables + each * warps;
-    if (smem < kSmemTables + 2048) smem = kSmemTables + 2048;   // (build_lane_tables)
+    const int smem = kSmemRing + each * warps;
     // Few units: eight to a CTA, which leaves SMs to the other launches of the step. A GefenMuon step of four small matrices
     // (three launches) takes 219 us, with one unit to a CTA 231; 512 units alone take 15.0 us, with one to a CTA 11.7, with
     // as many as there are warps 16.7.
