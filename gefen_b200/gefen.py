@@ -315,6 +315,8 @@ class Gefen(torch.optim.Optimizer):
         make = torch.zeros if fresh is None else torch.empty
         state["m_codebook_shape"] = tuple(grad_view.shape)
         state["m_codebook"] = make(grad_view.shape, dtype=torch.uint8, device=grad_view.device)
+        if fresh is not None:
+            fresh.append(state["m_codebook"])   # (before anything below can refuse the gradient)
         state_dtype = gefen_state_dtype_from_grad(grad_view)
         if grad_view.shape[1] == 1:
             d = self._period_one_divisor_for_numel(grad_view.numel())
@@ -326,7 +328,7 @@ class Gefen(torch.optim.Optimizer):
             raise ValueError("Expected grad_view second dimension to be positive, got {}".format(grad_view.shape[1]))
         state["m_magnitude"] = make((rows, 1), dtype=state_dtype, device=grad_view.device)
         if fresh is not None:
-            fresh += [state["m_codebook"], state["m_magnitude"]]
+            fresh.append(state["m_magnitude"])
 
     @staticmethod
     def _zeroed(fresh) -> None:
