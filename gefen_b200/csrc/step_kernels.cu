@@ -2095,10 +2095,10 @@ static int launch_ring(StepLaunch L, const StepRows& rows, long long max_unit, c
     L.tmem_columns = 32;
     while (L.tmem_columns < (warps + 3) / 4 * L.hold_columns) L.tmem_columns *= 2;
     const int smem = kSmemRing + each * warps;
-    // Few units: eight to a CTA, which leaves SMs to the other launches of the step. A GefenMuon step of four small matrices
-    // (three launches) takes 219 us, with one unit to a CTA 231; 512 units alone take 15.0 us, with one to a CTA 11.7, with
-    // as many as there are warps 16.7.
-    return launch_step(kernel, grid_for(L.total_blocks, warps < 8 ? warps : 8, 1), warps * 32, smem, L, rows, stream);
+    // Few units: one to a CTA where the launch is alone. Eight where others of the step overlap it and want SMs of their
+    // own: a GefenMuon step of four small matrices (three launches) takes 219 us so, with one unit to a CTA 231.
+    const int share = L.follows || L.leads ? (warps < 8 ? warps : 8) : 1;
+    return launch_step(kernel, grid_for(L.total_blocks, share, 1), warps * 32, smem, L, rows, stream);
 }
 
 template <typename S>
