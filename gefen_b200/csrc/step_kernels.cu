@@ -2016,6 +2016,16 @@ static int launch_step(K kernel, int grid, int threads, int smem, const StepLaun
     return GEFEN_B200_OK;
 }
 
+// Bytes of a warp's slice of staged momenta (max_unit: the largest need of the launch, see unit_floats; a slice starts on 16
+// bytes; 256 floats: build_lane_tables), and the slices of a CTA.
+static int stage_bytes_for(long long max_unit) { return static_cast<int>(((max_unit > 256 ? max_unit : 256) * 4 + 15) / 16 * 16); }
+static int staged_warps(int stage_bytes) {
+    int most = kVecThreads / 32;
+    if (warps_override() > 0 && warps_override() < most) most = warps_override();
+    const int fit = (kMaxSmem - kStaticSmemSlack - kSmemTables) / stage_bytes;
+    return fit < most ? fit : most;
+}
+
 template <typename S, int V, int GSRC, bool FULL, int HOLD = kShared>
 static int launch_vec_variant(StepLaunch L, const StepRows& rows, long long max_unit, cudaStream_t stream) {
     static bool configured[kMaxDevices];
@@ -2031,19 +2041,15 @@ static int launch_vec_variant(StepLaunch L, const StepRows& rows, long long max_
         }
     }
     // a warp stages one unit: one long block, or the 32 / lanes shorter blocks that share the warp
-    // (max_unit: the largest need of the launch, see unit_floats; a slice starts on 16 bytes)
-    const long long stage_bytes = ((HOLD == kShared && max_unit > 256 ? max_unit : 256) * 4 + 15) / 16 * 16;   // (256: build_lane_tables)
-    int max_warps = kVecThreads / 32;
-    if (warps_override() > 0 && warps_override() < max_warps) max_warps = warps_override();
-    int warps = static_cast<int>((kMaxSmem - kStaticSmemSlack - kSmemTables) / stage_bytes);
-    if (warps > max_warps) warps = max_warps;
+    const int stage_bytes = stage_bytes_for(HOLD == kShared ? max_unit : 0);
+    int warps = staged_warps(stage_bytes);
     if (warps < 1) return fail(GEFEN_B200_EINVAL, "internal: unit of %lld elements too large for the staged path", max_unit);
     if (L.total_blocks < warps) warps = static_cast<int>(L.total_blocks);
-    const int smem = kSmemTables + static_cast<int>(stage_bytes) * warps;
+    const int smem = kSmemTables + stage_bytes * warps;
     int ctas_per_sm = (kMaxSmem + kCtaReservedSmem) / (smem + kStaticSmemSlack + kCtaReservedSmem);
     if (ctas_per_sm > 2) ctas_per_sm = 2;
     if (ctas_per_sm < 1) ctas_per_sm = 1;
-    L.stage_floats = static_cast<int>(stage_bytes / 4);
+    L.stage_floats = stage_bytes / 4;
     const int grid = grid_for(L.total_blocks, warps, ctas_per_sm);
     return launch_step(kernel, grid, warps * 32, smem, L, rows, stream);
 }
@@ -2092,6 +2098,15 @@ static int launch_ring(StepLaunch L, const StepRows& rows, long long max_unit, c
     if (warps > (kMost - kSmemRing) / each) warps = (kMost - kSmemRing) / each;
     if (warps > 512 / L.hold_columns * 4) warps = 512 / L.hold_columns * 4;
     if (warps < 1) return fail(GEFEN_B200_EINVAL, "internal: unit of %lld elements too large for the ring", max_unit);
+    if constexpr (sizeof(S) == 4 && V == 8) {
+        // The buffers of long fp32 units leave fewer warps than staged momenta do (12 against 16 for units of 2048 elements).
+        // Where the units make one round of those and two of these, the staged kernel takes them: 1800 to 2300 units of
+        // 2048 from HBM 19.8 to 21.2 us here, 17.3 to 18.5 there, four blocks of 512 each 21.5 to 22.3 and 19.2 to 20.7;
+        // 1700 units 16.8 / 17.0, 2600 22.5 / 28.0.
+        if (L.total_blocks > static_cast<long long>(sm_count()) * warps &&
+            L.total_blocks <= static_cast<long long>(sm_count()) * staged_warps(stage_bytes_for(max_unit)))
+            return launch_vec_variant<S, V, 0, FULL>(L, rows, max_unit, stream);
+    }
     L.tmem_columns = 32;
     while (L.tmem_columns < (warps + 3) / 4 * L.hold_columns) L.tmem_columns *= 2;
     const int smem = kSmemRing + each * warps;
