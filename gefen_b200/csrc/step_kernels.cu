@@ -91,6 +91,8 @@ struct StepRows {
     gefen_b200_step_tensor_t row[kParamRows];
 };
 static_assert(sizeof(StepRows) + sizeof(StepLaunch) <= 4096, "kernel parameter space");
+// Buffers that a chunk of averaged gradients is read from; the multicast mapping is one.
+__host__ __device__ __forceinline__ int chunk_sources(const StepLaunch& L) { return L.grad_mc_delta != 0 ? 1 : L.n_grad_srcs; }
 
 // Set (never cleared by a kernel) when a bounded wait ran out and the CTA left without doing its
 // share of the step: bit 0 = the table staging or the inputs of a step kernel, bit 1 = its shared-memory layout does not fit. Read and cleared by
@@ -636,7 +638,24 @@ __host__ __device__ __forceinline__ int lanes_shift(long long nchunks, int v) { 
     while (shift < 5 && (1 << shift) < want) ++shift;
     return shift;
 }
-// Elements of one work unit of a tensor (what a warp stages at a time), blocks of nchunks chunks of v elements.
+// Averaged gradients of two-byte types in blocks of 24, 40, 48 and 64 elements: half as many lanes with up to four chunks
+// each where the sources are few. The staged slices have no conflicts (slice_stride), and a lane's loads are what is in
+// flight; many sources read better with more lanes on one line. 67 M bf16 elements, ms, two / four chunks per lane: two
+// sources, blocks of 24 0.339 / 0.271, 40 0.406 / 0.280, 48 0.346 / 0.244, 64 0.263 / 0.232 (32 0.264 / 0.336, 56 0.304 / 0.357);
+// three, blocks of 24 0.363 / 0.380, 40 0.433 / 0.329, 48 0.380 / 0.310; four, 40 0.406 / 0.372, 48 0.359 / 0.364; eight, 64
+// 0.469 / 0.747. The second moments stay a single process's: each half of a lane's chunks has a sum of its own, and they
+// are added as the first step over twice the lanes adds them. (Kernels of their own, GSRC == 3: the second sum cost those
+// of eight sources 6 to 9 %, those of four up to 3 %.)
+// `sources`: buffers that a chunk is read from (1: the switch's sum), 0 = this GPU's gradients.
+constexpr int kFewSources = 3;
+__host__ __device__ __forceinline__ bool deep_lanes(long long nchunks, int v, int es, int sources) {
+    if (v != 8 || es != 2 || sources < 1) return false;
+    return ((nchunks == 5 || nchunks == 6) && sources <= kFewSources) || ((nchunks == 3 || nchunks == 8) && sources <= 2);
+}
+__host__ __device__ __forceinline__ int lanes_shift(long long nchunks, int v, int es, int sources) {
+    return lanes_shift(nchunks, v) - (deep_lanes(nchunks, v, es, sources) ? 1 : 0);
+}
+// Elements of one work unit of a tensor (what a warp works on at a time), blocks of nchunks chunks of v elements.
 __host__ __device__ __forceinline__ long long unit_elements(long long period, int v) { return period << (5 - lanes_shift(period / v, v)); }
 // Floats from one block's staged momenta to the next one's in a warp's slice. Eight lanes make one 128-byte access;
 // where they belong to several blocks (fewer than eight lanes per block), the blocks' slices start on different banks.
@@ -644,13 +663,13 @@ __host__ __device__ __forceinline__ int slice_stride(int period, int shift, int 
     return v < 8 || shift >= 3 ? period : ((period + 31) & ~31) + (4 << shift);
 }
 // Floats that a warp stages for one unit.
-__host__ __device__ __forceinline__ long long unit_floats(long long period, int v) {
-    const int shift = lanes_shift(period / v, v);
+__host__ __device__ __forceinline__ long long unit_floats(long long period, int v, int es, int sources) {
+    const int shift = lanes_shift(period / v, v, es, sources);
     return static_cast<long long>(slice_stride(static_cast<int>(period), shift, v)) << (5 - shift);
 }
 // Work units (one warp pass each) of a tensor on the fast path.
-__host__ __device__ __forceinline__ long long vec_units(long long num_blocks, long long period, int v) {
-    const int shift = 5 - lanes_shift(period / v, v);
+__host__ __device__ __forceinline__ long long vec_units(long long num_blocks, long long period, int v, int es, int sources) {
+    const int shift = 5 - lanes_shift(period / v, v, es, sources);
     return (num_blocks + (1 << shift) - 1) >> shift;
 }
 
@@ -684,7 +703,7 @@ template <typename S> struct alignas(8) TensorSlot {
     int period, mag_dtype, v_dtype;
     uint32_t flags;
     float beta1, beta2, inv_bc1, bc2, eps, lr, wd_mul;
-    __device__ __forceinline__ void load(const gefen_b200_step_tensor_t* t, int v_elems) {
+    __device__ __forceinline__ void load(const gefen_b200_step_tensor_t* t, int v_elems, int sources) {
         g = static_cast<const S*>(t->g);
         p = static_cast<S*>(t->p);
         codes = t->codes;
@@ -694,7 +713,7 @@ template <typename S> struct alignas(8) TensorSlot {
         num_blocks = t->num_blocks;
         period = static_cast<int>(t->period);   // at most kFastMaxPeriod
         flags = t->flags;
-        units = vec_units(num_blocks, period, v_elems);
+        units = vec_units(num_blocks, period, v_elems, sizeof(S), sources);
         mag_dtype = t->mag_dtype;
         v_dtype = t->v_dtype;
         beta1 = t->beta1;
@@ -707,6 +726,17 @@ template <typename S> struct alignas(8) TensorSlot {
     }
 };
 
+// The sum of squares of a lane's other chunks (see deep_lanes): the two change places after every chunk.
+struct OtherHalf {
+    bool used;
+    f32x2 sum;
+    __device__ __forceinline__ void turn(f32x2& mine) {
+        const f32x2 was = mine;
+        mine = used ? sum : was;
+        sum = used ? was : sum;
+    }
+};
+
 // First pass over U chunks of one lane (chunks c0, c0 + LANES, ...): all loads first, then the
 // moment update, the running absmax and sum of squares, and the staging of the updated momenta.
 // SUMMED: g_blk is the multicast address of the block's gradients; a load returns the sum over the ranks,
@@ -714,7 +744,7 @@ template <typename S> struct alignas(8) TensorSlot {
 template <typename S, int V, int U, bool GUARD, bool SUMMED, bool STAGED = true>
 __device__ __forceinline__ void first_pass_group(const S* g_blk, const uint8_t* codes_in, float* stage, int half,
                                                  const LaneTables& t, int c0, int LANES, int nchunks, f32x2 mag2,
-                                                 f32x2 beta2_, f32x2 omb2_, float scale, float& absmax, f32x2& sumsq2) {
+                                                 f32x2 beta2_, f32x2 omb2_, float scale, float& absmax, f32x2& sumsq2, OtherHalf& other) {
     CodeChunk<V> craw[U];
     Chunk<S, V> graw[U];
 #pragma unroll
@@ -759,6 +789,7 @@ __device__ __forceinline__ void first_pass_group(const S* g_blk, const uint8_t* 
                     sumsq2 = fma2(g2, g2, sumsq2);
                 }
             }
+            if (SUMMED) other.turn(sumsq2);
             if (STAGED) stage_store<V>(stage, half, c, m);
         }
     }
@@ -813,11 +844,11 @@ __device__ __forceinline__ void first_pass_ring(uint32_t g_at, uint32_t codes_at
 // First pass of a block whose gradient is averaged over up to NSRC buffers. kSlots 16-byte (fp32:
 // 32-byte) loads per lane are in flight at a time: U chunks x a batch of BS sources; the sources of
 // a chunk are added batch after batch, in the order given.
-// EXACT: there are exactly NSRC sources (no test per source).
-template <typename S, int NSRC, bool EXACT = false>
+// EXACT: there are exactly NSRC sources (no test per source). TURNS: the blocks may be those of deep_lanes.
+template <typename S, bool TURNS, int NSRC, bool EXACT = false>
 __device__ __forceinline__ void reduce_pass(const StepLaunch& L, const S* g_blk, const uint8_t* codes_in, float* stage, int half,
                                             const LaneTables& t, int lane, int LANES, int nchunks,
-                                            float old_mag, float beta1, float omb1, float& absmax, f32x2& sumsq2) {
+                                            float old_mag, float beta1, float omb1, float& absmax, f32x2& sumsq2, OtherHalf& other) {
     constexpr int kSlots = sizeof(S) == 2 ? 4 : 2;
     constexpr int BS = NSRC < kSlots ? NSRC : kSlots;
     constexpr int U = kSlots / BS;
@@ -876,6 +907,7 @@ __device__ __forceinline__ void reduce_pass(const StepLaunch& L, const S* g_blk,
                 }
 #pragma unroll
                 for (int i = 0; i < 8; i += 2) sumsq2 = fma2(pair(g[i], g[i + 1]), pair(g[i], g[i + 1]), sumsq2);   // as first_pass_group
+                if constexpr (TURNS) other.turn(sumsq2);
                 stage_store<8>(stage, half, c, m);
             }
         }
@@ -1145,7 +1177,8 @@ __device__ __forceinline__ void second_pass_muon(const LaneTables& t, Momenta<S,
 // each (a power of two, uniform over the warp; FULL fixes it to 32 at compile
 // time, for blocks of more than 1024 elements). A block's slice of `stage` holds period floats (see stage_store).
 // GSRC: where the gradients come from: 0 = this GPU's buffer, 1 = averaged over the ranks' buffers with peer
-// loads, 2 = summed by the switch through the multicast mapping (StepLaunch::grad_mc_delta). Chunks below eight elements
+// loads, 2 = summed by the switch through the multicast mapping (StepLaunch::grad_mc_delta), 3 = as 1, over at most
+// kFewSources buffers and with the lanes of deep_lanes (blocks that share a warp, two-byte types). Chunks below eight elements
 // know 0 and 1 only: 1 is every launch with peers, gradients of this GPU's buffer (no sources) included.
 // In: how the unit's inputs arrive (RingInputs; DirectInputs: they are loaded here). False: a bounded wait for the inputs
 // ran out and nothing was done.
@@ -1159,7 +1192,8 @@ __device__ __forceinline__ bool warp_block_step(const TensorSlot<S>& t, long lon
     // (the shuffle tells the compiler that the period is the same in all lanes, which the loops' bounds profit from)
     const int period = __shfl_sync(0xffffffffu, t.period, 0);
     const int chunks = period / V;                     // of a block
-    const int shift = FULL ? 5 : lanes_shift(chunks, V);
+    constexpr bool kMayBeDeep = (GSRC == 2 || GSRC == 3) && !FULL && sizeof(S) == 2;
+    const int shift = FULL ? 5 : (kMayBeDeep ? lanes_shift(chunks, V, sizeof(S), chunk_sources(L)) : lanes_shift(chunks, V));
     const int LANES = 1 << shift;
     const int lane = warp_lane & (LANES - 1);          // lane within the block's group
     const int member = warp_lane >> shift;             // which block of the unit
@@ -1200,19 +1234,20 @@ __device__ __forceinline__ bool warp_block_step(const TensorSlot<S>& t, long lon
     float absmax = 0.0f;
     float sumsq = 0.0f;
     f32x2 sumsq2 = pair(0.0f, 0.0f);
-    if (GSRC == 1) {
+    OtherHalf other = {kMayBeDeep && deep_lanes(chunks, V, sizeof(S), chunk_sources(L)), pair(0.0f, 0.0f)};
+    if (GSRC == 1 || GSRC == 3) {
         // The gradient of this block is the average over the ranks' buffers (this GPU's and the
         // peers', read over NVLink), summed in fp32 in rank order and rounded to the gradient dtype,
         // as a reduce-scatter into that dtype would leave it.
         if constexpr (GSRC == 1 && V < 8) {
             reduce_pass_small<S, V>(L, g_blk, codes, stage, half, tables, lane, LANES, nchunks, old_mag, beta1, omb1, absmax, sumsq2);
-        } else if constexpr (GSRC == 1) {
+        } else if constexpr (GSRC == 1 || GSRC == 3) {
             const int n_src = L.n_grad_srcs;
-#define GEFEN_REDUCE_PASS(...) reduce_pass<S, __VA_ARGS__>(L, g_blk, codes, stage, half, tables, lane, LANES, nchunks, old_mag, beta1, omb1, absmax, sumsq2)
+#define GEFEN_REDUCE_PASS(...) reduce_pass<S, GSRC == 3, __VA_ARGS__>(L, g_blk, codes, stage, half, tables, lane, LANES, nchunks, old_mag, beta1, omb1, absmax, sumsq2, other)
             if (n_src == 2) GEFEN_REDUCE_PASS(2, true);
             else if (n_src < 2) GEFEN_REDUCE_PASS(2);
-            else if (n_src == 4) GEFEN_REDUCE_PASS(4, true);
-            else if (n_src < 4) GEFEN_REDUCE_PASS(4);
+            else if (GSRC == 1 && n_src == 4) GEFEN_REDUCE_PASS(4, true);
+            else if (GSRC == 3 || n_src < 4) GEFEN_REDUCE_PASS(4);
             else GEFEN_REDUCE_PASS(8);
 #undef GEFEN_REDUCE_PASS
         }
@@ -1246,16 +1281,20 @@ __device__ __forceinline__ bool warp_block_step(const TensorSlot<S>& t, long lon
         if (all_valid && sizeof(S) == 2) {   // (fp32: the second copy of the loop costs registers; measured slower)
             for (; c0 + LANES * U <= chunks; c0 += LANES * U)
                 first_pass_group<S, V, U, false, SUMMED, STAGED>(g_src, codes, stage, half, tables, c0 + lane, LANES, nchunks, mag2, beta2_, omb2_,
-                                                         scale, absmax, sumsq2);
+                                                         scale, absmax, sumsq2, other);
         }
         for (; c0 < chunks; c0 += LANES * U)
             first_pass_group<S, V, U, true, SUMMED, STAGED>(g_src, codes, stage, half, tables, c0 + lane, LANES, nchunks, mag2, beta2_, omb2_,
-                                                    scale, absmax, sumsq2);
+                                                    scale, absmax, sumsq2, other);
     }
-    {   // (the same two partial sums wherever the gradients come from: a rank's second moments are a single process's)
+    {   // (the same partial sums wherever the gradients come from: a rank's second moments are a single process's)
         float even, odd;
         unpair(sumsq2, even, odd);
         sumsq = even + odd;
+        if (other.used) {
+            unpair(other.sum, even, odd);
+            sumsq += even + odd;
+        }
     }
     absmax = group_max_nan(absmax, LANES);
 
@@ -1443,7 +1482,7 @@ __global__ void __launch_bounds__(kVecThreads, 1) step_vec_kernel(const __grid_c
     for (long long gb = warp_global; gb < L.total_blocks; gb += warp_stride) {
         if (gb < t_first || gb >= t_first + t_units) {
             const gefen_b200_step_tensor_t* found = table + find_tensor_warp(table, L.n_tensors, gb);
-            if (lane == 0) t.load(found, V);
+            if (lane == 0) t.load(found, V, chunk_sources(L));
             __syncwarp();
             t_first = t.first;
             t_units = t.units;
@@ -1522,7 +1561,7 @@ template <typename S, int V, bool FULL> struct RingInputs {
         if (unit < first || unit >= first + units) {
             const gefen_b200_step_tensor_t* found = table + find_tensor_warp(table, L.n_tensors, unit);
             slot ^= 1;
-            if (lane == 0) w.slot[slot].load(found, V);
+            if (lane == 0) w.slot[slot].load(found, V, 0);
             __syncwarp();
             first = w.slot[slot].first;
             units = w.slot[slot].units;
@@ -2135,6 +2174,8 @@ static int launch_vec(int cls, StepLaunch L, const StepRows& rows, long long max
             return launch_vec_variant<S, 8, 0, true>(L, rows, max_unit, stream);
         case 2:
             if (L.grad_mc_delta != 0) return launch_vec_variant<S, 8, 2, false>(L, rows, max_unit, stream);
+            if constexpr (sizeof(S) == 2)
+                if (L.n_grad_srcs <= kFewSources) return launch_vec_variant<S, 8, 3, false>(L, rows, max_unit, stream);
             return launch_vec_variant<S, 8, 1, false>(L, rows, max_unit, stream);
     }
     if (L.n_peers > 0 || L.n_grad_srcs > 0) {
@@ -2194,8 +2235,9 @@ static int tensor_class(const gefen_b200_step_tensor_t& t, int dtype) {
 }
 // Units of a tensor in its launch's index space: passes of a warp on the staged path, blocks elsewhere.
 // (4-bit codes with an odd period: a pair of blocks is one unit, see step_generic_kernel)
-static long long class_units(const gefen_b200_step_tensor_t& t, int cls, int dtype) {
-    if (staged_class(cls)) return vec_units(t.num_blocks, t.period, class_chunk(cls));
+// (sources: see deep_lanes)
+static long long class_units(const gefen_b200_step_tensor_t& t, int cls, int dtype, int sources) {
+    if (staged_class(cls)) return vec_units(t.num_blocks, t.period, class_chunk(cls), dtype_size(dtype), sources);
     const bool paired = (t.flags & GEFEN_B200_STEP_PACKED) != 0 && (t.period & 1) != 0;
     return paired ? (t.num_blocks + 1) / 2 : t.num_blocks;
 }
@@ -2241,7 +2283,7 @@ static int run_single(gefen_b200_step_tensor_t& t, int param_dtype, const float*
     L.n_tensors = 1;
     L.stage_floats = 0;
     const int cls = route(tensor_class(t, param_dtype), t.period, param_dtype, 0, 0);
-    L.total_blocks = class_units(t, cls, param_dtype);
+    L.total_blocks = class_units(t, cls, param_dtype, 0);
     L.ws = static_cast<const unsigned char*>(ws);
     L.stepsize = stepsize;
     L.n_peers = 0;
@@ -2253,7 +2295,7 @@ static int run_single(gefen_b200_step_tensor_t& t, int param_dtype, const float*
     L.follows = L.leads = 0;
     StepRows rows = {};
     rows.row[0] = t;
-    return launch_class(cls, param_dtype, L, rows, staged_class(cls) ? unit_floats(t.period, class_chunk(cls)) : t.period, stream);
+    return launch_class(cls, param_dtype, L, rows, staged_class(cls) ? unit_floats(t.period, class_chunk(cls), dtype_size(param_dtype), 0) : t.period, stream);
 }
 
 }  // namespace gefen
@@ -2613,13 +2655,14 @@ int gefen_b200_multi_tensor_step_multicast(gefen_b200_step_tensor_t* host_table,
         if (cls == 6 && (n_peers > 0 || n_grad_srcs > 0)) cls = generic_class(t);
         t.reserved_[0] = route(cls, t.period, param_dtype, n_peers, n_grad_srcs);
     }
+    const int sources = grad_multicast_delta != 0 ? 1 : n_grad_srcs;   // (chunk_sources)
     int last_run = 0;   // the first row of the last run with anything to do
     for (int begin = 0; begin < n_tensors;) {
         int end = begin;
         long long first = 0;
         while (end < n_tensors && host_table[end].reserved_[0] == host_table[begin].reserved_[0]) {
             host_table[end].first_block = first;   // in work units on the staged path, in blocks elsewhere
-            first += class_units(host_table[end], host_table[end].reserved_[0], param_dtype);
+            first += class_units(host_table[end], host_table[end].reserved_[0], param_dtype, sources);
             ++end;
         }
         host_table[begin].reserved_[1] = end - begin;  // run length, read back below
@@ -2639,11 +2682,11 @@ int gefen_b200_multi_tensor_step_multicast(gefen_b200_step_tensor_t* host_table,
     for (int begin = 0; begin < n_tensors;) {
         const int run = host_table[begin].reserved_[1];
         const gefen_b200_step_tensor_t& last = host_table[begin + run - 1];
-        const long long total = last.first_block + class_units(last, last.reserved_[0], param_dtype);
+        const long long total = last.first_block + class_units(last, last.reserved_[0], param_dtype, sources);
         long long max_period = 0;   // largest staging need of a warp: the elements of one unit on the staged path
         for (int i = begin; i < begin + run; ++i) {
             const int cls = host_table[begin].reserved_[0];
-            const long long need = staged_class(cls) ? unit_floats(host_table[i].period, class_chunk(cls)) : host_table[i].period;
+            const long long need = staged_class(cls) ? unit_floats(host_table[i].period, class_chunk(cls), dtype_size(param_dtype), sources) : host_table[i].period;
             max_period = need > max_period ? need : max_period;
         }
         if (total > 0) {
