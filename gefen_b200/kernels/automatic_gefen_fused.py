@@ -164,7 +164,7 @@ def automatic_gefen_step_cuda(p, grad_view, m_sign, m_magnitude, vmean, codebook
     require_state_dtype("vmean", vmean)
     require_codebook(codebook)
     require_index_count(m_sign, numel, False)
-    if not 0.0 <= beta2 <= 1.0:
+    if not period_one and not 0.0 <= beta2 <= 1.0:   # (as automatic_vmean_update_cuda; a moment per element takes any)
         raise ValueError("Expected beta2 to be in [0, 1], got {}.".format(beta2))
     if bias_correction_1 <= 0.0:
         raise ValueError("Expected bias_correction_1 to be positive, got {}".format(bias_correction_1))
