@@ -1111,21 +1111,10 @@ __global__ void __launch_bounds__(kElemThreads) ns_norm_kernel(const NsMatrix* _
     }
 }
 
-// The IEEE quotient by the matrix's norm, through its reciprocal where that gives it (see div_by_block_constant; a value whose
-// remainder could underflow, zeros and a norm outside the range are divided). 28 matrices, 0.2 G bf16
-// elements: 204 -> 164 us; 24 fp32 matrices, 42 M elements: 59 -> 54.
-struct NormDivider {
-    float norm, rnorm, least;   // |v| above `least` takes the reciprocal
-    __device__ __forceinline__ explicit NormDivider(float n)
-        : norm(n), rnorm(1.0f / n), least(div_range_ok(n) ? 1e-18f * fmaxf(n, 1.0f) : INFINITY) {}
-    __device__ __forceinline__ float operator()(float v) const {
-        if (fabsf(v) > least) return div_by_block_constant(v, norm, rnorm);
-        return v / norm;
-    }
-};
-
 // x0 <- bf16(src) / max(norm, eps), wide and padded with zeros; norm and quotient rounded to bf16 as torch's
-// x.div_(x.norm().clamp(min=eps)) on a bf16 tensor rounds them (reference: gefen_muon.py:38).
+// x.div_(x.norm().clamp(min=eps)) on a bf16 tensor rounds them (reference: gefen_muon.py:38). The quotient goes through the
+// norm's reciprocal where that gives the same bits (NormDivider): 28 matrices, 0.2 G bf16 elements, 204 -> 164 us; 24 fp32
+// matrices, 42 M elements, 59 -> 54.
 template <typename S>
 __global__ void __launch_bounds__(kElemThreads) ns_normalise_kernel(const NsMatrix* __restrict__ table, const float* __restrict__ parts, float eps) {
     __shared__ __align__(16) __nv_bfloat16 tile[kTile][kTilePitch];

@@ -15,8 +15,10 @@
 
 #if defined(__CUDACC__)
 #define GEFEN_HD __host__ __device__ __forceinline__
+#define GEFEN_HD_MEMBER GEFEN_HD
 #else
 #define GEFEN_HD static inline
+#define GEFEN_HD_MEMBER
 #endif
 
 namespace gefen {
@@ -171,7 +173,8 @@ GEFEN_HD uint32_t lut_query_fast(float x, const unsigned char* lut_bytes) {
 
 // ---------------------------------------------------------------------------------------------
 // a / b with b > 0 fixed per block and |a| <= b. `rb` must be the correctly rounded 1/b.
-// q0 = a*rb is within one ulp; the exact remainder (one FMA) corrects it to the IEEE quotient.
+// q0 = a*rb is within one ulp; the exact remainder (one FMA) corrects it to the IEEE quotient (P. W. Markstein,
+// Computation of elementary functions on the IBM RISC System/6000 processor, 1990).
 // Valid while b, rb and the products stay normal; callers fall back to a true division outside
 // [2^-100, 2^100] (see div_range_ok).
 GEFEN_HD float div_by_block_constant(float a, float b, float rb) {
@@ -182,5 +185,16 @@ GEFEN_HD float div_by_block_constant(float a, float b, float rb) {
 GEFEN_HD bool div_range_ok(float b) {
     return b >= 7.888609052210118e-31f && b <= 1.2676506002282294e+30f;
 }
+
+// The IEEE quotient of bf16 values by one norm (bf16 too, any sign and class), through its reciprocal where that gives it: a
+// value whose remainder could underflow, zeros, what is not finite and a norm outside the range are divided.
+struct NormDivider {
+    float norm, rnorm, least;   // |v| above `least` takes the reciprocal
+    GEFEN_HD_MEMBER explicit NormDivider(float n) : norm(n), rnorm(1.0f / n), least(div_range_ok(n) ? 1e-18f * fmaxf(n, 1.0f) : INFINITY) {}
+    GEFEN_HD_MEMBER float operator()(float v) const {
+        if (fabsf(v) > least) return div_by_block_constant(v, norm, rnorm);
+        return v / norm;
+    }
+};
 
 }  // namespace gefen
