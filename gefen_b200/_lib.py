@@ -92,6 +92,7 @@ def _declare(lib):
         "gefen_b200_step_classes": (i32, [vp, i32, i32, vp, vp]),
         "gefen_b200_step_status": (i32, [vp, i32]),
         "gefen_b200_debug_set_stage_spin_limit": (i32, [i64]),
+        "gefen_b200_debug_set_input_spin_limit": (i32, [i64]),
         "gefen_b200_exact_histogram": (i32, [vp, i32, i64, i64, vp, i32, vp]),
         "gefen_b200_average_within_block_variance": (i32, [vp, i32, i64, i64, i32, vp, vp]),
         "gefen_b200_average_within_block_coefficient_of_variation": (i32, [vp, i32, i64, i64, i32, vp, vp]),

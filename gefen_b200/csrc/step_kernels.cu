@@ -78,8 +78,8 @@ struct StepLaunch {
     // peer stores.
     long long grad_mc_delta;
     long long param_mc_delta;
-    // iteration limit of the waits for the staged tables and the ring's inputs (g_stage_spin_limit on the host)
-    unsigned int spin_limit;
+    // iteration limits of the waits for the staged tables and the ring's inputs (g_stage_spin_limit, g_input_spin_limit)
+    unsigned int spin_limit, input_limit;
     // the launch before this one (host only) and the one after it belong to the same step (see let_successor_in)
     int follows, leads;
 };
@@ -1257,7 +1257,7 @@ __device__ __forceinline__ bool warp_block_step(const TensorSlot<S>& t, long lon
         const uint32_t g_at = in.g_at(t.g + unit0) + static_cast<uint32_t>(member * period) * static_cast<uint32_t>(sizeof(S));
         const uint32_t codes_at = in.codes_at(t.codes + unit0) + static_cast<uint32_t>(member * period);
         const f32x2 mag2 = pair(old_mag, old_mag), beta2_ = pair(beta1, beta1), omb2_ = pair(omb1, omb1);
-        if (!in.arrived(L.spin_limit)) return false;
+        if (!in.arrived(L.input_limit)) return false;
         __syncwarp();   // (the lanes leave the wait one by one, tcgen05.st wants them together)
         int it = 0;
         for (; it + U <= full; it += U)
@@ -2025,16 +2025,18 @@ static int env_int(const char* name) {
     const int v = e != nullptr ? atoi(e) : 0;
     return v < 0 ? 0 : v;
 }
-// GEFEN_B200_STEP_WARPS=n caps the warps per CTA of the staged kernel (for measurements; read once).
+// GEFEN_B200_STEP_WARPS=n caps the warps per CTA of the staged and the ring kernel (for measurements; read once).
 static int warps_override() {
     static const int cached = env_int("GEFEN_B200_STEP_WARPS");
     return cached;
 }
 
-// Iteration limit of the step kernels' wait for their staged tables. gefen_b200_debug_set_stage_spin_limit
-// lowers it so that a test can watch the time-out path (status word, kernel returns) without a fault.
-constexpr unsigned int kDefaultStageSpinLimit = 4000000u;
-static unsigned int g_stage_spin_limit = kDefaultStageSpinLimit;
+// Iteration limits of the step kernels' wait for their staged tables and of a ring warp's wait for its inputs.
+// gefen_b200_debug_set_stage_spin_limit and gefen_b200_debug_set_input_spin_limit lower them so that a test can watch the
+// time-out paths (status word, kernel returns) without a fault.
+constexpr unsigned int kDefaultSpinLimit = 4000000u;
+static unsigned int g_stage_spin_limit = kDefaultSpinLimit, g_input_spin_limit = kDefaultSpinLimit;
+static unsigned int spin_limit_of(int64_t limit) { return limit < 0 || limit > 0xFFFFFFFFll ? kDefaultSpinLimit : static_cast<unsigned int>(limit); }
 
 template <typename K>
 static int launch_step(K kernel, int grid, int threads, int smem, const StepLaunch& L, const StepRows& rows,
@@ -2292,6 +2294,7 @@ static int run_single(gefen_b200_step_tensor_t& t, int param_dtype, const float*
     L.grad_mc_delta = 0;
     L.param_mc_delta = 0;
     L.spin_limit = g_stage_spin_limit;
+    L.input_limit = g_input_spin_limit;
     L.follows = L.leads = 0;
     StepRows rows = {};
     rows.row[0] = t;
@@ -2585,7 +2588,12 @@ int gefen_b200_step_status(int* host_status, int clear) {
 }
 
 int gefen_b200_debug_set_stage_spin_limit(int64_t limit) {
-    g_stage_spin_limit = (limit < 0 || limit > 0xFFFFFFFFll) ? kDefaultStageSpinLimit : static_cast<unsigned int>(limit);
+    g_stage_spin_limit = spin_limit_of(limit);
+    return GEFEN_B200_OK;
+}
+
+int gefen_b200_debug_set_input_spin_limit(int64_t limit) {
+    g_input_spin_limit = spin_limit_of(limit);
     return GEFEN_B200_OK;
 }
 
@@ -2706,6 +2714,7 @@ int gefen_b200_multi_tensor_step_multicast(gefen_b200_step_tensor_t* host_table,
             L.grad_mc_delta = grad_multicast_delta;
             L.param_mc_delta = param_multicast_delta;
             L.spin_limit = g_stage_spin_limit;
+            L.input_limit = g_input_spin_limit;
             L.follows = launched && n_peers == 0 && n_grad_srcs == 0;
             L.leads = begin < last_run && n_peers == 0 && n_grad_srcs == 0;
             launched = true;

@@ -214,18 +214,22 @@ int gefen_b200_step_launch_class(const gefen_b200_step_tensor_t* host_entry, int
 int gefen_b200_step_classes(const gefen_b200_step_tensor_t* host_table, int n_tensors, int param_dtype,
                             int32_t* tensor_classes, int32_t* launch_classes);
 
-/* Error status of the step kernels on the CURRENT device. Every wait inside them is bounded; a CTA
- * whose wait for its staged tables, or a warp whose wait for its next inputs, runs out leaves without
- * doing its share (the rest of its share) of the step and raises bit 0 of a status word; bit 1: the tables do not lie where the kernel was compiled to read them
- * (its static shared memory has outgrown its share), nothing was done. This call synchronises the device, writes the word to *host_status and,
- * with clear != 0, resets it. Non-zero means that a step since the last clear was incomplete. The
- * reference has no counterpart: its kernels do not wait on anything (errors there are exceptions
- * from C10_CUDA_KERNEL_LAUNCH_CHECK). */
+/* Error status of the step kernels on the CURRENT device. Every wait for a copy inside them is bounded: a CTA
+ * whose wait for its staged tables runs out leaves without doing its share of the step, a warp whose wait
+ * for its next inputs runs out without the rest of its share, and bit 0 of a status word is raised; bit 1:
+ * the tables do not lie where the kernel was compiled to read them (its static shared memory has outgrown
+ * its share), nothing was done. (One wait has no limit, the hardware's for tensor memory: it lasts while
+ * another CTA on the SM holds the columns, and those that can do not wait for this one.) This call
+ * synchronises the device, writes the word to *host_status and, with clear != 0, resets it. Non-zero means
+ * that a step since the last clear was incomplete. The reference has no counterpart: its kernels do not
+ * wait on anything (errors there are exceptions from C10_CUDA_KERNEL_LAUNCH_CHECK). */
 int gefen_b200_step_status(int* host_status, int clear);
 /* Test hook: the number of polls the step kernels grant the table staging (negative = default).
  * With 0 the wait runs out at once, the kernels return without touching their tensors and the
  * status word is set; nothing faults or hangs. Process-wide, not thread-safe. */
 int gefen_b200_debug_set_stage_spin_limit(int64_t limit);
+/* The same for the wait of a warp for its next inputs. */
+int gefen_b200_debug_set_input_spin_limit(int64_t limit);
 
 /* Replaces gefen_exact_histogram_cuda (gefen_cuda_binding.cpp:65-69;
  * exact_histogram_fused_kernel.cu:131-160): bin_counts[bin] += #elements, int64, exact. */
