@@ -1,6 +1,5 @@
-"""Averaged gradients in short blocks, where the lanes of a block depend on the number of buffers:
-the same bits as the plain
-step, second moments included, over several units per warp and a ragged last one."""
+"""Averaged gradients in short blocks, where the lanes of a block depend on the number of buffers: the same bits
+as the plain step, second moments included, over several units per warp and a ragged last one."""
 import pytest
 import torch
 
