@@ -6,6 +6,7 @@ import pytest
 import torch
 
 from tests.test_step_chunks import _run
+from tests.test_step_sources_gpu import _step
 from tests.util import make_grad, make_param, reference_like_codebook
 
 pytestmark = pytest.mark.gpu
@@ -24,7 +25,8 @@ def test_against_the_oracle(oracle, cuda_device, period, blocks, which):
 
 @pytest.mark.parametrize("which", ["two rounds of twelve", "one of sixteen"])
 @pytest.mark.parametrize("period,blocks", [(2048, 1), (512, 4), (1992, 1), (1000, 2)])
-def test_against_two_launches(cuda_device, period, blocks, which):
+@pytest.mark.parametrize("muon", [False, True])
+def test_against_two_launches(cuda_device, period, blocks, which, muon):
     from gefen_b200 import _lib
 
     lib = _lib.load()
@@ -43,7 +45,7 @@ def test_against_two_launches(cuda_device, period, blocks, which):
             for k, t in one.items():
                 host[k] = t[b0 if k in ("mag", "v") else b0 * period:].data_ptr()
             host["num_blocks"], host["period"], host["mag_dtype"], host["v_dtype"] = b1 - b0, period, _lib.F32, _lib.F32
-            host["flags"] = _lib.STEP_FUSE_VMEAN | _lib.STEP_WEIGHT_DECAY
+            host["flags"] = _lib.STEP_MUON | _lib.STEP_NESTEROV if muon else _lib.STEP_FUSE_VMEAN | _lib.STEP_WEIGHT_DECAY
             for k, value in (("beta1", 0.9), ("beta2", 0.999), ("lr", 3e-4), ("bc1", 0.3), ("bc2", 0.003), ("eps", 1e-8), ("wd_mul", 0.99997)):
                 host[k] = value
             _lib.check(lib.gefen_b200_multi_tensor_step(host.ctypes.data, _lib.ptr(table), 1, _lib.F32, _lib.ptr(ws), _lib.current_stream(cuda_device)))
@@ -53,3 +55,14 @@ def test_against_two_launches(cuda_device, period, blocks, which):
     together, apart = run([0, nb]), run([0, nb // 2, nb])
     for k in together:
         assert torch.equal(together[k], apart[k]), k
+
+
+@pytest.mark.parametrize("period,blocks", [(2048, 1), (512, 4)])
+def test_copies_of_the_parameters(cuda_device, period, blocks):
+    nb = _units(cuda_device, "one of sixteen") * blocks
+    plain = _step(cuda_device, torch.float32, nb, period, 0, 0)
+    got = _step(cuda_device, torch.float32, nb, period, 0, 2)
+    for copy in got[0]:
+        assert torch.equal(copy, plain[0][0])
+    for a, b in zip(got[1:], plain[1:]):
+        assert torch.equal(a, b)
