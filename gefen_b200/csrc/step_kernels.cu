@@ -19,8 +19,9 @@
 //    The codebook arrives by one bulk copy per CTA, which turns it into tables with a copy per lane (see LaneTables). No
 //    __syncthreads after set-up; the loops are short so the code stays in the instruction cache. What bounds it and what it
 //    measured stands at the kernel.
-//  * step_vec_kernel - the same without the ring: gradients averaged over ranks, chunks below eight with peer stores, and
-//    blocks too long for the buffers (see route); momenta in shared memory or formed twice (see Momenta).
+//  * step_vec_kernel - the same without the ring: gradients averaged over ranks, chunks below eight with peer stores or
+//    whose reads of the buffers would conflict, blocks too long for the buffers (see route), fp32 launches that make one
+//    round of it and two of the ring kernel (see launch_ring); momenta in shared memory or formed twice (see Momenta).
 //  * step_vector_kernel - period-1 tensors, one warp per magnitude, everything in registers.
 //  * step_generic_kernel - blocks of more than 8192 elements, fp64, 4-bit packed codes, and vectors of ranks with peers:
 //    two passes with scalar accesses, the second pass re-reading from L1/L2.
@@ -626,7 +627,7 @@ template <int V> __device__ __forceinline__ CodeChunk<V> row_codes(const uint32_
 // than 256 elements, as in a 2048-element block (8 lanes for 512 elements, 16 for 1024, all 32 from 1032 on), up to
 // four down to blocks of 72 elements, two below that (the blocks of a warp lie side by side in its buffer, so lanes with
 // four chunks of their own would read the same banks: 134 M bf16 elements in blocks of 64 / 32 0.60 / 0.58 ms with four,
-// 0.345 / 0.338 with two; before the buffers 0.349 / 0.357).
+// 0.342 / 0.336 with two; before the buffers 0.350 / 0.351). Averaged gradients differ, see deep_lanes.
 __host__ __device__ __forceinline__ int lanes_shift(long long nchunks, int v) {   // log2 of the lanes; chunks of v elements
     if (v < 8) {   // smaller chunks: about sixteen per lane, eight of them in flight
         int shift = 0;
@@ -979,7 +980,7 @@ __device__ __forceinline__ void reduce_pass_small(const StepLaunch& L, const S* 
 }
 
 // Where the second pass takes a chunk's updated momenta from:
-//   kShared  the warp's slice of shared memory (gradients of several ranks, and what route() leaves);
+//   kShared  the warp's slice of shared memory (gradients of several ranks, what route() and launch_ring leave);
 //   kTwice   computed once more from codes and gradients, which L2 still holds (blocks too long for the other two, see
 //            route); the next chunk's are requested while this one is worked on;
 //   kTensor  the warp's columns of tensor memory (step_ring_kernel).
@@ -1512,9 +1513,9 @@ __global__ void __launch_bounds__(kVecThreads, 1) step_vec_kernel(const __grid_c
 //    which leaves shared memory to those buffers and takes a quarter of the traffic off its data pipe.
 // Twenty warps of 96 registers (fp32: sixteen of 128) instead of sixteen of 128. Before, sixteen warps could not cover the
 // loads of the first pass (long scoreboard 2.06 of 7 cycles per issue, 56 % of the issue slots); now 70 % are used. 134 M
-// bf16 elements (67 M fp32) with second moment and decay, ms before and now: blocks of 2048 0.230 -> 0.199, 1664 0.242 ->
-// 0.188, 1120 0.293 -> 0.222, 512 0.238 -> 0.194, 128 0.333 -> 0.239; fp32 768 0.194 -> 0.166, 1152 0.186 -> 0.170; GefenMuon's
-// momentum, blocks of 2048, 0.242 -> 0.173; rows that are multiples of four only, 300 0.374 -> 0.254 (120 M), 1500 0.328 -> 0.250.
+// bf16 elements (67 M fp32) with second moment and decay, ms before and now: blocks of 2048 0.230 -> 0.198, 1664 0.244 ->
+// 0.191, 1120 0.297 -> 0.224, 512 0.240 -> 0.195, 128 0.335 -> 0.239; fp32 768 0.193 -> 0.165, 1152 0.179 -> 0.164; GefenMuon's
+// momentum, blocks of 2048, 0.244 -> 0.174; rows that are multiples of four only, 300 0.378 -> 0.256 (120 M), 1500 0.295 -> 0.223.
 template <typename S> constexpr int ring_threads() { return sizeof(S) == 2 ? 640 : 512; }
 // The warps' descriptors and buffers start behind the scratch of the tables: what the CTA has written there with ordinary
 // stores is not ordered before the bulk copies.
@@ -2099,8 +2100,8 @@ static int launch_vec_variant(StepLaunch L, const StepRows& rows, long long max_
 // whose momenta are formed twice; a class by itself = step_vec_kernel with staged momenta.
 constexpr int kTwiceClass = 7, kRing = 16;
 // The most that the ring kernel's buffers of a unit may take (codes and gradients; this much leaves six warps). Blocks of
-// 4096 fp32 elements: 0.224 ms with the momenta formed twice (66 M elements), 0.186 here; bf16, 134 M: 4096 0.264 against
-// 0.225, 5120 0.277 / 0.239, 8192 (24 KB) 0.300 / 0.323.
+// 4096 fp32 elements: 0.222 ms with the momenta formed twice (67 M elements), 0.194 here; bf16, 134 M: 4096 0.268 against
+// 0.227, 5120 0.294 / 0.242, 8192 (24 KB) 0.300 / 0.323.
 constexpr int kRingBytes = 20480;
 static int route(int cls, long long period, int dtype, int n_peers, int n_grad_srcs) {
     if (cls < 1 || cls > 5 || n_grad_srcs > 0) return cls;   // (averaged gradients: the staged kernels)
@@ -2212,8 +2213,8 @@ static int launch_generic(bool cta_per_block, const StepLaunch& L, const StepRow
     return launch_step(step_generic_kernel<S, 32>, grid_for(L.total_blocks, kWarps, 3), kThreads, smem, L, rows, stream);
 }
 
-// Class of a tensor: 1 = staged path in chunks of eight with whole-warp blocks, 2 = the same with several blocks
-// per warp pass (blocks of up to 1024 elements), 3 / 4 / 5 = staged path in chunks of four, two, one (the most that
+// Class of a tensor: 1 = fast path in chunks of eight with whole-warp blocks, 2 = the same with several blocks
+// per warp pass (blocks of up to 1024 elements), 3 / 4 / 5 = fast path in chunks of four, two, one (the most that
 // divides the block length and the alignment of all pointers), 6 = vectors (period 1, runs of up to 256 elements), 0 =
 // generic warp per block, -1 = generic CTA per block.
 static int generic_class(const gefen_b200_step_tensor_t& t) { return t.period > 2048 ? -1 : 0; }
@@ -2235,7 +2236,7 @@ static int tensor_class(const gefen_b200_step_tensor_t& t, int dtype) {
     }
     return generic_class(t);   // (a pointer that is not aligned to its own type)
 }
-// Units of a tensor in its launch's index space: passes of a warp on the staged path, blocks elsewhere.
+// Units of a tensor in its launch's index space: passes of a warp on the fast path, blocks elsewhere.
 // (4-bit codes with an odd period: a pair of blocks is one unit, see step_generic_kernel)
 // (sources: see deep_lanes)
 static long long class_units(const gefen_b200_step_tensor_t& t, int cls, int dtype, int sources) {
@@ -2669,7 +2670,7 @@ int gefen_b200_multi_tensor_step_multicast(gefen_b200_step_tensor_t* host_table,
         int end = begin;
         long long first = 0;
         while (end < n_tensors && host_table[end].reserved_[0] == host_table[begin].reserved_[0]) {
-            host_table[end].first_block = first;   // in work units on the staged path, in blocks elsewhere
+            host_table[end].first_block = first;   // in work units on the fast path, in blocks elsewhere
             first += class_units(host_table[end], host_table[end].reserved_[0], param_dtype, sources);
             ++end;
         }
@@ -2691,7 +2692,7 @@ int gefen_b200_multi_tensor_step_multicast(gefen_b200_step_tensor_t* host_table,
         const int run = host_table[begin].reserved_[1];
         const gefen_b200_step_tensor_t& last = host_table[begin + run - 1];
         const long long total = last.first_block + class_units(last, last.reserved_[0], param_dtype, sources);
-        long long max_period = 0;   // largest staging need of a warp: the elements of one unit on the staged path
+        long long max_period = 0;   // largest need of a warp: the elements of one unit on the fast path
         for (int i = begin; i < begin + run; ++i) {
             const int cls = host_table[begin].reserved_[0];
             const long long need = staged_class(cls) ? unit_floats(host_table[i].period, class_chunk(cls), dtype_size(param_dtype), sources) : host_table[i].period;

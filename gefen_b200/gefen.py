@@ -9,9 +9,9 @@ State per parameter (same keys, shapes and dtypes as the reference, so checkpoin
 state_dict() adds "gefen_global_step" and "gefen_codebook".
 
 `fused=True` (default) runs the whole step as a handful of multi-tensor launches that fuse the
-second-moment update, the decoupled weight decay and the 8-bit momentum step. `fused=False` keeps
-the reference's launch structure (one second-moment launch, one weight-decay multiply and one step
-launch per tensor) on the same kernels; there is no CPU path.
+second-moment update, the decoupled weight decay and the 8-bit momentum step. `fused=False` makes
+one call and one launch per tensor that does the same (float64 gradients: a second-moment launch, a
+multiplication by torch and a step launch); there is no CPU path.
 """
 from __future__ import annotations
 

@@ -849,7 +849,7 @@ class Zero1Gefen:
         return Gefen(named, lr=g0["lr"], betas=(g0["beta1"], g0["beta2"]), eps=g0["eps"], weight_decay=g0["weight_decay"])
 
     def _piece_is_staged(self, prm) -> bool:
-        """True if the local optimizer steps this piece with the staged (vectorised) kernel."""
+        """True if the local optimizer steps this piece with a vectorised kernel."""
         plan = getattr(self.local, "_plan", None)
         if plan is None:
             return False

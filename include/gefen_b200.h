@@ -185,7 +185,7 @@ int gefen_b200_multi_tensor_step_peers(gefen_b200_step_tensor_t* host_table, voi
  *    switch adds the ranks' copies, fp32 accumulation, one rounding to the gradient dtype), scales by
  *    grad_scale and rounds, instead of n_grad_srcs peer loads: 1/N of the ingress of the unicast
  *    reduce-scatter. The order of the switch's additions is not the rank order of the peer-load path.
- * Blocks that the staged kernel takes in chunks below eight elements, and the generic kernels, use the per-rank offsets, which must therefore be
+ * Blocks that are taken in chunks below eight elements, and the generic kernels, use the per-rank offsets, which must therefore be
  * given as well. Ordering between ranks is the caller's, as for gefen_b200_multi_tensor_step_peers. No
  * counterpart in the reference. */
 int gefen_b200_multi_tensor_step_multicast(gefen_b200_step_tensor_t* host_table, void* device_table,
@@ -202,11 +202,11 @@ int gefen_b200_multicast_sum(void* dst, const void* src_multicast, int dtype, in
                              void* stream);
 /* sizeof(gefen_b200_step_tensor_t) as compiled, for binding-side layout checks. */
 int gefen_b200_step_tensor_size(void);
-/* Kind of block of one table entry: 1 = staged path in chunks of eight elements with one block per
+/* Kind of block of one table entry: 1 = fast path in chunks of eight elements with one block per
  * warp pass, 2 = the same path with several blocks (of up to 1024 elements) per warp pass,
  * 0 = any other block of up to 2048 elements, -1 = any other longer block. */
 int gefen_b200_step_tensor_class(const gefen_b200_step_tensor_t* host_entry, int param_dtype);
-/* The launch a table entry goes to: 1 and 2 as above, 3 / 4 / 5 = staged path in chunks of four, two, one
+/* The launch a table entry goes to: 1 and 2 as above, 3 / 4 / 5 = fast path in chunks of four, two, one
  * element (blocks and pointers that are multiples of no more than that), 6 = period-1 vectors, 0 / -1 = generic. Rows
  * of equal launch class that are adjacent in the table share one launch. */
 int gefen_b200_step_launch_class(const gefen_b200_step_tensor_t* host_entry, int param_dtype);
